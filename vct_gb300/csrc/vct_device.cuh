@@ -90,43 +90,58 @@ __device__ __forceinline__ float4 unpack_h4(uint2 v) {
 // identical to the CPU oracle: window coordinates are snapped with
 // rint(w * 256) after clamping to +-2^20 pixels, edge functions are exact
 // 64-bit integers, and interpolation weights are e_k * (1 / area) in fp32.
-constexpr long long kSub = 256;
+constexpr int kSub = 256;
 
-__device__ __forceinline__ long long snap(float w) {
+__device__ __forceinline__ int snap(float w) {
     w = clampf(w, -1048576.0f, 1048576.0f);
-    return (long long)rintf(w * 256.0f);
+    return __float2int_rn(w * 256.0f);
 }
-__device__ __forceinline__ long long floordiv(long long a, long long b) {
-    long long q = a / b;
-    if ((a % b != 0) && ((a < 0) != (b < 0))) --q;
-    return q;
+
+// The fp32 value of 0 <= e < 2^46, rounded to nearest even as the conversion
+// of a 64-bit integer is: two 23-bit halves become floats exactly (as the low
+// bits of 2^23's significand), and one fused multiply-add rounds their sum.
+// The conversion instruction for 64-bit integers runs on the FP64 pipe, which
+// takes 16 cycles a warp on this chip: three of them per candidate pixel held
+// that pipe at 64% and the 2048^2 shadow pass at 0.67 ms.
+constexpr long long kHalvesLimit = 1LL << 46;
+__device__ __forceinline__ float halves_to_float(long long e) {
+    const uint32_t lo = (uint32_t)e, hi = (uint32_t)((unsigned long long)e >> 32);
+    const float h = __uint_as_float(0x4B000000u | __funnelshift_l(lo, hi, 9)) - 8388608.0f;
+    const float l = __uint_as_float(0x4B000000u | (lo & 0x7fffffu)) - 8388608.0f;
+    return fmaf(h, 8388608.0f, l);
 }
-__device__ __forceinline__ long long edge(long long ax, long long ay, long long bx, long long by, long long px,
-                                          long long py) {
-    return (bx - ax) * (py - ay) - (by - ay) * (px - ax);
+// `wide`: the triangle's area, which bounds its covered pixels' edge
+// functions, is past that range (it reaches some 2^29 pixels).  A call, so
+// that the conversion is branched around and not predicated.
+static __device__ __noinline__ float wide_to_float(long long e) { return __ll2float_rn(e); }
+__device__ __forceinline__ float edge_to_float(long long e, bool wide) {
+    return wide ? wide_to_float(e) : halves_to_float(e);
 }
 
 struct RasterTri {
-    long long X[3], Y[3];
-    long long area;
-    long long bias[3];
+    int X[3], Y[3];  // snapped coordinates, within 2^28
+    long long area;  // twice the area, positive
+    int bias[3];     // -1 for an edge that is not top-left
     int px0, px1, py0, py1;
     int perm1;  // 1: vertices 1 and 2 were swapped to make the triangle CCW
+    __device__ __forceinline__ bool wide() const { return area >= kHalvesLimit; }
+    __device__ __forceinline__ float area_float() const { return edge_to_float(area, wide()); }
 };
 
 __device__ __forceinline__ bool raster_setup(const float wx[3], const float wy[3], int W, int H, RasterTri& t) {
-    long long X[3], Y[3];
+    int X[3], Y[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         X[k] = snap(wx[k]);
         Y[k] = snap(wy[k]);
     }
-    long long area = edge(X[0], Y[0], X[1], Y[1], X[2], Y[2]);
+    long long area = (long long)(X[1] - X[0]) * (long long)(Y[2] - Y[0]) -
+                     (long long)(Y[1] - Y[0]) * (long long)(X[2] - X[0]);
     if (area == 0) return false;
     t.perm1 = area < 0;
     if (t.perm1) {
         area = -area;
-        long long tx = X[1], ty = Y[1];
+        const int tx = X[1], ty = Y[1];
         X[1] = X[2];
         Y[1] = Y[2];
         X[2] = tx;
@@ -141,47 +156,18 @@ __device__ __forceinline__ bool raster_setup(const float wx[3], const float wy[3
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         int a = (k + 1) % 3, b = (k + 2) % 3;
-        long long dx = X[b] - X[a], dy = Y[b] - Y[a];
+        const int dx = X[b] - X[a], dy = Y[b] - Y[a];
         bool tl = (dy < 0) || (dy == 0 && dx < 0);
         t.bias[k] = tl ? 0 : -1;
     }
-    long long minx = min(X[0], min(X[1], X[2])), maxx = max(X[0], max(X[1], X[2]));
-    long long miny = min(Y[0], min(Y[1], Y[2])), maxy = max(Y[0], max(Y[1], Y[2]));
-    long long x0 = -floordiv(-(minx - kSub / 2), kSub);
-    long long x1 = floordiv(maxx - kSub / 2, kSub);
-    long long y0 = -floordiv(-(miny - kSub / 2), kSub);
-    long long y1 = floordiv(maxy - kSub / 2, kSub);
-    x0 = max(x0, 0LL);
-    y0 = max(y0, 0LL);
-    x1 = min(x1, (long long)W - 1);
-    y1 = min(y1, (long long)H - 1);
-    if (x0 > x1 || y0 > y1) return false;
-    t.px0 = (int)x0;
-    t.px1 = (int)x1;
-    t.py0 = (int)y0;
-    t.py1 = (int)y1;
-    return true;
-}
-
-__device__ __forceinline__ bool raster_cover(const RasterTri& t, int px, int py, long long e[3]) {
-    long long sx = (long long)px * kSub + kSub / 2, sy = (long long)py * kSub + kSub / 2;
-    bool in = true;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        int a = (k + 1) % 3, b = (k + 2) % 3;
-        e[k] = edge(t.X[a], t.Y[a], t.X[b], t.Y[b], sx, sy);
-        in = in && (e[k] + t.bias[k] >= 0);
-    }
-    return in;
-}
-
-// Weights in the caller's original vertex order.
-__device__ __forceinline__ void raster_weights(const RasterTri& t, const long long e[3], float l[3]) {
-    float inv = __fdiv_rn(1.0f, __ll2float_rn(t.area));
-    float l0 = __ll2float_rn(e[0]) * inv, l1 = __ll2float_rn(e[1]) * inv, l2 = __ll2float_rn(e[2]) * inv;
-    l[0] = l0;
-    l[1] = t.perm1 ? l2 : l1;
-    l[2] = t.perm1 ? l1 : l2;
+    const int minx = min(X[0], min(X[1], X[2])), maxx = max(X[0], max(X[1], X[2]));
+    const int miny = min(Y[0], min(Y[1], Y[2])), maxy = max(Y[0], max(Y[1], Y[2]));
+    // pixel centres within [min, max]: ceil((min - 128) / 256) .. floor((max - 128) / 256)
+    t.px0 = max((minx - kSub / 2 + kSub - 1) >> 8, 0);
+    t.py0 = max((miny - kSub / 2 + kSub - 1) >> 8, 0);
+    t.px1 = min((maxx - kSub / 2) >> 8, W - 1);
+    t.py1 = min((maxy - kSub / 2) >> 8, H - 1);
+    return t.px0 <= t.px1 && t.py0 <= t.py1;
 }
 
 __device__ __forceinline__ float interp(const float l[3], float a, float b, float c) {

@@ -41,6 +41,9 @@ __device__ __forceinline__ unsigned long long* grab_counter(const VoxWork& W, in
     return reinterpret_cast<unsigned long long*>(W.block_off + (((long long)nblocks + 2) & ~1LL));
 }
 
+// Bit of a triangle's edge flags: its area is past halves_to_float's range.
+constexpr int kWide = 8;
+
 struct FragQueue {
     int tri[kQueue];       // triangle index within its scene
     uint32_t pix[kQueue];  // px | py << 11 | axis << 22 | scene << 24
@@ -120,8 +123,9 @@ __global__ void __launch_bounds__(kSetupThreads) voxelize_setup_kernel(const Sce
         int axis;
         if (project_triangle(P, t, rt, z, axis)) {
             const uint32_t bw = rt.px1 - rt.px0 + 1, bh = rt.py1 - rt.py0 + 1;
-            const uint32_t bias = (rt.bias[0] ? 1u : 0u) | (rt.bias[1] ? 2u : 0u) | (rt.bias[2] ? 4u : 0u);
-            const float inv = __fdiv_rn(1.0f, __ll2float_rn(rt.area));
+            const uint32_t bias = (rt.bias[0] ? 1u : 0u) | (rt.bias[1] ? 2u : 0u) | (rt.bias[2] ? 4u : 0u) |
+                                  (rt.wide() ? (uint32_t)kWide : 0u);
+            const float inv = __fdiv_rn(1.0f, rt.area_float());
             uint4* rec = W.tri_rec + 3 * g;
             rec[0] = make_uint4((uint32_t)rt.X[0], (uint32_t)rt.Y[0], (uint32_t)rt.X[1], (uint32_t)rt.Y[1]);
             rec[1] = make_uint4((uint32_t)rt.X[2], (uint32_t)rt.Y[2], __float_as_uint(z[0]), __float_as_uint(z[1]));
@@ -130,7 +134,7 @@ __global__ void __launch_bounds__(kSetupThreads) voxelize_setup_kernel(const Sce
             // of the triangle (the area over the rows, on average) and a
             // pixel each side.  A sliver's rows are short, so its units take
             // many rows.
-            const float row_px = (float)rt.area * (0.5f / (float)(kSub * kSub)) / (float)bh + 2.0f;
+            const float row_px = rt.area_float() * (0.5f / (float)(kSub * kSub)) / (float)bh + 2.0f;
             const uint32_t R = (uint32_t)fminf(fmaxf((float)(1u << W.unit_log2) / row_px, 1.0f), 1023.0f);
             rec[2] = make_uint4(__float_as_uint(z[2]), __float_as_uint(inv),
                                 (uint32_t)rt.px0 | ((uint32_t)rt.py0 << 11) | ((uint32_t)axis << 22) |
@@ -274,14 +278,15 @@ __device__ __forceinline__ void shade_fragment(const AccumParams& P, const FragQ
 
 // Coverage of pixel (px, py) by a set-up triangle (snapped vertices X, Y; edge
 // k runs from vertex a = k+1 to b = k+2 with deltas dX, dY; bit k of `bias`
-// set for an edge that is not top-left) and the fragment's barycentrics and
+// set for an edge that is not top-left, kWide for a triangle past
+// halves_to_float's range) and the fragment's barycentrics and
 // depth.  The edge function at the pixel centre is dX (sy - Ya) - dY (sx - Xa),
 // every factor within 32 bits (|snapped coordinates| <= 2^28), each product
 // exact in 64.  False outside the triangle or outside GL's depth clip.
 __device__ __forceinline__ bool pixel_fragment(const int X[3], const int Y[3], const int dX[3], const int dY[3],
                                                int bias, int perm1, float inv, const float z[3], int px, int py,
                                                float l[3], float& zf) {
-    const int sx = px * (int)kSub + (int)kSub / 2, sy = py * (int)kSub + (int)kSub / 2;
+    const int sx = px * kSub + kSub / 2, sy = py * kSub + kSub / 2;
     long long e[3];
     bool cov = true;
 #pragma unroll
@@ -291,7 +296,9 @@ __device__ __forceinline__ bool pixel_fragment(const int X[3], const int Y[3], c
         cov = cov && (e[k] - ((bias >> k) & 1) >= 0);
     }
     if (!cov) return false;
-    const float w0 = __ll2float_rn(e[0]) * inv, w1 = __ll2float_rn(e[1]) * inv, w2 = __ll2float_rn(e[2]) * inv;
+    const bool wide = (bias & kWide) != 0;
+    const float w0 = edge_to_float(e[0], wide) * inv, w1 = edge_to_float(e[1], wide) * inv,
+                w2 = edge_to_float(e[2], wide) * inv;
     l[0] = w0;
     l[1] = perm1 ? w2 : w1;
     l[2] = perm1 ? w1 : w2;
@@ -419,7 +426,7 @@ __global__ void __launch_bounds__(kWarps * 32, kRasterBlocksPerSM)
                 const int r = rb + lane;
                 int lo = 0, cnt = 0;
                 if (r <= r_b) {
-                    const int sy = (py0 + r) * (int)kSub + (int)kSub / 2;
+                    const int sy = (py0 + r) * kSub + kSub / 2;
                     float xmin = 3.0e38f, xmax = -3.0e38f;
 #pragma unroll
                     for (int k = 0; k < 3; ++k) {
@@ -539,12 +546,12 @@ __global__ void __launch_bounds__(kOccThreads) occupancy_kernel(const Scenes S, 
     if (ok) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            X[k] = (int)rt.X[k];
-            Y[k] = (int)rt.Y[k];
+            X[k] = rt.X[k];
+            Y[k] = rt.Y[k];
         }
-        bias = (rt.bias[0] ? 1 : 0) | (rt.bias[1] ? 2 : 0) | (rt.bias[2] ? 4 : 0);
+        bias = (rt.bias[0] ? 1 : 0) | (rt.bias[1] ? 2 : 0) | (rt.bias[2] ? 4 : 0) | (rt.wide() ? kWide : 0);
         perm1 = rt.perm1;
-        inv = __fdiv_rn(1.0f, __ll2float_rn(rt.area));
+        inv = __fdiv_rn(1.0f, rt.area_float());
         px0 = rt.px0;
         py0 = rt.py0;
         bw = rt.px1 - rt.px0 + 1;
