@@ -459,8 +459,8 @@ vct_status vct_batch_get_timers(vct_batch* batch, vct_timers* out);
  * pipeline and the compute shaders' local sizes).  Every setting gives
  * bit-identical results; only speed differs. */
 typedef struct vct_tuning {
-    int32_t voxel_unit_pixels;   /* candidate pixels (rows' spans of the triangle) per voxeliser work unit, about: power of two in [32, 8192] (512) */
-    int32_t voxel_blocks_per_sm; /* resident voxeliser raster CTAs per SM: 1..3 (3) */
+    int32_t voxel_unit_pixels;   /* voxeliser work share: the raster work is cut finer the smaller it is; power of two in [32, 8192] (512) */
+    int32_t voxel_blocks_per_sm; /* voxeliser raster CTAs per SM and share: 1..3 (3) */
     int32_t trace_tile_w;        /* pixel tile of one 256-thread trace CTA, tile_w * tile_h = 256: */
     int32_t trace_tile_h;        /*   tile_w a power of two in [4, 64] (16 x 16) */
     int32_t trace_warp_w;        /* pixel tile of one warp: warp_w x 32/warp_w, warp_w a power of two with */
@@ -600,8 +600,8 @@ vct_status vct_learned_trace_pixels(vct_ctx* ctx, vct_mlp* mlp, const vct_gbuffe
  * someone else, or a frame loop that must not allocate): vct_voxelize
  * (accumulate + normalise) into volumes the caller owns, with no context and
  * no device allocation by this library or anything it calls.  Its scratch
- * (accumulator records, occupancy mask, work-distribution arrays, counters)
- * is one fixed __device__ array of about 9 MiB that every GPU that loads the
+ * (accumulator records, occupancy mask, counters)
+ * is one fixed __device__ array of about 8 MiB that every GPU that loads the
  * library keeps until the process exits.
  *  - cfg->voxel_dim <= VCT_STATIC_MAX_DIM and tris->count <=
  *    VCT_STATIC_MAX_TRIANGLES, otherwise VCT_ERR_INVALID_ARGUMENT.
@@ -615,7 +615,7 @@ vct_status vct_learned_trace_pixels(vct_ctx* ctx, vct_mlp* mlp, const vct_gbuffe
  *    that first call before any stream capture.
  *  - With CUDA's lazy module loading (the default since CUDA 12.2) the array
  *    comes into being at that first call on each device: the driver then
- *    allocates its ~9 MiB.  Make the first call before reserving the rest of
+ *    allocates its ~8 MiB.  Make the first call before reserving the rest of
  *    the device's memory, or run with CUDA_MODULE_LOADING=EAGER so that the
  *    array is allocated when the context is created.  Later calls allocate
  *    nothing.

@@ -1,8 +1,10 @@
-"""The depth rasteriser of the set-up passes where its work is split: slivers
-along and across the lines it walks, triangles around the size that is left to
-the whole CTA, triangles that fill the image or reach far outside it,
-near-plane clips into two parts, triangle counts around the CTA's 256.  The
-shadow map and the G-buffer equal the oracle's bit for bit."""
+"""The line rasteriser of the set-up passes and of the voxeliser where its
+work is split: slivers along and across the lines it walks, triangles around
+the size whose edge functions leave 32 bits, triangles that fill the image or
+reach far outside it, near-plane clips into two parts, triangle counts around
+the CTA's 256.  The shadow map, the G-buffer and the radiance chain (lit by
+point lights inside and outside their range and through a shadow map that ends
+inside the volume) equal the oracle's bit for bit."""
 
 from __future__ import annotations
 
@@ -12,8 +14,8 @@ import numpy as np
 import pytest
 
 import oracle as O
-from helpers import GpuScene
-from vct_gb300 import scenes
+from helpers import GpuScene, read_chain
+from vct_gb300 import api, scenes
 
 pytestmark = pytest.mark.gpu
 
@@ -33,18 +35,46 @@ def _soup(kind: str, n: int, rng) -> np.ndarray:
     return far
 
 
-@pytest.mark.parametrize("n", [1, 31, 257, 1500])
-@pytest.mark.parametrize("kind", ["slivers", "sizes", "near", "far"])
-def test_depth_raster_matches_oracle(kind, n):
+def _scene(kind: str, n: int, dim: int):
     rng = np.random.default_rng((n, len(kind)))
-    base = scenes.tiny(seed=n, gbuffer=(321, 199), shadow=257)
+    base = scenes.tiny(seed=n, dim=dim, gbuffer=(321, 199), shadow=257)
     tris = _soup(kind, n, rng).reshape(n, 9).astype(np.float32)
     nrm = rng.normal(size=(n, 3, 3))
     nrm /= np.linalg.norm(nrm, axis=2, keepdims=True)
-    sc = dataclasses.replace(base, positions=tris, normals=nrm.reshape(n, 9).astype(np.float32),
-                             albedo=rng.uniform(0, 1, size=(n, 3)).astype(np.float32), shadow_size=(257, 140))
+    return dataclasses.replace(base, positions=tris, normals=nrm.reshape(n, 9).astype(np.float32),
+                               albedo=rng.uniform(0, 1, size=(n, 3)).astype(np.float32), shadow_size=(257, 140))
+
+
+@pytest.mark.parametrize("n", [1, 31, 257, 1500])
+@pytest.mark.parametrize("kind", ["slivers", "sizes", "near", "far"])
+def test_depth_raster_matches_oracle(kind, n):
+    sc = _scene(kind, n, 16)
     g = GpuScene(sc)
     sm, gbuf = g.host_inputs()
     assert np.array_equal(sm, O.render_shadowmap(sc))
     for got, want in zip(gbuf, O.render_gbuffer(sc)):
         assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("n,dim", [(1, 16), (31, 64), (257, 32), (1500, 128), (300, 256)])
+@pytest.mark.parametrize("kind", ["slivers", "sizes", "far"])
+def test_voxel_raster_matches_oracle(kind, n, dim):
+    sc = _scene(kind, n, dim)
+    # the shadow map covers the volume's middle only; one light far away, one whose range is 0
+    half = np.diag([2.0, 2.0, 1.0, 1.0]) @ sc.ls.reshape(4, 4).T
+    light = dict(position=np.array([0.1, -0.2, 0.3]), direction=np.array([0.0, -1.0, 0.0]), color=np.ones(3), range=0.5,
+                 intensity=1.0, shadow_caster=1, type=0)
+    extra = [light, dict(light, position=np.array([50.0, 0.0, 0.0]), shadow_caster=0), dict(light, range=0.0)]
+    sc = dataclasses.replace(sc, ls=scenes.colmajor(half), ls_inverse=scenes.colmajor(np.linalg.inv(half)),
+                             lights=sc.lights + extra)
+    g = GpuScene(sc)
+    sm, gbuf = g.host_inputs()
+    ref = O.frame(sc, shadowmap=sm, gbuf=gbuf, nthreads=8)
+    with api.Context(api.config_for(sc)) as ctx:
+        ctx.set_params(api.scene_params(sc))
+        irr, spec, col, samples = g.new_outputs()
+        ctx.frame(g.tris, g.lights, g.shadow, sc.eye, g.gb, api.trace_out(irr, spec, col, samples))
+        assert np.array_equal(read_chain(ctx), ref["chain"])
+        stats = ctx.stats()
+    for k in ("total_voxel_fragments", "unique_voxels", "max_fragments_per_voxel"):
+        assert stats[k] == ref["stats"][k]

@@ -25,7 +25,7 @@ struct vct_batch {
     char* d_blob = nullptr;
     char* h_blob = nullptr;        // staging of vct_batch_frame
     char* h_graph_blob = nullptr;  // staging read by the captured graph
-    void* work = nullptr;          // voxeliser work arrays over all triangles
+    void* work = nullptr;          // tessellation voxeliser's work arrays over all triangles
     long long work_bytes = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -53,7 +53,7 @@ struct BatchTotals {
 constexpr int kClearPre = 5;  // clear-list entries per scene before the voxeliser (one more after the resolve)
 
 // Validates the scene descriptors and fills the staging blob `h` (parameter
-// structs and prefix tables).  Allocates the voxeliser work arrays when the
+// structs and prefix tables).  Allocates the tessellation voxeliser's work arrays when the
 // batch grew (never during a capture: `allow_alloc` false).
 vct_status batch_stage(vct_batch* b, const vct_scene_desc* sc, int n, char* h, BatchTotals& tot, bool allow_alloc) {
     if (!sc || n != b->n) return fail(VCT_ERR_INVALID_ARGUMENT, "scene descriptors must match the batch's scene count");
@@ -178,7 +178,7 @@ vct_status batch_stage(vct_batch* b, const vct_scene_desc* sc, int n, char* h, B
     if (tot.tris > 0x7fffffffLL) return fail(VCT_ERR_INVALID_ARGUMENT, "a batch holds at most 2^31-1 triangles");
     if (b->ctx[0]->params.voxelize_tesselation && tot.tris > (1LL << 24))
         return fail(VCT_ERR_UNSUPPORTED, "the tessellation voxeliser takes at most 2^24 triangles per batch");
-    const long long need = accumulate_scratch_bytes(std::max(tot.tris, 1LL));
+    const long long need = b->ctx[0]->params.voxelize_tesselation ? tess_scratch_bytes(std::max(tot.tris, 1LL)) : 0;
     if (need > b->work_bytes) {
         if (!allow_alloc) return fail(VCT_ERR_STATE, "batch work arrays too small for the captured scenes");
         // A captured graph points at the old arrays: it goes with them.
@@ -225,18 +225,19 @@ vct_status batch_enqueue(vct_batch* b, const char* h, const BatchTotals& tot, cu
         VCT_CHECK_LAUNCH("batch: warp maps");
     }
     const long long* d_tables = reinterpret_cast<const long long*>(b->d_blob + b->off_tables);
-    AccumParams W0;
-    W0.ntri = tot.tris;
-    accumulate_bind_scratch(W0, b->work);
-    const VoxWork W = {W0.tri_rec, W0.tri_units, W0.tri_scan, W0.block_off, tot.tris,
-                       ilog2(b->tuning.voxel_unit_pixels)};
     if (timed) VCT_CUDA(cudaEventRecord(b->ev[0], st));
     if (tot.tris > 0) {
         const SceneBatch<AccumParams> SB{reinterpret_cast<const AccumParams*>(b->d_blob + b->off_accum), d_tables, n};
-        if (b->ctx[0]->params.voxelize_tesselation)
-            launch_tesselate_batch(SB, W, b->num_sms, st);
-        else
-            launch_accumulate_batch(SB, W, b->num_sms, b->tuning.voxel_blocks_per_sm, st);
+        if (b->ctx[0]->params.voxelize_tesselation) {
+            AccumParams W;
+            W.ntri = tot.tris;
+            tess_bind_scratch(W, b->work);
+            launch_tesselate_batch(SB, VoxWork{W.tri_rec, W.tri_units, W.tri_scan, W.block_off, tot.tris}, b->num_sms,
+                                   st);
+        } else {
+            launch_accumulate_batch(SB, tot.tris, ilog2(b->tuning.voxel_unit_pixels), b->num_sms,
+                                    b->tuning.voxel_blocks_per_sm, st);
+        }
         VCT_CHECK_LAUNCH("batch: accumulate");
     }
     if (timed) VCT_CUDA(cudaEventRecord(b->ev[1], st));

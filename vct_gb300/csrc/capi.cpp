@@ -7,6 +7,7 @@
 #include <cmath>
 #include <cstddef>
 #include <cstring>
+#include <limits>
 #include <new>
 #include <string>
 #include <vector>
@@ -249,6 +250,10 @@ void fill_accum_inputs(const vct_config& cfg, const vct_params& prm, const float
         hf3 ndn = hnorm(nd);
         L.neg_dir_n = {ndn.x, ndn.y, ndn.z};
         L.range075 = 0.75f * lights[i].range;
+        // (a relative 1e-6 covers the rounding of the squared distance and its root)
+        const float r = lights[i].range, beyond2 = (r * r) * 1.000002f;
+        L.beyond2 = r - L.range075 > 0.0f && beyond2 > 1e-30f && beyond2 < 1e30f ? beyond2
+                                                                                : std::numeric_limits<float>::infinity();
     }
     std::memcpy(P.mvp, mvp, sizeof P.mvp);
     P.vmin = to_f3(cfg.voxel_min);
@@ -366,7 +371,8 @@ vct_status fill_accum(vct_ctx* ctx, const vct_triangles* t, const vct_light* lig
     P.brick_exact = ctx->params.voxelize_tesselation ? ctx->brick_exact : nullptr;
     P.stats = ctx->stats;
     P.num_sms = ctx->num_sms;
-    const long long need = accumulate_scratch_bytes(t->count);
+    if (!ctx->params.voxelize_tesselation) return VCT_OK;
+    const long long need = tess_scratch_bytes(t->count);
     if (need > ctx->vox_scratch_bytes) {
         if (ctx->vox_scratch) cudaFree(ctx->vox_scratch);
         ctx->vox_scratch = nullptr;
@@ -378,7 +384,7 @@ vct_status fill_accum(vct_ctx* ctx, const vct_triangles* t, const vct_light* lig
         }
         ctx->vox_scratch_bytes = need;
     }
-    accumulate_bind_scratch(P, ctx->vox_scratch);
+    tess_bind_scratch(P, ctx->vox_scratch);
     return VCT_OK;
 }
 

@@ -36,7 +36,7 @@ struct vct_ctx {
     // with the voxeliser: `fork` / `join` order it against the caller's stream.
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
-    void* vox_scratch = nullptr;  // voxeliser work-distribution arrays
+    void* vox_scratch = nullptr;  // tessellation voxeliser's work-distribution arrays
     long long vox_scratch_bytes = 0;
     float4* pchain = nullptr;  // bordered fp32 radiance chain read by the software sampler
     bool pad_ready = false;   // pchain holds the current radiance chain

@@ -1,0 +1,349 @@
+// Line walking shared by the depth rasteriser (raster.cu) and the voxeliser
+// (voxelize.cu): the covered pixels of 256 set-up triangles, dealt out to a
+// CTA's warps 32 at a time.
+//
+// A triangle is walked in lines: rows, or columns when its bounding box is
+// more than twice as tall as wide, so that an upright sliver costs a few lines
+// and not its whole height.  A line's covered pixels are contiguous and found
+// from the triangle's crossings of it, with the edge functions at the first
+// one.  A CTA walks the lines of its 256 triangles together: a chunk of 512
+// lines at a time, a thread each, their pixel counts scanned; then the warps
+// take the pixels, 32 a step, whichever lines and triangles they belong to.
+//
+// No scratch memory is used, so work is not handed from one CTA to another:
+// the CTAs of gridDim.y set up the same 256 triangles and share their lines.
+#pragma once
+
+#include <algorithm>
+
+#include "vct_device.cuh"
+
+namespace vct {
+namespace lines {
+
+constexpr int kLineThreads = 256;
+constexpr int kChunkLines = 512;  // lines walked together (half as many of the big triangles')
+constexpr int kLineWarps = kLineThreads / 32;
+// A set-up triangle in shared memory.  For its lines, counter-clockwise:
+// {X0, Y0, X1, Y1}, {X2, Y2, x0 | y0 << 16, x1 | y1 << 16}, flags.  For its
+// pixels, in the caller's vertex order: what a pixel along a line adds to each
+// edge function (per sub-pixel unit) and 1 / area; the depths and the triangle;
+// two words of the caller's.  (Five uint4: the odd stride spreads the banks.)
+struct TriRec {
+    uint4 v0, v1;
+    int step[3];
+    float inv;
+    float z[3];
+    int tri;
+    uint32_t flags, user[2], unused;
+};
+static_assert(sizeof(TriRec) == 80, "a record's stride is five uint4");
+// Twice the area from which on 32 bits do not hold the edge functions.
+constexpr long long kBigArea = 1LL << 31;
+// Flags: bits 0-2 the edges that are not top-left.
+constexpr uint32_t kRecSwapped = 8u, kRecColumns = 16u;
+
+// Stores the record of a set-up triangle; its lines.  Columns only for boxes
+// four times as tall as wide: the pixels of a column are in as many sectors of
+// the image.
+__device__ __forceinline__ int store_rec(TriRec& r, const RasterTri& t, const float z[3], int tri) {
+    const int w = t.px1 - t.px0 + 1, h = t.py1 - t.py0 + 1;
+    const bool columns = 2 * w < h;
+    r.v0 = make_uint4((uint32_t)t.X[0], (uint32_t)t.Y[0], (uint32_t)t.X[1], (uint32_t)t.Y[1]);
+    r.v1 = make_uint4((uint32_t)t.X[2], (uint32_t)t.Y[2], (uint32_t)t.px0 | ((uint32_t)t.py0 << 16),
+                      (uint32_t)t.px1 | ((uint32_t)t.py1 << 16));
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int a = (k + 1) % 3, b = (k + 2) % 3;
+        const int s = columns ? t.X[b] - t.X[a] : t.Y[a] - t.Y[b];
+        if (k == 0)
+            r.step[0] = s;
+        else
+            r.step[t.perm1 ? 3 - k : k] = s;
+        r.z[k] = z[k];
+    }
+    r.inv = __fdiv_rn(1.0f, t.area_float());
+    r.tri = tri;
+    r.flags = (t.bias[0] ? 1u : 0u) | (t.bias[1] ? 2u : 0u) | (t.bias[2] ? 4u : 0u) |
+              (t.perm1 ? kRecSwapped : 0u) | (columns ? kRecColumns : 0u);
+    return columns ? w : h;
+}
+
+// The covered pixels of line `k` of a triangle, which are contiguous: how
+// many, the first one, and the edge functions there in the caller's vertex
+// order (modulo 2^32 unless BIG).  The triangle's crossings of the line are
+// computed in fp32, within 2^-21 of the coordinates' magnitude (the
+// differences' conversion, the division, the product and the sum each round
+// at 2^-24 or 2^-22).  Pixel centres further than 2^-20 of it and half a
+// sub-pixel unit from a crossing are decided by it; the few nearer ones by the
+// exact edge functions.
+template <bool BIG>
+__device__ __forceinline__ int line_pixels(const TriRec& r, int k, int& first, long long base[3]) {
+    const uint4 v0 = r.v0, v1 = r.v1;
+    const uint32_t flags = r.flags;
+    const int X[3] = {(int)v0.x, (int)v0.z, (int)v1.x}, Y[3] = {(int)v0.y, (int)v0.w, (int)v1.y};
+    const bool columns = (flags & kRecColumns) != 0u;
+    const int x0 = (int)(v1.z & 0xffffu), y0 = (int)(v1.z >> 16), x1 = (int)(v1.w & 0xffffu), y1 = (int)(v1.w >> 16);
+    const int at = ((columns ? x0 : y0) + k) * kSub + kSub / 2;
+    int U[3], V[3];  // along the line, and across
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        U[i] = columns ? Y[i] : X[i];
+        V[i] = columns ? X[i] : Y[i];
+    }
+    float lo = 3.0e38f, hi = -3.0e38f, big = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const int a = i, b = (i + 1) % 3;
+        const float ua = (float)U[a];
+        big = fmaxf(big, fabsf(ua));
+        if (min(V[a], V[b]) <= at && at <= max(V[a], V[b])) {
+            const int dv = V[b] - V[a];
+            // an edge along the line decides all of it
+            if (dv == 0 && ((flags >> ((i + 2) % 3)) & 1u)) return 0;
+            const float u = dv != 0 ? fmaf((float)(at - V[a]), __fdividef((float)(U[b] - U[a]), (float)dv), ua) : ua;
+            const float v = dv != 0 ? u : (float)U[b];
+            lo = fminf(lo, fminf(u, v));
+            hi = fmaxf(hi, fmaxf(u, v));
+        }
+    }
+    if (!(lo <= hi)) return 0;
+    const float eps = fmaf(big, 9.5367431640625e-7f, 0.5f), half = 0.5f * (float)kSub, rs = 1.0f / (float)kSub;
+    // the first and last pixel: certainly covered ones (in), possibly covered ones (out);
+    // clamped to the image's part as floats, since the crossings may lie far outside
+    const float p0 = (float)(columns ? y0 : x0), p1 = (float)(columns ? y1 : x1);
+    const int in0 = (int)fminf(fmaxf(ceilf((lo + eps - half) * rs), p0), p1 + 1.0f);
+    const int in1 = (int)fmaxf(fminf(floorf((hi - eps - half) * rs), p1), p0 - 1.0f);
+    first = (int)fminf(fmaxf(ceilf((lo - eps - half) * rs), p0), p1 + 1.0f);
+    int last = (int)fmaxf(fminf(floorf((hi + eps - half) * rs), p1), p0 - 1.0f);
+    if (first != in0 || last != in1) {
+        // (products of 32-bit factors, exact in 64)
+        auto covered = [&](int p) {
+            const int u = p * kSub + kSub / 2, sx = columns ? at : u, sy = columns ? u : at;
+            bool in = true;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const int ia = (i + 1) % 3, ib = (i + 2) % 3;
+                const long long e = (long long)(X[ib] - X[ia]) * (long long)(sy - Y[ia]) -
+                                    (long long)(Y[ib] - Y[ia]) * (long long)(sx - X[ia]);
+                in = in && e - (long long)((flags >> i) & 1u) >= 0;
+            }
+            return in;
+        };
+        while (last >= first && last != in1 && !covered(last)) --last;
+        while (first <= last && first != in0 && !covered(first)) ++first;
+    }
+    if (first > last) return 0;
+    const int u = first * kSub + kSub / 2, sx = columns ? at : u, sy = columns ? u : at;
+    const bool sw = (flags & kRecSwapped) != 0u;
+    long long e[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const int ia = (i + 1) % 3, ib = (i + 2) % 3;
+        if (BIG)
+            e[i] = (long long)(X[ib] - X[ia]) * (long long)(sy - Y[ia]) -
+                   (long long)(Y[ib] - Y[ia]) * (long long)(sx - X[ia]);
+        else
+            e[i] = (uint32_t)(X[ib] - X[ia]) * (uint32_t)(sy - Y[ia]) - (uint32_t)(Y[ib] - Y[ia]) * (uint32_t)(sx - X[ia]);
+    }
+    base[0] = e[0];
+    base[1] = sw ? e[2] : e[1];
+    base[2] = sw ? e[1] : e[2];
+    return last - first + 1;
+}
+
+// Inclusive scans of `v` over the CTA, the totals in `total`; `s` holds a
+// word per warp and value.  Callers put a barrier between two uses of one `s`.
+template <int N>
+__device__ __forceinline__ void cta_scan(int (&v)[N], int (*s)[kLineWarps], int (&total)[N]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            const int u = __shfl_up_sync(0xffffffffu, v[n], o);
+            if (lane >= o) v[n] += u;
+        }
+    }
+    if (lane == 31)
+        for (int n = 0; n < N; ++n) s[n][warp] = v[n];
+    __syncthreads();
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        total[n] = 0;
+#pragma unroll
+        for (int w = 0; w < kLineWarps; ++w) {
+            if (w == warp) v[n] += total[n];
+            total[n] += s[n][w];
+        }
+    }
+}
+
+struct LineShared {
+    TriRec recs[kLineThreads];
+    int line_off[kLineThreads];  // first line of each triangle among the CTA's
+    // lines with covered pixels, in order: the number of the first pixel among
+    // the lines'; the edge functions there (64 bits each for big triangles, in
+    // two halves of the array) and its place; the line's place | its
+    // triangle's record << 16
+    int pix_off[kChunkLines + 32];
+    uint4 pix_base[kChunkLines];
+    uint32_t pix_line[kChunkLines];
+    int scan[5][kLineWarps];
+    int next;  // the step that the next free warp takes
+};
+
+// One lane's share of a step: a covered pixel and its weights and depth.
+struct LinePixel {
+    bool on;
+    int px, py;
+    float l[3], z;
+    const TriRec* rec;
+};
+
+// Walks this slice's share of the lines of the CTA's triangles (`lines` of a
+// thread's own), handing their covered pixels to `sink`, STEPS times 32 at a
+// time (every lane of the warp calls it); a warp takes GRAB steps when it has
+// done its last.  BIG: triangles of any area; otherwise twice the area is
+// below 2^31 square sub-pixel units, and so are the covered pixels' edge
+// functions: 32 bits hold them, whatever the products on the way.
+template <bool BIG, int STEPS, int GRAB, class Sink>
+__device__ __forceinline__ void walk_triangles(LineShared& S, int lines, Sink& sink) {
+    constexpr int kChunk = BIG ? kChunkLines / 2 : kChunkLines;
+    const unsigned FULL = 0xffffffffu;
+    const int tid = threadIdx.x, lane = tid & 31;
+    int end[1] = {lines}, total[1];
+    cta_scan(end, S.scan, total);
+    S.line_off[tid] = end[0] - lines;
+    __syncthreads();
+    const int l_end = (int)((long long)total[0] * (blockIdx.y + 1) / gridDim.y);
+    for (int l0 = (int)((long long)total[0] * blockIdx.y / gridDim.y); l0 < l_end; l0 += kChunk) {
+        int npix = 0, nline = 0;
+#pragma unroll 1
+        for (int q = 0; q < kChunk / kLineThreads; ++q) {
+            const int l = l0 + q * kLineThreads + tid;
+            int first = 0, cnt = 0, rec = 0, k = 0;
+            long long base[3] = {0, 0, 0};
+            if (l < l_end) {
+                // the last triangle whose lines start at or before l
+#pragma unroll
+                for (int st = kLineThreads / 2; st > 0; st >>= 1)
+                    if (S.line_off[rec + st] <= l) rec += st;
+                k = l - S.line_off[rec];
+                cnt = line_pixels<BIG>(S.recs[rec], k, first, base);
+            }
+            int ends[2] = {cnt, cnt > 0 ? 1 : 0}, sums[2];  // covered pixels, lines that have any
+            cta_scan(ends, S.scan + 1 + 2 * (q & 1), sums);
+            const int at = nline + ends[1] - 1;
+            if (cnt > 0) {
+                S.pix_off[at] = npix + ends[0] - cnt;
+                if (BIG) {
+                    S.pix_base[at] = make_uint4((uint32_t)base[0], (uint32_t)(base[0] >> 32), (uint32_t)base[1],
+                                                (uint32_t)(base[1] >> 32));
+                    S.pix_base[kChunk + at] = make_uint4((uint32_t)base[2], (uint32_t)(base[2] >> 32), (uint32_t)first, 0u);
+                } else {
+                    S.pix_base[at] = make_uint4((uint32_t)base[0], (uint32_t)base[1], (uint32_t)base[2], (uint32_t)first);
+                }
+                const uint32_t box = S.recs[rec].v1.z;
+                const uint32_t place = ((S.recs[rec].flags & kRecColumns) ? (box & 0xffffu) : (box >> 16)) + (uint32_t)k;
+                S.pix_line[at] = place | ((uint32_t)rec << 16);
+            }
+            npix += sums[0];
+            nline += sums[1];
+        }
+        const int steps = (npix + 31) / 32;
+        if (tid < 32) S.pix_off[nline + tid] = 0x7fffffff;
+        if (tid == 32) S.next = 0;
+        __syncthreads();
+        for (;;) {
+            int s0 = 0;
+            if (lane == 0) s0 = atomicAdd(&S.next, GRAB);
+            s0 = __shfl_sync(FULL, s0, 0);
+            if (s0 >= steps) break;
+            const int s1 = min(s0 + GRAB, steps);
+            int j = 0;  // the line of the step's first pixel
+#pragma unroll
+            for (int st = kChunk / 2; st > 0; st >>= 1)
+                if (j + st < nline && S.pix_off[j + st] <= s0 * 32) j += st;
+            for (int st = s0; st < s1; st += STEPS) {
+                LinePixel f[STEPS];
+#pragma unroll
+                for (int h = 0; h < STEPS; ++h) {
+                    // A step's 32 pixels lie in at most 32 lines, from line j on:
+                    // a bit where each of the later ones starts gives every
+                    // lane its line.
+                    const int c0 = (st + h) * 32, c = c0 + lane;
+                    const int off = S.pix_off[j + lane] - c0;
+                    const unsigned starts = __reduce_or_sync(FULL, off > 0 && off < 32 ? 1u << off : 0u);
+                    const int i = __popc(starts & (0xffffffffu >> (31 - lane)));
+                    f[h].on = st + h < s1 && c < npix;
+                    if (f[h].on) {
+                        const uint32_t line = S.pix_line[j + i];
+                        const TriRec& r = S.recs[line >> 16];
+                        const int4 d = *reinterpret_cast<const int4*>(r.step);  // and 1 / area
+                        const int n = c - S.pix_off[j + i];
+                        const uint4 b0 = S.pix_base[j + i];
+                        float e[3];
+                        int u;
+                        if (BIG) {
+                            const uint4 b1 = S.pix_base[kChunk + j + i];
+                            const int m = n * kSub;
+                            const long long e0 = (long long)(((unsigned long long)b0.y << 32) | b0.x) + (long long)d.x * m,
+                                            e1 = (long long)(((unsigned long long)b0.w << 32) | b0.z) + (long long)d.y * m,
+                                            e2 = (long long)(((unsigned long long)b1.y << 32) | b1.x) + (long long)d.z * m;
+                            const bool wide = (e0 | e1 | e2) >= kHalvesLimit;
+                            e[0] = edge_to_float(e0, wide);
+                            e[1] = edge_to_float(e1, wide);
+                            e[2] = edge_to_float(e2, wide);
+                            u = (int)b1.z + n;
+                        } else {
+                            const uint32_t m = (uint32_t)(n * kSub);
+                            e[0] = __uint2float_rn(b0.x + (uint32_t)d.x * m);
+                            e[1] = __uint2float_rn(b0.y + (uint32_t)d.y * m);
+                            e[2] = __uint2float_rn(b0.z + (uint32_t)d.z * m);
+                            u = (int)b0.w + n;
+                        }
+                        const float inv = __int_as_float(d.w);
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) f[h].l[q] = e[q] * inv;
+                        f[h].z = interp(f[h].l, r.z[0], r.z[1], r.z[2]);
+                        const int v = (int)(line & 0xffffu);
+                        const bool columns = (r.flags & kRecColumns) != 0u;
+                        f[h].px = columns ? v : u;
+                        f[h].py = columns ? u : v;
+                        f[h].rec = &r;
+                    }
+                    j += __popc(starts);
+                    if (S.pix_off[j + 1] <= c0 + 32) ++j;  // that line's last pixel was the step's last
+                }
+                sink(f);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// Triangle of a thread: runs of RUN dealt out to the CTAs, since neighbours in
+// the array are often alike in size.
+template <int RUN>
+__device__ __forceinline__ long long my_triangle() {
+    return ((long long)(threadIdx.x / RUN) * gridDim.x + blockIdx.x) * RUN + (threadIdx.x % RUN);
+}
+
+// Every thread's set-up triangle: the small ones the 32-bit way, then the big
+// ones.
+template <int STEPS, int GRAB, class Sink>
+__device__ __forceinline__ void walk_all(LineShared& S, int lines, bool big, Sink& sink) {
+    walk_triangles<false, STEPS, GRAB>(S, big ? 0 : lines, sink);
+    if (__syncthreads_or(big)) walk_triangles<true, STEPS, GRAB>(S, big ? lines : 0, sink);
+}
+
+// Grid of a kernel over `ntri` triangles: as many CTAs to each 256 of them as
+// give `want` in all, at least two, at most 64.
+inline dim3 line_grid(long long ntri, long long want) {
+    const long long ctas = (ntri + kLineThreads - 1) / kLineThreads;
+    return dim3((unsigned)ctas, (unsigned)std::max(2LL, std::min((want + ctas - 1) / ctas, 64LL)));
+}
+
+}  // namespace lines
+}  // namespace vct

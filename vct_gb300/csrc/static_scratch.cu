@@ -7,13 +7,12 @@
 // allocate once a frame loop has started.  For them this entry point
 // voxelises a scene into output volumes the caller already owns, and keeps
 // everything else it needs (the 32-byte accumulator records, the occupancy
-// mask, the triangle set-up records and scans of the work distribution, and
-// the VoxelizeInfo counters) in one file-scope __device__ array of fixed
-// size.  Every GPU that loads the library holds that array until the process
+// mask and the VoxelizeInfo counters) in one file-scope __device__ array of
+// fixed size.  Every GPU that loads the library holds that array until the process
 // exits.
 //
 // Limits: grids up to VCT_STATIC_MAX_DIM^3 voxels and up to
-// VCT_STATIC_MAX_TRIANGLES triangles (about 9 MiB of device memory).
+// VCT_STATIC_MAX_TRIANGLES triangles (about 8 MiB of device memory).
 #include <mutex>
 
 #include "vct_device.cuh"
@@ -26,8 +25,7 @@ constexpr long long kMaxVoxels = (long long)VCT_STATIC_MAX_DIM * VCT_STATIC_MAX_
 constexpr long long kRecordBytes = align256(kMaxVoxels * kAccWords * 4);
 constexpr long long kOccBytes = align256((kMaxVoxels + 31) / 32 * 4);
 constexpr long long kStatsBytes = align256(sizeof(StatsDev));
-constexpr long long kWorkBytes = accumulate_scratch_bytes(VCT_STATIC_MAX_TRIANGLES);
-constexpr long long kScratchBytes = kRecordBytes + kOccBytes + kStatsBytes + kWorkBytes;
+constexpr long long kScratchBytes = kRecordBytes + kOccBytes + kStatsBytes;
 
 // The shared scratch.  Host code must not use this name as a device address:
 // on the host it is only a stand-in symbol, so the device address is looked
@@ -111,7 +109,6 @@ extern "C" vct_status vct_voxelize_static(const vct_config* cfg, const vct_param
     uint32_t* acc = reinterpret_cast<uint32_t*>(base);
     uint32_t* occ = reinterpret_cast<uint32_t*>(base + kRecordBytes);
     StatsDev* st_dev = reinterpret_cast<StatsDev*>(base + kRecordBytes + kOccBytes);
-    void* work = base + kRecordBytes + kOccBytes + kStatsBytes;
 
     // The array keeps whatever the previous call left; the records, the mask
     // and the counters must start at zero.
@@ -133,7 +130,6 @@ extern "C" vct_status vct_voxelize_static(const vct_config* cfg, const vct_param
     A.occ = occ;
     A.stats = st_dev;
     A.num_sms = num_sms;
-    accumulate_bind_scratch(A, work);
     launch_accumulate(A, st);
 
     NormalizeParams N;

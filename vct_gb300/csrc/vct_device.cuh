@@ -209,6 +209,34 @@ __device__ __forceinline__ float pcf5(const float* __restrict__ sm, int sw, int 
     float sz = (c[2] + 1.0f) * 0.5f;
     float frag = sz - 0.01f;
     if (frag > 1.0f) return 0.0f;
+    // The five taps' footprints share texels: when their corners are one texel
+    // apart (they nearly always are; the offsets are added before rounding)
+    // and inside the map, 12 loads from one address replace 20 with their
+    // border tests.
+    const float x[3] = {(sx * (float)sw + -1.0f) - 0.5f, (sx * (float)sw + 0.0f) - 0.5f, (sx * (float)sw + 1.0f) - 0.5f};
+    const float y[3] = {(sy * (float)sh + -1.0f) - 0.5f, (sy * (float)sh + 0.0f) - 0.5f, (sy * (float)sh + 1.0f) - 0.5f};
+    const float fx = floorf(x[1]), fy = floorf(y[1]);
+    if (floorf(x[0]) == fx - 1.0f && floorf(x[2]) == fx + 1.0f && floorf(y[0]) == fy - 1.0f &&
+        floorf(y[2]) == fy + 1.0f && fx >= 1.0f && fy >= 1.0f && fx < (float)(sw - 2) && fy < (float)(sh - 2)) {
+        const float* p = sm + ((int)fy * sw + (int)fx);  // at most 2^30 texels
+        const float *pu = p - sw, *pd = p + sw, *pd2 = pd + sw;
+        const float t00 = __ldg(p), t10 = __ldg(p + 1), t01 = __ldg(pd), t11 = __ldg(pd + 1);
+        const float l0 = __ldg(p - 1), l1 = __ldg(pd - 1), r0 = __ldg(p + 2), r1 = __ldg(pd + 2);
+        const float u0 = __ldg(pu), u1 = __ldg(pu + 1), d0 = __ldg(pd2), d1 = __ldg(pd2 + 1);
+        auto tap = [](float t00, float t10, float t01, float t11, float a, float b) {
+            const float bot = t00 * (1.0f - a) + t10 * a, top = t01 * (1.0f - a) + t11 * a;
+            return bot * (1.0f - b) + top * b;
+        };
+        const float a = x[1] - fx, b = y[1] - fy;
+        const float al = x[0] - (fx - 1.0f), ar = x[2] - (fx + 1.0f), bu = y[0] - (fy - 1.0f), bd = y[2] - (fy + 1.0f);
+        float n = 0.0f;
+        n += frag > tap(t00, t10, t01, t11, a, b) ? 1.0f : 0.0f;
+        n += frag > tap(t10, r0, t11, r1, ar, b) ? 1.0f : 0.0f;
+        n += frag > tap(t01, t11, d0, d1, a, bd) ? 1.0f : 0.0f;
+        n += frag > tap(l0, t00, l1, t01, al, b) ? 1.0f : 0.0f;
+        n += frag > tap(u0, u1, t00, t10, a, bu) ? 1.0f : 0.0f;
+        return __fdiv_rn(n, 5.0f);
+    }
     const int ox[5] = {0, 1, 0, -1, 0};
     const int oy[5] = {0, 0, 1, 0, -1};
     float f = 0.0f;

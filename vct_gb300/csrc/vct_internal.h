@@ -60,6 +60,10 @@ struct LightDev {
     // same fp32 operations the shader evaluates per fragment.
     f3 neg_dir_n;
     float range075;
+    // Squared distance past which a point light's attenuation is exactly 0
+    // (its smoothstep's quotient is at least 1); infinite for ranges for which
+    // that does not hold.
+    float beyond2;
 };
 
 struct StatsDev {
@@ -89,13 +93,13 @@ struct AccumParams {
     uint32_t* brick_exact;  // with `carry`: per 16^3 brick, set by the carry pass for the bricks it rewrote
     StatsDev* stats;
     int num_sms;
-    int unit_log2;      // log2 of the candidate pixels per work unit (whole rows of the bounding box)
+    int unit_log2;      // log2 of the pixels of a share of the raster work, about
     int blocks_per_sm;  // raster CTAs per SM (1..3)
     WarpDev warp;
     f3 vmin, vcenter, ext;  // voxelLinearPosition of the tessellation voxeliser
     float max_tess_level;   // GL_MAX_TESS_GEN_LEVEL
-    // Work distribution scratch (sized for ntri; see voxelize.cu).
-    uint4* tri_rec;          // 3 x uint4 per triangle
+    // Work distribution scratch of the tessellation voxeliser (sized for ntri).
+    uint4* tri_rec;          // uint4 per triangle
     uint32_t* tri_units;     // work units per triangle
     uint32_t* tri_scan;      // block-local exclusive scan of tri_units
     uint32_t* block_off;     // exclusive scan of per-block unit totals (+ total at [nblocks])
@@ -113,28 +117,27 @@ struct SceneBatch {
     int n;
 };
 
-// Voxeliser work distribution over all triangles of one launch (one scene, or
-// the concatenated triangles of a batch).
+// The tessellation voxeliser's work distribution over all triangles of one
+// launch (one scene, or the concatenated triangles of a batch).
 struct VoxWork {
     uint4* tri_rec;
     uint32_t* tri_units;
     uint32_t* tri_scan;
     uint32_t* block_off;
     long long ntri;
-    int unit_log2;
 };
 
 constexpr int kSetupThreads = 256;  // triangles per setup block
 constexpr long long align256(long long b) { return (b + 255) & ~255LL; }
-// Scratch bytes the voxeliser needs for `ntri` triangles: a 48-byte setup
-// record, a unit count and a scan entry per triangle, one offset per block
-// (+ the total), then an 8-byte work counter.
-constexpr long long accumulate_scratch_bytes(long long ntri) {
-    return align256(ntri * 48) + align256(ntri * 4) * 2 +
-           align256(((ntri + kSetupThreads - 1) / kSetupThreads + 2) * 4 + 8);
+// Scratch bytes the tessellation voxeliser needs for `ntri` triangles: a
+// 16-byte set-up record, a unit count and a scan entry per triangle, one
+// offset per block (+ the total).  The rasterising voxeliser needs none.
+constexpr long long tess_scratch_bytes(long long ntri) {
+    return align256(ntri * 16) + align256(ntri * 4) * 2 +
+           align256(((ntri + kSetupThreads - 1) / kSetupThreads + 1) * 4);
 }
 // Carves the scratch buffer into the AccumParams work arrays.
-void accumulate_bind_scratch(AccumParams& P, void* scratch);
+void tess_bind_scratch(AccumParams& P, void* scratch);
 
 // One 32-byte accumulator record per voxel: {count, r, g, b, nx, ny, nz, 0}.
 // Sums are of 16-bit fixed point (round(x * 65535)); they are updated as
@@ -329,8 +332,8 @@ void launch_fill_u32(uint32_t* p, uint32_t v, long long n, cudaStream_t s);
 
 // Batched frame stages: one launch covers the work of every scene.
 int accumulate_batch_max_scenes();
-void launch_accumulate_batch(const SceneBatch<AccumParams>& B, const VoxWork& W, int num_sms, int blocks_per_sm,
-                             cudaStream_t s);
+void launch_accumulate_batch(const SceneBatch<AccumParams>& B, long long ntri, int unit_log2, int num_sms,
+                             int blocks_per_sm, cudaStream_t s);
 void launch_tesselate_batch(const SceneBatch<AccumParams>& B, const VoxWork& W, int num_sms, cudaStream_t s);
 void launch_inject_mark_batch(const SceneBatch<InjectParams>& B, long long ntexels, cudaStream_t s);
 void launch_resolve_batch(const SceneBatch<ResolveParams>& B, long long nbricks, bool exact, cudaStream_t s);

@@ -1,83 +1,48 @@
 // Triangle voxelisation: shaders/voxelize.geom:25-73 + voxelize.frag:75-280.
 //
-// Three launches, balanced at fragment granularity (triangle sizes vary by
-// more than three orders of magnitude in one scene), for one scene or for the
-// concatenated triangles of a batch of scenes:
-//  1. voxelize_setup_kernel, one thread per triangle: the geometry-shader
-//     part (dominant axis from the summed vertex normals, per-axis ortho
-//     projection, snapping to the 1/256 sub-pixel grid, bounding box) into a
-//     48-byte record, and the triangle's share of work: its bounding box's
-//     rows in units of about 2^unit_log2 candidate pixels (a tuning
-//     setting), with a block-local exclusive scan;
-//  2. voxelize_scan_kernel, one CTA: exclusive scan of the per-block totals;
-//  3. voxelize_raster_kernel, persistent: warps take work units from a
-//     shared counter, narrow each row to the triangle's span, test 32 pixel
-//     centres at a time for coverage, compact
-//     covered fragments (clipped to the depth range) with a ballot into a
-//     per-warp ring queue in shared memory, and whenever 32 are queued each
-//     lane lights one fragment (all enabled lights, 5-tap PCF for shadow
-//     casters) and adds it into the voxel's 32-byte accumulator record with
-//     fire-and-forget 64-bit reductions.
+// One launch for one scene or for the concatenated triangles of a batch of
+// scenes (voxelize_raster_kernel): a thread does the geometry-shader part of a
+// triangle (dominant axis from the summed vertex normals, per-axis ortho
+// projection, snapping to the 1/256 sub-pixel grid), the CTA walks the covered
+// runs of its triangles' lines (lines.cuh), and each lane of a step lights one
+// fragment (all enabled lights, 5-tap PCF for shadow casters) and adds it into
+// the voxel's 32-byte accumulator record with fire-and-forget 64-bit
+// reductions.
+//
+// What bounds it: issue (59% of peak at 3 CTAs, 24 warps, per SM; stalls on
+// shared and global loads), some 700 instructions per 32 fragments, most of
+// them the lighting's.  262,144 triangles, 5 lights, 6.7 M fragments into
+// 256^3: 0.29 ms, 300 MB of records read and 167 MB written.  The form before
+// had triangle set-up and a scan as kernels of their own, units of bounding-box
+// rows taken by warps from a shared counter, an edge test per candidate pixel
+// and a queue of the covered ones: 0.35 ms, and 0.10 against 0.016 ms for 1,290
+// triangles in 64^3, where ten walls' units left most warps idle.  Runs of 32
+// triangles to a CTA keep neighbouring triangles' records in the L2 together
+// (0.29 ms; runs of 64: 0.31, 16: 0.32, 256: 0.35).
 //
 // Integer sums make the result independent of fragment order: it is
 // bit-exact against the CPU oracle.  Compiled with --fmad=false (see
 // vct_device.cuh).
-#include "vct_device.cuh"
+#include "lines.cuh"
 
 namespace vct {
 
 namespace {
 
-constexpr int kWarps = 8;
-constexpr int kQueue = 64;
-constexpr int kRasterBlocksPerSM = 3;  // register budget: up to 3 raster CTAs per SM
-constexpr int kMaxBatchScenes = 256;  // scene id travels in 8 bits of a queue entry
-constexpr int kGrabUnits = 2;          // work units a warp takes from the shared counter at a time
-constexpr int kStagedBlocks = 4096;    // setup-block offsets copied to shared memory when they fit
+using namespace lines;
 
-// The raster warps' shared work counter: 8 bytes after block_off[nblocks]
-// (zeroed by the setup kernel).
-__device__ __forceinline__ unsigned long long* grab_counter(const VoxWork& W, int nblocks) {
-    return reinterpret_cast<unsigned long long*>(W.block_off + (((long long)nblocks + 2) & ~1LL));
-}
+constexpr int kWarps = 8;
+constexpr int kRasterBlocksPerSM = 3;  // register budget: up to 3 raster CTAs per SM
+constexpr int kMaxBatchScenes = 256;   // per-scene fragment counters in shared memory
 
 // Bit of a triangle's edge flags: its area is past halves_to_float's range.
 constexpr int kWide = 8;
-
-struct FragQueue {
-    int tri[kQueue];       // triangle index within its scene
-    uint32_t pix[kQueue];  // px | py << 11 | axis << 22 | scene << 24
-    float l0[kQueue], l1[kQueue], l2[kQueue], z[kQueue];
-};
 
 __device__ __forceinline__ float shadow_factor(const AccumParams& P, f3 wp) {
     return pcf5(P.shadowmap, P.sw, P.sh, P.ls, wp);
 }
 
-// Block-local exclusive scan of the per-triangle unit counts of one setup
-// block into tri_scan, and the block's total into block_off[blockIdx.x].
-__device__ __forceinline__ void block_scan_units(const VoxWork& W, long long g, uint32_t units) {
-    __shared__ uint32_t warp_tot[kSetupThreads / 32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    uint32_t incl = units;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-    }
-    if (lane == 31) warp_tot[wid] = incl;
-    __syncthreads();
-    uint32_t before = 0, total = 0;
-#pragma unroll
-    for (int w = 0; w < kSetupThreads / 32; ++w) {
-        before += (w < wid) ? warp_tot[w] : 0u;
-        total += warp_tot[w];
-    }
-    if (g < W.ntri) W.tri_scan[g] = before + incl - units;
-    if (threadIdx.x == 0) W.block_off[blockIdx.x] = total;
-}
-
-// ------------------------------------------------------------- 1. setup
+// ------------------------------------------------------------- set-up
 // voxelize.geom:25-73 for triangle t of P: the dominant axis of the summed
 // normals (strict >, ties to z, or the override), the projection through
 // that axis' orthographic matrix into the N x N viewport, and the snapped
@@ -111,75 +76,7 @@ __device__ __forceinline__ bool project_triangle(const AccumParams& P, long long
     return raster_setup(wx, wy, N, N, rt);
 }
 
-template <class Scenes>
-__global__ void __launch_bounds__(kSetupThreads) voxelize_setup_kernel(const Scenes S, const VoxWork W) {
-    const long long g = (long long)blockIdx.x * kSetupThreads + threadIdx.x;
-    uint32_t units = 0;
-    if (g < W.ntri) {
-        long long t;
-        const AccumParams& P = S.get(S.find(g, t));
-        RasterTri rt;
-        float z[3];
-        int axis;
-        if (project_triangle(P, t, rt, z, axis)) {
-            const uint32_t bw = rt.px1 - rt.px0 + 1, bh = rt.py1 - rt.py0 + 1;
-            const uint32_t bias = (rt.bias[0] ? 1u : 0u) | (rt.bias[1] ? 2u : 0u) | (rt.bias[2] ? 4u : 0u) |
-                                  (rt.wide() ? (uint32_t)kWide : 0u);
-            const float inv = __fdiv_rn(1.0f, rt.area_float());
-            uint4* rec = W.tri_rec + 3 * g;
-            rec[0] = make_uint4((uint32_t)rt.X[0], (uint32_t)rt.Y[0], (uint32_t)rt.X[1], (uint32_t)rt.Y[1]);
-            rec[1] = make_uint4((uint32_t)rt.X[2], (uint32_t)rt.Y[2], __float_as_uint(z[0]), __float_as_uint(z[1]));
-            // A work unit is R whole rows of the bounding box, R chosen so that
-            // the unit holds about 2^unit_log2 candidate pixels: a row's span
-            // of the triangle (the area over the rows, on average) and a
-            // pixel each side.  A sliver's rows are short, so its units take
-            // many rows.
-            const float row_px = rt.area_float() * (0.5f / (float)(kSub * kSub)) / (float)bh + 2.0f;
-            const uint32_t R = (uint32_t)fminf(fmaxf((float)(1u << W.unit_log2) / row_px, 1.0f), 1023.0f);
-            rec[2] = make_uint4(__float_as_uint(z[2]), __float_as_uint(inv),
-                                (uint32_t)rt.px0 | ((uint32_t)rt.py0 << 11) | ((uint32_t)axis << 22) |
-                                    ((uint32_t)rt.perm1 << 24) | (bias << 25),
-                                bw | (bh << 11) | (R << 22));
-            units = (bh + R - 1) / R;
-        }
-        W.tri_units[g] = units;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) *grab_counter(W, gridDim.x) = 0ull;
-    block_scan_units(W, g, units);
-}
-
-// --------------------------------------------------------------- 2. scan
-__global__ void __launch_bounds__(1024) voxelize_scan_kernel(uint32_t* block_off, int nblocks) {
-    __shared__ uint32_t warp_tot[32];
-    __shared__ uint32_t carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int base = 0; base < nblocks; base += 1024) {
-        const int i = base + threadIdx.x;
-        const uint32_t v = i < nblocks ? block_off[i] : 0u;
-        uint32_t incl = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t s = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += s;
-        }
-        if (lane == 31) warp_tot[wid] = incl;
-        __syncthreads();
-        uint32_t before = carry, total = 0;
-        for (int w = 0; w < 32; ++w) {
-            before += (w < wid) ? warp_tot[w] : 0u;
-            total += warp_tot[w];
-        }
-        if (i < nblocks) block_off[i] = before + incl - v;
-        __syncthreads();
-        if (threadIdx.x == 0) carry += total;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) block_off[nblocks] = carry;
-}
-
-// ------------------------------------------------------------- 3. raster
+// ------------------------------------------------------------- raster
 // Voxel of a fragment: voxelize.frag:79-108.  Without warping the axis
 // swizzle resolves to integers: the projected coordinates are the pixel
 // indices and the depth axis is trunc(N * (1 - u.z)).  With warping the
@@ -219,16 +116,35 @@ __device__ __forceinline__ bool fragment_voxel(const AccumParams& P, int px, int
     return !(vx < 0 || vy < 0 || vz < 0 || vx >= N || vy >= N || vz >= N);
 }
 
-// voxelize.frag:186-280 for one queued fragment.
-__device__ __forceinline__ void shade_fragment(const AccumParams& P, const FragQueue& q, int e) {
-    const long long t = q.tri[e];
-    const uint32_t pix = q.pix[e];
-    const int px = (int)(pix & 0x7ffu), py = (int)((pix >> 11) & 0x7ffu), axis = (int)((pix >> 22) & 3u);
+// A warp's fragments on their way to the records: the four 64-bit words each
+// adds and where (null: nothing).
+struct RecordStage {
+    ulonglong2 words[32][2];
+    unsigned long long* rec[32];
+};
+
+// Adds the staged fragments with fire-and-forget reductions (no result is
+// waited for): four lanes take the four words of one record, so an
+// instruction's 32 reductions fall into 8 sectors.  A lane adding all of its
+// own record's words sends a sector per word (6.7 M fragments: 40 M requests to
+// the L2 against 17 M).
+__device__ __forceinline__ void flush_stage(const RecordStage& st, int lane) {
+    const unsigned long long* w = reinterpret_cast<const unsigned long long*>(st.words);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        unsigned long long* rec = st.rec[8 * i + (lane >> 2)];
+        if (rec) atomicAdd(rec + (lane & 3), w[32 * i + lane]);
+    }
+}
+
+// voxelize.frag:186-280 for one fragment: triangle t of the scene, pixel
+// (px, py) of its dominant axis' view, weights l and depth z.
+__device__ __forceinline__ void shade_fragment(const AccumParams& P, long long t, int axis, int px, int py,
+                                               const float l[3], float z, RecordStage& st, int lane) {
     int vx, vy, vz;
-    if (!fragment_voxel(P, px, py, axis, q.z[e], vx, vy, vz)) return;
+    if (!fragment_voxel(P, px, py, axis, z, vx, vy, vz)) return;
     const int N = P.dim;
     const long long v = ((long long)vz * N + vy) * N + vx;
-    const float l[3] = {q.l0[e], q.l1[e], q.l2[e]};
     const float* Pp = P.pos + t * 9;
     const float* Pn = P.nrm + t * 9;
     const f3 p0 = ld3(Pp), p1 = ld3(Pp + 3), p2 = ld3(Pp + 6);
@@ -245,8 +161,18 @@ __device__ __forceinline__ void shade_fragment(const AccumParams& P, const FragQ
             f3 lit = mk(0.0f, 0.0f, 0.0f);
             if (L.type == 0u) {
                 f3 d = sub(L.position, wp);
+                // Out of the light's range the attenuation is exactly 0, and
+                // for a surface turned well away (by more than rounding) the
+                // cosine is: the light then adds +-0, unless its product with
+                // the albedo overflows.  Four point lights of range 0.3-0.8 in a
+                // volume of side 2 leave one in nine fragments inside one.
+                const f3 base = mulv(mul(color, L.intensity), L.color);
+                const float d2 = dot(d, d), nd = dot(Nf, d);
+                if ((d2 > L.beyond2 || (nd < 0.0f && nd * nd > 1e-6f * d2 && d2 > 1e-30f && L.beyond2 < 3.0e38f)) &&
+                    fmaxf(fmaxf(fabsf(base.x), fabsf(base.y)), fabsf(base.z)) < 3.0e38f)
+                    continue;
                 float ndl = fmaxf(0.0f, dot(Nf, normalize(d)));
-                lit = mul(mulv(mul(color, L.intensity), L.color), ndl);
+                lit = mul(base, ndl);
                 float att = 1.0f - smoothstep(L.range075, L.range, length(d));
                 lit = mul(lit, att);
             } else if (L.type == 1u) {
@@ -266,15 +192,102 @@ __device__ __forceinline__ void shade_fragment(const AccumParams& P, const FragQ
     unsigned long long* rec = reinterpret_cast<unsigned long long*>(P.acc + kAccWords * record_slot(v, P.dim));
     const unsigned long long qr = quant16(color.x), qg = quant16(color.y), qb = quant16(color.z);
     const unsigned long long qx = quant16(n01.x), qy = quant16(n01.y), qz = quant16(n01.z);
-    // Fire-and-forget reductions: no result is waited for.  (Setting the
-    // occupancy bit only for the fragment that finds the count at 0 waits
-    // for the first add's result and is slower.)
-    atomicAdd(rec + 0, 1ull | (qr << 32));
-    atomicAdd(rec + 1, qg | (qb << 32));
-    atomicAdd(rec + 2, qx | (qy << 32));
-    atomicAdd(rec + 3, qz);
+    st.words[lane][0] = make_ulonglong2(1ull | (qr << 32), qg | (qb << 32));
+    st.words[lane][1] = make_ulonglong2(qx | (qy << 32), qz);
+    st.rec[lane] = rec;
+    // (Setting the occupancy bit only for the fragment that finds the count at
+    // 0 waits for the first add's result and is slower.)
     atomicOr(P.occ + (v >> 5), 1u << (v & 31));
 }
+
+// Lights 32 fragments, one per lane, and counts them for
+// VoxelizeInfo.totalVoxelFragments: covered and inside GL's depth clip.
+template <class Scenes>
+struct VoxelSink {
+    const Scenes& S;
+    RecordStage& stage;
+    unsigned* frag_count;  // per scene, in shared memory
+    int lane;
+    __device__ __forceinline__ void operator()(const LinePixel (&f)[1]) {
+        const unsigned FULL = 0xffffffffu;
+        const bool on = f[0].on && f[0].z >= -1.0f && f[0].z <= 1.0f;
+        const unsigned m = __ballot_sync(FULL, on);
+        if (!m) return;
+        const int scene = on ? (int)f[0].rec->user[1] : 0;
+        if (S.count() == 1) {
+            if (lane == 0) atomicAdd(frag_count, (unsigned)__popc(m));
+        } else if (on) {
+            atomicAdd(frag_count + scene, 1u);
+        }
+        stage.rec[lane] = nullptr;
+        if (on)
+            shade_fragment(S.get(scene), f[0].rec->tri, (int)f[0].rec->user[0], f[0].px, f[0].py, f[0].l, f[0].z, stage,
+                           lane);
+        __syncwarp();
+        flush_stage(stage, lane);
+        __syncwarp();
+    }
+};
+
+template <class Scenes>
+__global__ void __launch_bounds__(kLineThreads, kRasterBlocksPerSM)
+    voxelize_raster_kernel(const Scenes S, long long ntri) {
+    __shared__ LineShared L;
+    __shared__ RecordStage stages[kWarps];
+    __shared__ unsigned frag_count[kMaxBatchScenes];
+    const int nscenes = S.count();
+    for (int i = threadIdx.x; i < nscenes; i += blockDim.x) frag_count[i] = 0;
+    const long long g = my_triangle<32>();
+    int lines = 0;
+    bool big = false;
+    if (g < ntri) {
+        long long t;
+        const int scene = S.find(g, t);
+        RasterTri rt;
+        float z[3];
+        int axis;
+        if (project_triangle(S.get(scene), t, rt, z, axis)) {
+            TriRec& r = L.recs[threadIdx.x];
+            lines = store_rec(r, rt, z, (int)t);
+            r.user[0] = (uint32_t)axis;
+            r.user[1] = (uint32_t)scene;
+            big = rt.area >= kBigArea;
+        }
+    }
+    VoxelSink<Scenes> sink = {S, stages[threadIdx.x >> 5], frag_count, (int)(threadIdx.x & 31)};
+    walk_all<1, 2>(L, lines, big, sink);
+    __syncthreads();
+    for (int i = threadIdx.x; i < nscenes; i += blockDim.x)
+        if (frag_count[i]) atomicAdd(&S.get(i).stats->total_voxel_fragments, frag_count[i]);
+}
+
+// By default (units of 512 pixels, 3 CTAs per SM) 9 CTAs per SM, three times
+// as many as are resident; smaller units share the lines out further.  Each
+// CTA that sets the same triangles up again costs some 7 us of latency (loads,
+// projection, scans), each CTA too few leaves SMs idle at the end: with 6, 12
+// and 24 per SM 38,000 triangles in 128^3 take 53, 66 and 96 us, 74,752 in
+// 256^3 0.304, 0.281 and (24 not measured); past 300,000 triangles the least,
+// two to each 256, is best (519,552: 0.497 with one, 0.460 with two).
+template <class Scenes>
+void launch_voxelize(const Scenes& S, long long ntri, int unit_log2, int num_sms, int blocks_per_sm, cudaStream_t s) {
+    if (ntri <= 0) return;
+    const int bps = blocks_per_sm < 1 ? 1 : (blocks_per_sm > kRasterBlocksPerSM ? kRasterBlocksPerSM : blocks_per_sm);
+    const dim3 grid = line_grid(ntri, (((long long)num_sms * bps * 3) << 9) >> unit_log2);
+    voxelize_raster_kernel<Scenes><<<grid, kLineThreads, 0, s>>>(S, ntri);
+    note_launches(1);
+}
+
+// ================================================ warp-map occupancy pass
+// voxelize.frag:187-192: the occupancy voxelisation that the warp map is
+// built from (Application.cpp:235-285), the same rasterisation rule as above
+// at a 32^2 viewport, unwarped and unshaded.  Nearly every triangle of a
+// scene covers a handful of pixels at that size, so that
+// sharing out lines and pixels would cost far more than the pixels: one thread takes one triangle,
+// sets it up and walks a bounding box of up to kOccLanePixels pixels itself;
+// the warp walks the larger ones together, 32 pixels at a time.  The result
+// is an OR of bits, so the order of the walks does not matter.
+constexpr int kOccThreads = 256;
+constexpr int kOccLanePixels = 32;
 
 // Coverage of pixel (px, py) by a set-up triangle (snapped vertices X, Y; edge
 // k runs from vertex a = k+1 to b = k+2 with deltas dX, dY; bit k of `bias`
@@ -305,218 +318,6 @@ __device__ __forceinline__ bool pixel_fragment(const int X[3], const int Y[3], c
     zf = interp(l, z[0], z[1], z[2]);
     return zf >= -1.0f && zf <= 1.0f;  // GL clipping
 }
-
-template <class Scenes>
-__device__ __forceinline__ long long unit_start(const VoxWork& W, long long g) {
-    return (long long)W.block_off[g / kSetupThreads] + W.tri_scan[g];
-}
-
-template <class Scenes>
-__global__ void __launch_bounds__(kWarps * 32, kRasterBlocksPerSM)
-    voxelize_raster_kernel(const Scenes S, const VoxWork W, int nblocks) {
-    __shared__ FragQueue queues[kWarps];
-    __shared__ unsigned frag_count[kMaxBatchScenes];  // VoxelizeInfo.totalVoxelFragments per scene
-    __shared__ uint32_t s_boff[kStagedBlocks + 1];
-    const int lane = threadIdx.x & 31;
-    FragQueue& q = queues[threadIdx.x >> 5];
-    const unsigned FULL = 0xffffffffu;
-    const int nscenes = S.count();
-    for (int i = threadIdx.x; i < nscenes; i += blockDim.x) frag_count[i] = 0;
-    const bool staged = nblocks <= kStagedBlocks;
-    if (staged)
-        for (int i = threadIdx.x; i <= nblocks; i += blockDim.x) s_boff[i] = W.block_off[i];
-    __syncthreads();
-    auto boff = [&](long long b) -> long long { return staged ? s_boff[b] : W.block_off[b]; };
-    const long long total = boff(nblocks);
-    unsigned long long* grab = grab_counter(W, nblocks);
-    // The queue is a ring of kQueue entries: fragments [head, head + qn).
-    int qn = 0, head = 0;  // warp-uniform
-
-    // Shades the 32 oldest queued fragments (or `nact`), one per lane.
-    auto shade32 = [&](int nact) {
-        __syncwarp();
-        if (lane < nact) {
-            const int e = (head + lane) & (kQueue - 1);
-            shade_fragment(S.get((int)(q.pix[e] >> 24)), q, e);
-        }
-        __syncwarp();
-    };
-    // VoxelizeInfo.totalVoxelFragments: covered fragments are counted where
-    // they are queued, for the unit's scene, and added to the CTA's
-    // per-scene counter when the scene changes.
-    int cur_scene = 0;
-    unsigned pending = 0;
-    auto flush_count = [&]() {
-        if (lane == 0 && pending) atomicAdd(&frag_count[cur_scene], pending);
-        pending = 0;
-    };
-
-    // Warps take kGrabUnits work units at a time from a shared counter until
-    // none are left, so that every warp ends at about the same time whatever
-    // the units cost (their pixel counts and coverage vary by orders of
-    // magnitude).  Fragments are summed as integers, so the order in which
-    // warps take the units does not change the result.
-    for (;;) {
-        unsigned long long gu = 0;
-        if (lane == 0) gu = atomicAdd(grab, (unsigned long long)kGrabUnits);
-        gu = __shfl_sync(FULL, gu, 0);
-        if ((long long)gu >= total) break;
-        const long long u0 = (long long)gu, u1 = min(u0 + (long long)kGrabUnits, total);
-        // Triangle owning unit u0: binary search over the block offsets, then
-        // the block-local scan, 8 entries per lane: the number of entries <=
-        // u0 is one past the last triangle starting at or before u0.
-        int lo = 0, hi = nblocks - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (boff(mid) <= u0)
-                lo = mid;
-            else
-                hi = mid - 1;
-        }
-        const long long gbase = (long long)lo * kSetupThreads;
-        const int in_block = (int)min((long long)kSetupThreads, W.ntri - gbase);
-        const uint32_t rel = (uint32_t)(u0 - boff(lo));
-        int below = 0;
-#pragma unroll
-        for (int j = 0; j < kSetupThreads / 32; ++j) {
-            const int k = lane * (kSetupThreads / 32) + j;
-            below += (k < in_block && __ldg(W.tri_scan + gbase + k) <= rel) ? 1 : 0;
-        }
-        below = __reduce_add_sync(FULL, below);
-        long long g = gbase + max(below - 1, 0);
-        long long start = boff(lo) + W.tri_scan[g];
-        uint32_t nunits = W.tri_units[g];
-        for (long long u = u0; u < u1; ++u) {
-            while (u >= start + nunits) {
-                ++g;
-                start = boff(g / kSetupThreads) + W.tri_scan[g];
-                nunits = W.tri_units[g];
-            }
-            long long tl;
-            const int scene = S.find(g, tl);
-            if (scene != cur_scene) {
-                flush_count();
-                cur_scene = scene;
-            }
-            const uint4* rp = W.tri_rec + 3 * g;
-            const uint4 r0 = __ldg(rp), r1 = __ldg(rp + 1), r2 = __ldg(rp + 2);
-            const int X[3] = {(int)r0.x, (int)r0.z, (int)r1.x};
-            const int Y[3] = {(int)r0.y, (int)r0.w, (int)r1.y};
-            const float z[3] = {__uint_as_float(r1.z), __uint_as_float(r1.w), __uint_as_float(r2.x)};
-            const float inv = __uint_as_float(r2.y);
-            const int px0 = (int)(r2.z & 0x7ffu), py0 = (int)((r2.z >> 11) & 0x7ffu);
-            const int axis = (int)((r2.z >> 22) & 3u), perm1 = (int)((r2.z >> 24) & 1u), bias = (int)(r2.z >> 25);
-            const int bw = (int)(r2.w & 0x7ffu), bh = (int)((r2.w >> 11) & 0x7ffu), R = (int)(r2.w >> 22);
-            int dX[3], dY[3];  // edge k: vertex k+2 minus vertex k+1
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                dX[k] = X[(k + 2) % 3] - X[(k + 1) % 3];
-                dY[k] = Y[(k + 2) % 3] - Y[(k + 1) % 3];
-            }
-            // The unit's rows of the bounding box, 32 at a time: each lane takes
-            // one row and narrows it to the pixels between the triangle's
-            // crossings of the row's centre line (widened by one pixel each
-            // side, so that float rounding never drops a covered pixel); the
-            // warp then tests the rows' candidates 32 at a time.
-            const int r_a = (int)(u - start) * R, r_b = min(r_a + R, bh) - 1;
-            float slope[3];  // x per unit y along edge k
-#pragma unroll
-            for (int k = 0; k < 3; ++k) slope[k] = dY[k] != 0 ? __fdividef((float)dX[k], (float)dY[k]) : 0.0f;
-            for (int rb = r_a; rb <= r_b; rb += 32) {
-                const int r = rb + lane;
-                int lo = 0, cnt = 0;
-                if (r <= r_b) {
-                    const int sy = (py0 + r) * kSub + kSub / 2;
-                    float xmin = 3.0e38f, xmax = -3.0e38f;
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) {
-                        const int a = (k + 1) % 3, bb = (k + 2) % 3;
-                        if (min(Y[a], Y[bb]) <= sy && sy <= max(Y[a], Y[bb])) {
-                            const float x0 = dY[k] != 0 ? fmaf((float)(sy - Y[a]), slope[k], (float)X[a]) : (float)X[a];
-                            const float x1 = dY[k] != 0 ? x0 : (float)X[bb];
-                            xmin = fminf(xmin, fminf(x0, x1));
-                            xmax = fmaxf(xmax, fmaxf(x0, x1));
-                        }
-                    }
-                    if (xmin <= xmax) {
-                        const float rs = 1.0f / (float)kSub, hs = 0.5f * (float)kSub;
-                        const int s0 = (int)ceilf((xmin - hs) * rs) - 1 - px0;
-                        const int s1 = (int)floorf((xmax - hs) * rs) + 1 - px0;
-                        lo = max(0, s0);
-                        cnt = max(min(bw - 1, s1) - lo + 1, 0);
-                    }
-                }
-                int excl = cnt;  // exclusive prefix of the rows' candidate counts
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int v = __shfl_up_sync(FULL, excl, o);
-                    if (lane >= o) excl += v;
-                }
-                const int ncand = __shfl_sync(FULL, excl, 31);
-                excl -= cnt;
-                for (int k0 = 0; k0 < ncand; k0 += 32) {
-                    const int kc = k0 + lane;
-                    int j = 0;  // the last row whose candidates start at or before kc
-#pragma unroll
-                    for (int st = 16; st > 0; st >>= 1)
-                        if (__shfl_sync(FULL, excl, j + st) <= kc) j += st;
-                    const int lo_j = __shfl_sync(FULL, lo, j), ex_j = __shfl_sync(FULL, excl, j);
-                    bool cov = false;
-                    float l[3] = {0.f, 0.f, 0.f}, zf = 0.f;
-                    const int py = py0 + rb + j, px = px0 + lo_j + (kc - ex_j);
-                    if (kc < ncand) cov = pixel_fragment(X, Y, dX, dY, bias, perm1, inv, z, px, py, l, zf);
-                    const unsigned m = __ballot_sync(FULL, cov);
-                    if (cov) {
-                        const int slot = (head + qn + __popc(m & ((1u << lane) - 1u))) & (kQueue - 1);
-                        q.tri[slot] = (int)tl;
-                        q.pix[slot] = (uint32_t)px | ((uint32_t)py << 11) | ((uint32_t)axis << 22) |
-                                      ((uint32_t)scene << 24);
-                        q.l0[slot] = l[0];
-                        q.l1[slot] = l[1];
-                        q.l2[slot] = l[2];
-                        q.z[slot] = zf;
-                    }
-                    qn += __popc(m);
-                    pending += (unsigned)__popc(m);
-                    if (qn >= 32) {
-                        shade32(32);
-                        head = (head + 32) & (kQueue - 1);
-                        qn -= 32;
-                    }
-                }
-            }
-        }
-    }
-    shade32(qn);
-    flush_count();
-    __syncthreads();
-    for (int i = threadIdx.x; i < nscenes; i += blockDim.x)
-        if (frag_count[i]) atomicAdd(&S.get(i).stats->total_voxel_fragments, frag_count[i]);
-}
-
-template <class Scenes>
-void launch_voxelize(const Scenes& S, const VoxWork& W, int num_sms, int blocks_per_sm, cudaStream_t s) {
-    if (W.ntri <= 0) return;
-    const int nblocks = (int)((W.ntri + kSetupThreads - 1) / kSetupThreads);
-    voxelize_setup_kernel<Scenes><<<nblocks, kSetupThreads, 0, s>>>(S, W);
-    voxelize_scan_kernel<<<1, 1024, 0, s>>>(W.block_off, nblocks);
-    const int bps = blocks_per_sm < 1 ? 1 : (blocks_per_sm > kRasterBlocksPerSM ? kRasterBlocksPerSM : blocks_per_sm);
-    voxelize_raster_kernel<Scenes><<<num_sms * bps, kWarps * 32, 0, s>>>(S, W, nblocks);
-    note_launches(3);
-}
-
-// ================================================ warp-map occupancy pass
-// voxelize.frag:187-192: the occupancy voxelisation that the warp map is
-// built from (Application.cpp:235-285), the same rasterisation rule as above
-// at a 32^2 viewport, unwarped and unshaded.  Nearly every triangle of a
-// scene covers a handful of pixels at that size, so the persistent raster's
-// work units (one shared-counter grab, a search and three dependent loads
-// each) would cost far more than the pixels: one thread takes one triangle,
-// sets it up and walks a bounding box of up to kOccLanePixels pixels itself;
-// the warp walks the larger ones together, 32 pixels at a time.  The result
-// is an OR of bits, so the order of the walks does not matter.
-constexpr int kOccThreads = 256;
-constexpr int kOccLanePixels = 32;
 
 __device__ __forceinline__ void occupancy_fragment(const AccumParams& P, int axis, int px, int py, float zf) {
     int vx, vy, vz;
@@ -615,6 +416,64 @@ __global__ void __launch_bounds__(kOccThreads) occupancy_kernel(const Scenes S, 
 // Tessellation levels after GL's equal_spacing rounding, packed 7 bits each:
 // inner n | outer[0] << 7 | outer[1] << 14 | outer[2] << 21 (1..64 each).
 constexpr int kTessUnit = 32;
+
+// Block-local exclusive scan of the per-triangle unit counts of one setup
+// block into tri_scan, and the block's total into block_off[blockIdx.x].
+__device__ __forceinline__ void block_scan_units(const VoxWork& W, long long g, uint32_t units) {
+    __shared__ uint32_t warp_tot[kSetupThreads / 32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    uint32_t incl = units;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) warp_tot[wid] = incl;
+    __syncthreads();
+    uint32_t before = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < kSetupThreads / 32; ++w) {
+        before += (w < wid) ? warp_tot[w] : 0u;
+        total += warp_tot[w];
+    }
+    if (g < W.ntri) W.tri_scan[g] = before + incl - units;
+    if (threadIdx.x == 0) W.block_off[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(1024) voxelize_scan_kernel(uint32_t* block_off, int nblocks) {
+    __shared__ uint32_t warp_tot[32];
+    __shared__ uint32_t carry;
+    if (threadIdx.x == 0) carry = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int base = 0; base < nblocks; base += 1024) {
+        const int i = base + threadIdx.x;
+        const uint32_t v = i < nblocks ? block_off[i] : 0u;
+        uint32_t incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            uint32_t s = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += s;
+        }
+        if (lane == 31) warp_tot[wid] = incl;
+        __syncthreads();
+        uint32_t before = carry, total = 0;
+        for (int w = 0; w < 32; ++w) {
+            before += (w < wid) ? warp_tot[w] : 0u;
+            total += warp_tot[w];
+        }
+        if (i < nblocks) block_off[i] = before + incl - v;
+        __syncthreads();
+        if (threadIdx.x == 0) carry += total;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) block_off[nblocks] = carry;
+}
+
+template <class Scenes>
+__device__ __forceinline__ long long unit_start(const VoxWork& W, long long g) {
+    return (long long)W.block_off[g / kSetupThreads] + W.tri_scan[g];
+}
 
 // Float-to-int truncation of ivec3(): NaN -> 0, saturating (cvt.rzi.s32.f32).
 __device__ __forceinline__ int trunc_sat(float x) { return __float2int_rz(x); }
@@ -733,7 +592,7 @@ __global__ void __launch_bounds__(kSetupThreads) tess_setup_kernel(const Scenes 
         const AccumParams& P = S.get(scene);
         uint32_t packed = 0, npts = 0;
         if (!tess_levels(P, P.pos + t * 9, packed, npts)) npts = 0;
-        W.tri_rec[3 * g] = make_uint4(packed, npts, (uint32_t)scene, (uint32_t)t);
+        W.tri_rec[g] = make_uint4(packed, npts, (uint32_t)scene, (uint32_t)t);
         units = (npts + kTessUnit - 1) / kTessUnit;
         W.tri_units[g] = units;
     }
@@ -910,7 +769,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4) tess_points_kernel(const Scene
                 start = unit_start<Scenes>(W, g);
                 nunits = W.tri_units[g];
             }
-            const uint4 r = __ldg(W.tri_rec + 3 * g);
+            const uint4 r = __ldg(W.tri_rec + g);
             const int base = (int)(u - start) * kTessUnit;
             const int cnt = min(kTessUnit, (int)r.y - base);
             if (lane < cnt) {
@@ -961,7 +820,7 @@ void launch_tess(const Scenes& S, const VoxWork& W, int num_sms, cudaStream_t s)
 // The tessellation voxeliser: setup, scan, points (the same scratch as the
 // rasteriser's).
 void launch_tesselate(const AccumParams& P, cudaStream_t s) {
-    const VoxWork W = {P.tri_rec, P.tri_units, P.tri_scan, P.block_off, P.ntri, 0};
+    const VoxWork W = {P.tri_rec, P.tri_units, P.tri_scan, P.block_off, P.ntri};
     launch_tess(OneScene<AccumParams>{P}, W, P.num_sms, s);
     if (P.carry) {
         carry_fixup_kernel<<<dim3(kCarrySlots / 256, 1), 256, 0, s>>>(OneScene<AccumParams>{P});
@@ -975,11 +834,11 @@ void launch_tesselate_batch(const SceneBatch<AccumParams>& B, const VoxWork& W, 
     note_launches(1);
 }
 
-void accumulate_bind_scratch(AccumParams& P, void* scratch) {
+void tess_bind_scratch(AccumParams& P, void* scratch) {
     char* p = static_cast<char*>(scratch);
     const long long ntri = P.ntri;
     P.tri_rec = reinterpret_cast<uint4*>(p);
-    p += align256(ntri * 48);
+    p += align256(ntri * 16);
     P.tri_units = reinterpret_cast<uint32_t*>(p);
     p += align256(ntri * 4);
     P.tri_scan = reinterpret_cast<uint32_t*>(p);
@@ -1002,15 +861,14 @@ void launch_occupancy_batch(const SceneBatch<AccumParams>& B, long long ntri, cu
 }
 
 void launch_accumulate(const AccumParams& P, cudaStream_t s) {
-    const VoxWork W = {P.tri_rec, P.tri_units, P.tri_scan, P.block_off, P.ntri, P.unit_log2};
-    launch_voxelize(OneScene<AccumParams>{P}, W, P.num_sms, P.blocks_per_sm, s);
+    launch_voxelize(OneScene<AccumParams>{P}, P.ntri, P.unit_log2, P.num_sms, P.blocks_per_sm, s);
 }
 
 int accumulate_batch_max_scenes() { return kMaxBatchScenes; }
 
-void launch_accumulate_batch(const SceneBatch<AccumParams>& B, const VoxWork& W, int num_sms, int blocks_per_sm,
-                             cudaStream_t s) {
-    launch_voxelize(ManyScenes<AccumParams>{B}, W, num_sms, blocks_per_sm, s);
+void launch_accumulate_batch(const SceneBatch<AccumParams>& B, long long ntri, int unit_log2, int num_sms,
+                             int blocks_per_sm, cudaStream_t s) {
+    launch_voxelize(ManyScenes<AccumParams>{B}, ntri, unit_log2, num_sms, blocks_per_sm, s);
 }
 
 }  // namespace vct
