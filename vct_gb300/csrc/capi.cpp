@@ -260,6 +260,8 @@ void fill_accum_inputs(const vct_config& cfg, const vct_params& prm, const float
     P.vcenter = to_f3(cfg.voxel_center);
     P.ext = {cfg.voxel_max[0] - cfg.voxel_min[0], cfg.voxel_max[1] - cfg.voxel_min[1],
              cfg.voxel_max[2] - cfg.voxel_min[2]};
+    int exponent = 0;
+    P.ext_rcp = std::frexp(P.ext.x, &exponent) == 0.5f && exponent > -100 && exponent < 100 ? 1.0f / P.ext.x : 0.0f;
     P.max_tess_level = prm.max_tess_level;
     if (sh) {
         std::memcpy(P.ls, sh->ls, sizeof P.ls);

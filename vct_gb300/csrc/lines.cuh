@@ -338,11 +338,14 @@ __device__ __forceinline__ void walk_all(LineShared& S, int lines, bool big, Sin
     if (__syncthreads_or(big)) walk_triangles<true, STEPS, GRAB>(S, big ? lines : 0, sink);
 }
 
-// Grid of a kernel over `ntri` triangles: as many CTAs to each 256 of them as
-// give `want` in all, at least two, at most 64.
-inline dim3 line_grid(long long ntri, long long want) {
+// Grid of a kernel over `ntri` triangles: as many CTAs to each 256 of them (at
+// most 64) as give `want` in all, but no more than have some `share` pixels
+// each if the triangles cover `pixels`, and at least `least` where there are
+// more sets of 256 than SMs hold CTAs.
+inline dim3 line_grid(long long ntri, long long want, long long pixels, long long share, int num_sms, long long least) {
     const long long ctas = (ntri + kLineThreads - 1) / kLineThreads;
-    return dim3((unsigned)ctas, (unsigned)std::max(2LL, std::min((want + ctas - 1) / ctas, 64LL)));
+    const long long n = std::min((want + ctas - 1) / ctas, pixels / (ctas * share));
+    return dim3((unsigned)ctas, (unsigned)std::max(ctas > 4LL * num_sms ? least : 1LL, std::min(n, 64LL)));
 }
 
 }  // namespace lines

@@ -224,9 +224,11 @@ __global__ void gbuffer_resolve_kernel(const GbufferRasterParams P) {
 }  // namespace
 
 namespace {
+// Shares of about 2,048 pixels if the image is covered eight times over.
 template <class Pass>
 void launch_depth_raster(const Pass& P, cudaStream_t s) {
-    depth_raster_kernel<Pass><<<line_grid(P.ntri, P.num_sms * 24LL), kLineThreads, 0, s>>>(P, P.ntri);
+    const dim3 grid = line_grid(P.ntri, P.num_sms * 24LL, 8LL * P.w * P.h, 2048, P.num_sms, 2);
+    depth_raster_kernel<Pass><<<grid, kLineThreads, 0, s>>>(P, P.ntri);
     note_launches(1);
 }
 }  // namespace

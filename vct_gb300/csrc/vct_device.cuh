@@ -52,9 +52,10 @@ __device__ __forceinline__ f3 mul(f3 a, float s) { return {a.x * s, a.y * s, a.z
 __device__ __forceinline__ f3 mulv(f3 a, f3 b) { return {a.x * b.x, a.y * b.y, a.z * b.z}; }
 __device__ __forceinline__ float dot(f3 a, f3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 __device__ __forceinline__ f3 ld3(const float* p) { return {p[0], p[1], p[2]}; }
-// normalize(v) = v * (1 / sqrt(dot(v, v))), both operations IEEE-rounded.
+// normalize(v) = v * (1 / sqrt(dot(v, v))), both operations IEEE-rounded (the
+// rounded reciprocal is the rounded quotient of 1).
 __device__ __forceinline__ f3 normalize(f3 v) {
-    float inv = __fdiv_rn(1.0f, __fsqrt_rn(dot(v, v)));
+    float inv = __frcp_rn(__fsqrt_rn(dot(v, v)));
     return mul(v, inv);
 }
 __device__ __forceinline__ float length(f3 v) { return __fsqrt_rn(dot(v, v)); }
@@ -246,7 +247,7 @@ __device__ __forceinline__ float pcf5(const float* __restrict__ sm, int sw, int 
     return __fdiv_rn(f, 5.0f);
 }
 
-__device__ __forceinline__ uint32_t quant16(float x) { return __float2uint_rn(clampf(x, 0.0f, 1.0f) * 65535.0f); }
+__device__ __forceinline__ uint32_t quant16(float x) { return __float2uint_rn(__saturatef(x) * 65535.0f); }
 
 // ------------------------------------------------------------ scene sets
 // Kernels are templated on a scene set: OneScene keeps the parameters in

@@ -97,6 +97,7 @@ struct AccumParams {
     int blocks_per_sm;  // raster CTAs per SM (1..3)
     WarpDev warp;
     f3 vmin, vcenter, ext;  // voxelLinearPosition of the tessellation voxeliser
+    float ext_rcp;          // 1 / ext when ext (the volume is cubic) is a power of two, else 0
     float max_tess_level;   // GL_MAX_TESS_GEN_LEVEL
     // Work distribution scratch of the tessellation voxeliser (sized for ntri).
     uint4* tri_rec;          // uint4 per triangle
@@ -125,16 +126,19 @@ struct VoxWork {
     uint32_t* tri_scan;
     uint32_t* block_off;
     long long ntri;
+    int run_log2;  // log2 of the most points of an edge that one item holds
 };
+int tess_run_log2(long long ntri);
 
 constexpr int kSetupThreads = 256;  // triangles per setup block
 constexpr long long align256(long long b) { return (b + 255) & ~255LL; }
 // Scratch bytes the tessellation voxeliser needs for `ntri` triangles: a
 // 16-byte set-up record, a unit count and a scan entry per triangle, one
-// offset per block (+ the total).  The rasterising voxeliser needs none.
+// offset per block (+ the total), an 8-byte work counter.  The rasterising
+// voxeliser needs none.
 constexpr long long tess_scratch_bytes(long long ntri) {
     return align256(ntri * 16) + align256(ntri * 4) * 2 +
-           align256(((ntri + kSetupThreads - 1) / kSetupThreads + 1) * 4);
+           align256(((ntri + kSetupThreads - 1) / kSetupThreads + 2) * 4 + 8);
 }
 // Carves the scratch buffer into the AccumParams work arrays.
 void tess_bind_scratch(AccumParams& P, void* scratch);
@@ -332,8 +336,9 @@ void launch_fill_u32(uint32_t* p, uint32_t v, long long n, cudaStream_t s);
 
 // Batched frame stages: one launch covers the work of every scene.
 int accumulate_batch_max_scenes();
-void launch_accumulate_batch(const SceneBatch<AccumParams>& B, long long ntri, int unit_log2, int num_sms,
-                             int blocks_per_sm, cudaStream_t s);
+// (`faces`: the sum of the grids' dim^2)
+void launch_accumulate_batch(const SceneBatch<AccumParams>& B, long long ntri, long long faces, int unit_log2,
+                             int num_sms, int blocks_per_sm, cudaStream_t s);
 void launch_tesselate_batch(const SceneBatch<AccumParams>& B, const VoxWork& W, int num_sms, cudaStream_t s);
 void launch_inject_mark_batch(const SceneBatch<InjectParams>& B, long long ntexels, cudaStream_t s);
 void launch_resolve_batch(const SceneBatch<ResolveParams>& B, long long nbricks, bool exact, cudaStream_t s);

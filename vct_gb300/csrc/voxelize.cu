@@ -269,10 +269,12 @@ __global__ void __launch_bounds__(kLineThreads, kRasterBlocksPerSM)
 // 256^3 0.304, 0.281 and (24 not measured); past 300,000 triangles the least,
 // two to each 256, is best (519,552: 0.497 with one, 0.460 with two).
 template <class Scenes>
-void launch_voxelize(const Scenes& S, long long ntri, int unit_log2, int num_sms, int blocks_per_sm, cudaStream_t s) {
+void launch_voxelize(const Scenes& S, long long ntri, long long faces, int unit_log2, int num_sms, int blocks_per_sm,
+                     cudaStream_t s) {
     if (ntri <= 0) return;
     const int bps = blocks_per_sm < 1 ? 1 : (blocks_per_sm > kRasterBlocksPerSM ? kRasterBlocksPerSM : blocks_per_sm);
-    const dim3 grid = line_grid(ntri, (((long long)num_sms * bps * 3) << 9) >> unit_log2);
+    const dim3 grid = line_grid(ntri, (((long long)num_sms * bps * 3) << 9) >> unit_log2, 64 * faces, 1LL << (unit_log2 + 1),
+                                num_sms, 2);
     voxelize_raster_kernel<Scenes><<<grid, kLineThreads, 0, s>>>(S, ntri);
     note_launches(1);
 }
@@ -407,15 +409,36 @@ __global__ void __launch_bounds__(kOccThreads) occupancy_kernel(const Scenes S, 
 }
 
 // ====================================================== tessellation voxeliser
-// testTesselation.tesc/.tese (Application.cpp:585-662) in three launches of
-// the same shape as the rasteriser's: per-triangle tessellation levels and
-// point counts (tess_setup_kernel), the scan of the block totals, and a
-// persistent kernel in which every warp takes an equal range of 32-point
-// work units, queues the points of its units and stores 32 at a time.
+// testTesselation.tesc/.tese (Application.cpp:585-662) in three launches:
+// per-triangle tessellation levels and edge counts (tess_setup_kernel), the
+// scan of the block totals, and a persistent kernel (tess_points_kernel).
+//
+// The points of a patch fall into few voxels (on the 262,144-triangle scene, 14
+// points to each voxel that a triangle reaches), but not in the order of its
+// rings.  A lane therefore walks a sequence of points that is likely to stay in
+// one voxel (TessItem) and sums it in registers while it does; a finished run
+// goes to a queue in shared memory, and 32 queued runs are added to the records
+// together.  Integer sums: any grouping gives the same record.
+//
+// What bounds it is issue (82% of peak), some 300 instructions per 32 points:
+// half of them the exact position, a tenth each the normal, the runs' queue and
+// their additions, the rest each item's set-up.  53,248 column slivers and
+// 24,576 box triangles (181 M points, 38 M runs) in 256^3: 1.89 ms.  The form
+// before, one point per lane with neighbouring pairs merged, spent 4.85 ms on 28
+// times as many reductions; lanes that walk whole ring edges, which finish a
+// run every 1.6 points, 2.65 ms.  Triangles of ordinary shape, whose points are
+// about a voxel apart in every direction, have nothing to gain: 3,568 of them
+// take 0.095 against 0.076 ms.
 //
 // Tessellation levels after GL's equal_spacing rounding, packed 7 bits each:
-// inner n | outer[0] << 7 | outer[1] << 14 | outer[2] << 21 (1..64 each).
-constexpr int kTessUnit = 32;
+// inner n | outer[0] << 7 | outer[1] << 14 | outer[2] << 21 (1..64 each) |
+// 1 + the type of the edges that a sliver is walked along (0: none) << 28.
+constexpr int kTessUnit = 32;  // items per work unit
+constexpr int kTessBlocksPerSM = 3;
+constexpr int kTessSliver = 8; // inner level from which slivers are walked across
+constexpr int kTessGrab = 8;  // units a warp takes at a time, when there are that many
+constexpr int kTessSpread = 8192;  // places in the unit order that are worked on at a time
+constexpr int kMaxTess = VCT_MAX_TESS_LEVEL;
 
 // Block-local exclusive scan of the per-triangle unit counts of one setup
 // block into tri_scan, and the block's total into block_off[blockIdx.x].
@@ -529,59 +552,120 @@ __device__ __forceinline__ bool tess_levels(const AccumParams& P, const float* P
               m2 = tess_round(oy, P.max_tess_level);
     int n = tess_round(inner, P.max_tess_level);
     if (n == 1 && (m0 > 1 || m1 > 1 || m2 > 1)) n = 2;  // inner 1 + epsilon
-    packed = (uint32_t)n | ((uint32_t)m0 << 7) | ((uint32_t)m1 << 14) | ((uint32_t)m2 << 21);
+    // A sliver (one edge under a quarter of the other two, which the levels cut
+    // into steps of a voxel or more) is walked across, parallel to that edge:
+    // type 0 from vertex 0 to 1, type 1 from 1 to 2, type 2 from 2 to 0.
+    uint32_t across = 0;
+    if (n >= kTessSliver) {
+        if (4.0f * lz < fminf(lx, ly)) across = 1;
+        if (4.0f * lx < fminf(ly, lz)) across = 2;
+        if (4.0f * ly < fminf(lx, lz)) across = 3;
+    }
+    packed = (uint32_t)n | ((uint32_t)m0 << 7) | ((uint32_t)m1 << 14) | ((uint32_t)m2 << 21) | (across << 28);
     npts = tess_point_count(n, m0, m1, m2);
     return true;
 }
 
-// gl_TessCoord of point `i` in the order of tess_point_count.  The outer
-// edges are u = 0 (from vertex 1 to 2, outer[0]), v = 0 (2 to 0, outer[1]),
-// w = 0 (0 to 1, outer[2]), at j / m.  Ring k's corners lie where the
+// The work items of a patch.  Point (c, k, j) is j / q of the way along the
+// edge of ring k from corner c to corner c + 1 (type c).  The outer edges
+// (k = 0) are u = 0 (from vertex 1 to 2, outer[0] segments), v = 0 (2 to 0,
+// outer[1]), w = 0 (0 to 1, outer[2]); the inner rings (inner level n >= 2)
+// have q = n - 2k segments an edge, and their corners lie where the
 // perpendiculars through the inner subdivision points nearest each corner
-// meet: (1 - 2t, t, t) and rotations, t = 2k / (3n); its edges are split
-// into n - 2k equal segments.
-__device__ __forceinline__ f3 tess_coord(uint32_t packed, int i) {
-    const int n = (int)(packed & 127u), m0 = (int)((packed >> 7) & 127u), m1 = (int)((packed >> 14) & 127u),
-              m2 = (int)((packed >> 21) & 127u);
-    if (i < 3) return i == 0 ? mk(1.0f, 0.0f, 0.0f) : i == 1 ? mk(0.0f, 1.0f, 0.0f) : mk(0.0f, 0.0f, 1.0f);
-    i -= 3;
-    if (i < m0 - 1) {
-        const float s = __fdiv_rn((float)(i + 1), (float)m0);
-        return mk(0.0f, 1.0f - s, s);
-    }
-    i -= m0 - 1;
-    if (i < m1 - 1) {
-        const float s = __fdiv_rn((float)(i + 1), (float)m1);
-        return mk(s, 0.0f, 1.0f - s);
-    }
-    i -= m1 - 1;
-    if (i < m2 - 1) {
-        const float s = __fdiv_rn((float)(i + 1), (float)m2);
-        return mk(1.0f - s, s, 0.0f);
-    }
-    i -= m2 - 1;
-    int k = 1, q = n - 2;
-    while (q > 0 && i >= 3 * q) {
-        i -= 3 * q;
-        ++k;
-        q -= 2;
-    }
-    if (q <= 0) {  // the centre of an even inner level
-        const float third = __fdiv_rn(1.0f, 3.0f);
-        return mk(third, third, third);
-    }
-    const float t = __fdiv_rn((float)(2 * k), (float)(3 * n));
-    const float h = 1.0f - 2.0f * t;
-    const int e = i / q, j = i - e * q;
-    const float s = __fdiv_rn((float)j, (float)q);
-    // corners c_e and c_{e+1} of the ring: c0 = (h,t,t), c1 = (t,h,t), c2 = (t,t,h)
-    const int e1 = e == 2 ? 0 : e + 1;
-    const float a0 = e == 0 ? h : t, a1 = e == 1 ? h : t, a2 = e == 2 ? h : t;
-    const float b0 = e1 == 0 ? h : t, b1 = e1 == 1 ? h : t, b2 = e1 == 2 ? h : t;
-    return mk(a0 + s * (b0 - a0), a1 + s * (b1 - a1), a2 + s * (b2 - a2));
+// meet: (h, t, t) and rotations, t = 2k / (3n), h = 1 - 2t.  An edge's last
+// corner belongs to the next one.  An even inner level has a centre.
+//
+// An item is a sequence of points (c, k0 + dk i, j0 + dj i).  Edges are items
+// of up to 2^run_log2 points.  The edges of ring k advance by 1 / n a point,
+// whatever k, so in a sliver, where every such step of the two long types
+// crosses a voxel or more, they are not walked along but across: parallel to
+// the short type, that is (k + 3, j - 2) on the type after it and (k + 3,
+// j - 4) on the one after that.  With w = 2k + 3j (4k + 3j) those diagonals
+// are w = 2 .. 3n - 7 (4 .. 3n - 5), of up to n / 6 points; they are numbered so
+// that neighbours are about as long (one from the side where the length rises
+// by 1/6 of a point, two from the side where it falls by 1/12, or the other way
+// round).
+struct TessItem {
+    int c, k, j, dk, dj, cnt;
+};
+
+// Runs 0 .. r of the inner edges of one type: run s has K - s h rings, as far as
+// positive.
+__device__ __forceinline__ int tess_rings_before(int K, int h, int r) {
+    r = min(r + 1, (K + h - 1) / h);
+    return r * K - h * (r * (r - 1) / 2);
+}
+__device__ __forceinline__ int tess_runs(int m, int rl) { return (m + (1 << rl) - 1) >> rl; }
+
+__device__ __forceinline__ uint32_t tess_item_count(uint32_t packed, int rl) {
+    const int n = (int)(packed & 127u);
+    int c = tess_runs((int)((packed >> 7) & 127u), rl) + tess_runs((int)((packed >> 14) & 127u), rl) +
+            tess_runs((int)((packed >> 21) & 127u), rl);
+    if (n < 2) return (uint32_t)c;
+    const int rings = tess_rings_before((n - 1) / 2, 1 << (rl - 1), n >> rl);
+    return (uint32_t)(c + ((packed >> 28) ? rings + 2 * (3 * n - 8) : 3 * rings) + ((n & 1) ? 0 : 1));
 }
 
-// Record of a triangle: {packed levels, points, scene, index within its scene}.
+__device__ __forceinline__ TessItem tess_item(uint32_t packed, int i, int rl) {
+    const int n = (int)(packed & 127u), across = (int)(packed >> 28);
+    TessItem t = {0, 0, 0, 0, 1, 1};
+    // most of a sliver's items are diagonals: first, with nothing to search
+    const int diagonals = across ? 3 * n - 8 : 0;
+    if (i < 2 * diagonals) {
+        const bool second = i >= diagonals;
+        if (second) i -= diagonals;
+        const int g = i / 3, r = i - 3 * g, f = second ? 4 : 2;
+        const int w = second ? (r == 0 ? 3 * n - 5 - g : 3 + 2 * g + r) : (r == 0 ? 2 + g : 3 * n - 6 - 2 * g - r);
+        const int last = (3 * n - w - 1) >> (second ? 1 : 2);  // j < q
+        const int rest = (second ? w : 2 * w) % 3;             // w - f k a multiple of 3
+        t.c = across - 1 + (second ? 2 : 1);
+        if (t.c >= 3) t.c -= 3;
+        t.k = rest ? rest : 3;
+        t.j = (w - f * t.k) / 3;
+        t.dk = 3;
+        t.dj = -f;
+        const int kmax = min(w >> (second ? 2 : 1), last);
+        t.cnt = kmax >= t.k ? (kmax - t.k) / 3 + 1 : 0;
+        return t;
+    }
+    i -= 2 * diagonals;
+    // The inner edges, first runs first: run r has (n - 1) / 2 - r h rings (as far
+    // as positive), h = 2^(rl - 1), so the ones before it have a quadratic in r.
+    const int types = across ? 1 : 3, K = n > 1 ? (n - 1) / 2 : 0, h = 1 << (rl - 1), all = tess_rings_before(K, h, n >> rl);
+    if (i < types * all) {
+        const int ring = across ? i : i / 3;
+        const float b = (float)K + 0.5f * (float)h;
+        int r = (int)((b - sqrtf(fmaxf(b * b - 2.0f * (float)h * (float)ring, 0.0f))) / (float)h);
+        while (r > 0 && tess_rings_before(K, h, r - 1) > ring) --r;
+        while (tess_rings_before(K, h, r) <= ring) ++r;  // the runs up to r
+        t.k = 1 + ring - tess_rings_before(K, h, r - 1);
+        t.c = across ? across - 1 : i - 3 * ring;
+        t.j = r << rl;
+        t.cnt = min(n - 2 * t.k - t.j, 1 << rl);
+        return t;
+    }
+    i -= types * all;
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+        const int m = (int)((packed >> (7 + 7 * e)) & 127u), runs = tess_runs(m, rl);
+        if (i >= 0 && i < runs) {
+            t.c = e == 2 ? 0 : e + 1;
+            t.j = i << rl;
+            t.cnt = min(m - t.j, 1 << rl);
+            return t;
+        }
+        i -= runs;
+    }
+    t.k = n / 2;  // the centre: q = 0
+    return t;
+}
+
+// The points warps' shared work counter: 8 bytes after block_off[nblocks].
+__device__ __forceinline__ unsigned long long* grab_counter(const VoxWork& W, int nblocks) {
+    return reinterpret_cast<unsigned long long*>(W.block_off + (((long long)nblocks + 2) & ~1LL));
+}
+
+// Record of a triangle: {packed levels, items, scene, index within its scene}.
 template <class Scenes>
 __global__ void __launch_bounds__(kSetupThreads) tess_setup_kernel(const Scenes S, const VoxWork W) {
     const long long g = (long long)blockIdx.x * kSetupThreads + threadIdx.x;
@@ -592,109 +676,199 @@ __global__ void __launch_bounds__(kSetupThreads) tess_setup_kernel(const Scenes 
         const AccumParams& P = S.get(scene);
         uint32_t packed = 0, npts = 0;
         if (!tess_levels(P, P.pos + t * 9, packed, npts)) npts = 0;
-        W.tri_rec[g] = make_uint4(packed, npts, (uint32_t)scene, (uint32_t)t);
-        units = (npts + kTessUnit - 1) / kTessUnit;
+        const uint32_t items = npts ? tess_item_count(packed, W.run_log2) : 0u;
+        W.tri_rec[g] = make_uint4(packed, items, (uint32_t)scene, (uint32_t)t);
+        units = (items + kTessUnit - 1) / kTessUnit;
         W.tri_units[g] = units;
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *grab_counter(W, gridDim.x) = 0ull;
     block_scan_units(W, g, units);
 }
 
-struct TessQueue {
-    int tri[2 * kTessUnit];       // triangle index within its scene
-    uint32_t pt[2 * kTessUnit];   // point index within the triangle | scene << 16
-    uint32_t lev[2 * kTessUnit];  // packed levels
+// A warp's queued items, and its finished runs of points on their way to the
+// records (a ring): the four 64-bit words of each, its voxel and scene.
+struct TessStage {
+    int tri[2 * kTessUnit];        // triangle index within its scene
+    uint32_t item[2 * kTessUnit];  // item of the triangle | scene << 16
+    uint32_t lev[2 * kTessUnit];   // packed levels
+    ulonglong2 words[64][2];
+    uint32_t vox[64], scene[64];
 };
 
-// testTesselation.tese:101-133 for the queued points, one per lane (lanes
-// >= nact idle), stored with 64-bit reductions.  Summing every group of
-// lanes that hit one voxel first (__match_any_sync, __reduce_add_sync)
-// measured 2.2x slower on the large frame than plain reductions; merging
-// adjacent pairs, and setting the occupancy bit only on a voxel's first
-// store, are what pays.  Integer sums: any grouping gives the same record.
+// Adds the `n` (at most 32) oldest queued runs to their records, four lanes to
+// a record.
+//
+// Exact past 65,536 points: the old values show every crossing of 2^32 by r, g,
+// b, nx and ny (the count itself never gets near one; nz's carries land in the
+// last word's unused high half).  The add that takes the count past 65,536
+// lists the voxel even without a crossing, so that the carry pass rewrites
+// every voxel whose nz may have carried.  The voxel's occupancy bit is set by
+// the add that found its count at 0.
 template <class Scenes>
-__device__ __forceinline__ void tess_store32(const Scenes& S, const TessQueue& q, int nact, int lane) {
-    bool valid = false;
-    uint32_t v = 0, qr = 0, qg = 0, qb = 0, qx = 0, qy = 0, qz = 0;
-    const AccumParams& P = S.get(lane < nact ? (int)(q.pt[lane] >> 16) : 0);
+__device__ __forceinline__ void tess_flush(const Scenes& S, const TessStage& st, int head, int n, int lane) {
+    const int w = lane & 3;
+    unsigned long long add[4], was[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = 8 * i + (lane >> 2), e = (head + r) & 63;
+        add[i] = was[i] = 0ull;
+        if (r < n) {
+            add[i] = reinterpret_cast<const unsigned long long*>(st.words)[4 * e + w];
+            // (the record's place is found here and not where the run is queued: that is done every step)
+            const AccumParams& P = S.get((int)st.scene[e]);
+            was[i] = atomicAdd(reinterpret_cast<unsigned long long*>(P.acc + kAccWords * record_slot(st.vox[e], P.dim)) + w,
+                               add[i]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        // the sum carried out of the low field, out of the high one; the count
+        // was 0, or passes 65,536
+        const unsigned long long sum = was[i] + add[i];
+        const uint32_t c0 = (uint32_t)was[i], c1 = (uint32_t)sum;
+        const bool lo = c1 < c0, hi = sum < was[i];
+        const bool first = w == 0 && c0 == 0u && add[i] != 0ull, listed = w == 0 && c0 <= 65536u && c1 > 65536u;
+        if (w != 3 && (lo || hi || first || listed)) {
+            const int e = (head + 8 * i + (lane >> 2)) & 63;
+            const AccumParams& P = S.get((int)st.scene[e]);
+            const uint32_t v = st.vox[e];
+            if (first) atomicOr(P.occ + (v >> 5), 1u << (v & 31));
+            if (P.carry && (lo || hi || listed)) {
+                const uint32_t ev[kCarryEvents] = {w == 0 && hi, w == 1 && lo, w == 1 && hi, w == 2 && lo, w == 2 && hi};
+                carry_add(P.carry, v, ev, P.stats);
+            }
+        }
+    }
+}
+
+// The quotients of the points' places, IEEE-rounded: j / q, j < q, and 2k / (3n)
+// for the rings k < n / 2 of inner level n.
+struct TessTables {
+    float quot[kMaxTess * (kMaxTess + 1) / 2];
+    float ring[kMaxTess + 1][kMaxTess / 2];
+};
+__device__ __forceinline__ void fill_tables(TessTables& T) {
+    for (int i = threadIdx.x; i < kMaxTess * kMaxTess; i += blockDim.x) {
+        const int q = i / kMaxTess + 1, j = i % kMaxTess;
+        if (j < q) T.quot[q * (q - 1) / 2 + j] = __fdiv_rn((float)j, (float)q);
+        if (j < kMaxTess / 2) T.ring[q][j] = __fdiv_rn((float)(2 * j), (float)(3 * q));
+    }
+}
+
+// testTesselation.tese:101-133 for the queued items, one per lane (lanes >=
+// nact idle).
+template <class Scenes>
+__device__ __forceinline__ uint32_t tess_walk32(const Scenes& S, TessStage& st, const TessTables& T, int nact, int lane,
+                                                int rl, int& head, int& count) {
+    const unsigned FULL = 0xffffffffu;
+    constexpr uint32_t kNone = 0xffffffffu;
+    f3 p0 = mk(0.f, 0.f, 0.f), p1 = p0, p2 = p0, n0 = p0, n1 = p0, n2 = p0;
+    uint32_t qrg = 0, qb = 0;  // quantised albedo
+    TessItem it = {0, 0, 0, 0, 0, 0};
+    int scene = 0, at = 0, step = 0;  // the place in T.quot, what a point adds to it
+    const float* ring = T.ring[1];
+    float third = 0.0f;  // the centre's coordinates
     if (lane < nact) {
-        const long long t = q.tri[lane];
-        const f3 bc = tess_coord(q.lev[lane], (int)(q.pt[lane] & 0xffffu));
+        scene = (int)(st.item[lane] >> 16);
+        const AccumParams& P = S.get(scene);
+        const long long t = st.tri[lane];
+        const uint32_t packed = st.lev[lane];
+        it = tess_item(packed, (int)(st.item[lane] & 0xffffu), rl);
+        const int n = (int)(packed & 127u);
+        ring = T.ring[n] + it.k;
+        // (an outer edge's segments: outer[0] from corner 1, outer[1] from 2, outer[2] from 0)
+        int q = it.k ? n - 2 * it.k : (int)((packed >> (it.c == 0 ? 21 : 7 * it.c)) & 127u);
+        if (q == 0) {
+            q = 1;
+            ring = T.ring[1];
+            third = __fdiv_rn(1.0f, 3.0f);
+        }
+        at = q * (q - 1) / 2 + it.j;
+        step = it.dj - (it.dk ? 6 * q - 21 : 0);  // q falls by 6 with k + 3
         const float* Pp = P.pos + t * 9;
         const float* Pn = P.nrm + t * 9;
-        const f3 p0 = ld3(Pp), p1 = ld3(Pp + 3), p2 = ld3(Pp + 6);
-        const f3 n0 = ld3(Pn), n1 = ld3(Pn + 3), n2 = ld3(Pn + 6);
-        const f3 pos = add(add(mul(p0, bc.x), mul(p1, bc.y)), mul(p2, bc.z));
-        const f3 nrm = add(add(mul(n0, bc.x), mul(n1, bc.y)), mul(n2, bc.z));
-        const int N = P.dim;
-        const float fN = (float)N;
-        f3 tc;
-        if (P.warp.mode == VCT_WARP_PERSPECTIVE) {  // voxelTesselationWarpedPosition
-            tc = perspective_tc(P.warp, pos);
-        } else {  // voxelLinearPosition (the evaluation shader passes warpVoxels = false)
-            tc = mk(__fdiv_rn((pos.x - P.vcenter.x) - P.vmin.x, P.ext.x),
-                    __fdiv_rn((pos.y - P.vcenter.y) - P.vmin.y, P.ext.y),
-                    __fdiv_rn((pos.z - P.vcenter.z) - P.vmin.z, P.ext.z));
+        p0 = ld3(Pp), p1 = ld3(Pp + 3), p2 = ld3(Pp + 6);
+        n0 = ld3(Pn), n1 = ld3(Pn + 3), n2 = ld3(Pn + 6);
+        const f3 col = ld3(P.albedo + t * 3);
+        qrg = quant16(col.x) | (quant16(col.y) << 16);
+        qb = quant16(col.z);
+    }
+    const int cnt = it.cnt;
+    const AccumParams& P = S.get(scene);
+    const int N = P.dim;
+    const float fN = (float)N;
+    uint32_t cur = kNone, run = 0, sx = 0, sy = 0, sz = 0;
+    // Queues the finished runs of the lanes with `push`; 32 queued ones go out.
+    auto finish = [&](bool push) {
+        const unsigned m = __ballot_sync(FULL, push);
+        if (!m) return;
+        if (push) {
+            const int e = (head + count + __popc(m & ((1u << lane) - 1u))) & 63;
+            st.words[e][0] = make_ulonglong2((unsigned long long)run | ((unsigned long long)((qrg & 0xffffu) * run) << 32),
+                                             (unsigned long long)((qrg >> 16) * run) |
+                                                 ((unsigned long long)(qb * run) << 32));
+            st.words[e][1] = make_ulonglong2((unsigned long long)sx | ((unsigned long long)sy << 32), (unsigned long long)sz);
+            st.vox[e] = cur;
+            st.scene[e] = (uint32_t)scene;
         }
-        const int vx = trunc_sat(fN * tc.x), vy = trunc_sat(fN * tc.y), vz = trunc_sat(fN * tc.z);
-        if (!(vx < 0 || vy < 0 || vz < 0 || vx >= N || vy >= N || vz >= N)) {
-            valid = true;
-            v = (uint32_t)(((long long)vz * N + vy) * N + vx);
-            const f3 Nf = normalize(nrm);  // voxelStore: normalize(normal) * 0.5 + 0.5
-            const f3 col = ld3(P.albedo + t * 3);
-            qr = quant16(col.x);
-            qg = quant16(col.y);
-            qb = quant16(col.z);
-            qx = quant16(Nf.x * 0.5f + 0.5f);
-            qy = quant16(Nf.y * 0.5f + 0.5f);
-            qz = quant16(Nf.z * 0.5f + 0.5f);
+        count += __popc(m);
+        __syncwarp();
+        if (count >= 32) {
+            tess_flush(S, st, head, 32, lane);
+            head = (head + 32) & 63;
+            count -= 32;
+            __syncwarp();
+        }
+    };
+    const int steps = __reduce_max_sync(FULL, cnt);
+    for (int i = 0; i < steps; ++i) {
+        uint32_t v = kNone, qx = 0, qy = 0, qz = 0;
+        if (i < cnt) {
+            // corner c's coordinate falls from h to t, the next one's rises from t to h, the third's is t
+            const float s = T.quot[at], t = third != 0.0f ? third : *ring;
+            const float h = third != 0.0f ? third : 1.0f - 2.0f * t, d = h - t;
+            const float from = h + s * -d, to = t + s * d;
+            const f3 bc = mk(it.c == 0 ? from : it.c == 2 ? to : t, it.c == 1 ? from : it.c == 0 ? to : t,
+                             it.c == 2 ? from : it.c == 1 ? to : t);
+            at += step;
+            if (it.dk) step += 36;
+            ring += it.dk;
+            const f3 pos = add(add(mul(p0, bc.x), mul(p1, bc.y)), mul(p2, bc.z));
+            f3 tc;  // times N
+            if (P.warp.mode == VCT_WARP_PERSPECTIVE) {  // voxelTesselationWarpedPosition
+                tc = mul(perspective_tc(P.warp, pos), fN);
+            } else {  // voxelLinearPosition (the evaluation shader passes warpVoxels = false)
+                tc = sub(sub(pos, P.vcenter), P.vmin);
+                if (P.ext_rcp != 0.0f)  // the extents are a power of two, as N is: the product is the quotient's
+                    tc = mul(tc, P.ext_rcp * fN);
+                else
+                    tc = mul(mk(__fdiv_rn(tc.x, P.ext.x), __fdiv_rn(tc.y, P.ext.y), __fdiv_rn(tc.z, P.ext.z)), fN);
+            }
+            const int vx = trunc_sat(tc.x), vy = trunc_sat(tc.y), vz = trunc_sat(tc.z);
+            if ((uint32_t)(vx | vy | vz) < (uint32_t)N) {  // all in [0, N): N is a power of two
+                v = (uint32_t)((vz * N + vy) * N + vx);
+                const f3 nrm = add(add(mul(n0, bc.x), mul(n1, bc.y)), mul(n2, bc.z));
+                const f3 Nf = normalize(nrm);  // voxelStore: normalize(normal) * 0.5 + 0.5
+                qx = quant16(Nf.x * 0.5f + 0.5f);
+                qy = quant16(Nf.y * 0.5f + 0.5f);
+                qz = quant16(Nf.z * 0.5f + 0.5f);
+            }
+        }
+        const bool change = i < cnt && v != cur;
+        finish(change && run > 0);
+        if (change) {
+            cur = v;
+            run = sx = sy = sz = 0;
+        }
+        if (v != kNone) {
+            ++run;
+            sx += qx;
+            sy += qy;
+            sz += qz;
         }
     }
-    // Neighbouring points of a ring edge often share a voxel: an even lane
-    // takes its odd neighbour's sums when both hit the same voxel (one
-    // shuffle per word), so the pair costs one set of reductions.
-    const unsigned key = valid ? v : 0xffffffffu;
-    const unsigned partner = __shfl_xor_sync(0xffffffffu, key, 1);  // every lane takes part
-    const bool pair = valid && partner == key;
-    const uint32_t pr = __shfl_xor_sync(0xffffffffu, qr, 1), pg = __shfl_xor_sync(0xffffffffu, qg, 1),
-                   pb = __shfl_xor_sync(0xffffffffu, qb, 1), px = __shfl_xor_sync(0xffffffffu, qx, 1),
-                   py = __shfl_xor_sync(0xffffffffu, qy, 1), pz = __shfl_xor_sync(0xffffffffu, qz, 1);
-    if (!valid || (pair && (lane & 1))) return;
-    unsigned long long cnt = 1;
-    if (pair) {
-        cnt = 2;
-        qr += pr;
-        qg += pg;
-        qb += pb;
-        qx += px;
-        qy += py;
-        qz += pz;
-    }
-    unsigned long long* rec = reinterpret_cast<unsigned long long*>(P.acc + kAccWords * record_slot(v, P.dim));
-    const unsigned long long a0 = cnt | ((unsigned long long)qr << 32);
-    const unsigned long long a1 = (unsigned long long)qg | ((unsigned long long)qb << 32);
-    const unsigned long long a2 = (unsigned long long)qx | ((unsigned long long)qy << 32);
-    const unsigned long long was = atomicAdd(rec + 0, a0);
-    if (P.carry) {
-        // Exact past 65,536 points: the old values show every crossing of
-        // 2^32 by r, g, b, nx and ny (the count itself never gets near one;
-        // nz's carries land in the last word's unused high half).  The store
-        // that takes the count past 65,536 lists the voxel even without a
-        // crossing, so that the carry pass rewrites every voxel whose nz may
-        // have carried.
-        const unsigned long long w1 = atomicAdd(rec + 1, a1), w2 = atomicAdd(rec + 2, a2);
-        atomicAdd(rec + 3, (unsigned long long)qz);
-        const uint32_t ev[kCarryEvents] = {wrap_hi(was, a0), carry_lo(w1, a1), wrap_hi(w1, a1),
-                                           carry_lo(w2, a2), wrap_hi(w2, a2)};
-        const unsigned long long c0 = was & 0xffffffffull;
-        if ((ev[0] | ev[1] | ev[2] | ev[3] | ev[4]) || (c0 <= 65536ull && c0 + cnt > 65536ull))
-            carry_add(P.carry, v, ev, P.stats);
-    } else {
-        atomicAdd(rec + 1, a1);
-        atomicAdd(rec + 2, a2);
-        atomicAdd(rec + 3, (unsigned long long)qz);
-    }
-    // The voxel's occupancy bit, once: by the store that found its count at 0.
-    if ((was & 0xffffffffull) == 0ull) atomicOr(P.occ + (v >> 5), 1u << (v & 31));
+    finish(run > 0);
+    return (uint32_t)cnt;
 }
 
 // The carry pass: every voxel listed in a scene's carry table gets its six
@@ -726,46 +900,77 @@ __global__ void __launch_bounds__(256) carry_fixup_kernel(const Scenes S) {
     P.brick_exact[((z / 16) * bpa + y / 16) * bpa + x / 16] = 1u;
 }
 
+// Warps take units from a shared counter, whose values are
+// spread over the unit order (kTessSpread places in turn): neighbouring units,
+// which belong to neighbouring triangles and add to the same records, are then
+// not worked on at the same time.
 template <class Scenes>
-__global__ void __launch_bounds__(kWarps * 32, 4) tess_points_kernel(const Scenes S, const VoxWork W, int nblocks) {
-    __shared__ TessQueue queues[kWarps];
-    __shared__ unsigned point_count[kMaxBatchScenes];  // generated points per scene
+__global__ void __launch_bounds__(kWarps * 32, kTessBlocksPerSM) tess_points_kernel(const Scenes S, const VoxWork W, int nblocks) {
+    __shared__ TessStage stages[kWarps];
+    __shared__ TessTables tables;
+    __shared__ unsigned point_count[kMaxBatchScenes];      // generated points per scene
+    const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    TessQueue& q = queues[threadIdx.x >> 5];
+    TessStage& q = stages[threadIdx.x >> 5];
     const int nscenes = S.count();
     for (int i = threadIdx.x; i < nscenes; i += blockDim.x) point_count[i] = 0;
+    fill_tables(tables);
     __syncthreads();
-    const long long nw = (long long)gridDim.x * kWarps;
-    const long long w = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5);
     const long long total = W.block_off[nblocks];
-    const long long u0 = total * w / nw, u1 = total * (w + 1) / nw;
-    int qn = 0;                // queued points (warp-uniform)
-    int cur_scene = 0;         // generated points of the current scene, not yet counted
-    unsigned pending = 0;
-    if (u0 < u1) {
-        int lo = 0, hi = nblocks - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if ((long long)W.block_off[mid] <= u0)
-                lo = mid;
-            else
-                hi = mid - 1;
+    const int grab = (int)max(1LL, min((long long)kTessGrab, total / ((long long)gridDim.x * kWarps)));
+    const long long grabs = (total + grab - 1) / grab, stretch = (grabs + kTessSpread - 1) / kTessSpread;
+    unsigned long long* counter = grab_counter(W, nblocks);
+    int qn = 0;               // queued items (warp-uniform)
+    int head = 0, count = 0;  // the ring of finished runs (warp-uniform)
+    uint32_t points = 0;      // this lane's, of a single scene
+    auto walk = [&](int nact) {
+        const int scene = lane < nact ? (int)(q.item[lane] >> 16) : 0;
+        const uint32_t pts = tess_walk32(S, q, tables, nact, lane, W.run_log2, head, count);
+        if (nscenes > 1) {
+            if (pts) atomicAdd(&point_count[scene], pts);
+        } else {
+            points += pts;
         }
-        long long glo = (long long)lo * kSetupThreads;
-        long long ghi = min(glo + kSetupThreads, W.ntri) - 1;
-        while (glo < ghi) {
-            const long long mid = (glo + ghi + 1) >> 1;
-            if (unit_start<Scenes>(W, mid) <= u0)
-                glo = mid;
-            else
-                ghi = mid - 1;
-        }
-        long long g = glo;
-        long long start = unit_start<Scenes>(W, g);
-        uint32_t nunits = W.tri_units[g];
+    };
+    for (;;) {
+        unsigned long long gu = 0;
+        if (lane == 0) gu = atomicAdd(counter, 1ull);
+        const long long c = (long long)__shfl_sync(FULL, gu, 0);
+        if (c >= stretch * kTessSpread) break;
+        const long long u0 = ((c % kTessSpread) * stretch + c / kTessSpread) * grab, u1 = min(u0 + grab, total);
+        if (u0 >= total) continue;
+        long long g = 0, start = 0;
+        uint32_t nunits = 0;
         for (long long u = u0; u < u1; ++u) {
-            while (u >= start + nunits) {
-                ++g;
+            if (u != u0 && u >= start + nunits) {  // often the next triangle's
+                g = min(g + 1, W.ntri - 1);
+                start = unit_start<Scenes>(W, g);
+                nunits = W.tri_units[g];
+            }
+            if (u == u0 || u >= start + nunits) {
+                // Triangle owning unit u: binary search over the block offsets,
+                // then the block-local scan, 8 entries per lane: the number of
+                // entries <= u is one past the last triangle starting at or
+                // before u.
+                int lo = 0, hi = nblocks - 1;
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if ((long long)W.block_off[mid] <= u)
+                        lo = mid;
+                    else
+                        hi = mid - 1;
+                }
+                const long long gbase = (long long)lo * kSetupThreads;
+                const int in_block = (int)min((long long)kSetupThreads, W.ntri - gbase);
+                const uint32_t rel = (uint32_t)(u - W.block_off[lo]);
+                int below = 0;
+#pragma unroll
+                for (int j = 0; j < kSetupThreads / 32; ++j) {
+                    const int k = lane * (kSetupThreads / 32) + j;
+                    below += (k < in_block && __ldg(W.tri_scan + gbase + k) <= rel) ? 1 : 0;
+                }
+                below = __reduce_add_sync(FULL, below);
+                g = gbase + max(below - 1, 0);
                 start = unit_start<Scenes>(W, g);
                 nunits = W.tri_units[g];
             }
@@ -774,23 +979,17 @@ __global__ void __launch_bounds__(kWarps * 32, 4) tess_points_kernel(const Scene
             const int cnt = min(kTessUnit, (int)r.y - base);
             if (lane < cnt) {
                 q.tri[qn + lane] = (int)r.w;
-                q.pt[qn + lane] = (uint32_t)(base + lane) | (r.z << 16);
+                q.item[qn + lane] = (uint32_t)(base + lane) | (r.z << 16);
                 q.lev[qn + lane] = r.x;
             }
-            if ((int)r.z != cur_scene) {
-                if (lane == 0 && pending) atomicAdd(&point_count[cur_scene], pending);
-                cur_scene = (int)r.z;
-                pending = 0;
-            }
-            pending += (unsigned)cnt;
             __syncwarp();
             qn += cnt;
             if (qn >= kTessUnit) {
-                tess_store32(S, q, kTessUnit, lane);
+                walk(kTessUnit);
                 __syncwarp();
                 if (lane < qn - kTessUnit) {
                     q.tri[lane] = q.tri[kTessUnit + lane];
-                    q.pt[lane] = q.pt[kTessUnit + lane];
+                    q.item[lane] = q.item[kTessUnit + lane];
                     q.lev[lane] = q.lev[kTessUnit + lane];
                 }
                 __syncwarp();
@@ -798,8 +997,9 @@ __global__ void __launch_bounds__(kWarps * 32, 4) tess_points_kernel(const Scene
             }
         }
     }
-    tess_store32(S, q, qn, lane);
-    if (lane == 0 && pending) atomicAdd(&point_count[cur_scene], pending);
+    walk(qn);
+    tess_flush(S, q, head, count, lane);
+    if (points) atomicAdd(&point_count[0], points);
     __syncthreads();
     for (int i = threadIdx.x; i < nscenes; i += blockDim.x)
         if (point_count[i] && S.get(i).stats) atomicAdd(&S.get(i).stats->total_voxel_fragments, point_count[i]);
@@ -811,16 +1011,19 @@ void launch_tess(const Scenes& S, const VoxWork& W, int num_sms, cudaStream_t s)
     const int nblocks = (int)((W.ntri + kSetupThreads - 1) / kSetupThreads);
     tess_setup_kernel<Scenes><<<nblocks, kSetupThreads, 0, s>>>(S, W);
     voxelize_scan_kernel<<<1, 1024, 0, s>>>(W.block_off, nblocks);
-    tess_points_kernel<Scenes><<<num_sms * 4, kWarps * 32, 0, s>>>(S, W, nblocks);
+    tess_points_kernel<Scenes><<<num_sms * kTessBlocksPerSM, kWarps * 32, 0, s>>>(S, W, nblocks);
     note_launches(3);
 }
 
 }  // namespace
 
+// Points of an edge item: with few triangles, the fewer the more warps have any.
+int tess_run_log2(long long ntri) { return ntri < 16384 ? 2 : 3; }
+
 // The tessellation voxeliser: setup, scan, points (the same scratch as the
 // rasteriser's).
 void launch_tesselate(const AccumParams& P, cudaStream_t s) {
-    const VoxWork W = {P.tri_rec, P.tri_units, P.tri_scan, P.block_off, P.ntri};
+    const VoxWork W = {P.tri_rec, P.tri_units, P.tri_scan, P.block_off, P.ntri, tess_run_log2(P.ntri)};
     launch_tess(OneScene<AccumParams>{P}, W, P.num_sms, s);
     if (P.carry) {
         carry_fixup_kernel<<<dim3(kCarrySlots / 256, 1), 256, 0, s>>>(OneScene<AccumParams>{P});
@@ -861,14 +1064,14 @@ void launch_occupancy_batch(const SceneBatch<AccumParams>& B, long long ntri, cu
 }
 
 void launch_accumulate(const AccumParams& P, cudaStream_t s) {
-    launch_voxelize(OneScene<AccumParams>{P}, P.ntri, P.unit_log2, P.num_sms, P.blocks_per_sm, s);
+    launch_voxelize(OneScene<AccumParams>{P}, P.ntri, (long long)P.dim * P.dim, P.unit_log2, P.num_sms, P.blocks_per_sm, s);
 }
 
 int accumulate_batch_max_scenes() { return kMaxBatchScenes; }
 
-void launch_accumulate_batch(const SceneBatch<AccumParams>& B, long long ntri, int unit_log2, int num_sms,
-                             int blocks_per_sm, cudaStream_t s) {
-    launch_voxelize(ManyScenes<AccumParams>{B}, ntri, unit_log2, num_sms, blocks_per_sm, s);
+void launch_accumulate_batch(const SceneBatch<AccumParams>& B, long long ntri, long long faces, int unit_log2,
+                             int num_sms, int blocks_per_sm, cudaStream_t s) {
+    launch_voxelize(ManyScenes<AccumParams>{B}, ntri, faces, unit_log2, num_sms, blocks_per_sm, s);
 }
 
 }  // namespace vct
