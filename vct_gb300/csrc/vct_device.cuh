@@ -75,10 +75,8 @@ __device__ __forceinline__ void mat_vec(const float* m, float x, float y, float 
 __device__ __forceinline__ uint16_t f2h(float f) { return __half_as_ushort(__float2half_rn(f)); }
 __device__ __forceinline__ float h2f(uint16_t h) { return __half2float(__ushort_as_half(h)); }
 __device__ __forceinline__ uint2 pack_h4(float a, float b, float c, float d) {
-    uint2 r;
-    r.x = (uint32_t)f2h(a) | ((uint32_t)f2h(b) << 16);
-    r.y = (uint32_t)f2h(c) | ((uint32_t)f2h(d) << 16);
-    return r;
+    const __half2 lo = __floats2half2_rn(a, b), hi = __floats2half2_rn(c, d);
+    return make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
 }
 __device__ __forceinline__ float4 unpack_h4(uint2 v) {
     float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&v.x));

@@ -163,6 +163,16 @@ __device__ __forceinline__ void brick_mips(uint2* s0, uint2* s1, int nlev, uint2
     }
 }
 
+// a / b rounded to nearest, given y = RN(1 / b): the quotient a y is within a
+// unit in the last place, its remainder is exact in one fused multiply-add, and
+// the corrected quotient is the rounded one (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev.
+// 34, 1990).  For 0 <= a < 2^32 and b = 65535 c; six quotients share y.
+__device__ __forceinline__ float quotient(float a, float b, float y) {
+    const float q = a * y;
+    return fmaf(fmaf(-q, b, a), y, q);
+}
+
 // ----------------------------------------------------------- brick resolve
 // FUSED = false: transferVoxels.comp (radiance level 0 = (0,0,0,alpha)).
 // FUSED = true : additionally applies injectRadiance's stores (voxels marked
@@ -171,6 +181,13 @@ __device__ __forceinline__ void brick_mips(uint2* s0, uint2* s1, int nlev, uint2
 //                result equals normalise; inject; filter because the value
 //                injectRadiance stores into a voxel depends only on that
 //                voxel (its stores are idempotent).
+//
+// What bounds it: DRAM, at 73% of its peak (256^3 with the hybrid sampler's two
+// copies of the chain: 1.10 GB in 0.189 ms; 0.161 ms at the copy rate).  With
+// IEEE divisions it took 0.255 ms: six a voxel, and a quotient of 0, which
+// every unlit voxel has three of, goes through the division's slow path.  Four
+// CTAs per SM (64 registers) 0.199 ms, two 0.228; the texture copy written from
+// registers, a texel in each of 32 sectors an instruction, 0.192.
 //
 // EXACT = false: every brick the carry pass did not flag (all of them for
 // the rasterising voxeliser).  EXACT = true: only the flagged bricks, whose
@@ -246,12 +263,10 @@ __global__ void __launch_bounds__(kThreads, 3) resolve_kernel(const Scenes S) {
                     nrm[j] = pack_h4(__fdiv_rn(sum(rec[j][1].x), denom), __fdiv_rn(sum(rec[j][1].y), denom),
                                      __fdiv_rn(sum(rec[j][1].z), denom), 1.0f);
                 } else {
-                    col[j] = pack_h4(__fdiv_rn(__uint2float_rn(rec[j][0].y), denom),
-                                     __fdiv_rn(__uint2float_rn(rec[j][0].z), denom),
-                                     __fdiv_rn(__uint2float_rn(rec[j][0].w), denom), alpha);
-                    nrm[j] = pack_h4(__fdiv_rn(__uint2float_rn(rec[j][1].x), denom),
-                                     __fdiv_rn(__uint2float_rn(rec[j][1].y), denom),
-                                     __fdiv_rn(__uint2float_rn(rec[j][1].z), denom), 1.0f);
+                    const float y = __frcp_rn(denom);
+                    auto mean = [denom, y](uint32_t f) { return quotient(__uint2float_rn(f), denom, y); };
+                    col[j] = pack_h4(mean(rec[j][0].y), mean(rec[j][0].z), mean(rec[j][0].w), alpha);
+                    nrm[j] = pack_h4(mean(rec[j][1].x), mean(rec[j][1].y), mean(rec[j][1].z), 1.0f);
                 }
             }
             // transferVoxels.comp:53-62: radiance seed.
@@ -276,19 +291,20 @@ __global__ void __launch_bounds__(kThreads, 3) resolve_kernel(const Scenes S) {
         if (!FUSED || R.radiance_levels[0]) store4((FUSED ? R.radiance_levels[0] : P.radiance) + v0, rad);
         if (FUSED) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                s0[(lz * kBrick + ly) * kBrick + lx + j] = rad[j];
-                if (R.surf[0]) surf3Dwrite(rad[j], R.surf[0], (x + j) * (int)sizeof(uint2), y, z);
-            }
+            for (int j = 0; j < 4; ++j) s0[(lz * kBrick + ly) * kBrick + lx + j] = rad[j];
         }
     }
     if (FUSED) __syncthreads();
-    if (FUSED && R.pad_levels[0]) {
-        // The sampler's bordered copy of level 0 from the brick in shared
-        // memory: each half-warp writes one row of 16 texels (256 bytes).
-        for (int t = threadIdx.x; t < kBrickVox; t += kThreads)
-            R.pad_levels[0][pad_index(bx * kBrick + (t & 15), by * kBrick + ((t >> 4) & 15), bz * kBrick + (t >> 8), N)] =
-                unpack_h4(s0[t]);
+    if (FUSED && (R.pad_levels[0] || R.surf[0])) {
+        // The sampler's copies of level 0 from the brick in shared memory: each
+        // half-warp writes one row of 16 texels (256 bytes of the bordered
+        // copy, 128 of the texture).
+        for (int t = threadIdx.x; t < kBrickVox; t += kThreads) {
+            const int x = bx * kBrick + (t & 15), y = by * kBrick + ((t >> 4) & 15), z = bz * kBrick + (t >> 8);
+            const uint2 v = s0[t];
+            if (R.pad_levels[0]) R.pad_levels[0][pad_index(x, y, z, N)] = unpack_h4(v);
+            if (R.surf[0]) surf3Dwrite(v, R.surf[0], x * (int)sizeof(uint2), y, z);
+        }
     }
     block_stats(P.stats, uniq, mx, flags);
     if (FUSED) {
