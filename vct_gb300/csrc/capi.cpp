@@ -202,6 +202,13 @@ uint2* level_ptr(uint2* chain, const vct_ctx* ctx, int l) { return chain + ctx->
 
 f3 to_f3(const float* p) { return {p[0], p[1], p[2]}; }
 
+// 1 / x for a power of two in (2^-100, 2^100), whose products are the quotients
+// by x; else 0.
+float exact_reciprocal(float x) {
+    int exponent = 0;
+    return std::frexp(x, &exponent) == 0.5f && exponent > -100 && exponent < 100 ? 1.0f / x : 0.0f;
+}
+
 }  // namespace host
 }  // namespace vct
 
@@ -260,8 +267,7 @@ void fill_accum_inputs(const vct_config& cfg, const vct_params& prm, const float
     P.vcenter = to_f3(cfg.voxel_center);
     P.ext = {cfg.voxel_max[0] - cfg.voxel_min[0], cfg.voxel_max[1] - cfg.voxel_min[1],
              cfg.voxel_max[2] - cfg.voxel_min[2]};
-    int exponent = 0;
-    P.ext_rcp = std::frexp(P.ext.x, &exponent) == 0.5f && exponent > -100 && exponent < 100 ? 1.0f / P.ext.x : 0.0f;
+    P.ext_rcp = exact_reciprocal(P.ext.x);
     P.max_tess_level = prm.max_tess_level;
     if (sh) {
         std::memcpy(P.ls, sh->ls, sizeof P.ls);
@@ -427,6 +433,9 @@ void fill_inject(vct_ctx* ctx, const vct_shadow_desc* s, const float* eye, Injec
     P.shadowmap = s->shadowmap_dev;
     P.sw = s->width;
     P.sh = s->height;
+    P.sw_rcp = 1.0f / (float)s->width;
+    P.sh_rcp = 1.0f / (float)s->height;
+    P.ext_rcp = exact_reciprocal(ctx->cfg.voxel_max[0] - ctx->cfg.voxel_min[0]);  // the volume is cubic
     // The dispatch covers ceil(size/16)*16 invocations and the bounds test in
     // injectRadiance.comp:44 is `>`, so index == size also runs when size is
     // not a multiple of 16.
@@ -1277,6 +1286,9 @@ vct_status vct_shade(vct_ctx* c, const vct_gbuffer* g, const float eye[3], const
     P.shininess = pr.shininess;
     P.ambient_scale = pr.ambient_scale;
     P.reflect_scale = pr.reflect_scale;
+    P.tame = pr.roughness >= 0.01f && pr.roughness <= 100.0f && std::fabs(pr.metallic) <= 100.0f;
+    for (int i = 0; i < n; ++i)
+        for (int k = 0; k < 3; ++k) P.tame = P.tame && std::fabs(lights[i].color[k]) < 1e15f;
     launch_shade(P, as_stream(stream));
     VCT_CHECK_LAUNCH("shade");
     return VCT_OK;

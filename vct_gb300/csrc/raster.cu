@@ -92,7 +92,12 @@ struct ShadowPass : ShadowRasterParams {
         for (int k = 0; k < 3; ++k) {
             float c[4];
             mat_vec(ls, Pp[3 * k], Pp[3 * k + 1], Pp[3 * k + 2], 1.0f, c);
-            float nx = __fdiv_rn(c[0], c[3]), ny = __fdiv_rn(c[1], c[3]), nz = __fdiv_rn(c[2], c[3]);
+            float nx = c[0], ny = c[1], nz = c[2];
+            if (c[3] != 1.0f) {  // x / 1 = x: no division for a directional light
+                nx = __fdiv_rn(nx, c[3]);
+                ny = __fdiv_rn(ny, c[3]);
+                nz = __fdiv_rn(nz, c[3]);
+            }
             wx[k] = (nx + 1.0f) * 0.5f * (float)w;
             wy[k] = (ny + 1.0f) * 0.5f * (float)h;
             d[k] = (nz + 1.0f) * 0.5f;
@@ -180,8 +185,8 @@ __device__ __forceinline__ f3 crossf(f3 a, f3 b) {
 }
 
 __global__ void gbuffer_resolve_kernel(const GbufferRasterParams P) {
-    const long long n = (long long)P.w * P.h;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const unsigned n = (unsigned)P.w * (unsigned)P.h;  // at most 2^28
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const unsigned long long key = P.keys[i];
         if (key == ~0ull) {
             P.gpos[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -189,7 +194,7 @@ __global__ void gbuffer_resolve_kernel(const GbufferRasterParams P) {
             P.galb[i] = make_float4(0.f, 0.f, 0.f, 0.f);
             continue;
         }
-        const int px = (int)(i % P.w), py = (int)(i / P.w);
+        const int py = (int)(i / (unsigned)P.w), px = (int)(i - (unsigned)py * (unsigned)P.w);
         const long long t = (long long)(key & 0xffffffffull);
         const float* Pp = P.pos + t * 9;
         const float* Pn = P.nrm + t * 9;

@@ -21,12 +21,12 @@ struct Lighting {
 
 __device__ __forceinline__ float pow2(float x) { return x * x; }
 
-__device__ __forceinline__ Lighting cook_torrance(f3 dc, f3 lc, f3 N, f3 V, f3 L, f3 H, float r, float m) {
+// `f_lambert`: dc / kPi.
+__device__ __forceinline__ Lighting cook_torrance(f3 dc, f3 f_lambert, f3 lc, f3 N, f3 V, f3 L, f3 H, float r, float m) {
     const float n_dot_l = fmaxf(0.0f, dot(N, L));
     const float n_dot_v = fmaxf(0.0f, dot(N, V));
     const float n_dot_h = fmaxf(0.0f, dot(N, H));
     const float h_dot_v = fmaxf(0.0f, dot(H, V));
-    const f3 f_lambert = mk(dc.x / kPi, dc.y / kPi, dc.z / kPi);
     // D_ggxtr
     const float alpha2 = pow2(r);
     const float D = alpha2 / (kPi * pow2(pow2(n_dot_h) * (alpha2 - 1.0f) + 1.0f));
@@ -41,7 +41,13 @@ __device__ __forceinline__ Lighting cook_torrance(f3 dc, f3 lc, f3 N, f3 V, f3 L
     const float p5 = powf(1.0f - h_dot_v, 5.0f);
     const f3 F = mk(F0.x + (1.0f - F0.x) * p5, F0.y + (1.0f - F0.y) * p5, F0.z + (1.0f - F0.z) * p5);
     const float den = fmaxf(4.0f * n_dot_l * n_dot_v, 0.001f);
-    const f3 fct = mk(D * G * F.x / den, D * G * F.y / den, D * G * F.z / den);
+    f3 fct = mul(F, D * G);
+    if (fmaxf(fmaxf(fabsf(fct.x), fabsf(fct.y)), fabsf(fct.z)) < 1e30f && den < 1e30f) {
+        const float y = __frcp_rn(den);  // (den is at least 0.001)
+        fct = mk(quotient(fct.x, den, y), quotient(fct.y, den, y), quotient(fct.z, den, y));
+    } else {
+        fct = mk(fct.x / den, fct.y / den, fct.z / den);
+    }
     const f3 kd = mk((1.0f - F.x) * (1.0f - m), (1.0f - F.y) * (1.0f - m), (1.0f - F.z) * (1.0f - m));
     Lighting out;
     out.diffuse = mk(lc.x * n_dot_l * kd.x * f_lambert.x, lc.y * n_dot_l * kd.y * f_lambert.y,
@@ -63,7 +69,12 @@ __device__ __forceinline__ Lighting blinn_phong(f3 dc, const LightDev& Lt, f3 N,
     return out;
 }
 
-__global__ void __launch_bounds__(256) shade_kernel(const ShadeParams P) {
+// What bounds it: issue (68% of peak) and the latency of the shadow map's taps;
+// 1920x1080 with 5 lights 0.055 ms, against 0.029 ms for its 199 MB.  Before, with
+// every light in range evaluated whole, IEEE divisions (those of 0 slow) and 79
+// registers, 0.088 ms.  Six CTAs per SM (40 registers): with 78 registers 0.071,
+// four 0.0575, five 0.0577 ms.
+__global__ void __launch_bounds__(256, 6) shade_kernel(const ShadeParams P) {
     const long long n = (long long)P.width * P.height;
     for (long long pix = (long long)blockIdx.x * blockDim.x + threadIdx.x; pix < n;
          pix += (long long)gridDim.x * blockDim.x) {
@@ -79,17 +90,25 @@ __global__ void __launch_bounds__(256) shade_kernel(const ShadeParams P) {
         const f3 dc = mk(ga.x, ga.y, ga.z);
         const f3 V = normalize(sub(P.eye, Pw));
         f3 dsum = mk(0.f, 0.f, 0.f), ssum = mk(0.f, 0.f, 0.f);
+        const f3 f_lambert = mk(dc.x / kPi, dc.y / kPi, dc.z / kPi);
+        // whether a light that the surface is turned away from adds exactly 0
+        // whatever its other factors (all finite): it is then not evaluated
+        const bool tame = P.tame && fmaxf(fmaxf(fabsf(dc.x), fabsf(dc.y)), fabsf(dc.z)) < 1e15f;
         for (int i = 0; i < P.nlights; ++i) {
             const LightDev& Lt = P.lights[i];
             if (!Lt.enabled) continue;
             Lighting lg = {mk(0.f, 0.f, 0.f), mk(0.f, 0.f, 0.f)};
             if (Lt.type == 0u) {  // calculatePointLight
-                const float dist = length(sub(Lt.position, Pw));
+                const f3 d = sub(Lt.position, Pw);
+                const float d2 = dot(d, d);
+                if (d2 > Lt.beyond2) continue;  // past the range, by more than rounding
+                const float dist = __fsqrt_rn(d2);
                 if (dist > Lt.range) continue;
                 const float att = 1.0f - smoothstep(0.75f * Lt.range, Lt.range, dist);
-                const f3 L = normalize(sub(Lt.position, Pw));
+                const f3 L = normalize(d);
                 if (P.cooktorrance) {
-                    lg = cook_torrance(dc, Lt.color, N, V, L, normalize(add(V, L)), P.roughness, P.metallic);
+                    if (tame && !(dot(N, L) > 0.0f)) continue;
+                    lg = cook_torrance(dc, f_lambert, Lt.color, N, V, L, normalize(add(V, L)), P.roughness, P.metallic);
                     lg.diffuse = mul(lg.diffuse, att);
                     lg.specular = mul(lg.specular, att);
                 } else {
@@ -97,8 +116,9 @@ __global__ void __launch_bounds__(256) shade_kernel(const ShadeParams P) {
                 }
             } else if (Lt.type == 1u) {  // calculateDirectionalLight
                 const f3 L = Lt.neg_dir_n;
+                if (P.cooktorrance && tame && !(dot(N, L) > 0.0f)) continue;
                 if (P.cooktorrance)
-                    lg = cook_torrance(dc, Lt.color, N, V, L, normalize(add(V, L)), P.roughness, P.metallic);
+                    lg = cook_torrance(dc, f_lambert, Lt.color, N, V, L, normalize(add(V, L)), P.roughness, P.metallic);
                 else
                     lg = blinn_phong(dc, Lt, N, V, L, P.shininess, 1.0f);
             }

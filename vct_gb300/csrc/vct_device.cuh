@@ -52,6 +52,17 @@ __device__ __forceinline__ f3 mul(f3 a, float s) { return {a.x * s, a.y * s, a.z
 __device__ __forceinline__ f3 mulv(f3 a, f3 b) { return {a.x * b.x, a.y * b.y, a.z * b.z}; }
 __device__ __forceinline__ float dot(f3 a, f3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 __device__ __forceinline__ f3 ld3(const float* p) { return {p[0], p[1], p[2]}; }
+// a / b rounded to nearest, given y = RN(1 / b): the quotient a y is within a
+// unit in the last place, its remainder is exact in one fused multiply-add, and
+// the corrected quotient is the rounded one (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev.
+// 34, 1990), as long as nothing on the way overflows or underflows; a = 0 gives
+// 0.  Cheaper than the division where y is at hand or shared, and above all for
+// a = 0, which takes the division's slow path.
+__device__ __forceinline__ float quotient(float a, float b, float y) {
+    const float q = a * y;
+    return fmaf(fmaf(-q, b, a), y, q);
+}
 // normalize(v) = v * (1 / sqrt(dot(v, v))), both operations IEEE-rounded (the
 // rounded reciprocal is the rounded quotient of 1).
 __device__ __forceinline__ f3 normalize(f3 v) {
@@ -185,8 +196,17 @@ __device__ __forceinline__ float shadow_bilinear(const float* __restrict__ sm, i
     float fx = floorf(x), fy = floorf(y);
     float a = x - fx, b = y - fy;
     int i = (int)fx, j = (int)fy;
-    float t00 = shadow_fetch(sm, W, H, i, j), t10 = shadow_fetch(sm, W, H, i + 1, j);
-    float t01 = shadow_fetch(sm, W, H, i, j + 1), t11 = shadow_fetch(sm, W, H, i + 1, j + 1);
+    float t00, t10, t01, t11;
+    if (i >= 0 && j >= 0 && i < W - 1 && j < H - 1) {
+        const float* p = sm + (j * W + i);  // at most 2^30 texels
+        t00 = __ldg(p);
+        t10 = __ldg(p + 1);
+        t01 = __ldg(p + W);
+        t11 = __ldg(p + W + 1);
+    } else {
+        t00 = shadow_fetch(sm, W, H, i, j), t10 = shadow_fetch(sm, W, H, i + 1, j);
+        t01 = shadow_fetch(sm, W, H, i, j + 1), t11 = shadow_fetch(sm, W, H, i + 1, j + 1);
+    }
     float bot = t00 * (1.0f - a) + t10 * a;
     float top = t01 * (1.0f - a) + t11 * a;
     return bot * (1.0f - b) + top * b;
@@ -234,7 +254,7 @@ __device__ __forceinline__ float pcf5(const float* __restrict__ sm, int sw, int 
         n += frag > tap(t01, t11, d0, d1, a, bd) ? 1.0f : 0.0f;
         n += frag > tap(l0, t00, l1, t01, al, b) ? 1.0f : 0.0f;
         n += frag > tap(u0, u1, t00, t10, a, bu) ? 1.0f : 0.0f;
-        return __fdiv_rn(n, 5.0f);
+        return quotient(n, 5.0f, 0.2f);
     }
     const int ox[5] = {0, 1, 0, -1, 0};
     const int oy[5] = {0, 0, 1, 0, -1};
@@ -242,7 +262,7 @@ __device__ __forceinline__ float pcf5(const float* __restrict__ sm, int sw, int 
 #pragma unroll
     for (int s = 0; s < 5; ++s)
         if (frag > shadow_bilinear(sm, sw, sh, sx, sy, ox[s], oy[s])) f += 1.0f;
-    return __fdiv_rn(f, 5.0f);
+    return quotient(f, 5.0f, 0.2f);
 }
 
 __device__ __forceinline__ uint32_t quant16(float x) { return __float2uint_rn(__saturatef(x) * 65535.0f); }

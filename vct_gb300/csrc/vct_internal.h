@@ -202,6 +202,8 @@ struct InjectParams {
     int dim;
     const float* shadowmap;
     int sw, sh;
+    float sw_rcp, sh_rcp;  // 1 / sw, 1 / sh, rounded
+    float ext_rcp;         // 1 / (vmax - vmin) when that is a power of two, else 0
     int nx, ny;  // texel threads that pass the shader's bounds test
     float ls_inverse[16];
     f3 vmin, vmax, vcenter;
@@ -471,6 +473,7 @@ struct ShadeParams {
     int cooktorrance, enable_diffuse, enable_specular, enable_indirect, enable_reflections, draw_occlusion,
         enable_postprocess;
     float roughness, metallic, shininess, ambient_scale, reflect_scale;
+    int tame;  // roughness, metalness and lights are finite and of ordinary size
 };
 void launch_shade(const ShadeParams& P, cudaStream_t s);
 

@@ -163,16 +163,6 @@ __device__ __forceinline__ void brick_mips(uint2* s0, uint2* s1, int nlev, uint2
     }
 }
 
-// a / b rounded to nearest, given y = RN(1 / b): the quotient a y is within a
-// unit in the last place, its remainder is exact in one fused multiply-add, and
-// the corrected quotient is the rounded one (P. Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev.
-// 34, 1990).  For 0 <= a < 2^32 and b = 65535 c; six quotients share y.
-__device__ __forceinline__ float quotient(float a, float b, float y) {
-    const float q = a * y;
-    return fmaf(fmaf(-q, b, a), y, q);
-}
-
 // ----------------------------------------------------------- brick resolve
 // FUSED = false: transferVoxels.comp (radiance level 0 = (0,0,0,alpha)).
 // FUSED = true : additionally applies injectRadiance's stores (voxels marked
@@ -316,16 +306,23 @@ __global__ void __launch_bounds__(kThreads, 3) resolve_kernel(const Scenes S) {
 // injectRadiance.comp:40-56: texel -> voxel.  Returns false when the shader
 // would return early.
 __device__ __forceinline__ bool inject_voxel(const InjectParams& P, int x, int y, int& ix, int& iy, int& iz) {
-    float u = __fdiv_rn((float)x, (float)P.sw), v = __fdiv_rn((float)y, (float)P.sh);
+    float u = quotient((float)x, (float)P.sw, P.sw_rcp), v = quotient((float)y, (float)P.sh, P.sh_rcp);
     float depth = shadow_bilinear(P.shadowmap, P.sw, P.sh, u, v, 0, 0);
     float ndx = u * 2.0f - 1.0f, ndy = v * 2.0f - 1.0f, ndz = depth * 2.0f - 1.0f;
     float w[4];
     mat_vec(P.ls_inverse, ndx, ndy, ndz, 1.0f, w);
     f3 ext = sub(P.vmax, P.vmin);
     float N = (float)P.dim;
-    float tx = __fdiv_rn((w[0] - P.vcenter.x) - P.vmin.x, ext.x);
-    float ty = __fdiv_rn((w[1] - P.vcenter.y) - P.vmin.y, ext.y);
-    float tz = __fdiv_rn((w[2] - P.vcenter.z) - P.vmin.z, ext.z);
+    float tx = (w[0] - P.vcenter.x) - P.vmin.x, ty = (w[1] - P.vcenter.y) - P.vmin.y, tz = (w[2] - P.vcenter.z) - P.vmin.z;
+    if (P.ext_rcp != 0.0f) {  // the extents are a power of two: the product is the quotient
+        tx *= P.ext_rcp;
+        ty *= P.ext_rcp;
+        tz *= P.ext_rcp;
+    } else {
+        tx = __fdiv_rn(tx, ext.x);
+        ty = __fdiv_rn(ty, ext.y);
+        tz = __fdiv_rn(tz, ext.z);
+    }
     if (P.warp.mode != VCT_WARP_NONE) {  // getVoxelPosition (common.glsl:44-60)
         const f3 t = P.warp.mode == VCT_WARP_PERSPECTIVE ? perspective_tc(P.warp, mk(w[0], w[1], w[2]))
                                                          : apply_warp(P.warp, mk(tx, ty, tz));
@@ -374,7 +371,8 @@ __global__ void __launch_bounds__(kThreads) inject_mark_kernel(const Scenes S, l
     if (g >= ntexels) return;
     long long local;
     const InjectParams& P = S.get(S.find(g, local));
-    const int y = (int)(local / P.nx), x = (int)(local - (long long)y * P.nx);
+    const unsigned texel = (unsigned)local;  // at most 2^15 + 1 a side
+    const int y = (int)(texel / (unsigned)P.nx), x = (int)(texel - (unsigned)y * (unsigned)P.nx);
     int ix, iy, iz;
     if (!inject_voxel(P, x, y, ix, iy, iz)) return;
     const int N = P.dim;

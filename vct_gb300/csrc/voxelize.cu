@@ -68,8 +68,13 @@ __device__ __forceinline__ bool project_triangle(const AccumParams& P, long long
     for (int k = 0; k < 3; ++k) {
         float c[4];
         mat_vec(M, Pp[3 * k], Pp[3 * k + 1], Pp[3 * k + 2], 1.0f, c);
-        float nx = __fdiv_rn(c[0], c[3]), ny = __fdiv_rn(c[1], c[3]);
-        z[k] = __fdiv_rn(c[2], c[3]);
+        float nx = c[0], ny = c[1];
+        z[k] = c[2];
+        if (c[3] != 1.0f) {  // (x / 1 = x; the projections are orthographic)
+            nx = __fdiv_rn(nx, c[3]);
+            ny = __fdiv_rn(ny, c[3]);
+            z[k] = __fdiv_rn(z[k], c[3]);
+        }
         wx[k] = (nx + 1.0f) * 0.5f * (float)N;
         wy[k] = (ny + 1.0f) * 0.5f * (float)N;
     }
@@ -104,8 +109,8 @@ __device__ __forceinline__ bool fragment_voxel(const AccumParams& P, int px, int
             vz = iz;
         }
     } else {
-        const float fN = (float)N;
-        const float ux = __fdiv_rn((float)px + 0.5f, fN), uy = __fdiv_rn((float)py + 0.5f, fN);
+        const float fN = (float)N, rN = __frcp_rn(fN);  // N is a power of two: the products are the quotients
+        const float ux = ((float)px + 0.5f) * rN, uy = ((float)py + 0.5f) * rN;
         f3 u = axis == 0 ? mk(1.0f - uz, uy, ux) : axis == 1 ? mk(ux, 1.0f - uz, uy) : mk(ux, uy, uz);
         u.z = 1.0f - u.z;
         u = apply_warp(P.warp, u);
