@@ -960,23 +960,29 @@ vct_status vct_build_mips(vct_ctx* c, int32_t volume, void* stream) {
     if (volume == VCT_VOLUME_RADIANCE) {
         vct_status s = sync_linear(c, st);
         if (s != VCT_OK) return s;
-        launch_mips(mip_levels(c, c->radiance, c->levels), 0, st);
-        VCT_CHECK_LAUNCH("build mips");
-        if (filter_uses_texture(c->params.trace_filter)) {
-            vct_status s = refresh_texture(c, st);
-            if (s != VCT_OK) return s;
-        }
-        if (filter_uses_bordered(c->params.trace_filter)) {
-            launch_pad_copy(c->radiance, c->pchain, c->dim, c->levels, st);
+        const bool hw = filter_uses_texture(c->params.trace_filter), pad = filter_uses_bordered(c->params.trace_filter);
+        if (hw && (s = ensure_texture(c)) != VCT_OK) return s;
+        if (c->levels > 1) {  // one pass writes the levels and the sampler's copies of the whole chain
+            MipLevels M = mip_levels(c, c->radiance, c->levels);
+            for (int l = 0; l < c->levels; ++l) {
+                M.surf[l] = hw ? c->surf[l] : 0;
+                M.pad[l] = pad ? c->pchain + padded_level_offset(c->dim, l) : nullptr;
+            }
+            launch_mips(M, 0, true, st);
+            VCT_CHECK_LAUNCH("build mips");
+        } else {
+            if (hw && (s = refresh_texture(c, st)) != VCT_OK) return s;
+            if (pad) launch_pad_copy(c->radiance, c->pchain, c->dim, c->levels, st);
             VCT_CHECK_LAUNCH("bordered chain copy");
-            c->pad_ready = true;
         }
+        c->tex_ready = c->tex_ready || hw;
+        c->pad_ready = c->pad_ready || pad;
         c->mips_ready = true;
         return VCT_OK;
     }
     if (volume == VCT_VOLUME_COLOR) {
         if (c->color_levels < 2) return fail(VCT_ERR_UNSUPPORTED, "context created without VCT_CONFIG_COLOR_MIPS");
-        launch_mips(mip_levels(c, c->color, c->color_levels), 0, st);
+        launch_mips(mip_levels(c, c->color, c->color_levels), 0, false, st);
         VCT_CHECK_LAUNCH("build colour mips");
         return VCT_OK;
     }
@@ -1108,7 +1114,7 @@ vct_status frame_volume(vct_ctx* c, const vct_triangles* tris, const vct_light* 
             M.surf[l] = hw ? c->surf[l] : 0;
             M.pad[l] = pad ? c->pchain + padded_level_offset(c->dim, l) : nullptr;
         }
-        launch_mips(M, 4, st);
+        launch_mips(M, 4, false, st);
         VCT_CHECK_LAUNCH("frame: coarse mips");
     }
     c->tex_ready = hw;

@@ -244,6 +244,7 @@ struct MipLevels {
     int dim;
     int levels;
     int first;  // mip tail: the level the remaining levels are built from
+    int copy_first;  // mip_tail: write the sampler's copies of level `first` too
 };
 
 struct TraceParams {
@@ -328,7 +329,9 @@ void launch_inject(const InjectParams& P, cudaStream_t s);
 void launch_inject_mark(const InjectParams& P, cudaStream_t s);
 void launch_resolve(const ResolveParams& P, cudaStream_t s);
 // Builds levels [first+1, levels) from level `first`.
-void launch_mips(const MipLevels& M, int first, cudaStream_t s);
+// Levels first + 1 .. of a chain, with the sampler's copies (surf, pad) of each;
+// `copy`: of level `first` too.
+void launch_mips(const MipLevels& M, int first, bool copy, cudaStream_t s);
 void launch_trace(const TraceParams& P, cudaStream_t s);
 // Sampler throughput microbenchmark (vct_sampler_rate): blocks x 256 threads x iters samples.
 void launch_sampler_rate(const TraceParams& P, int filter, int blocks, int iters, float* sink, cudaStream_t s);
