@@ -41,6 +41,7 @@ size_t up256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 struct BatchTotals {
     long long tris = 0, texels = 0, bricks = 0, tiles = 0;
+    int cones = kConesPlain;  // the kind of the scenes' cone marches
     // The frame's clears, zeroed by one launch each: before the voxeliser
     // (statistics, lit masks; carry tables and brick flags of the tessellation
     // voxeliser; the occupancy masks of the warp maps) at [0, n_pre) of the blob's clear list, and after the resolve
@@ -120,6 +121,7 @@ vct_status batch_stage(vct_batch* b, const vct_scene_desc* sc, int n, char* h, B
         TraceParams T;
         if ((s = fill_trace(c, &d.gbuffer, d.eye, &d.out, T)) != VCT_OK) return s;
         apply_tuning(b->tuning, T);
+        tot.cones = i ? cone_kind_of(tot.cones, trace_kind(T)) : trace_kind(T);
         std::memcpy(h + b->off_accum + i * sizeof(AccumParams), &A, sizeof A);
         std::memcpy(h + b->off_inject + i * sizeof(InjectParams), &I, sizeof I);
         std::memcpy(h + b->off_resolve + i * sizeof(ResolveParams), &R, sizeof R);
@@ -259,7 +261,7 @@ vct_status batch_enqueue(vct_batch* b, const char* h, const BatchTotals& tot, cu
     if (timed) VCT_CUDA(cudaEventRecord(b->ev[2], st));
     launch_trace_batch(SceneBatch<TraceParams>{reinterpret_cast<const TraceParams*>(b->d_blob + b->off_trace),
                                               d_tables + 3 * (n + 1), n},
-                       b->ctx[0]->params.trace_filter, tot.tiles, st);
+                       b->ctx[0]->params.trace_filter, tot.cones, tot.tiles, st);
     VCT_CHECK_LAUNCH("batch: trace");
     if (timed) VCT_CUDA(cudaEventRecord(b->ev[3], st));
     const int filter = b->ctx[0]->params.trace_filter;

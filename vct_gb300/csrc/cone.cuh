@@ -23,21 +23,17 @@ __device__ __forceinline__ float4 texel0(const float4* __restrict__ pchain, int 
     return __ldg(pchain + (((k + 1) * Pd + (j + 1)) * Pd + (i + 1)));
 }
 
-__device__ __forceinline__ float4 lerp4(float4 p, float4 q, float t) {
-    return make_float4(fmaf(t, q.x, fmaf(-t, p.x, p.x)), fmaf(t, q.y, fmaf(-t, p.y, p.y)),
-                       fmaf(t, q.z, fmaf(-t, p.z, p.z)), fmaf(t, q.w, fmaf(-t, p.w, p.w)));
-}
-
 // RGBA as two packed fp32 pairs: Blackwell issues one FFMA2/FMUL2 per pair.
 struct rgba2 {
     float2 rg, ba;
 };
 
+__device__ __forceinline__ rgba2 from_float4(float4 v) { return {make_float2(v.x, v.y), make_float2(v.z, v.w)}; }
+
 // The bordered chain holds each binary16 texel widened to fp32 (exactly), so
 // a texel is one 16-byte read-only load with no conversion.
 __device__ __forceinline__ rgba2 ld_texel(const float4* __restrict__ p) {
-    const float4 v = __ldg(p);
-    return {make_float2(v.x, v.y), make_float2(v.z, v.w)};
+    return from_float4(__ldg(p));
 }
 
 // t*q + (p - t*p) on both pairs: two FFMA2 per pair.
@@ -48,28 +44,65 @@ __device__ __forceinline__ rgba2 lerp2(rgba2 p, rgba2 q, float t) {
 
 __device__ __forceinline__ float4 to_float4(rgba2 v) { return make_float4(v.rg.x, v.rg.y, v.ba.x, v.ba.y); }
 
+// The place of a lane in its warp's 2^wl x 2^(5-wl) pixels: eight lanes, which
+// a 16-byte load serves at a time, take a 4 x 2 block (rather than a row of
+// 8), whose footprints share more texels and lines.
+__device__ __forceinline__ int lane_x(int lane, int wl) {
+    return wl < 2 || wl > 4 ? lane & ((1 << wl) - 1) : (lane & 3) | (((lane >> 3) & ((1 << (wl - 2)) - 1)) << 2);
+}
+__device__ __forceinline__ int lane_y(int lane, int wl) {
+    return wl < 2 || wl > 4 ? lane >> wl : ((lane >> 2) & 1) | ((lane >> (wl + 1)) << 1);
+}
+
+// What a sample needs to know of a level: the side S as a float, the row and
+// slice strides of the bordered level, and the texel offset at which integers
+// taken from the float trick below index it.
+struct __align__(16) Level {
+    float side;
+    uint32_t row, slice, base;
+};
+
+// floor of a float by adding 1.5 x 2^23, rounding down: the sum's bits are the
+// integer plus kRoundBits.
+constexpr float kRound = 12582912.0f;
+constexpr uint32_t kRoundBits = 0x4B400000u;
+
+__device__ __forceinline__ Level level_of(int dim, int l) {
+    Level v;
+    v.side = (float)(dim >> l);
+    v.row = (uint32_t)(dim >> l) + 2u;
+    v.slice = v.row * v.row;
+    // (the lower corner -1 of a footprint is texel 0)
+    v.base = (uint32_t)padded_level_offset(dim, l) - (kRoundBits - 1u) * (1u + v.row + v.slice);
+    return v;
+}
+__device__ __forceinline__ void fill_levels(const TraceParams& P, Level* lv) {
+    if (threadIdx.x < VCT_MAX_LEVELS)
+        lv[threadIdx.x] = level_of(P.dim, min((int)threadIdx.x, P.levels - 1));
+}
+
 // GL_LINEAR within level l with a (0,0,0,0) border, read from the bordered
 // chain: for a position in [0,1]^3 the footprint's lower corner is in
 // [-1, S-1]^3, i.e. [0, S]^3 of the (S+2)^3 bordered level, so the eight
 // texels are plain loads at constant offsets with no bounds tests.
 //
-// With `guard` (positions warped about an eye outside the volume, or
-// projected by the perspective warp, can leave [0,1]^3) the footprint is
-// checked first: the bordered level holds texel
-// indices -1..S, i.e. u = p S - 1/2 in [-1, S); outside that every texel of
+// The floors come from additions and the texel index from the sums' bits:
+// no rounding or conversion instructions, which run at a quarter of the rate.
+//
+// With `guard` (warped positions: about an eye outside the volume, or
+// projected by the perspective warp, they can leave [0,1]^3) the footprint is
+// checked first: the bordered level holds texel indices -1..S, i.e. u = p S - 1/2 in [-1, S); outside that every texel of
 // the footprint is border and the sample is (0,0,0,0).
-__device__ __forceinline__ rgba2 trilinear2(const TraceParams& P, const int* __restrict__ off, int l, f3 p,
-                                            bool guard = false) {
-    const int S = P.dim >> l, Pd = S + 2;
-    const float4* base = P.pchain + off[l];
-    const float u = fmaf(p.x, (float)S, -0.5f), v = fmaf(p.y, (float)S, -0.5f), w = fmaf(p.z, (float)S, -0.5f);
-    if (guard && !(u >= -1.0f && v >= -1.0f && w >= -1.0f && u < (float)S && v < (float)S && w < (float)S))
+__device__ __forceinline__ rgba2 trilinear2(const float4* __restrict__ pchain, const Level lv, f3 p, bool guard = false) {
+    const float S = lv.side;
+    const float u = fmaf(p.x, S, -0.5f), v = fmaf(p.y, S, -0.5f), w = fmaf(p.z, S, -0.5f);
+    if (guard && !(u >= -1.0f && v >= -1.0f && w >= -1.0f && u < S && v < S && w < S))
         return {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-    const float fu = floorf(u), fv = floorf(v), fw = floorf(w);
-    const float a = u - fu, b = v - fv, c = w - fw;
-    const int i = (int)fu + 1, j = (int)fv + 1, k = (int)fw + 1;
-    const float4* q = base + ((k * Pd + j) * Pd + i);
-    const int sy = Pd, sz = Pd * Pd;
+    const float ru = __fadd_rd(u, kRound), rv = __fadd_rd(v, kRound), rw = __fadd_rd(w, kRound);
+    const float a = u - (ru - kRound), b = v - (rv - kRound), c = w - (rw - kRound);
+    const uint32_t at = lv.base + __float_as_uint(ru) + __float_as_uint(rv) * lv.row + __float_as_uint(rw) * lv.slice;
+    const float4* q = pchain + at;
+    const uint32_t sy = lv.row, sz = lv.slice;
     const rgba2 t0 = ld_texel(q), t1 = ld_texel(q + 1), t2 = ld_texel(q + sy), t3 = ld_texel(q + sy + 1);
     const rgba2 t4 = ld_texel(q + sz), t5 = ld_texel(q + sz + 1), t6 = ld_texel(q + sz + sy),
                 t7 = ld_texel(q + sz + sy + 1);
@@ -78,87 +111,134 @@ __device__ __forceinline__ rgba2 trilinear2(const TraceParams& P, const int* __r
     return lerp2(lerp2(x00, x10, b), lerp2(x01, x11, b), c);
 }
 
-__device__ __forceinline__ float4 trilinear(const TraceParams& P, const int* off, int l, f3 p, bool guard = false) {
-    return to_float4(trilinear2(P, off, l, p, guard));
+__device__ __forceinline__ float4 trilinear(const float4* pchain, const Level lv, f3 p, bool guard = false) {
+    return to_float4(trilinear2(pchain, lv, p, guard));
+}
+
+// The level choice of textureLod at `lambda`: level l and, with weight f, the
+// next one; magnification (lambda <= 0) and the chain's last level (lambda >=
+// its index) read one.
+struct __align__(16) Lod {
+    float h;       // the cone step's distance from the start, in voxels
+    float lambda;
+    float f;
+    int l;         // level, or one of:
+};
+constexpr int kLodNearest = -1, kLodLast = -2, kLodStop = -3;  // kLodStop: the cone has no such step
+
+__device__ __forceinline__ Lod choose_lod(float h, float lambda, int last) {
+    Lod d = {h, lambda, 0.0f, kLodNearest};
+    if (!(lambda <= 0.0f)) {
+        const float fl = floorf(lambda);
+        d.f = lambda - fl;
+        d.l = lambda >= (float)last ? kLodLast : (int)fl;
+    }
+    return d;
 }
 
 template <int MODE>
-__device__ __forceinline__ float4 sample_lod(const TraceParams& P, const int* off, f3 p, float lambda) {
-    if (MODE == VCT_FILTER_HARDWARE) return tex3DLod<float4>(P.tex, p.x, p.y, p.z, lambda);
+__device__ __forceinline__ rgba2 sample_lod(const TraceParams& P, const Level* lv, f3 p, const Lod d, bool guard) {
+    if (MODE == VCT_FILTER_HARDWARE) return from_float4(tex3DLod<float4>(P.tex, p.x, p.y, p.z, d.lambda));
     const int q = P.levels - 1;
     if (MODE == VCT_FILTER_HARDWARE_LEVELS) {
         // Texture units filter within each level; the two levels are blended
         // with the exact fp32 fraction (GL_LINEAR_MIPMAP_LINEAR level choice).
-        if (lambda <= 0.0f) return tex3DLod<float4>(P.tex, p.x, p.y, p.z, 0.0f);
-        if (lambda >= (float)q) return tex3DLod<float4>(P.tex, p.x, p.y, p.z, (float)q);
-        const float fl = floorf(lambda);
-        return lerp4(tex3DLod<float4>(P.tex, p.x, p.y, p.z, fl), tex3DLod<float4>(P.tex, p.x, p.y, p.z, fl + 1.0f),
-                     lambda - fl);
+        if (d.l == kLodNearest) return from_float4(tex3DLod<float4>(P.tex, p.x, p.y, p.z, 0.0f));
+        if (d.l == kLodLast) return from_float4(tex3DLod<float4>(P.tex, p.x, p.y, p.z, (float)q));
+        return lerp2(from_float4(tex3DLod<float4>(P.tex, p.x, p.y, p.z, (float)d.l)),
+                     from_float4(tex3DLod<float4>(P.tex, p.x, p.y, p.z, (float)(d.l + 1))), d.f);
     }
-    if (MODE == VCT_FILTER_HYBRID && lambda > 0.0f && lambda < (float)q) {
+    if (MODE == VCT_FILTER_HYBRID && d.l >= 0) {
         // The level with the larger weight exactly, the other one by the
         // texture units at its integral level: the texture units' fixed-point
         // filter weights then enter the sample scaled by at most 1/2.  (The
-        // step's level is the same in every lane, so the branch is uniform.)
-        const float fl = floorf(lambda);
-        const int d1 = (int)fl;
-        const float f = lambda - fl;
-        const bool guard = warp_leaves_volume(P.warp.mode);
-        if (f <= 0.5f) {
-            const rgba2 fine = trilinear2(P, off, d1, p, guard);
-            const float4 c = tex3DLod<float4>(P.tex, p.x, p.y, p.z, fl + 1.0f);
-            return to_float4(lerp2(fine, {make_float2(c.x, c.y), make_float2(c.z, c.w)}, f));
+        // step's level is the same in every lane, so the choice is uniform.)
+        if (d.f <= 0.5f) {
+            const rgba2 fine = trilinear2(P.pchain, lv[d.l], p, guard);
+            return lerp2(fine, from_float4(tex3DLod<float4>(P.tex, p.x, p.y, p.z, (float)(d.l + 1))), d.f);
         }
-        const float4 c = tex3DLod<float4>(P.tex, p.x, p.y, p.z, fl);
-        const rgba2 coarse = trilinear2(P, off, d1 + 1, p, guard);
-        return to_float4(lerp2({make_float2(c.x, c.y), make_float2(c.z, c.w)}, coarse, f));
+        const float4 c = tex3DLod<float4>(P.tex, p.x, p.y, p.z, (float)d.l);
+        return lerp2(from_float4(c), trilinear2(P.pchain, lv[d.l + 1], p, guard), d.f);
     }
-    if (lambda <= 0.0f) {  // magnification: GL_NEAREST on level 0 (index S = border)
+    if (d.l == kLodNearest) {  // magnification: GL_NEAREST on level 0 (index S = border)
         const int S = P.dim;
-        return texel0(P.pchain + off[0], S, (int)floorf(p.x * S), (int)floorf(p.y * S), (int)floorf(p.z * S));
+        return from_float4(texel0(P.pchain + padded_level_offset(P.dim, 0), S, (int)floorf(p.x * S),
+                                  (int)floorf(p.y * S), (int)floorf(p.z * S)));
     }
-    const bool guard = warp_leaves_volume(P.warp.mode);
-    if (lambda >= (float)q) return trilinear(P, off, q, p, guard);
-    float fl = floorf(lambda);
-    int d1 = (int)fl;
-    float f = lambda - fl;
-    if (guard) return to_float4(lerp2(trilinear2(P, off, d1, p, true), trilinear2(P, off, d1 + 1, p, true), f));
-    return to_float4(lerp2(trilinear2(P, off, d1, p), trilinear2(P, off, d1 + 1, p), f));
+    if (d.l == kLodLast) return trilinear2(P.pchain, lv[q], p, guard);
+    return lerp2(trilinear2(P.pchain, lv[d.l], p, guard), trilinear2(P.pchain, lv[d.l + 1], p, guard), d.f);
 }
 
-// `tanh` is tanf(c.cone_angle * 0.5f), which callers with many cones of one
-// setting compute once.
-template <int MODE>
-__device__ __forceinline__ float4 trace_cone(const TraceParams& P, const int* off, f3 pos, f3 n, f3 dir,
-                                             const vct_cone_settings c, float maxd, unsigned& ns, float tanh) {
+// A cone's steps do not depend on what it meets: their distances and levels
+// are the same for every cone of a setting, so a CTA computes them once (by
+// the recurrence, h += h tan(angle / 2)) and the march reads them.
+constexpr int kConeSteps = kConeTableSteps;
+struct ConeTable {
+    Lod step[kConeSteps + 1];  // the step after the last one stops
+};
+// By threads first .. first + kConeSteps of the CTA.
+__device__ __forceinline__ void fill_cone(const TraceParams& P, const vct_cone_settings& c, float maxd, ConeTable& T,
+                                          int first) {
+    const int i = (int)threadIdx.x - first;
+    if (i < 0 || i >= kConeSteps || i > c.steps) return;  // (the step after the last one stops)
+    const float scale = 1.0f / (float)P.dim, tanh = tanf(c.cone_angle * 0.5f);
+    float h = c.cone_initial_height;
+    for (int k = 0; k < i; ++k) h += h * tanh;
+    Lod d = choose_lod(h, __log2f(fmaxf(1.0f, 2.0f * (h * tanh))) + c.lod_offset, P.levels - 1);
+    if (i >= c.steps || h * scale > maxd) d.l = kLodStop;
+    T.step[i] = d;
+    if (i == 0) T.step[kConeSteps].l = kLodStop;
+}
+
+// KIND: no more steps than the table holds and no warp, the
+// same with the warp map, or any.
+template <int MODE, int KIND>
+__device__ __forceinline__ float4 trace_cone(const TraceParams& P, const Level* lv, const ConeTable& T, f3 pos, f3 n,
+                                             f3 dir, const vct_cone_settings& c, float maxd, unsigned& ns) {
     dir = fnormalize(dir);
     const float scale = 1.0f / (float)P.dim;
     const f3 start = add(pos, mul(mul(n, c.bias), scale));
-    float h = c.cone_initial_height;
-    float alpha = 0.0f;
-    f3 col = mk(0.f, 0.f, 0.f);
-    for (int i = 0; i < c.steps && alpha < 0.95f; ++i) {
-        float r = h * tanh;
-        float lod = __log2f(fmaxf(1.0f, 2.0f * r));
-        const f3 dh = mul(dir, h);
+    const bool guard = KIND == kConesAny && P.warp.mode != VCT_WARP_NONE;
+    rgba2 acc = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};  // colour, and the opacity
+    // One step: false when the cone leaves the volume.
+    auto march = [&](const Lod d) {
+        const f3 dh = mul(dir, d.h);
         const f3 sp = mk(fmaf(dh.x, scale, start.x), fmaf(dh.y, scale, start.y), fmaf(dh.z, scale, start.z));
         // any(notEqual(p, clamp(p, 0, 1))): outside, or NaN
-        if (!(sp.x >= 0.f && sp.y >= 0.f && sp.z >= 0.f && sp.x <= 1.f && sp.y <= 1.f && sp.z <= 1.f)) break;
-        if (h * scale > maxd) break;
-        float4 s = sample_lod<MODE>(P, off, P.warp.mode ? apply_warp(P.warp, sp) : sp, lod + c.lod_offset);
+        if (!(sp.x >= 0.f && sp.y >= 0.f && sp.z >= 0.f && sp.x <= 1.f && sp.y <= 1.f && sp.z <= 1.f)) return false;
+        f3 wp = sp;
+        if (KIND == kConesMapped) {
+            // saturated: a sample's footprint has to lie in the bordered level
+            wp = warp_lookup<true>(P.warp.mapf, sp);
+            wp = mk(__saturatef(wp.x), __saturatef(wp.y), __saturatef(wp.z));
+        } else if (KIND == kConesAny) {
+            wp = apply_warp(P.warp, sp);
+        }
+        const rgba2 s = sample_lod<MODE>(P, lv, wp, d, guard);
         ++ns;
-        float a = 1.0f - alpha;
-        col = mk(fmaf(s.x, a, col.x), fmaf(s.y, a, col.y), fmaf(s.z, a, col.z));
-        alpha = fmaf(a, s.w, alpha);
-        h += r;
+        const float a = 1.0f - acc.ba.y;
+        const float2 aa = make_float2(a, a);
+        acc = {__ffma2_rn(s.rg, aa, acc.rg), __ffma2_rn(s.ba, aa, acc.ba)};
+        return acc.ba.y < 0.95f;
+    };
+    bool on = true;
+    const Lod* step = T.step;
+    for (; on; ++step) {
+        const Lod d = *step;
+        if (d.l == kLodStop) break;
+        on = march(d);
     }
-    return make_float4(col.x, col.y, col.z, alpha);
-}
-
-template <int MODE>
-__device__ __forceinline__ float4 trace_cone(const TraceParams& P, const int* off, f3 pos, f3 n, f3 dir,
-                                             const vct_cone_settings c, float maxd, unsigned& ns) {
-    return trace_cone<MODE>(P, off, pos, n, dir, c, maxd, ns, tanf(c.cone_angle * 0.5f));
+    if (KIND == kConesAny && on && c.steps > kConeSteps && step == T.step + kConeSteps) {
+        // the steps past the table
+        const float tanh = tanf(c.cone_angle * 0.5f);
+        float h = T.step[kConeSteps - 1].h;
+        for (int i = kConeSteps; i < c.steps && on; ++i) {
+            h += h * tanh;
+            if (h * scale > maxd) break;
+            on = march(choose_lod(h, __log2f(fmaxf(1.0f, 2.0f * (h * tanh))) + c.lod_offset, P.levels - 1));
+        }
+    }
+    return to_float4(acc);
 }
 
 }  // namespace cone

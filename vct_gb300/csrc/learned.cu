@@ -9,6 +9,7 @@
 #include <cuda_bf16.h>
 
 #include <cmath>
+#include <type_traits>
 
 #include "cone.cuh"
 #include "umma.cuh"
@@ -123,11 +124,6 @@ __device__ __forceinline__ f3 volume_coord(const TraceParams& P, float4 gp) {
               ((gp.z - P.vcenter.z) - P.vmin.z) / ext.z);
 }
 
-__device__ __forceinline__ void level_offsets(const TraceParams& P, int* s_off) {
-    if (threadIdx.x < VCT_MAX_LEVELS)
-        s_off[threadIdx.x] = (int)threadIdx.x < P.levels ? (int)padded_level_offset(P.dim, threadIdx.x) : 0;
-}
-
 // ------------------------------------------------------- cheap trace
 // Quarter-resolution features: for each 4x4 pixel block, at its first
 // covered pixel (centre pixels first), two 90-degree cones along
@@ -141,8 +137,8 @@ __device__ __forceinline__ void level_offsets(const TraceParams& P, int* s_off) 
 __constant__ unsigned char kRepOrder[16] = {5, 10, 6, 9, 0, 1, 2, 3, 4, 7, 8, 11, 12, 13, 14, 15};
 
 __global__ void __launch_bounds__(256) learned_features_kernel(const LearnedParams P) {
-    __shared__ int s_off[VCT_MAX_LEVELS];
-    level_offsets(P.T, s_off);
+    __shared__ cone::Level s_lv[VCT_MAX_LEVELS];
+    cone::fill_levels(P.T, s_lv);
     __syncthreads();
     const int qx = blockIdx.x * 16 + (threadIdx.x & 15), qy = blockIdx.y * 16 + (threadIdx.x >> 4);
     if (qx >= P.wq || qy >= P.hq) return;
@@ -183,7 +179,7 @@ __global__ void __launch_bounds__(256) learned_features_kernel(const LearnedPara
                 if (inside) {
                     const f3 wp = T.warp.mode ? apply_warp(T.warp, sp) : sp;
                     const float4 smp =
-                        cone::trilinear(T, s_off, min(i + 1, T.levels - 1), wp, warp_leaves_volume(T.warp.mode));
+                        cone::trilinear(T.pchain, s_lv[min(i + 1, T.levels - 1)], wp, T.warp.mode != VCT_WARP_NONE);
                     const float a = 1.0f - alpha;
                     col = mk(fmaf(smp.x, a, col.x), fmaf(smp.y, a, col.y), fmaf(smp.z, a, col.z));
                     alpha = fmaf(a, smp.w, alpha);
@@ -231,8 +227,8 @@ __device__ __forceinline__ void pixel_features(const LearnedParams& P, long long
     const f3 sp = mk(fmaf(N.x, step, vp.x), fmaf(N.y, step, vp.y), fmaf(N.z, step, vp.z));
     float4 near = make_float4(0.f, 0.f, 0.f, 0.f);
     if (sp.x >= 0.f && sp.y >= 0.f && sp.z >= 0.f && sp.x <= 1.f && sp.y <= 1.f && sp.z <= 1.f) {
-        const int off[2] = {(int)padded_level_offset(T.dim, 0), (int)padded_level_offset(T.dim, 1)};
-        near = cone::trilinear(T, off, 1, T.warp.mode ? apply_warp(T.warp, sp) : sp, warp_leaves_volume(T.warp.mode));
+        near = cone::trilinear(T.pchain, cone::level_of(T.dim, 1), T.warp.mode ? apply_warp(T.warp, sp) : sp,
+                               T.warp.mode != VCT_WARP_NONE);
     }
     f[16] = bf16x2(N.x, N.y);
     f[17] = bf16x2(N.z, dist * P.depth_scale);
@@ -262,8 +258,9 @@ __global__ void __launch_bounds__(256) learned_rows_kernel(const LearnedParams P
 // ------------------------------------------------------- 16-cone trace
 // Irradiance of the 16-cone reference set: cones of the Fibonacci hemisphere
 // set in the (T, B, N) frame, each weighted by its cosine, summed.
-__device__ __forceinline__ float4 irradiance16(const LearnedParams& P, const int* off, const float (*dirs)[4],
-                                               float4 gp, float4 gn, unsigned& ns) {
+template <int KIND>
+__device__ __forceinline__ float4 irradiance16(const LearnedParams& P, const cone::Level* lv, const cone::ConeTable& tab,
+                                               const float (*dirs)[4], float4 gp, float4 gn, unsigned& ns) {
     const TraceParams& T = P.T;
     const f3 N = cone::fnormalize(mk(gn.x, gn.y, gn.z));
     f3 Tg, Bg;
@@ -273,7 +270,7 @@ __device__ __forceinline__ float4 irradiance16(const LearnedParams& P, const int
 #pragma unroll 1
     for (int c = 0; c < 16; ++c) {
         const f3 d = add(add(mul(Tg, dirs[c][0]), mul(Bg, dirs[c][1])), mul(N, dirs[c][2]));
-        const float4 cr = cone::trace_cone<VCT_FILTER_SOFTWARE>(T, off, vp, N, d, P.ref_cone, T.max_distance, ns);
+        const float4 cr = cone::trace_cone<VCT_FILTER_SOFTWARE, KIND>(T, lv, tab, vp, N, d, P.ref_cone, T.max_distance, ns);
         const float w = dirs[c][3];
         acc = make_float4(fmaf(w, cr.x, acc.x), fmaf(w, cr.y, acc.y), fmaf(w, cr.z, acc.z), fmaf(w, cr.w, acc.w));
     }
@@ -285,10 +282,13 @@ __device__ __forceinline__ void load_dirs(const LearnedParams& P, float (*s_dirs
 }
 
 // 16-cone irradiance of whole 16x16 tiles (every tile, or the listed ones).
-__global__ void __launch_bounds__(256) trace16_kernel(const LearnedParams P, int listed) {
-    __shared__ int s_off[VCT_MAX_LEVELS];
+template <int KIND>
+__global__ void __launch_bounds__(256, 4) trace16_kernel(const LearnedParams P, int listed) {
+    __shared__ cone::Level s_lv[VCT_MAX_LEVELS];
+    __shared__ cone::ConeTable s_cone;
     __shared__ float s_dirs[16][4];
-    level_offsets(P.T, s_off);
+    cone::fill_levels(P.T, s_lv);
+    cone::fill_cone(P.T, P.ref_cone, P.T.max_distance, s_cone, 64);
     load_dirs(P, s_dirs);
     __syncthreads();
     const TraceParams& T = P.T;
@@ -298,13 +298,13 @@ __global__ void __launch_bounds__(256) trace16_kernel(const LearnedParams P, int
     unsigned ns = 0;
     for (long long t = blockIdx.x; t < total; t += gridDim.x) {
         const long long tile = listed ? (long long)P.list[t] : t;
-        const int x = (int)(tile % tiles_x) * kLearnTile + (wid & 1) * 8 + (lane & 7);
-        const int y = (int)(tile / tiles_x) * kLearnTile + (wid >> 1) * 4 + (lane >> 3);
+        const int x = (int)(tile % tiles_x) * kLearnTile + (wid & 1) * 8 + cone::lane_x(lane, 3);
+        const int y = (int)(tile / tiles_x) * kLearnTile + (wid >> 1) * 4 + cone::lane_y(lane, 3);
         if (x >= T.width || y >= T.height) continue;
         const long long pix = (long long)y * T.width + x;
         const float4 gp = __ldg(T.gpos + pix);
         float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (gp.w != 0.0f) r = irradiance16(P, s_off, s_dirs, gp, __ldg(T.gnrm + pix), ns);
+        if (gp.w != 0.0f) r = irradiance16<KIND>(P, s_lv, s_cone, s_dirs, gp, __ldg(T.gnrm + pix), ns);
         P.out[pix] = make_float4(r.x, r.y, r.z, 0.0f);
     }
 }
@@ -318,8 +318,8 @@ __global__ void __launch_bounds__(256) trace16_kernel(const LearnedParams P, int
 __global__ void __launch_bounds__(256) learned_flag_kernel(const LearnedParams P) {
     const int W = P.T.width, H = P.T.height, tiles_x = (W + 15) / 16;
     const int tile = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int x = (tile % tiles_x) * 16 + (warp & 1) * 8 + (lane & 7);
-    const int y = (tile / tiles_x) * 16 + (warp >> 1) * 4 + (lane >> 3);
+    const int x = (tile % tiles_x) * 16 + (warp & 1) * 8 + cone::lane_x(lane, 3);
+    const int y = (tile / tiles_x) * 16 + (warp >> 1) * 4 + cone::lane_y(lane, 3);
     const long long i = (long long)y * W + x;
     const float n = P.frame_sums[1];
     const float bound = P.threshold * sqrtf(n > 0.0f ? P.frame_sums[0] / n : 0.0f);
@@ -344,18 +344,21 @@ __global__ void __launch_bounds__(256) learned_flag_kernel(const LearnedParams P
 // 16-cone irradiance of the listed pixels (the per-pixel fallback), one
 // thread per list entry; the grid covers the longest possible list and
 // threads past the list's length return at once.
+template <int KIND>
 __global__ void __launch_bounds__(256, 4) trace16_pixels_kernel(const LearnedParams P) {
-    __shared__ int s_off[VCT_MAX_LEVELS];
+    __shared__ cone::Level s_lv[VCT_MAX_LEVELS];
+    __shared__ cone::ConeTable s_cone;
     __shared__ float s_dirs[16][4];
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if ((long long)blockIdx.x * blockDim.x >= (long long)*P.count) return;  // the whole CTA is past the list
-    level_offsets(P.T, s_off);
+    cone::fill_levels(P.T, s_lv);
+    cone::fill_cone(P.T, P.ref_cone, P.T.max_distance, s_cone, 64);
     load_dirs(P, s_dirs);
     __syncthreads();
     if (i >= (long long)*P.count) return;
     const long long pix = (long long)P.list[i];
     unsigned ns = 0;
-    const float4 r = irradiance16(P, s_off, s_dirs, __ldg(P.T.gpos + pix), __ldg(P.T.gnrm + pix), ns);
+    const float4 r = irradiance16<KIND>(P, s_lv, s_cone, s_dirs, __ldg(P.T.gpos + pix), __ldg(P.T.gnrm + pix), ns);
     P.out[pix] = make_float4(r.x, r.y, r.z, 0.0f);
 }
 
@@ -366,11 +369,14 @@ __global__ void __launch_bounds__(256, 4) trace16_pixels_kernel(const LearnedPar
 // a warp holds two probes' 16 cones, two warps a tile.
 constexpr int kProbeThreads = 256;  // 4 tiles per CTA
 
+template <int KIND>
 __global__ void __launch_bounds__(kProbeThreads) learned_probe_kernel(const LearnedParams P) {
-    __shared__ int s_off[VCT_MAX_LEVELS];
+    __shared__ cone::Level s_lv[VCT_MAX_LEVELS];
+    __shared__ cone::ConeTable s_cone;
     __shared__ float s_dirs[16][4];
     __shared__ float s_part[kProbeThreads / 32][2];
-    level_offsets(P.T, s_off);
+    cone::fill_levels(P.T, s_lv);
+    cone::fill_cone(P.T, P.ref_cone, P.T.max_distance, s_cone, 64);
     load_dirs(P, s_dirs);
     __syncthreads();
     const TraceParams& T = P.T;
@@ -395,7 +401,7 @@ __global__ void __launch_bounds__(kProbeThreads) learned_probe_kernel(const Lear
                 onb(N, Tg, Bg);
                 const f3 vp = volume_coord(T, gp);
                 const f3 d = add(add(mul(Tg, s_dirs[c][0]), mul(Bg, s_dirs[c][1])), mul(N, s_dirs[c][2]));
-                const float4 cr = cone::trace_cone<VCT_FILTER_SOFTWARE>(T, s_off, vp, N, d, P.ref_cone, T.max_distance, ns);
+                const float4 cr = cone::trace_cone<VCT_FILTER_SOFTWARE, KIND>(T, s_lv, s_cone, vp, N, d, P.ref_cone, T.max_distance, ns);
                 const float w = s_dirs[c][3];
                 rc = make_float4(w * cr.x, w * cr.y, w * cr.z, 0.0f);
             }
@@ -1000,10 +1006,23 @@ void launch_mlp_infer(const LearnedParams& P, int num_sms, cudaStream_t s) {
     note_launches(1);
 }
 
+// f(integral constant) with the kind of the 16 cones' march.
+template <class F>
+static void with_kind(const LearnedParams& P, F f) {
+    const int kind = cone_kind(P.T.warp, P.ref_cone.steps);
+    if (kind == kConesPlain)
+        f(std::integral_constant<int, kConesPlain>());
+    else if (kind == kConesMapped)
+        f(std::integral_constant<int, kConesMapped>());
+    else
+        f(std::integral_constant<int, kConesAny>());
+}
+
 void launch_learned_probe(const LearnedParams& P, cudaStream_t s) {
     const long long tiles = (long long)((P.T.width + kLearnTile - 1) / kLearnTile) *
                             ((P.T.height + kLearnTile - 1) / kLearnTile);
-    learned_probe_kernel<<<(unsigned)((tiles + kProbeThreads / 64 - 1) / (kProbeThreads / 64)), kProbeThreads, 0, s>>>(P);
+    const unsigned grid = (unsigned)((tiles + kProbeThreads / 64 - 1) / (kProbeThreads / 64));
+    with_kind(P, [&](auto kind) { learned_probe_kernel<kind.value><<<grid, kProbeThreads, 0, s>>>(P); });
     note_launches(1);
 }
 
@@ -1012,8 +1031,10 @@ void launch_trace16(const LearnedParams& P, bool listed, int num_sms, cudaStream
                             ((P.T.height + kLearnTile - 1) / kLearnTile);
     // Persistent over the listed tiles: as many CTAs as fit (8 per SM).
     const long long cap = (long long)num_sms * 8;
-    const long long grid = listed ? cap : (tiles < cap * 4 ? tiles : cap * 4);
-    trace16_kernel<<<(unsigned)(grid > 0 ? grid : 1), 256, 0, s>>>(P, listed ? 1 : 0);
+    const long long grid = listed ? cap : tiles;
+    with_kind(P, [&](auto kind) {
+        trace16_kernel<kind.value><<<(unsigned)(grid > 0 ? grid : 1), 256, 0, s>>>(P, listed ? 1 : 0);
+    });
     note_launches(1);
 }
 
@@ -1021,7 +1042,7 @@ void launch_trace16_pixels(const LearnedParams& P, cudaStream_t s) {
     const long long n = (long long)P.T.width * P.T.height;
     const long long tiles = (long long)((P.T.width + 15) / 16) * ((P.T.height + 15) / 16);  // one CTA each
     learned_flag_kernel<<<(unsigned)tiles, 256, 0, s>>>(P);
-    trace16_pixels_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P);
+    with_kind(P, [&](auto kind) { trace16_pixels_kernel<kind.value><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P); });
     note_launches(2);
 }
 

@@ -356,7 +356,20 @@ struct ClearRange {
 // Zeroes n ranges (a device array) in one launch; max_words sizes the grid.
 void launch_clear_ranges(const ClearRange* ranges, int n, long long max_words, cudaStream_t s);
 long long trace_tiles(int width, int height, int tile_w_log2, int tile_h_log2);
-void launch_trace_batch(const SceneBatch<TraceParams>& B, int filter, long long tiles, cudaStream_t s);
+// What the march of a scene's cones has to provide for (a kernel for each):
+// no more steps than the marcher's table holds and no warp, the same with the
+// warp map, or any warp and any number of steps.  The general march checks
+// every footprint and holds the march's body twice.
+enum { kConesPlain = 0, kConesMapped = 1, kConesAny = 2 };
+constexpr int kConeTableSteps = 64;
+inline int cone_kind(const WarpDev& W, int steps) {
+    if (steps > kConeTableSteps) return kConesAny;
+    return W.mode == VCT_WARP_NONE ? kConesPlain : W.mode == VCT_WARP_TEXTURE ? kConesMapped : kConesAny;
+}
+// (of several scenes)
+inline int cone_kind_of(int a, int b) { return a == b ? a : kConesAny; }
+int trace_kind(const TraceParams& P);
+void launch_trace_batch(const SceneBatch<TraceParams>& B, int filter, int kind, long long tiles, cudaStream_t s);
 void launch_trace_views(const ViewSet& V, int filter, cudaStream_t s);
 // ------------------------------------------------------------- learned path
 // MLP 42-64-64-64-4: irradiance RGB and the network's estimate of its own

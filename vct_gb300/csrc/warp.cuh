@@ -47,15 +47,31 @@ constexpr int kWarpPad = kWarpDim + 2;
 // lerped along x, then y, then z.  The footprint's lower corner is clamped to
 // the border, so the eight loads are constant offsets from one address and
 // read the texels the clamped indices would; x and y are interpolated as
-// packed fp32 pairs (each element rounds as the scalar product and sum do).
+// packed fp32 pairs (whose products and sums the compiler fuses).
+//
+// INSIDE: p is in [0,1]^3, so the footprint needs no clamp, and its floors
+// come from additions of 1.5 x 2^23 rounded down, whose bits are the integers
+// plus 0x4B400000 (no rounding and conversion instructions).
+template <bool INSIDE = false>
 __device__ __forceinline__ f3 warp_lookup(const float4* __restrict__ mapf, f3 p) {
     const float u = p.x * (float)kWarpDim - 0.5f, v = p.y * (float)kWarpDim - 0.5f, w = p.z * (float)kWarpDim - 0.5f;
-    const float fu = floorf(u), fv = floorf(v), fw = floorf(w);
-    const float a = u - fu, b = v - fv, c = w - fw;
-    const int i = min(max((int)fu + 1, 0), kWarpDim), j = min(max((int)fv + 1, 0), kWarpDim),
-              k = min(max((int)fw + 1, 0), kWarpDim);
-    const float4* q = mapf + ((k * kWarpPad + j) * kWarpPad + i);
     constexpr int sy = kWarpPad, sz = kWarpPad * kWarpPad;
+    float fu, fv, fw;
+    uint32_t at;
+    if (INSIDE) {
+        constexpr float big = 12582912.0f;
+        const float ru = __fadd_rd(u, big), rv = __fadd_rd(v, big), rw = __fadd_rd(w, big);
+        fu = ru - big, fv = rv - big, fw = rw - big;
+        at = __float_as_uint(rw) * sz + __float_as_uint(rv) * sy + __float_as_uint(ru) -
+             (0x4B400000u - 1u) * (uint32_t)(sz + sy + 1);
+    } else {
+        fu = floorf(u), fv = floorf(v), fw = floorf(w);
+        const int i = min(max((int)fu + 1, 0), kWarpDim), j = min(max((int)fv + 1, 0), kWarpDim),
+                  k = min(max((int)fw + 1, 0), kWarpDim);
+        at = (uint32_t)((k * kWarpPad + j) * kWarpPad + i);
+    }
+    const float a = u - fu, b = v - fv, c = w - fw;
+    const float4* q = mapf + at;
     const float4 t0 = __ldg(q), t1 = __ldg(q + 1), t2 = __ldg(q + sy), t3 = __ldg(q + sy + 1);
     const float4 t4 = __ldg(q + sz), t5 = __ldg(q + sz + 1), t6 = __ldg(q + sz + sy), t7 = __ldg(q + sz + sy + 1);
     // p * (1 - s) + q * s on the (x, y) pair and on z
@@ -103,11 +119,6 @@ __device__ __forceinline__ f3 perspective_from_tc(const WarpDev& W, f3 t) {
     w.y = (t.y * W.ext.y + W.vcenter.y) + W.vmin.y;
     w.z = (t.z * W.ext.z + W.vcenter.z) + W.vmin.z;
     return perspective_tc(W, w);
-}
-
-// Warps that can move a position off [0,1]^3 (the samplers check the footprint).
-__device__ __forceinline__ bool warp_leaves_volume(int mode) {
-    return mode == VCT_WARP_ANALYTIC || mode == VCT_WARP_PERSPECTIVE;
 }
 
 __device__ __forceinline__ f3 apply_warp(const WarpDev& W, f3 p) {
