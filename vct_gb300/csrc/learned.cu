@@ -107,6 +107,15 @@ __device__ __forceinline__ void tc_sync() {
     fence_after_sync();
 }
 
+// Programmatic dependent launch: a kernel launched with launch_overlapped may
+// start once every CTA of the kernel before it has called
+// grid_launch_dependents (or ended), and waits in grid_wait for that kernel's
+// end before it touches anything that other kernels read or write.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Orthonormal basis (T, B) around unit N: Duff et al. 2017, "Building an
 // Orthonormal Basis, Revisited" (JCGT 6(1)), as the cone tracer uses it.
 __device__ __forceinline__ void onb(f3 N, f3& T, f3& B) {
@@ -457,7 +466,7 @@ constexpr int kInferGroups = 2;
 constexpr int kInferTiles = 2;
 constexpr int kInferThreads = 128 * kInferGroups;
 constexpr int kInferTile = 128 * kMlpHidden * 2;
-constexpr int kInferSmem = kImgFwd + kInferGroups * kInferTiles * kInferTile;
+constexpr int kInferSmem = kImgAll + kInferGroups * kInferTiles * kInferTile;
 constexpr int kInferCols = 64 * kInferTiles * kInferGroups;  // TMEM columns per CTA
 constexpr int kInferBlocksPerSM = 2;                        // 2 x 88 KB of shared memory, 2 x 256 TMEM columns
 
@@ -489,7 +498,7 @@ __global__ void __launch_bounds__(kInferThreads, kInferBlocksPerSM) mlp_infer_ke
     __shared__ uint32_t s_tmem;
     __shared__ int s_done[kInferGroups];
     const int tid = threadIdx.x, warp = tid >> 5, grp = warp >> 2, row = tid & 127;
-    for (int i = tid; i < kImgFwd / 16; i += kInferThreads)
+    for (int i = tid; i < kImgAll / 16; i += kInferThreads)
         reinterpret_cast<uint4*>(smem)[i] = __ldg(reinterpret_cast<const uint4*>(P.img) + i);
     for (int i = tid; i < kBiasPad; i += kInferThreads) s_bias[i] = P.bias[i];
     if (tid < kInferGroups) mbar_init(smem_u32(&mbar[tid]), 1);
@@ -505,7 +514,7 @@ __global__ void __launch_bounds__(kInferThreads, kInferBlocksPerSM) mlp_infer_ke
     uint32_t tm[kInferTiles], a0[kInferTiles];
 #pragma unroll
     for (int k = 0; k < kInferTiles; ++k) {
-        sa[k] = smem + kImgFwd + (grp * kInferTiles + k) * kInferTile;
+        sa[k] = smem + kImgAll + (grp * kInferTiles + k) * kInferTile;
         a0[k] = smem_u32(sa[k]);
         tm[k] = s_tmem + 64u * (uint32_t)(grp * kInferTiles + k);
     }
@@ -639,60 +648,66 @@ __global__ void __launch_bounds__(kInferThreads, kInferBlocksPerSM) mlp_infer_ke
 }
 
 // ------------------------------------------------------- MLP training
-// One CTA per SM (210 KB of shared memory, all 512 TMEM columns), 128
-// samples per tile.  Forward as in inference, keeping each hidden layer's
-// ReLU mask in registers and its BF16 activations transposed (features x
-// samples) for the weight gradients.  Backward, per layer l:
+// A CTA of eight warps takes tiles of 128 samples: a thread a sample (a TMEM
+// lane) and half of a layer's columns.  Forward as in inference, keeping each
+// hidden layer's ReLU mask in registers and its BF16 activations in shared
+// memory.  Backward, per layer l:
 //   dZ_l = (dZ_{l+1} W_{l+1}) * mask_l           (MMA into the 64 scratch columns)
 //   dW_l^T += H_{l-1}^T dZ_l                     (MMA, accumulated in TMEM over the CTA's tiles)
-// The transposed activation tiles are padded to 128 rows (M = 128) with one
-// row of ones below the features, so the same MMA also accumulates the bias
-// gradient.  At the end each CTA adds its TMEM gradients to the global fp32
-// gradient with fire-and-forget atomics.  Loss: mean squared error over the
+// Every operand is stored once, samples x features, and the weight-gradient
+// MMAs read H and dZ transposed (as the backward ones read W).  A column of
+// ones after an activation tile's features makes the same MMA accumulate the
+// bias gradient; M = 128 rows also reads what follows the tile, into rows of
+// the accumulator that nothing uses.  A layer's weight gradient is issued
+// after the MMAs that the next layer waits for and runs beside its epilogue.
+// At the end each CTA stores its TMEM gradients as its part, which the update
+// kernel sums.
+//
+// What bounds it: the chain of eight MMAs, waits and epilogues that a tile is,
+// and the launch.  A step of 16,384 rows takes 15 us with its update (a tile to
+// a CTA; 10 us of them this kernel).  With 128 threads a CTA, transposed copies
+// of every operand stored in 2-byte pieces over zeroed tiles, and atomics from
+// 128 CTAs into one gradient (6 us of contention) it took 30 us, and 45 with the
+// two memsets, the update and a copy of the loss.
+// Loss: mean squared error over the
 // n x 3 irradiance outputs, plus kMlpConfidenceWeight times the mean over the
 // n samples of (e - |y - t|)^2, where e is the fourth output (the error
 // estimate) and |y - t| the Euclidean error of the sample's irradiance, held
 // constant (no gradient flows from this term into the irradiance outputs).
-constexpr int kTrW = 0;
-constexpr int kTrA = kImgAll;                      // 128 x 64 A operand
-constexpr int kTrT = kTrA + 128 * 64 * 2;          // 4 transposed activation tiles, 128 x 128 each
-constexpr int kTrTile = 128 * 128 * 2;
-constexpr int kTrDZT = kTrT + 4 * kTrTile;         // 64 x 128
-constexpr int kTrDYT = kTrDZT + 64 * 128 * 2;      // 16 x 128
-constexpr int kTrDY = kTrDYT + 16 * 128 * 2;       // 128 x 16
+constexpr int kTrThreads = 256;
+constexpr int kTrX = kImgAll;                      // input tile: 48 features, the ones' chunk
+constexpr int kTrH = kTrX + 7 * 128 * 16;          // three activation tiles: 64 features, the ones' chunk
+constexpr int kTrHTile = 9 * 128 * 16;
+constexpr int kTrDZ = kTrH + 3 * kTrHTile;         // three dZ tiles, 128 x 64
+constexpr int kTrDZTile = 128 * 64 * 2;
+constexpr int kTrDY = kTrDZ + 3 * kTrDZTile;       // 128 x 16
 constexpr int kTrSmem = kTrDY + 128 * 16 * 2;
 static_assert(kTrSmem <= 227 * 1024 - 2048, "training tiles exceed shared memory");
+// an M = 128 operand at the last activation tile reads 16 chunks
+static_assert(kTrH + 2 * kTrHTile + 16 * 128 * 16 <= kTrSmem, "transposed operand exceeds shared memory");
 // TMEM columns: scratch, dW1^T, dW2^T, dW3^T, dW4^T.
 constexpr uint32_t kColFb = 0, kColW1 = 64, kColW2 = 128, kColW3 = 192, kColW4 = 256;
-constexpr uint16_t kBf16One = 0x3F80u;
+constexpr uint32_t kBf16One = 0x3F80u;
 
-// Element (row, col) of an R-row operand tile.
-__device__ __forceinline__ void st_t(uint8_t* base, int row, int col, uint16_t v, int R = 128) {
-    *reinterpret_cast<uint16_t*>(base + tile_offset(row, col, R)) = v;
-}
-
-__global__ void __launch_bounds__(128, 1) mlp_train_kernel(const TrainParams P) {
+__global__ void __launch_bounds__(kTrThreads, 1) mlp_train_kernel(const TrainParams P) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ float s_bias[kBiasPad];
+    __shared__ __align__(16) float s_bias[kBiasPad];
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t s_tmem;
     __shared__ float s_loss[4], s_closs[4];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int i = tid; i < kImgAll / 16; i += 128)
-        reinterpret_cast<uint4*>(smem + kTrW)[i] = __ldg(reinterpret_cast<const uint4*>(P.mlp.img) + i);
-    for (int i = tid; i < kBiasPad; i += 128) s_bias[i] = P.mlp.bias[i];
-    for (int i = tid; i < (kTrSmem - kTrT) / 16; i += 128)
-        reinterpret_cast<uint4*>(smem + kTrT)[i] = make_uint4(0u, 0u, 0u, 0u);
-    __syncthreads();
-    uint8_t* sa = smem + kTrA;
-    uint8_t* T0 = smem + kTrT;
-    uint8_t* Th[3] = {smem + kTrT + kTrTile, smem + kTrT + 2 * kTrTile, smem + kTrT + 3 * kTrTile};
-    uint8_t* dzt = smem + kTrDZT;
-    uint8_t* dyt = smem + kTrDYT;
-    uint8_t* dy = smem + kTrDY;
-    // rows of ones: bias gradients
-    st_t(T0, kMlpInPad, tid, kBf16One);
-    for (int l = 0; l < 3; ++l) st_t(Th[l], kMlpHidden, tid, kBf16One);
+    const int row = tid & 127, half = tid >> 7;
+    uint8_t* const xt = smem + kTrX;
+    uint8_t* const dy = smem + kTrDY;
+    // columns of ones: bias gradients
+    const uint4 ones = make_uint4(kBf16One, 0u, 0u, 0u);
+    if (half == 0) {
+        *reinterpret_cast<uint4*>(xt + tile_offset(row, kMlpInPad, 128)) = ones;
+        *reinterpret_cast<uint4*>(dy + tile_offset(row, 8, 128)) = make_uint4(0u, 0u, 0u, 0u);
+    } else {
+        for (int l = 0; l < 3; ++l)
+            *reinterpret_cast<uint4*>(smem + kTrH + l * kTrHTile + tile_offset(row, kMlpHidden, 128)) = ones;
+    }
     if (tid == 0) {
         mbar_init(smem_u32(&mbar), 1);
         fence_mbar_init();
@@ -701,11 +716,16 @@ __global__ void __launch_bounds__(128, 1) mlp_train_kernel(const TrainParams P) 
         tmem_alloc(smem_u32(&s_tmem), 512);
         tmem_relinquish();
     }
-    fence_async_smem();
+    const uint32_t w0 = smem_u32(smem);
+    grid_wait();  // nothing above reads what a kernel before this one writes
+    for (int i = tid; i < kImgAll / 16; i += kTrThreads)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(w0 + 16u * (uint32_t)i),
+                     "l"(P.mlp.img + 16 * (long long)i)
+                     : "memory");
+    const float bias = tid < kBiasPad ? P.mlp.bias[tid] : 0.0f;  // stored with the first tile's input
     tc_sync();
-    const uint32_t tm = s_tmem, mb = smem_u32(&mbar), w0 = smem_u32(smem + kTrW);
-    const uint32_t a0 = smem_u32(sa), t0 = smem_u32(T0), dzt0 = smem_u32(dzt), dyt0 = smem_u32(dyt), dy0 = smem_u32(dy);
-    const uint32_t th0[3] = {smem_u32(Th[0]), smem_u32(Th[1]), smem_u32(Th[2])};
+    const uint32_t tm = s_tmem, mb = smem_u32(&mbar);
+    const uint32_t x0 = w0 + kTrX, h0 = w0 + kTrH, dz0 = w0 + kTrDZ, dy0 = w0 + kTrDY;
     const uint32_t id64 = idesc_bf16_f32(128, 64), id16 = idesc_bf16_f32(128, 16);
     const long long ntiles = (P.n + 127) / 128;
     uint32_t phase = 0;
@@ -713,81 +733,86 @@ __global__ void __launch_bounds__(128, 1) mlp_train_kernel(const TrainParams P) 
     bool first = true;
     float loss = 0.0f, closs = 0.0f;
 
-    // Issues nothing itself: waits for the MMAs committed by thread 0.
-    auto wait_mma = [&]() -> int {
-        int done = 1;
-        if (tid == 0) {
-            commit(mb);
-            done = mbar_wait(mb, phase) ? 1 : 0;
-        }
+    // Waits for the MMAs committed by thread 0.  Every thread does, and after a
+    // wait that gave up goes on without waiting (the barriers stay matched;
+    // what it computes is not used).
+    auto wait_mma = [&]() {
+        if (ok) ok = mbar_wait(mb, phase) ? 1 : 0;
         phase ^= 1u;
-        const int r = __syncthreads_and(done);
         fence_after_sync();
-        return r;
     };
 
-    for (long long t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-        const long long idx = t * 128 + tid;
+    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const long long idx = t * 128 + row;
         const bool valid = idx < P.n;
-        const long long row = valid ? (P.index ? (long long)P.index[idx] : idx) : 0;
-        // ---- input
-        uint32_t f[24];
+        const long long src = valid ? (P.index ? (long long)P.index[idx] : idx) : 0;
+        // ---- input: 24 of the 48 features each
+        float target[3] = {0.f, 0.f, 0.f};
+        {
+            uint32_t f[12];
+            const float2* rp = reinterpret_cast<const float2*>(P.rows + src * kMlpIn) + 12 * half;
 #pragma unroll
-        for (int i = 0; i < 24; ++i) f[i] = 0u;
-        if (valid) {
-            const float2* r = reinterpret_cast<const float2*>(P.rows + row * kMlpIn);
-#pragma unroll
-            for (int i = 0; i < kMlpIn / 2; ++i) {
-                const float2 v = __ldg(r + i);
-                f[i] = bf16x2(v.x, v.y);
+            for (int i = 0; i < 12; ++i) {
+                f[i] = 0u;
+                if (valid && (i < kMlpIn / 2 - 12 || half == 0)) {
+                    const float2 v = __ldg(rp + i);
+                    f[i] = bf16x2(v.x, v.y);
+                }
             }
+            if (valid && half == 0) {
+#pragma unroll
+                for (int o = 0; o < 3; ++o) target[o] = __ldg(P.targets + src * 3 + o);
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                *reinterpret_cast<uint4*>(xt + tile_offset(row, 24 * half + 8 * c, 128)) =
+                    make_uint4(f[4 * c], f[4 * c + 1], f[4 * c + 2], f[4 * c + 3]);
         }
-#pragma unroll
-        for (int c = 0; c < 6; ++c)
-            *reinterpret_cast<uint4*>(sa + tile_offset(tid, 8 * c, 128)) =
-                make_uint4(f[4 * c], f[4 * c + 1], f[4 * c + 2], f[4 * c + 3]);
-#pragma unroll
-        for (int k = 0; k < kMlpIn; ++k) st_t(T0, k, tid, (uint16_t)((f[k >> 1] >> ((k & 1) * 16)) & 0xFFFFu));
+        if (first) {
+            if (tid < kBiasPad) s_bias[tid] = bias;
+            asm volatile("cp.async.wait_all;" ::: "memory");
+        }
         fence_async_smem();
         tc_sync();
         // ---- forward, hidden layers
-        uint64_t mask[3] = {0, 0, 0};
-#pragma unroll 1
-        for (int layer = 0; layer < 3 && ok; ++layer) {
-            const int K = layer == 0 ? kMlpInPad : kMlpHidden;
-            const uint32_t b = w0 + (layer == 0 ? kImgW1 : layer == 1 ? kImgW2 : kImgW3);
-            if (tid == 0)
-                for (int j = 0; j < K / 16; ++j) mma_bf16(tm + kColFb, tile_desc(a0, 128, j), tile_desc(b, 64, j), id64, j > 0);
-            if (!(ok = wait_mma())) break;
-            const float* bb = s_bias + kMlpHidden * layer;
-            uint64_t m = 0;
+        uint32_t mask[3] = {0, 0, 0};
 #pragma unroll
-            for (int c = 0; c < kMlpHidden; c += 16) {
-                float v[16];
-                tmem_ld16(tmem_addr(tm + kColFb, warp, c), v);
-                uint32_t pk[8];
+        for (int layer = 0; layer < 3; ++layer) {
+            if (tid == 0) {
+                const uint32_t a = layer == 0 ? x0 : h0 + (layer - 1) * kTrHTile;
+                const uint32_t b = w0 + (layer == 0 ? kImgW1 : layer == 1 ? kImgW2 : kImgW3);
+                for (int j = 0; j < (layer == 0 ? kMlpInPad : kMlpHidden) / 16; ++j)
+                    mma_bf16(tm + kColFb, tile_desc(a, 128, j), tile_desc(b, 64, j), id64, j > 0);
+                commit(mb);
+            }
+            wait_mma();
+            const float* bb = s_bias + kMlpHidden * layer + 32 * half;
+            uint8_t* h = smem + kTrH + layer * kTrHTile;
+            float v[32];
+            tmem_ld32(tmem_addr(tm + kColFb, warp, 32 * half), v);
+            uint32_t m = 0;
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    v[i] = fmaxf(v[i] + bb[c + i], 0.0f);
-                    if (v[i] > 0.0f) m |= 1ull << (c + i);
-                }
-#pragma unroll
-                for (int i = 0; i < 8; ++i) pk[i] = bf16x2(v[2 * i], v[2 * i + 1]);
-                *reinterpret_cast<uint4*>(sa + tile_offset(tid, c, 128)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                *reinterpret_cast<uint4*>(sa + tile_offset(tid, c + 8, 128)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-#pragma unroll
-                for (int i = 0; i < 16; ++i) st_t(Th[layer], c + i, tid, (uint16_t)((pk[i >> 1] >> ((i & 1) * 16)) & 0xFFFFu));
+            for (int i = 0; i < 32; ++i) {
+                v[i] = fmaxf(v[i] + bb[i], 0.0f);
+                if (v[i] > 0.0f) m |= 1u << i;
             }
             mask[layer] = m;
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                *reinterpret_cast<uint4*>(h + tile_offset(row, 32 * half + 8 * c, 128)) =
+                    make_uint4(bf16x2(v[8 * c], v[8 * c + 1]), bf16x2(v[8 * c + 2], v[8 * c + 3]),
+                               bf16x2(v[8 * c + 4], v[8 * c + 5]), bf16x2(v[8 * c + 6], v[8 * c + 7]));
             fence_async_smem();
             tc_sync();
         }
-        if (!ok) break;
         // ---- output layer, loss and dY
-        if (tid == 0)
-            for (int j = 0; j < 4; ++j) mma_bf16(tm + kColFb, tile_desc(a0, 128, j), tile_desc(w0 + kImgW4, 16, j), id16, j > 0);
-        if (!(ok = wait_mma())) break;
-        {
+        if (tid == 0) {
+            for (int j = 0; j < 4; ++j)
+                mma_bf16(tm + kColFb, tile_desc(h0 + 2 * kTrHTile, 128, j), tile_desc(w0 + kImgW4, 16, j), id16, j > 0);
+            commit(mb);
+        }
+        wait_mma();
+        if (half == 0) {
             float v[16];
             tmem_ld16(tmem_addr(tm + kColFb, warp, 0), v);
             float d[4] = {0.f, 0.f, 0.f, 0.f};
@@ -795,7 +820,7 @@ __global__ void __launch_bounds__(128, 1) mlp_train_kernel(const TrainParams P) 
                 float e2 = 0.0f;
 #pragma unroll
                 for (int o = 0; o < 3; ++o) {
-                    const float diff = (v[o] + s_bias[3 * kMlpHidden + o]) - __ldg(P.targets + row * 3 + o);
+                    const float diff = (v[o] + s_bias[3 * kMlpHidden + o]) - target[o];
                     loss += diff * diff;
                     e2 += diff * diff;
                     d[o] = P.scale * diff;
@@ -805,87 +830,80 @@ __global__ void __launch_bounds__(128, 1) mlp_train_kernel(const TrainParams P) 
                 closs += dc * dc;
                 d[3] = P.conf_scale * dc;
             }
-            const uint32_t p01 = bf16x2(d[0], d[1]), p23 = bf16x2(d[2], d[3]);
-            *reinterpret_cast<uint4*>(dy + tile_offset(tid, 0, 128)) = make_uint4(p01, p23, 0u, 0u);
-            st_t(dyt, 0, tid, (uint16_t)(p01 & 0xFFFFu), 16);
-            st_t(dyt, 1, tid, (uint16_t)(p01 >> 16), 16);
-            st_t(dyt, 2, tid, (uint16_t)(p23 & 0xFFFFu), 16);
-            st_t(dyt, 3, tid, (uint16_t)(p23 >> 16), 16);
+            *reinterpret_cast<uint4*>(dy + tile_offset(row, 0, 128)) =
+                make_uint4(bf16x2(d[0], d[1]), bf16x2(d[2], d[3]), 0u, 0u);
         }
         fence_async_smem();
         tc_sync();
-        // ---- backward
-        // dW4^T += H3^T dY ; dH3 = dY W4
+        // ---- backward: dH3 = dY W4; dW4^T += H3^T dY
         if (tid == 0) {
+            mma_bf16(tm + kColFb, tile_desc(dy0, 128, 0), tile_desc_t(w0 + kImgW4, 16, 0), id64 | kTransB, 0u);
+            commit(mb);
             for (int j = 0; j < 8; ++j)
-                mma_bf16(tm + kColW4, tile_desc(th0[2], 128, j), tile_desc(dyt0, 16, j), id16, (!first || j > 0) ? 1u : 0u);
-            mma_bf16(tm + kColFb, tile_desc(dy0, 128, 0), tile_desc(w0 + kImgW4t, 64, 0), id64, 0u);
+                mma_bf16(tm + kColW4, tile_desc_t(h0 + 2 * kTrHTile, 128, j), tile_desc_t(dy0, 128, j),
+                         id16 | kTransA | kTransB, (!first || j > 0) ? 1u : 0u);
         }
-        if (!(ok = wait_mma())) break;
-#pragma unroll 1
+        wait_mma();
+#pragma unroll
         for (int layer = 2; layer >= 0; --layer) {
-            // dZ_layer = dH * mask -> A operand (for dH of the layer below) and transposed (for dW)
+            // dZ_layer = dH * mask
+            const uint32_t dz = dz0 + layer * kTrDZTile;
+            {
+                float v[32];
+                tmem_ld32(tmem_addr(tm + kColFb, warp, 32 * half), v);
 #pragma unroll
-            for (int c = 0; c < kMlpHidden; c += 16) {
-                float v[16];
-                tmem_ld16(tmem_addr(tm + kColFb, warp, c), v);
-                uint32_t pk[8];
+                for (int i = 0; i < 32; ++i) v[i] = (mask[layer] >> i) & 1u ? v[i] : 0.0f;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float a = (mask[layer] >> (c + 2 * i)) & 1ull ? v[2 * i] : 0.0f;
-                    const float b = (mask[layer] >> (c + 2 * i + 1)) & 1ull ? v[2 * i + 1] : 0.0f;
-                    pk[i] = bf16x2(a, b);
-                }
-                if (layer > 0) {
-                    *reinterpret_cast<uint4*>(sa + tile_offset(tid, c, 128)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                    *reinterpret_cast<uint4*>(sa + tile_offset(tid, c + 8, 128)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-                }
-#pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    *reinterpret_cast<uint16_t*>(dzt + tile_offset(c + i, tid, 64)) =
-                        (uint16_t)((pk[i >> 1] >> ((i & 1) * 16)) & 0xFFFFu);
+                for (int c = 0; c < 4; ++c)
+                    *reinterpret_cast<uint4*>(smem + kTrDZ + layer * kTrDZTile + tile_offset(row, 32 * half + 8 * c, 128)) =
+                        make_uint4(bf16x2(v[8 * c], v[8 * c + 1]), bf16x2(v[8 * c + 2], v[8 * c + 3]),
+                                   bf16x2(v[8 * c + 4], v[8 * c + 5]), bf16x2(v[8 * c + 6], v[8 * c + 7]));
             }
             fence_async_smem();
             tc_sync();
             if (tid == 0) {
-                // dW_layer^T += H_{layer-1}^T dZ_layer   (H_{-1} = X)
-                const uint32_t hT = layer == 0 ? t0 : th0[layer - 1];
-                const uint32_t col = layer == 0 ? kColW1 : layer == 1 ? kColW2 : kColW3;
-                for (int j = 0; j < 8; ++j)
-                    mma_bf16(tm + col, tile_desc(hT, 128, j), tile_desc(dzt0, 64, j), id64, (!first || j > 0) ? 1u : 0u);
                 if (layer > 0) {
                     // dH_{layer-1} = dZ_layer W_layer
-                    const uint32_t wt = w0 + (layer == 2 ? kImgW3t : kImgW2t);
+                    const uint32_t w = w0 + (layer == 2 ? kImgW3 : kImgW2);
                     for (int j = 0; j < 4; ++j)
-                        mma_bf16(tm + kColFb, tile_desc(a0, 128, j), tile_desc(wt, 64, j), id64, j > 0);
+                        mma_bf16(tm + kColFb, tile_desc(dz, 128, j), tile_desc_t(w, 64, j), id64 | kTransB, j > 0);
+                    commit(mb);
                 }
+                // dW_layer^T += H_{layer-1}^T dZ_layer   (H_{-1} = X)
+                const uint32_t h = layer == 0 ? x0 : h0 + (layer - 1) * kTrHTile;
+                const uint32_t col = layer == 0 ? kColW1 : layer == 1 ? kColW2 : kColW3;
+                for (int j = 0; j < 8; ++j)
+                    mma_bf16(tm + col, tile_desc_t(h, 128, j), tile_desc_t(dz, 128, j), id64 | kTransA | kTransB,
+                             (!first || j > 0) ? 1u : 0u);
+                // the tile's last MMAs: nothing of it is read after them
+                if (layer == 0) commit(mb);
             }
-            if (!(ok = wait_mma())) break;
+            wait_mma();
         }
         first = false;
     }
-    // ---- gradients out
-    if (ok && !first) {
-        float* g = P.mlp.grad;
-        const int r = tid;  // TMEM lane = row of dW^T = input feature (or the bias row)
+    grid_launch_dependents();
+    ok = __syncthreads_and(ok);
+    // ---- gradients out: this CTA's part (zeros after a wait that gave up)
+    float* const part = P.mlp.parts + (long long)blockIdx.x * kPartStride;
+    {
+        const int r = row;  // TMEM lane = row of dW^T = input feature (or the bias row)
 #pragma unroll 1
         for (int layer = 0; layer < 4; ++layer) {
             const int in = layer == 0 ? kMlpIn : kMlpHidden;
             const int bias_row = layer == 0 ? kMlpInPad : kMlpHidden;
-            const int nout = layer == 3 ? kMlpOut : kMlpHidden;
             const uint32_t col = layer == 0 ? kColW1 : layer == 1 ? kColW2 : layer == 2 ? kColW3 : kColW4;
             const int offw = layer == 0 ? kOffW1 : layer == 1 ? kOffW2 : layer == 2 ? kOffW3 : kOffW4;
             const int offb = layer == 0 ? kOffB1 : layer == 1 ? kOffB2 : layer == 2 ? kOffB3 : kOffB4;
-            for (int c = 0; c < (layer == 3 ? 16 : 64); c += 16) {
-                float v[16];
-                tmem_ld16(tmem_addr(tm + col, warp, c), v);
+            const int nout = layer == 3 ? (half == 0 ? kMlpOut : 0) : 32;
+            float v[32];
+            tmem_ld32(tmem_addr(tm + col, warp, layer == 3 ? 0 : 32 * half), v);
+            float* p = r < in ? part + offw + r + 32 * half * in : part + offb + 32 * half;
+            const int stride = r < in ? in : 1;
+            if (r < in || r == bias_row) {
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const int o = c + i;
-                    if (o >= nout) continue;
-                    if (r < in) atomicAdd(g + offw + o * in + r, v[i]);
-                    else if (r == bias_row) atomicAdd(g + offb + o, v[i]);
-                }
+                for (int i = 0; i < 32; ++i)
+                    if (i < nout) p[i * stride] = ok ? v[i] : 0.0f;
             }
         }
     }
@@ -894,30 +912,71 @@ __global__ void __launch_bounds__(128, 1) mlp_train_kernel(const TrainParams P) 
         loss += __shfl_xor_sync(0xffffffffu, loss, o);
         closs += __shfl_xor_sync(0xffffffffu, closs, o);
     }
-    if (lane == 0) {
+    if (lane == 0 && half == 0) {
         s_loss[warp] = loss;
         s_closs[warp] = closs;
     }
     if (!ok && tid == 0) atomicOr(P.status, 1u);
     tc_sync();
     if (tid == 0)
-        atomicAdd(P.mlp.loss, (s_loss[0] + s_loss[1] + s_loss[2] + s_loss[3]) * (0.5f * P.scale) +
-                                  (s_closs[0] + s_closs[1] + s_closs[2] + s_closs[3]) * (0.5f * P.conf_scale));
+        part[kMlpParams] = (s_loss[0] + s_loss[1] + s_loss[2] + s_loss[3]) * (0.5f * P.scale) +
+                           (s_closs[0] + s_closs[1] + s_closs[2] + s_closs[3]) * (0.5f * P.conf_scale);
     if (warp == 0) tmem_dealloc(tm, 512);
 }
 
 // ------------------------------------------------------- optimiser
-// Adam on the fp32 master parameters (optional), then the BF16 operand
+// The sum of the parts' gradients (eight threads a parameter, an eighth of the
+// parts each), Adam on the fp32 master parameters, then the BF16 operand
 // images and the padded bias vector the kernels read.
-__global__ void mlp_update_kernel(const MlpDev M, float lr, float beta1, float beta2, float eps, float c1, float c2,
-                                  int update) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kMlpParams) return;
-    float w = M.params[i];
-    if (update) {
-        const float g = M.grad[i];
-        const float m = beta1 * M.m[i] + (1.0f - beta1) * g;
-        const float v = beta2 * M.v[i] + (1.0f - beta2) * g * g;
+constexpr int kUpdateThreads = 512, kUpdateSlices = 8, kUpdateParams = kUpdateThreads / kUpdateSlices;
+
+__global__ void __launch_bounds__(kUpdateThreads) mlp_update_kernel(const MlpDev M, int what, int nparts, float lr,
+                                                                    float beta1, float beta2, float eps, float c1,
+                                                                    float c2, float* loss_out) {
+    __shared__ float s_sum[kUpdateSlices][kUpdateParams];
+    const int slice = threadIdx.x / kUpdateParams, k = threadIdx.x % kUpdateParams;
+    const int i = blockIdx.x * kUpdateParams + k;
+    float w = 0.0f, m = 0.0f, v = 0.0f;
+    const bool mine = slice == 0 && i < kMlpParams;
+    if (mine && what == kUpdateAdam) {
+        // the training kernel, which this one may overlap, started after the
+        // end of everything that writes these
+        w = M.params[i];
+        m = M.m[i];
+        v = M.v[i];
+    }
+    grid_wait();
+    grid_launch_dependents();
+    if (what != kUpdateImages) {
+        float g = 0.0f;
+        if (i < kMlpParams) {
+#pragma unroll 16
+            for (int p = slice; p < nparts; p += kUpdateSlices) g += __ldcg(M.parts + (long long)p * kPartStride + i);
+        }
+        s_sum[slice][k] = g;
+        if (blockIdx.x == 0 && threadIdx.x < 32) {
+            float l = 0.0f;
+            for (int p = threadIdx.x; p < nparts; p += 32) l += __ldcg(M.parts + (long long)p * kPartStride + kMlpParams);
+            for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+            if (threadIdx.x == 0) {
+                *M.loss = l;
+                if (loss_out) *loss_out = l;
+            }
+        }
+        __syncthreads();
+    }
+    if (!mine) return;
+    if (what == kUpdateImages) {
+        w = M.params[i];
+    } else {
+        const float g = ((s_sum[0][k] + s_sum[1][k]) + (s_sum[2][k] + s_sum[3][k])) +
+                        ((s_sum[4][k] + s_sum[5][k]) + (s_sum[6][k] + s_sum[7][k]));
+        if (what == kUpdateGradient) {
+            M.grad[i] = g;
+            return;
+        }
+        m = beta1 * m + (1.0f - beta1) * g;
+        v = beta2 * v + (1.0f - beta2) * g * g;
         M.m[i] = m;
         M.v[i] = v;
         w = w - lr * (m * c1) / (sqrtf(v * c2) + eps);
@@ -933,19 +992,16 @@ __global__ void mlp_update_kernel(const MlpDev M, float lr, float beta1, float b
     } else if (i < kOffB2) {
         const int o = (i - kOffW2) / kMlpHidden, f = (i - kOffW2) % kMlpHidden;
         *reinterpret_cast<uint16_t*>(img + kImgW2 + tile_offset(o, f, 64)) = h;
-        *reinterpret_cast<uint16_t*>(img + kImgW2t + tile_offset(f, o, 64)) = h;
     } else if (i < kOffW3) {
         M.bias[kMlpHidden + i - kOffB2] = w;
     } else if (i < kOffB3) {
         const int o = (i - kOffW3) / kMlpHidden, f = (i - kOffW3) % kMlpHidden;
         *reinterpret_cast<uint16_t*>(img + kImgW3 + tile_offset(o, f, 64)) = h;
-        *reinterpret_cast<uint16_t*>(img + kImgW3t + tile_offset(f, o, 64)) = h;
     } else if (i < kOffW4) {
         M.bias[2 * kMlpHidden + i - kOffB3] = w;
     } else if (i < kOffB4) {
         const int o = (i - kOffW4) / kMlpHidden, f = (i - kOffW4) % kMlpHidden;
         *reinterpret_cast<uint16_t*>(img + kImgW4 + tile_offset(o, f, 16)) = h;
-        *reinterpret_cast<uint16_t*>(img + kImgW4t + tile_offset(f, o, 64)) = h;
     } else {
         M.bias[3 * kMlpHidden + i - kOffB4] = w;
     }
@@ -1046,21 +1102,37 @@ void launch_trace16_pixels(const LearnedParams& P, cudaStream_t s) {
     note_launches(2);
 }
 
-void launch_mlp_train(const TrainParams& P, int num_sms, cudaStream_t s) {
-    if (P.n <= 0) return;
-    const long long tiles = (P.n + 127) / 128;
-    const long long grid = tiles < num_sms ? tiles : num_sms;
-    cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrSmem);
-    mlp_train_kernel<<<(unsigned)grid, 128, kTrSmem, s>>>(P);
+template <class... K, class... A>
+static void launch_overlapped(void (*kernel)(K...), int grid, int threads, int smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
     note_launches(1);
 }
 
-void launch_mlp_update(const MlpDev& M, int step, float lr, float beta1, float beta2, float eps, int update,
-                       cudaStream_t s) {
-    const double c1 = update ? 1.0 / (1.0 - std::pow((double)beta1, (double)step)) : 1.0;
-    const double c2 = update ? 1.0 / (1.0 - std::pow((double)beta2, (double)step)) : 1.0;
-    mlp_update_kernel<<<(kMlpParams + 255) / 256, 256, 0, s>>>(M, lr, beta1, beta2, eps, (float)c1, (float)c2, update);
-    note_launches(1);
+int launch_mlp_train(const TrainParams& P, int num_sms, cudaStream_t s) {
+    const long long tiles = (P.n + 127) / 128;
+    const int grid = (int)(tiles < num_sms ? tiles : num_sms);
+    cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrSmem);
+    launch_overlapped(mlp_train_kernel, grid, kTrThreads, kTrSmem, s, P);
+    return grid;
+}
+
+void launch_mlp_update(const MlpDev& M, int what, int nparts, int step, float lr, float beta1, float beta2, float eps,
+                       float* loss_out, cudaStream_t s) {
+    const bool adam = what == kUpdateAdam;
+    const double c1 = adam ? 1.0 / (1.0 - std::pow((double)beta1, (double)step)) : 1.0;
+    const double c2 = adam ? 1.0 / (1.0 - std::pow((double)beta2, (double)step)) : 1.0;
+    launch_overlapped(mlp_update_kernel, (kMlpParams + kUpdateParams - 1) / kUpdateParams, kUpdateThreads, 0, s, M, what,
+                      nparts, lr, beta1, beta2, eps, (float)c1, (float)c2, loss_out);
 }
 
 }  // namespace vct

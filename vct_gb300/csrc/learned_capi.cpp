@@ -4,6 +4,7 @@
 // reference, the learned trace with its per-tile or per-pixel fallback).
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -16,8 +17,10 @@ using namespace vct::host;
 struct vct_mlp {
     int device = 0, num_sms = 0;
     MlpDev dev = {};
-    uint32_t* status = nullptr;
+    uint32_t* status = nullptr;  // the word behind the parameters
     int step = 0;
+    std::mutex staging_lock;
+    float* staging = nullptr;  // pinned: the parameters and the status word
 };
 
 namespace {
@@ -52,7 +55,7 @@ vct_status upload_params(vct_mlp* m, const float* host, cudaStream_t st) {
     VCT_CUDA(cudaMemcpyAsync(m->dev.params, host, sizeof(float) * kMlpParams, cudaMemcpyHostToDevice, st));
     VCT_CUDA(cudaMemsetAsync(m->dev.m, 0, sizeof(float) * kMlpParams, st));
     VCT_CUDA(cudaMemsetAsync(m->dev.v, 0, sizeof(float) * kMlpParams, st));
-    launch_mlp_update(m->dev, 1, 0.f, 0.f, 0.f, 0.f, 0, st);
+    launch_mlp_update(m->dev, kUpdateImages, 0, 1, 0.f, 0.f, 0.f, 0.f, nullptr, st);
     VCT_CHECK_LAUNCH("mlp operand images");
     m->step = 0;
     return VCT_OK;
@@ -212,10 +215,11 @@ vct_status vct_mlp_create(int32_t device, uint64_t seed, vct_mlp** out) {
     struct {
         void** p;
         size_t bytes;
-    } allocs[] = {{(void**)&m->dev.params, pf},           {(void**)&m->dev.grad, pf},
+    } allocs[] = {{(void**)&m->dev.params, pf + sizeof(uint32_t)}, {(void**)&m->dev.grad, pf},
+                  {(void**)&m->dev.parts, sizeof(float) * kPartStride * (size_t)m->num_sms},
                   {(void**)&m->dev.m, pf},                {(void**)&m->dev.v, pf},
                   {(void**)&m->dev.img, (size_t)kImgAll}, {(void**)&m->dev.bias, sizeof(float) * kBiasPad},
-                  {(void**)&m->dev.loss, sizeof(float)},  {(void**)&m->status, sizeof(uint32_t)}};
+                  {(void**)&m->dev.loss, sizeof(float)}};
     for (auto& a : allocs) {
         cudaError_t e = cudaMalloc(a.p, a.bytes);
         if (e == cudaSuccess) e = cudaMemset(*a.p, 0, a.bytes);
@@ -224,6 +228,12 @@ vct_status vct_mlp_create(int32_t device, uint64_t seed, vct_mlp** out) {
             vct_mlp_destroy(m);
             return fail(VCT_ERR_OUT_OF_MEMORY, std::string("mlp buffers: ") + cudaGetErrorString(e));
         }
+    }
+    m->status = reinterpret_cast<uint32_t*>(m->dev.params + kMlpParams);
+    if (cudaMallocHost(reinterpret_cast<void**>(&m->staging), pf + sizeof(uint32_t)) != cudaSuccess) {
+        cudaGetLastError();
+        vct_mlp_destroy(m);
+        return fail(VCT_ERR_OUT_OF_MEMORY, "mlp buffers: pinned host memory");
     }
     std::vector<float> p;
     init_params(seed, p);
@@ -241,9 +251,10 @@ vct_status vct_mlp_create(int32_t device, uint64_t seed, vct_mlp** out) {
 vct_status vct_mlp_destroy(vct_mlp* m) {
     if (!m) return VCT_OK;
     DeviceScope ds(m->device);
-    void* ptrs[] = {m->dev.params, m->dev.grad, m->dev.m, m->dev.v, m->dev.img, m->dev.bias, m->dev.loss, m->status};
+    void* ptrs[] = {m->dev.params, m->dev.grad, m->dev.parts, m->dev.m, m->dev.v, m->dev.img, m->dev.bias, m->dev.loss};
     for (void* p : ptrs)
         if (p) cudaFree(p);
+    if (m->staging) cudaFreeHost(m->staging);
     delete m;
     return VCT_OK;
 }
@@ -267,8 +278,14 @@ vct_status vct_mlp_get_params(vct_mlp* m, float* host, int64_t count, void* stre
     DeviceScope ds(m->device);
     VCT_CUDA(ds.err);
     cudaStream_t st = as_stream(stream);
-    VCT_CUDA(cudaMemcpyAsync(host, m->dev.params, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost, st));
-    return check_status(m, st);
+    // one copy brings the parameters and the status word behind them
+    std::lock_guard<std::mutex> hold(m->staging_lock);
+    VCT_CUDA(cudaMemcpyAsync(m->staging, m->dev.params, sizeof(float) * (kMlpParams + 1), cudaMemcpyDeviceToHost, st));
+    VCT_CUDA(cudaStreamSynchronize(st));
+    std::memcpy(host, m->staging, sizeof(float) * kMlpParams);
+    uint32_t h;
+    std::memcpy(&h, m->staging + kMlpParams, sizeof h);
+    return h ? check_status(m, st) : VCT_OK;
 }
 
 vct_status vct_mlp_forward(vct_mlp* m, const float* rows, int64_t n, float* out, void* stream) {
@@ -292,13 +309,11 @@ vct_status vct_mlp_forward(vct_mlp* m, const float* rows, int64_t n, float* out,
 }
 
 static vct_status train_launch(vct_mlp* m, const float* rows, const float* targets, const int32_t* index, int64_t n,
-                               cudaStream_t st) {
+                               cudaStream_t st, int& nparts) {
     vct_status s = validate_rows(rows, n);
     if (s != VCT_OK) return s;
     if (n < 1) return fail(VCT_ERR_INVALID_ARGUMENT, "training needs at least one row");
     if (!targets) return fail(VCT_ERR_INVALID_ARGUMENT, "targets is NULL");
-    VCT_CUDA(cudaMemsetAsync(m->dev.grad, 0, sizeof(float) * kMlpParams, st));
-    VCT_CUDA(cudaMemsetAsync(m->dev.loss, 0, sizeof(float), st));
     TrainParams P;
     std::memset(&P, 0, sizeof P);
     P.mlp = m->dev;
@@ -309,7 +324,7 @@ static vct_status train_launch(vct_mlp* m, const float* rows, const float* targe
     P.scale = (float)(2.0 / (3.0 * (double)n));
     P.conf_scale = (float)(2.0 * (double)kMlpConfidenceWeight / (double)n);
     P.status = m->status;
-    launch_mlp_train(P, m->num_sms, st);
+    nparts = launch_mlp_train(P, m->num_sms, st);
     VCT_CHECK_LAUNCH("mlp training kernel");
     return VCT_OK;
 }
@@ -320,8 +335,11 @@ vct_status vct_mlp_gradients(vct_mlp* m, const float* rows, const float* targets
     DeviceScope ds(m->device);
     VCT_CUDA(ds.err);
     cudaStream_t st = as_stream(stream);
-    vct_status s = train_launch(m, rows, targets, nullptr, n, st);
+    int nparts = 0;
+    vct_status s = train_launch(m, rows, targets, nullptr, n, st, nparts);
     if (s != VCT_OK) return s;
+    launch_mlp_update(m->dev, kUpdateGradient, nparts, 0, 0.f, 0.f, 0.f, 0.f, nullptr, st);
+    VCT_CHECK_LAUNCH("gradient sum");
     VCT_CUDA(cudaMemcpyAsync(grad_dev, m->dev.grad, sizeof(float) * kMlpParams, cudaMemcpyDeviceToDevice, st));
     if (loss_dev) VCT_CUDA(cudaMemcpyAsync(loss_dev, m->dev.loss, sizeof(float), cudaMemcpyDeviceToDevice, st));
     return check_status(m, st);
@@ -336,12 +354,16 @@ vct_status vct_mlp_train_step(vct_mlp* m, const float* rows, const float* target
     DeviceScope ds(m->device);
     VCT_CUDA(ds.err);
     cudaStream_t st = as_stream(stream);
-    vct_status s = train_launch(m, rows, targets, index, n, st);
+    int nparts = 0;
+    vct_status s = train_launch(m, rows, targets, index, n, st, nparts);
     if (s != VCT_OK) return s;
     ++m->step;
-    launch_mlp_update(m->dev, m->step, opt->lr, opt->beta1, opt->beta2, opt->eps, 1, st);
+    // the update stores the loss, unless that is not in a float's place
+    const bool place = reinterpret_cast<uintptr_t>(loss_dev) % sizeof(float) == 0;
+    launch_mlp_update(m->dev, kUpdateAdam, nparts, m->step, opt->lr, opt->beta1, opt->beta2, opt->eps,
+                      place ? loss_dev : nullptr, st);
     VCT_CHECK_LAUNCH("adam");
-    if (loss_dev) VCT_CUDA(cudaMemcpyAsync(loss_dev, m->dev.loss, sizeof(float), cudaMemcpyDeviceToDevice, st));
+    if (!place) VCT_CUDA(cudaMemcpyAsync(loss_dev, m->dev.loss, sizeof(float), cudaMemcpyDeviceToDevice, st));
     return VCT_OK;
 }
 

@@ -45,9 +45,19 @@ __device__ __forceinline__ uint64_t tile_desc(uint32_t saddr, int R, int j) {
     return smem_desc(saddr + (uint32_t)(j * 2 * R * 16), (uint32_t)(R * 16), 128u);
 }
 
+// The same bytes as the transposed operand: M (or N) runs along the tile's
+// columns and K along its R rows, K step `j` (16 rows).  In the canonical
+// no-swizzle MN-major layout the leading-dimension byte offset is the one
+// between core matrices adjacent in K, the stride-dimension byte offset the
+// one between those adjacent in M or N.
+__device__ __forceinline__ uint64_t tile_desc_t(uint32_t saddr, int R, int j) {
+    return smem_desc(saddr + (uint32_t)(j * 256), 128u, (uint32_t)(R * 16));
+}
+
 // Instruction descriptor of kind::f16: D FP32 (bits 4-5 = 1), A and B BF16
-// (bits 7-9 and 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 in bits
-// 17-22, M >> 4 in bits 24-28.
+// (bits 7-9 and 10-12 = 1), K-major (bits 15, 16 = 0; set for a transposed A
+// or B, kTransA and kTransB), N >> 3 in bits 17-22, M >> 4 in bits 24-28.
+constexpr uint32_t kTransA = 1u << 15, kTransB = 1u << 16;
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
@@ -81,8 +91,9 @@ __device__ __forceinline__ uint64_t global_ns() {
 // Waits for the completion of the mbarrier phase of parity `parity`, for at
 // most `limit_ns` nanoseconds.  Returns false on timeout.
 __device__ __forceinline__ bool mbar_wait_for(uint32_t mbar, uint32_t parity, uint64_t limit_ns) {
-    const uint64_t t0 = global_ns();
-    while (true) {
+    // (the timer is read after the first try: reading it takes as long as a wait)
+    uint64_t t0 = 0;
+    for (int n = 0;; ++n) {
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -92,7 +103,10 @@ __device__ __forceinline__ bool mbar_wait_for(uint32_t mbar, uint32_t parity, ui
             : "r"(mbar), "r"(parity)
             : "memory");
         if (done) return true;
-        if (global_ns() - t0 > limit_ns) return false;
+        if (n == 0)
+            t0 = global_ns();
+        else if (global_ns() - t0 > limit_ns)
+            return false;
     }
 }
 

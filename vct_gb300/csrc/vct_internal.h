@@ -381,11 +381,10 @@ constexpr int kOffW1 = 0, kOffB1 = 2688, kOffW2 = 2752, kOffB2 = 6848, kOffW3 = 
 // Weight of the error-estimate term in the training loss (relative to the
 // mean squared error of the irradiance).
 constexpr float kMlpConfidenceWeight = 0.5f;
-// BF16 operand images in the tensor core's shared-memory tile layout:
-// forward B operands W1 (64 x 48), W2, W3 (64 x 64), W4 (16 x 64), then the
-// transposes used by the backward pass W4^T (64 x 16), W3^T, W2^T (64 x 64).
-constexpr int kImgW1 = 0, kImgW2 = 6144, kImgW3 = 14336, kImgW4 = 22528, kImgFwd = 24576, kImgW4t = 24576,
-              kImgW3t = 26624, kImgW2t = 34816, kImgAll = 43008;
+// BF16 operand images in the tensor core's shared-memory tile layout: W1
+// (64 x 48), W2, W3 (64 x 64), W4 (16 x 64); the forward passes' B operands,
+// and the backward pass's transposed ones.
+constexpr int kImgW1 = 0, kImgW2 = 6144, kImgW3 = 14336, kImgW4 = 22528, kImgAll = 24576;
 // Bias vector padded for the kernels: b1 | b2 | b3 | b4 (16).
 constexpr int kBiasPad = 208;
 // Quarter-resolution cheap trace: 2 cones x 4 levels x RGBA, BF16.
@@ -393,9 +392,11 @@ constexpr int kCheapFeatures = 32;
 // Per-tile error probes of the learned trace and its 16 x 16 tiles.
 constexpr int kProbes = 4, kLearnTile = 16;
 
+constexpr int kPartStride = kMlpParams + 4;
 struct MlpDev {
     float* params;  // fp32 master
     float* grad;
+    float* parts;   // kPartStride floats for each CTA of the training kernel: its gradient, its loss
     float* m;
     float* v;
     uint8_t* img;   // kImgAll bytes
@@ -446,9 +447,14 @@ void launch_trace16(const LearnedParams& P, bool listed, int num_sms, cudaStream
 // The per-pixel fallback after inference with `est` set: the list of flagged
 // pixels, then their 16-cone trace.
 void launch_trace16_pixels(const LearnedParams& P, cudaStream_t s);
-void launch_mlp_train(const TrainParams& P, int num_sms, cudaStream_t s);
-void launch_mlp_update(const MlpDev& M, int step, float lr, float beta1, float beta2, float eps, int update,
-                       cudaStream_t s);
+// Returns the number of CTAs, i.e. of parts.
+int launch_mlp_train(const TrainParams& P, int num_sms, cudaStream_t s);
+// What the update kernel does: the operand images of the parameters; the sum
+// of a training pass's `nparts` gradients, and its loss; both with an Adam step
+// between (`loss_out`, if given, gets the loss too).
+enum { kUpdateImages = 0, kUpdateGradient = 1, kUpdateAdam = 2 };
+void launch_mlp_update(const MlpDev& M, int what, int nparts, int step, float lr, float beta1, float beta2, float eps,
+                       float* loss_out, cudaStream_t s);
 
 // Injection through the lit mask (marked by launch_inject_mark): every marked
 // voxel's store computed once from the radiance seeded this frame.
