@@ -1222,7 +1222,8 @@ def irradiance_accuracy(gpu: np.ndarray, ref: np.ndarray, covered: np.ndarray, f
     return out
 
 
-KERNEL_SOURCES = ("cone.cuh", "vct_device.cuh", "vct_internal.h", "warp.cuh", "voxelize.cu", "volume.cu", "trace.cu")
+KERNEL_SOURCES = ("cone.cuh", "lines.cuh", "trace.cuh", "vct_device.cuh", "vct_internal.h", "warp.cuh", "voxelize.cu",
+                  "volume.cu", "trace.cu", "trace_split.cu")
 
 
 def kernel_sources_digest() -> str:

@@ -1,6 +1,6 @@
 """The cone march around the size of its step table (64 steps a cone), for each
 of its variants (no warp, the warp map, any warp): irradiance, specular light
-and sample counts against the fp32 oracle."""
+and sample counts against the fp32 oracle; and the tracer's two kernels against each other."""
 
 from __future__ import annotations
 
@@ -34,4 +34,30 @@ def test_cone_steps_match_oracle(steps, warp):
     assert rel_l2(rgb(irr.cpu().numpy()), rgb(ref["irradiance"])) <= 1e-4
     assert rel_l2(rgb(spec.cpu().numpy()), rgb(ref["specular"])) <= 1e-4
     assert int(samples.item()) == pytest.approx(ref["samples"], rel=1e-3)
+    ctx.close()
+
+
+@pytest.mark.parametrize("filt", [L.VCT_FILTER_SOFTWARE, L.VCT_FILTER_HYBRID])
+def test_few_and_many_pixels_give_the_same_bits(filt):
+    """An image of 5,000 tiles (a warp to 32 pixels) and its bands of 80 to 1,120
+    tiles (four warps): every output, and the number of samples."""
+    import torch
+
+    W, H = 1277, 990
+    sc = scenes.cornell(seed=4, gbuffer=(W, H))
+    g = GpuScene(sc)
+    ctx = api.Context(api.config_for(sc))
+    ctx.set_params(api.scene_params(sc, trace_filter=filt))
+    ctx.frame_volume(g.tris, g.lights, g.shadow, sc.eye)
+    whole, bands = g.new_outputs(), g.new_outputs()
+    ctx.trace(g.gb, sc.eye, api.trace_out(*whole))
+    rows = lambda t, r0, r1: t[r0 * W * 4:r1 * W * 4]  # noqa: E731
+    cuts = [0, 1, 17, 241, 465, 689, 913, H]
+    for r0, r1 in zip(cuts, cuts[1:]):
+        gb = api.gbuffer(rows(g.gpos, r0, r1), rows(g.gnrm, r0, r1), rows(g.galb, r0, r1), W, r1 - r0)
+        ctx.trace(gb, sc.eye, api.trace_out(*(rows(t, r0, r1) for t in bands[:3]), bands[3]))
+    torch.cuda.synchronize()
+    assert float(whole[0].abs().sum()) > 0
+    for a, b in zip(whole, bands):
+        assert torch.equal(a.view(torch.int32), b.view(torch.int32))
     ctx.close()

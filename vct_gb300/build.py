@@ -36,6 +36,7 @@ CUDA_SOURCES = [
     ("volume.cu", ["--fmad=false"]),
     ("raster.cu", ["--fmad=false"]),
     ("trace.cu", ["--fmad=false"]),
+    ("trace_split.cu", ["--fmad=false"]),
     ("static_scratch.cu", []),
     ("learned.cu", ["--fmad=false"]),
     ("shade.cu", ["--fmad=false"]),

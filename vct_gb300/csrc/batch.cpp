@@ -261,7 +261,7 @@ vct_status batch_enqueue(vct_batch* b, const char* h, const BatchTotals& tot, cu
     if (timed) VCT_CUDA(cudaEventRecord(b->ev[2], st));
     launch_trace_batch(SceneBatch<TraceParams>{reinterpret_cast<const TraceParams*>(b->d_blob + b->off_trace),
                                               d_tables + 3 * (n + 1), n},
-                       b->ctx[0]->params.trace_filter, tot.cones, tot.tiles, st);
+                       b->ctx[0]->params.trace_filter, tot.cones, tot.tiles, b->num_sms, st);
     VCT_CHECK_LAUNCH("batch: trace");
     if (timed) VCT_CUDA(cudaEventRecord(b->ev[3], st));
     const int filter = b->ctx[0]->params.trace_filter;

@@ -579,6 +579,7 @@ vct_status fill_trace(vct_ctx* ctx, const vct_gbuffer* g, const float eye[3], co
     P.ref_tbn_quirk = pr.ref_tbn_quirk;
     P.filter = pr.trace_filter;
     P.tex = ctx->tex;
+    P.num_sms = ctx->num_sms;
     P.warp = warp_dev(ctx, eye);
     apply_tuning(ctx->tuning, P);
     for (auto p : {(const void*)g->position_dev, (const void*)g->normal_dev, (const void*)g->albedo_dev,

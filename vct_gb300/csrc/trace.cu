@@ -19,21 +19,11 @@
 // instantiations of the kernel give bit-identical results.
 #include <algorithm>
 
-#include "cone.cuh"
+#include "trace.cuh"
 
 namespace vct {
 
 namespace {
-
-using namespace cone;
-
-__constant__ float kConeDir[6][3] = {{0.f, 1.f, 0.f},
-                                     {0.f, 0.5f, 0.866025f},
-                                     {0.823639f, 0.5f, 0.267617f},
-                                     {0.509037f, 0.5f, -0.700629f},
-                                     {-0.5909037f, 0.5f, -0.700629f},  // sic, phong.frag:475
-                                     {-0.823639f, 0.5f, 0.267617f}};
-__constant__ float kConeWeight[6] = {0.25f, 0.15f, 0.15f, 0.15f, 0.15f, 0.15f};
 
 // Bound by the L1 data pipe: a warp's 16-byte texel load takes four passes or
 // more (5 on average), and the pipe is busy 78% of the time; the loads mostly
@@ -45,18 +35,12 @@ __constant__ float kConeWeight[6] = {0.25f, 0.15f, 0.15f, 0.15f, 0.15f, 0.15f};
 // software sampler's 565 us (602).
 template <int MODE, int KIND, class Scenes>
 __global__ void __launch_bounds__(256, 4) trace_kernel(const Scenes S) {
-    // One CTA per tile of 2^tile_w_log2 x 2^tile_h_log2 = 256 pixels (a
-    // tuning setting; tiles of every scene of the launch in a row), one warp
-    // per 2^warp_w_log2 x 32/2^warp_w_log2 sub-tile.
+    // One CTA per tile (tiles of every scene of the launch in a row), one warp
+    // per sub-tile.
     long long tile;
     const TraceParams& P = S.get(S.find(blockIdx.x, tile));
-    const int twl = P.tile_w_log2, thl = P.tile_h_log2, wwl = P.warp_w_log2;
-    const int tiles_x = (P.width + (1 << twl) - 1) >> twl;
-    const int tx = (int)(tile % tiles_x), ty = (int)(tile / tiles_x);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int wxl = twl - wwl;  // log2 of warps per tile row
-    const int x = (tx << twl) + ((wid & ((1 << wxl) - 1)) << wwl) + lane_x(lane, wwl);
-    const int y = (ty << thl) + ((wid >> wxl) << (5 - wwl)) + lane_y(lane, wwl);
+    int x, y;
+    tile_pixel(P, tile, threadIdx.x >> 5, threadIdx.x & 31, x, y);
     __shared__ Level s_lv[VCT_MAX_LEVELS];
     __shared__ ConeTable s_cone[2];  // the diffuse and the specular cones' steps
     fill_levels(P, s_lv);
@@ -69,66 +53,28 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const Scenes S) {
         float4 irr = make_float4(0.f, 0.f, 0.f, 0.f), spc = irr, out = irr;
         const float4 gp = __ldg(P.gpos + pix);
         if (gp.w != 0.0f) {
-            const float4 gn = __ldg(P.gnrm + pix);
-            const f3 N = fnormalize(mk(gn.x, gn.y, gn.z));
-            f3 rgb;
             if (P.enable_indirect) {
-                const f3 ext = sub(P.vmax, P.vmin);
-                const f3 vp = mk(((gp.x - P.vcenter.x) - P.vmin.x) / ext.x, ((gp.y - P.vcenter.y) - P.vmin.y) / ext.y,
-                                 ((gp.z - P.vcenter.z) - P.vmin.z) / ext.z);
-                // Orthonormal basis from N: Duff et al. 2017, "Building an
-                // Orthonormal Basis, Revisited" (JCGT 6(1)).
-                const float sgn = N.z >= 0.0f ? 1.0f : -1.0f;
-                const float ca = -1.0f / (sgn + N.z);
-                const float cb = N.x * N.y * ca;
-                const f3 T = mk(1.0f + sgn * N.x * N.x * ca, sgn * cb, -sgn * N.x);
-                const f3 B = mk(cb, sgn + N.y * N.y * ca, -N.y);
-                float4 ind = make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 gn = __ldg(P.gnrm + pix);
+                const f3 N = fnormalize(mk(gn.x, gn.y, gn.z));
+                const f3 vp = volume_position(P, gp);
+                f3 T, B;
+                tangents(N, T, B);
 #pragma unroll 1
                 for (int c = 0; c < 6; ++c) {
-                    const float dx = kConeDir[c][0], dy = kConeDir[c][1], dz = kConeDir[c][2];
-                    f3 d = P.ref_tbn_quirk ? add(add(mul(T, dx), mul(B, dy)), mul(N, dz))
-                                           : sub(add(mul(T, dx), mul(N, dy)), mul(B, dz));
-                    float4 cr = trace_cone<MODE, KIND>(P, s_lv, s_cone[0], vp, N, d, P.diffuse, P.max_distance, ns);
-                    const float w = kConeWeight[c];
-                    ind = make_float4(fmaf(w, cr.x, ind.x), fmaf(w, cr.y, ind.y), fmaf(w, cr.z, ind.z),
-                                      fmaf(w, cr.w, ind.w));
+                    const float4 cr = trace_cone<MODE, KIND>(P, s_lv, s_cone[0], vp, N, diffuse_direction(P, c, N, T, B),
+                                                             P.diffuse, P.max_distance, ns);
+                    irr = add_cone(irr, kConeWeight[c], cr);
                 }
-                irr = ind;
-                const float occ = 1.0f - clampf(ind.w, 0.0f, 1.0f);
-                rgb = mk(ind.x, ind.y, ind.z);
-                if (P.enable_reflections) {
-                    // the position is read again rather than kept live across the diffuse cones
-                    const float4 gq = __ldg(P.gpos + pix);
-                    const f3 I = sub(mk(gq.x, gq.y, gq.z), P.eye);
-                    const f3 R = sub(I, mul(N, 2.0f * dot(N, I)));
-                    spc = trace_cone<MODE, KIND>(P, s_lv, s_cone[1], vp, N, R, P.specular_cone, P.max_distance, ns);
-                    rgb = add(rgb, mul(mk(spc.x, spc.y, spc.z), P.reflect_scale));
-                }
-                // the albedo is loaded after the cones: it is not live across them
-                const float4 ga = __ldg(P.galb + pix);
-                const float as = P.ambient_scale;
-                rgb = mk(rgb.x * (as * ga.x), rgb.y * (as * ga.y), rgb.z * (as * ga.z));
-                if (P.draw_occlusion) rgb = mul(rgb, occ);
-            } else {
-                const float4 ga = __ldg(P.galb + pix);
-                rgb = mk(P.ambient_scale * ga.x, P.ambient_scale * ga.y, P.ambient_scale * ga.z);
+                // (the position is read again rather than kept live across the diffuse cones)
+                if (P.enable_reflections)
+                    spc = trace_cone<MODE, KIND>(P, s_lv, s_cone[1], vp, N, reflected(P, __ldg(P.gpos + pix), N),
+                                                 P.specular_cone, P.max_distance, ns);
             }
-            if (P.enable_postprocess) {
-                const float g = 1.0f / 2.2f;
-                rgb = mk(powf(rgb.x / (rgb.x + 1.0f), g), powf(rgb.y / (rgb.y + 1.0f), g),
-                         powf(rgb.z / (rgb.z + 1.0f), g));
-            }
-            out = make_float4(rgb.x, rgb.y, rgb.z, 1.0f);
+            out = composite(P, pix, irr, spc);
         }
-        if (P.irradiance) P.irradiance[pix] = irr;
-        if (P.specular) P.specular[pix] = spc;
-        if (P.color) P.color[pix] = out;
+        store_pixel(P, pix, irr, spc, out);
     }
-    if (P.samples) {
-        unsigned tot = __reduce_add_sync(0xffffffffu, ns);
-        if (lane == 0 && tot) atomicAdd(P.samples, (unsigned long long)tot);
-    }
+    count_samples(P, ns);
 }
 
 // Peak rate of textureLod samples (the denominator of the cone tracer's
@@ -175,29 +121,29 @@ void launch_sampler_rate(const TraceParams& P, int filter, int blocks, int iters
     note_launches(1);
 }
 
-template <int KIND, class Scenes>
-void launch_trace_kind(const Scenes& S, int filter, long long tiles, cudaStream_t s) {
-    if (filter == VCT_FILTER_HARDWARE)
-        trace_kernel<VCT_FILTER_HARDWARE, KIND><<<(unsigned)tiles, 256, 0, s>>>(S);
-    else if (filter == VCT_FILTER_HARDWARE_LEVELS)
-        trace_kernel<VCT_FILTER_HARDWARE_LEVELS, KIND><<<(unsigned)tiles, 256, 0, s>>>(S);
-    else if (filter == VCT_FILTER_HYBRID)
-        trace_kernel<VCT_FILTER_HYBRID, KIND><<<(unsigned)tiles, 256, 0, s>>>(S);
-    else
-        trace_kernel<VCT_FILTER_SOFTWARE, KIND><<<(unsigned)tiles, 256, 0, s>>>(S);
+namespace {
+
+// Up to this many tiles per SM (two rounds of the CTAs that it holds) a launch
+// takes the split kernel.  1,200 tiles (640 x 480): 139 us against 173 with the
+// software sampler over 64^3, 130 against 138 with the hybrid one over 256^3;
+// 1,450 tiles 127 against 166 and 121 against 110, 2,040 tiles 174 against 174 and
+// 160 against 153.
+constexpr long long kSplitTilesPerSM = 8;
+
+template <class Scenes>
+void launch_trace_set(const Scenes& S, int filter, int kind, long long tiles, int num_sms, cudaStream_t s) {
+    if (tiles <= 0) return;
+    if (tiles <= kSplitTilesPerSM * num_sms) {
+        launch_trace_split(S, filter, kind, tiles, s);
+        return;
+    }
+    with_trace_mode(filter, kind, [&](auto mode, auto cones) {
+        trace_kernel<mode.value, cones.value><<<(unsigned)tiles, 256, 0, s>>>(S);
+    });
     note_launches(1);
 }
 
-template <class Scenes>
-void launch_trace_set(const Scenes& S, int filter, int kind, long long tiles, cudaStream_t s) {
-    if (tiles <= 0) return;
-    if (kind == kConesPlain)
-        launch_trace_kind<kConesPlain>(S, filter, tiles, s);
-    else if (kind == kConesMapped)
-        launch_trace_kind<kConesMapped>(S, filter, tiles, s);
-    else
-        launch_trace_kind<kConesAny>(S, filter, tiles, s);
-}
+}  // namespace
 
 int trace_kind(const TraceParams& P) {
     return cone_kind(P.warp, std::max(P.diffuse.steps, P.specular_cone.steps));
@@ -210,17 +156,18 @@ long long trace_tiles(int width, int height, int tile_w_log2, int tile_h_log2) {
 
 void launch_trace(const TraceParams& P, cudaStream_t s) {
     launch_trace_set(OneScene<TraceParams>{P}, P.filter, trace_kind(P), trace_tiles(P.width, P.height, P.tile_w_log2, P.tile_h_log2),
-                     s);
+                     P.num_sms, s);
 }
 
-void launch_trace_batch(const SceneBatch<TraceParams>& B, int filter, int kind, long long tiles, cudaStream_t s) {
-    launch_trace_set(ManyScenes<TraceParams>{B}, filter, kind, tiles, s);
+void launch_trace_batch(const SceneBatch<TraceParams>& B, int filter, int kind, long long tiles, int num_sms,
+                        cudaStream_t s) {
+    launch_trace_set(ManyScenes<TraceParams>{B}, filter, kind, tiles, num_sms, s);
 }
 
 void launch_trace_views(const ViewSet& V, int filter, cudaStream_t s) {
     int kind = trace_kind(V.p[0]);
     for (int k = 1; k < V.n; ++k) kind = cone_kind_of(kind, trace_kind(V.p[k]));
-    launch_trace_set(FewScenes{V}, filter, kind, V.off[V.n], s);
+    launch_trace_set(FewScenes{V}, filter, kind, V.off[V.n], V.p[0].num_sms, s);
 }
 
 }  // namespace vct

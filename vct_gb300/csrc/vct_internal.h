@@ -268,6 +268,7 @@ struct TraceParams {
     // Pixel tile of one 256-thread CTA (tile_w x tile_h) and of one warp
     // (warp_w x 32/warp_w), as log2.
     int tile_w_log2, tile_h_log2, warp_w_log2;
+    int num_sms;
     WarpDev warp;
 };
 
@@ -369,7 +370,8 @@ inline int cone_kind(const WarpDev& W, int steps) {
 // (of several scenes)
 inline int cone_kind_of(int a, int b) { return a == b ? a : kConesAny; }
 int trace_kind(const TraceParams& P);
-void launch_trace_batch(const SceneBatch<TraceParams>& B, int filter, int kind, long long tiles, cudaStream_t s);
+void launch_trace_batch(const SceneBatch<TraceParams>& B, int filter, int kind, long long tiles, int num_sms,
+                        cudaStream_t s);
 void launch_trace_views(const ViewSet& V, int filter, cudaStream_t s);
 // ------------------------------------------------------------- learned path
 // MLP 42-64-64-64-4: irradiance RGB and the network's estimate of its own
