@@ -39,11 +39,12 @@ def test_cone_steps_match_oracle(steps, warp):
 
 @pytest.mark.parametrize("filt", [L.VCT_FILTER_SOFTWARE, L.VCT_FILTER_HYBRID])
 def test_few_and_many_pixels_give_the_same_bits(filt):
-    """An image of 5,000 tiles (a warp to 32 pixels) and its bands of 80 to 1,120
-    tiles (four warps): every output, and the number of samples."""
+    """An image of 5,000 tiles (a warp to 32 pixels) and its bands of 20 to 1,120
+    tiles (four warps; two steps at a time up to 38 tiles): every output, and
+    the number of samples."""
     import torch
 
-    W, H = 1277, 990
+    W, H = 317, 3990
     sc = scenes.cornell(seed=4, gbuffer=(W, H))
     g = GpuScene(sc)
     ctx = api.Context(api.config_for(sc))
@@ -52,7 +53,7 @@ def test_few_and_many_pixels_give_the_same_bits(filt):
     whole, bands = g.new_outputs(), g.new_outputs()
     ctx.trace(g.gb, sc.eye, api.trace_out(*whole))
     rows = lambda t, r0, r1: t[r0 * W * 4:r1 * W * 4]  # noqa: E731
-    cuts = [0, 1, 17, 241, 465, 689, 913, H]
+    cuts = [0, 1, 17, 49, 273, 1169, 2065, 2961, 3857, H]
     for r0, r1 in zip(cuts, cuts[1:]):
         gb = api.gbuffer(rows(g.gpos, r0, r1), rows(g.gnrm, r0, r1), rows(g.galb, r0, r1), W, r1 - r0)
         ctx.trace(gb, sc.eye, api.trace_out(*(rows(t, r0, r1) for t in bands[:3]), bands[3]))

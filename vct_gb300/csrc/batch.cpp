@@ -42,16 +42,16 @@ size_t up256(size_t b) { return (b + 255) & ~(size_t)255; }
 struct BatchTotals {
     long long tris = 0, texels = 0, bricks = 0, tiles = 0;
     int cones = kConesPlain;  // the kind of the scenes' cone marches
-    // The frame's clears, zeroed by one launch each: before the voxeliser
-    // (statistics, lit masks; carry tables and brick flags of the tessellation
-    // voxeliser; the occupancy masks of the warp maps) at [0, n_pre) of the blob's clear list, and after the resolve
-    // (occupancy masks, for the next frame's accumulation) at [kClearPre n, +n).
+    // The frame's clears, zeroed by one launch before the voxeliser (statistics,
+    // lit masks; carry tables and brick flags of the tessellation voxeliser;
+    // the occupancy masks of the warp maps): [0, n_pre) of the blob's clear list.
     int n_pre = 0;
-    long long max_pre = 0, max_post = 0;
+    long long max_pre = 0;
+    int max_occ = 0;  // words of the largest occupancy mask
     bool any_map = false;  // some scene builds a warp map (VCT_WARP_TEXTURE)
 };
 
-constexpr int kClearPre = 5;  // clear-list entries per scene before the voxeliser (one more after the resolve)
+constexpr int kClearPre = 5;  // clear-list entries per scene
 
 // Validates the scene descriptors and fills the staging blob `h` (parameter
 // structs and prefix tables).  Allocates the tessellation voxeliser's work arrays when the
@@ -118,6 +118,9 @@ vct_status batch_stage(vct_batch* b, const vct_scene_desc* sc, int n, char* h, B
             M.pad[l] = pad ? c->pchain + padded_level_offset(c->dim, l) : nullptr;
         }
         M.first = std::min(4, c->levels - 1);
+        M.occ = c->occ;
+        M.occ_words = (int)((c->nv + 31) / 32);
+        tot.max_occ = std::max(tot.max_occ, M.occ_words);
         TraceParams T;
         if ((s = fill_trace(c, &d.gbuffer, d.eye, &d.out, T)) != VCT_OK) return s;
         apply_tuning(b->tuning, T);
@@ -170,8 +173,6 @@ vct_status batch_stage(vct_batch* b, const vct_scene_desc* sc, int n, char* h, B
             pre(c->carry, (long long)(kCarryBytes / 4));
             pre(c->brick_exact, c->nv / 4096 + 1);
         }
-        clr[kClearPre * n + i] = ClearRange{c->occ, mask_words};
-        tot.max_post = std::max(tot.max_post, mask_words);
     }
     tri_off[n] = tot.tris;
     tex_off[n] = tot.texels;
@@ -253,10 +254,8 @@ vct_status batch_enqueue(vct_batch* b, const char* h, const BatchTotals& tot, cu
                                                   d_tables + 2 * (n + 1), n},
                          tot.bricks, b->ctx[0]->params.voxelize_tesselation != 0, st);
     VCT_CHECK_LAUNCH("batch: resolve");
-    launch_clear_ranges(d_clear + kClearPre * n, n, tot.max_post, st);
-    VCT_CHECK_LAUNCH("batch: clear occupancy");
     launch_mip_tail_batch(SceneBatch<MipLevels>{reinterpret_cast<const MipLevels*>(b->d_blob + b->off_mips), nullptr, n},
-                          st);
+                          tot.max_occ, st);
     VCT_CHECK_LAUNCH("batch: coarse mips");
     if (timed) VCT_CUDA(cudaEventRecord(b->ev[2], st));
     launch_trace_batch(SceneBatch<TraceParams>{reinterpret_cast<const TraceParams*>(b->d_blob + b->off_trace),
@@ -319,7 +318,7 @@ vct_status vct_batch_create(const vct_config* scene_cfg, int32_t n, vct_batch** 
     b->off_tables = off;
     off = up256(off + sizeof(long long) * 4 * (n + 1));
     b->off_clear = off;
-    off = up256(off + sizeof(ClearRange) * (kClearPre + 1) * n);
+    off = up256(off + sizeof(ClearRange) * kClearPre * n);
     b->off_occ = off;
     off = up256(off + sizeof(AccumParams) * n);
     b->off_wmap = off;

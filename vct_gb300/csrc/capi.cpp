@@ -1003,7 +1003,7 @@ vct_status vct_trace(vct_ctx* c, const vct_gbuffer* g, const float eye[3], const
     if (filter_uses_bordered(c->params.trace_filter) && (s = ensure_padded_chain(c, st)) != VCT_OK) return s;
     TraceParams P;
     if ((s = fill_trace(c, g, eye, out, P)) != VCT_OK) return s;
-    launch_trace(P, st);
+    launch_trace(P, false, st);
     VCT_CHECK_LAUNCH("trace");
     if (c->timers_on && c->volume_timed) {  // render stage of a timed vct_frame_volume
         VCT_CUDA(cudaEventRecord(c->ev[4], st));
@@ -1106,18 +1106,17 @@ vct_status frame_volume(vct_ctx* c, const vct_triangles* tris, const vct_light* 
         R.surf[l] = hw ? c->surf[l] : 0;
         R.pad_levels[l] = pad ? c->pchain + padded_level_offset(c->dim, l) : nullptr;
     }
-    launch_resolve(R, st);
+    launch_resolve(R, c->num_sms, st);
     VCT_CHECK_LAUNCH("frame: resolve");
-    VCT_CUDA(cudaMemsetAsync(c->occ, 0, (size_t)((c->nv + 31) / 32) * 4, st));
-    if (c->levels > 5) {
-        MipLevels M = mip_levels(c, c->radiance, c->levels);
-        for (int l = 0; l < c->levels; ++l) {
-            M.surf[l] = hw ? c->surf[l] : 0;
-            M.pad[l] = pad ? c->pchain + padded_level_offset(c->dim, l) : nullptr;
-        }
-        launch_mips(M, 4, false, st);
-        VCT_CHECK_LAUNCH("frame: coarse mips");
+    MipLevels M = mip_levels(c, c->radiance, c->levels);
+    for (int l = 0; l < c->levels; ++l) {
+        M.surf[l] = hw ? c->surf[l] : 0;
+        M.pad[l] = pad ? c->pchain + padded_level_offset(c->dim, l) : nullptr;
     }
+    M.occ = c->occ;
+    M.occ_words = (int)((c->nv + 31) / 32);
+    launch_mips(M, R.mip_levels, false, st);
+    VCT_CHECK_LAUNCH("frame: coarse mips");
     c->tex_ready = hw;
     c->pad_ready = pad;
     c->linear_stale = stale;
@@ -1163,7 +1162,7 @@ vct_status vct_frame(vct_ctx* c, const vct_triangles* tris, const vct_light* lig
     if ((s = frame_volume(c, tris, lights, n, shadow, eye, st)) != VCT_OK) return s;
     TraceParams T;
     if ((s = fill_trace(c, g, eye, out, T)) != VCT_OK) return s;
-    launch_trace(T, st);
+    launch_trace(T, true, st);
     VCT_CHECK_LAUNCH("frame: trace");
     if (c->volume_timed) {
         VCT_CUDA(cudaEventRecord(c->ev[4], st));

@@ -192,7 +192,12 @@ __device__ __forceinline__ void fill_cone(const TraceParams& P, const vct_cone_s
 
 // KIND: no more steps than the table holds and no warp, the
 // same with the warp map, or any.
-template <int MODE, int KIND>
+//
+// PAIRS (for kernels of few warps, with registers to spare; no warp): two
+// steps at a time where both blend two levels, the second one's texels loaded
+// before the first one's colour is added, and dropped where the march ends
+// with the first.
+template <int MODE, int KIND, bool PAIRS = false>
 __device__ __forceinline__ float4 trace_cone(const TraceParams& P, const Level* lv, const ConeTable& T, f3 pos, f3 n,
                                              f3 dir, const vct_cone_settings& c, float maxd, unsigned& ns) {
     dir = fnormalize(dir);
@@ -200,12 +205,24 @@ __device__ __forceinline__ float4 trace_cone(const TraceParams& P, const Level* 
     const f3 start = add(pos, mul(mul(n, c.bias), scale));
     const bool guard = KIND == kConesAny && P.warp.mode != VCT_WARP_NONE;
     rgba2 acc = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};  // colour, and the opacity
-    // One step: false when the cone leaves the volume.
-    auto march = [&](const Lod d) {
+    auto position = [&](const Lod d) {
         const f3 dh = mul(dir, d.h);
-        const f3 sp = mk(fmaf(dh.x, scale, start.x), fmaf(dh.y, scale, start.y), fmaf(dh.z, scale, start.z));
-        // any(notEqual(p, clamp(p, 0, 1))): outside, or NaN
-        if (!(sp.x >= 0.f && sp.y >= 0.f && sp.z >= 0.f && sp.x <= 1.f && sp.y <= 1.f && sp.z <= 1.f)) return false;
+        return mk(fmaf(dh.x, scale, start.x), fmaf(dh.y, scale, start.y), fmaf(dh.z, scale, start.z));
+    };
+    // (not outside, nor NaN)
+    auto inside = [](f3 p) { return p.x >= 0.f && p.y >= 0.f && p.z >= 0.f && p.x <= 1.f && p.y <= 1.f && p.z <= 1.f; };
+    // Adds a sample: false when the cone is full.
+    auto take = [&](const rgba2 s) {
+        ++ns;
+        const float a = 1.0f - acc.ba.y;
+        const float2 aa = make_float2(a, a);
+        acc = {__ffma2_rn(s.rg, aa, acc.rg), __ffma2_rn(s.ba, aa, acc.ba)};
+        return acc.ba.y < 0.95f;
+    };
+    // One step: false when the cone leaves the volume or is full.
+    auto march = [&](const Lod d) {
+        const f3 sp = position(d);
+        if (!inside(sp)) return false;
         f3 wp = sp;
         if (KIND == kConesMapped) {
             // saturated: a sample's footprint has to lie in the bordered level
@@ -214,15 +231,27 @@ __device__ __forceinline__ float4 trace_cone(const TraceParams& P, const Level* 
         } else if (KIND == kConesAny) {
             wp = apply_warp(P.warp, sp);
         }
-        const rgba2 s = sample_lod<MODE>(P, lv, wp, d, guard);
-        ++ns;
-        const float a = 1.0f - acc.ba.y;
-        const float2 aa = make_float2(a, a);
-        acc = {__ffma2_rn(s.rg, aa, acc.rg), __ffma2_rn(s.ba, aa, acc.ba)};
-        return acc.ba.y < 0.95f;
+        return take(sample_lod<MODE>(P, lv, wp, d, guard));
     };
     bool on = true;
     const Lod* step = T.step;
+    if (PAIRS) {
+        static_assert(!PAIRS || (KIND == kConesPlain && MODE == VCT_FILTER_SOFTWARE), "pairs of plain software samples");
+        while (on) {
+            const Lod d0 = step[0];
+            if (d0.l < 0) break;
+            const Lod d1 = step[1];
+            if (d1.l < 0) break;
+            const f3 p0 = position(d0), q = position(d1);
+            if (!inside(p0)) return to_float4(acc);
+            const bool second = inside(q);
+            const f3 p1 = second ? q : p0;
+            const rgba2 a0 = trilinear2(P.pchain, lv[d0.l], p0), a1 = trilinear2(P.pchain, lv[d0.l + 1], p0);
+            const rgba2 b0 = trilinear2(P.pchain, lv[d1.l], p1), b1 = trilinear2(P.pchain, lv[d1.l + 1], p1);
+            on = take(lerp2(a0, a1, d0.f)) && second && take(lerp2(b0, b1, d1.f));
+            step += 2;
+        }
+    }
     for (; on; ++step) {
         const Lod d = *step;
         if (d.l == kLodStop) break;

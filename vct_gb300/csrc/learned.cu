@@ -107,15 +107,6 @@ __device__ __forceinline__ void tc_sync() {
     fence_after_sync();
 }
 
-// Programmatic dependent launch: a kernel launched with launch_overlapped may
-// start once every CTA of the kernel before it has called
-// grid_launch_dependents (or ended), and waits in grid_wait for that kernel's
-// end before it touches anything that other kernels read or write.
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_launch_dependents() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 // Orthonormal basis (T, B) around unit N: Duff et al. 2017, "Building an
 // Orthonormal Basis, Revisited" (JCGT 6(1)), as the cone tracer uses it.
 __device__ __forceinline__ void onb(f3 N, f3& T, f3& B) {
@@ -722,7 +713,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_kernel(const TrainPar
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(w0 + 16u * (uint32_t)i),
                      "l"(P.mlp.img + 16 * (long long)i)
                      : "memory");
-    const float bias = tid < kBiasPad ? P.mlp.bias[tid] : 0.0f;  // stored with the first tile's input
+    const float bias = tid < kBiasPad ? __ldca(P.mlp.bias + tid) : 0.0f;  // stored with the first tile's input
     tc_sync();
     const uint32_t tm = s_tmem, mb = smem_u32(&mbar);
     const uint32_t x0 = w0 + kTrX, h0 = w0 + kTrH, dz0 = w0 + kTrDZ, dy0 = w0 + kTrDY;
@@ -745,7 +736,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_kernel(const TrainPar
     for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const long long idx = t * 128 + row;
         const bool valid = idx < P.n;
-        const long long src = valid ? (P.index ? (long long)P.index[idx] : idx) : 0;
+        const long long src = valid ? (P.index ? (long long)__ldca(P.index + idx) : idx) : 0;
         // ---- input: 24 of the 48 features each
         float target[3] = {0.f, 0.f, 0.f};
         {
@@ -755,13 +746,13 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_kernel(const TrainPar
             for (int i = 0; i < 12; ++i) {
                 f[i] = 0u;
                 if (valid && (i < kMlpIn / 2 - 12 || half == 0)) {
-                    const float2 v = __ldg(rp + i);
+                    const float2 v = __ldca(rp + i);  // (ordinary loads: they stay behind grid_wait)
                     f[i] = bf16x2(v.x, v.y);
                 }
             }
             if (valid && half == 0) {
 #pragma unroll
-                for (int o = 0; o < 3; ++o) target[o] = __ldg(P.targets + src * 3 + o);
+                for (int o = 0; o < 3; ++o) target[o] = __ldca(P.targets + src * 3 + o);
             }
 #pragma unroll
             for (int c = 0; c < 3; ++c)
@@ -1102,27 +1093,11 @@ void launch_trace16_pixels(const LearnedParams& P, cudaStream_t s) {
     note_launches(2);
 }
 
-template <class... K, class... A>
-static void launch_overlapped(void (*kernel)(K...), int grid, int threads, int smem, cudaStream_t s, A... args) {
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = s;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, args...);
-    note_launches(1);
-}
-
 int launch_mlp_train(const TrainParams& P, int num_sms, cudaStream_t s) {
     const long long tiles = (P.n + 127) / 128;
     const int grid = (int)(tiles < num_sms ? tiles : num_sms);
     cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrSmem);
-    launch_overlapped(mlp_train_kernel, grid, kTrThreads, kTrSmem, s, P);
+    launch_overlapped(mlp_train_kernel, dim3((unsigned)grid), kTrThreads, kTrSmem, s, P);
     return grid;
 }
 
@@ -1131,7 +1106,7 @@ void launch_mlp_update(const MlpDev& M, int what, int nparts, int step, float lr
     const bool adam = what == kUpdateAdam;
     const double c1 = adam ? 1.0 / (1.0 - std::pow((double)beta1, (double)step)) : 1.0;
     const double c2 = adam ? 1.0 / (1.0 - std::pow((double)beta2, (double)step)) : 1.0;
-    launch_overlapped(mlp_update_kernel, (kMlpParams + kUpdateParams - 1) / kUpdateParams, kUpdateThreads, 0, s, M, what,
+    launch_overlapped(mlp_update_kernel, dim3((kMlpParams + kUpdateParams - 1) / kUpdateParams), kUpdateThreads, 0, s, M, what,
                       nparts, lr, beta1, beta2, eps, (float)c1, (float)c2, loss_out);
 }
 

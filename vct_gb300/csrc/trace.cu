@@ -46,6 +46,7 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const Scenes S) {
     fill_levels(P, s_lv);
     fill_cone(P, P.diffuse, P.max_distance, s_cone[0], 64);
     fill_cone(P, P.specular_cone, P.max_distance, s_cone[1], 128);
+    grid_wait();  // (the chain's addresses come from the tables behind the barrier)
     __syncthreads();
     unsigned ns = 0;
     if (x < P.width && y < P.height) {
@@ -131,16 +132,15 @@ namespace {
 constexpr long long kSplitTilesPerSM = 8;
 
 template <class Scenes>
-void launch_trace_set(const Scenes& S, int filter, int kind, long long tiles, int num_sms, cudaStream_t s) {
+void launch_trace_set(const Scenes& S, int filter, int kind, long long tiles, int num_sms, bool overlap, cudaStream_t s) {
     if (tiles <= 0) return;
     if (tiles <= kSplitTilesPerSM * num_sms) {
-        launch_trace_split(S, filter, kind, tiles, s);
+        launch_trace_split(S, filter, kind, tiles, num_sms, overlap, s);
         return;
     }
     with_trace_mode(filter, kind, [&](auto mode, auto cones) {
-        trace_kernel<mode.value, cones.value><<<(unsigned)tiles, 256, 0, s>>>(S);
+        launch_tiles(trace_kernel<mode.value, cones.value, Scenes>, S, tiles, overlap, s);
     });
-    note_launches(1);
 }
 
 }  // namespace
@@ -154,20 +154,20 @@ long long trace_tiles(int width, int height, int tile_w_log2, int tile_h_log2) {
     return ((width + tw - 1) / tw) * ((height + th - 1) / th);
 }
 
-void launch_trace(const TraceParams& P, cudaStream_t s) {
+void launch_trace(const TraceParams& P, bool overlap, cudaStream_t s) {
     launch_trace_set(OneScene<TraceParams>{P}, P.filter, trace_kind(P), trace_tiles(P.width, P.height, P.tile_w_log2, P.tile_h_log2),
-                     P.num_sms, s);
+                     P.num_sms, overlap, s);
 }
 
 void launch_trace_batch(const SceneBatch<TraceParams>& B, int filter, int kind, long long tiles, int num_sms,
                         cudaStream_t s) {
-    launch_trace_set(ManyScenes<TraceParams>{B}, filter, kind, tiles, num_sms, s);
+    launch_trace_set(ManyScenes<TraceParams>{B}, filter, kind, tiles, num_sms, false, s);
 }
 
 void launch_trace_views(const ViewSet& V, int filter, cudaStream_t s) {
     int kind = trace_kind(V.p[0]);
     for (int k = 1; k < V.n; ++k) kind = cone_kind_of(kind, trace_kind(V.p[k]));
-    launch_trace_set(FewScenes{V}, filter, kind, V.off[V.n], V.p[0].num_sms, s);
+    launch_trace_set(FewScenes{V}, filter, kind, V.off[V.n], V.p[0].num_sms, false, s);
 }
 
 }  // namespace vct

@@ -12,7 +12,7 @@ namespace vct {
 
 // The split kernel, over the tiles of `S`.
 template <class Scenes>
-void launch_trace_split(const Scenes& S, int filter, int kind, long long tiles, cudaStream_t s);
+void launch_trace_split(const Scenes& S, int filter, int kind, long long tiles, int num_sms, bool overlap, cudaStream_t s);
 
 namespace {
 
@@ -100,6 +100,16 @@ __device__ __forceinline__ void count_samples(const TraceParams& P, unsigned ns)
     if (P.samples) {
         unsigned tot = __reduce_add_sync(0xffffffffu, ns);
         if ((threadIdx.x & 31) == 0 && tot) atomicAdd(P.samples, (unsigned long long)tot);
+    }
+}
+
+template <class Scenes>
+void launch_tiles(void (*kernel)(Scenes), const Scenes& S, long long ctas, bool overlap, cudaStream_t s) {
+    if (overlap) {
+        launch_overlapped(kernel, dim3((unsigned)ctas), 256, 0, s, S);
+    } else {
+        kernel<<<(unsigned)ctas, 256, 0, s>>>(S);
+        note_launches(1);
     }
 }
 

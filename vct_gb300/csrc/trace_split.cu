@@ -17,9 +17,12 @@ namespace {
 // 38), 320 x 180 over 64^3 36 (60), 640 x 360 88 (101).  Where it does, the three
 // warps that wait for the fourth cost more than the shorter chain gains:
 // 1920 x 1080 over 256^3 675 (560).
+//
+// PAIRS: the marches take two steps at a time.  For launches of a CTA to an SM
+// at most, which have the registers: the 47 x 31 pixels' frame 37 us (43).
 constexpr int kSplit = 4;
-template <int MODE, int KIND, class Scenes>
-__global__ void __launch_bounds__(256, 4) trace_split_kernel(const Scenes S) {
+template <int MODE, int KIND, bool PAIRS, class Scenes>
+__global__ void __launch_bounds__(256, PAIRS ? 1 : 4) trace_split_kernel(const Scenes S) {
     long long tile;
     const TraceParams& P = S.get(S.find(blockIdx.x / kSplit, tile));
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -32,6 +35,7 @@ __global__ void __launch_bounds__(256, 4) trace_split_kernel(const Scenes S) {
     fill_levels(P, s_lv);
     fill_cone(P, P.diffuse, P.max_distance, s_cone[0], 64);
     fill_cone(P, P.specular_cone, P.max_distance, s_cone[1], 128);
+    grid_wait();  // (the chain's addresses come from the tables behind the barrier)
     __syncthreads();
     unsigned ns = 0;
     const bool inside = x < P.width && y < P.height;
@@ -47,10 +51,10 @@ __global__ void __launch_bounds__(256, 4) trace_split_kernel(const Scenes S) {
             tangents(N, T, B);
 #pragma unroll 1
             for (int c = 2 * group; c < 2 * group + 2; ++c)
-                s_out[c][slot] = trace_cone<MODE, KIND>(P, s_lv, s_cone[0], vp, N, diffuse_direction(P, c, N, T, B),
+                s_out[c][slot] = trace_cone<MODE, KIND, PAIRS>(P, s_lv, s_cone[0], vp, N, diffuse_direction(P, c, N, T, B),
                                                         P.diffuse, P.max_distance, ns);
         } else if (P.enable_reflections) {
-            s_out[6][slot] = trace_cone<MODE, KIND>(P, s_lv, s_cone[1], vp, N, reflected(P, gp, N), P.specular_cone,
+            s_out[6][slot] = trace_cone<MODE, KIND, PAIRS>(P, s_lv, s_cone[1], vp, N, reflected(P, gp, N), P.specular_cone,
                                                     P.max_distance, ns);
         }
     }
@@ -72,15 +76,18 @@ __global__ void __launch_bounds__(256, 4) trace_split_kernel(const Scenes S) {
 }  // namespace
 
 template <class Scenes>
-void launch_trace_split(const Scenes& S, int filter, int kind, long long tiles, cudaStream_t s) {
+void launch_trace_split(const Scenes& S, int filter, int kind, long long tiles, int num_sms, bool overlap, cudaStream_t s) {
+    if (filter == VCT_FILTER_SOFTWARE && kind == kConesPlain && tiles * kSplit <= num_sms) {
+        launch_tiles(trace_split_kernel<VCT_FILTER_SOFTWARE, kConesPlain, true, Scenes>, S, tiles * kSplit, overlap, s);
+        return;
+    }
     with_trace_mode(filter, kind, [&](auto mode, auto cones) {
-        trace_split_kernel<mode.value, cones.value><<<(unsigned)(tiles * kSplit), 256, 0, s>>>(S);
+        launch_tiles(trace_split_kernel<mode.value, cones.value, false, Scenes>, S, tiles * kSplit, overlap, s);
     });
-    note_launches(1);
 }
 
-template void launch_trace_split(const OneScene<TraceParams>&, int, int, long long, cudaStream_t);
-template void launch_trace_split(const ManyScenes<TraceParams>&, int, int, long long, cudaStream_t);
-template void launch_trace_split(const FewScenes&, int, int, long long, cudaStream_t);
+template void launch_trace_split(const OneScene<TraceParams>&, int, int, long long, int, bool, cudaStream_t);
+template void launch_trace_split(const ManyScenes<TraceParams>&, int, int, long long, int, bool, cudaStream_t);
+template void launch_trace_split(const FewScenes&, int, int, long long, int, bool, cudaStream_t);
 
 }  // namespace vct

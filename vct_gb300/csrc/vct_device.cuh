@@ -301,6 +301,33 @@ struct ManyScenes {
     }
 };
 
+// Programmatic dependent launch: a kernel launched with launch_overlapped may
+// start once every CTA of the kernel before it has called
+// grid_launch_dependents (or ended), and waits in grid_wait for that kernel's
+// end before it touches anything that other kernels read or write.  (Read-only
+// loads may be moved before the wait by the compiler: use ordinary ones behind
+// it, or addresses that a barrier behind it makes known.)
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <class... K, class... A>
+inline void launch_overlapped(void (*kernel)(K...), dim3 grid, int threads, int smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+    note_launches(1);
+}
+
 // The viewpoints of a ViewSet (at most kMaxViews): found by a linear scan.
 struct FewScenes {
     ViewSet v;

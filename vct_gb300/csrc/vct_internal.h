@@ -245,6 +245,8 @@ struct MipLevels {
     int levels;
     int first;  // mip tail: the level the remaining levels are built from
     int copy_first;  // mip_tail: write the sampler's copies of level `first` too
+    uint32_t* occ;   // mip_tail: an occupancy mask to zero, of occ_words words (0: none)
+    int occ_words;
 };
 
 struct TraceParams {
@@ -328,12 +330,14 @@ void launch_tesselate(const AccumParams& P, cudaStream_t s);
 void launch_normalize(const NormalizeParams& P, cudaStream_t s);
 void launch_inject(const InjectParams& P, cudaStream_t s);
 void launch_inject_mark(const InjectParams& P, cudaStream_t s);
-void launch_resolve(const ResolveParams& P, cudaStream_t s);
+void launch_resolve(const ResolveParams& R, int num_sms, cudaStream_t s);
 // Builds levels [first+1, levels) from level `first`.
 // Levels first + 1 .. of a chain, with the sampler's copies (surf, pad) of each;
 // `copy`: of level `first` too.
 void launch_mips(const MipLevels& M, int first, bool copy, cudaStream_t s);
-void launch_trace(const TraceParams& P, cudaStream_t s);
+// `overlap`: the trace follows the volume pass's last kernel in the stream and
+// may start during it; the G-buffer is older than that pass.
+void launch_trace(const TraceParams& P, bool overlap, cudaStream_t s);
 // Sampler throughput microbenchmark (vct_sampler_rate): blocks x 256 threads x iters samples.
 void launch_sampler_rate(const TraceParams& P, int filter, int blocks, int iters, float* sink, cudaStream_t s);
 void launch_shadow_raster(const ShadowRasterParams& P, cudaStream_t s);
@@ -348,7 +352,7 @@ void launch_accumulate_batch(const SceneBatch<AccumParams>& B, long long ntri, l
 void launch_tesselate_batch(const SceneBatch<AccumParams>& B, const VoxWork& W, int num_sms, cudaStream_t s);
 void launch_inject_mark_batch(const SceneBatch<InjectParams>& B, long long ntexels, cudaStream_t s);
 void launch_resolve_batch(const SceneBatch<ResolveParams>& B, long long nbricks, bool exact, cudaStream_t s);
-void launch_mip_tail_batch(const SceneBatch<MipLevels>& B, cudaStream_t s);
+void launch_mip_tail_batch(const SceneBatch<MipLevels>& B, int max_occ_words, cudaStream_t s);
 // A device range of 32-bit words to zero (p 16-byte aligned, as cudaMalloc returns).
 struct ClearRange {
     uint32_t* p;

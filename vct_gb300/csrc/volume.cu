@@ -8,6 +8,8 @@
 // occupied voxels touch their 32-byte accumulator record, and the colour,
 // normal and radiance outputs leave as 32-byte vector stores.  The fused
 // resolve also reduces the brick's first four mip levels in shared memory.
+#include <algorithm>
+
 #include "vct_device.cuh"
 
 namespace vct {
@@ -138,6 +140,7 @@ __device__ __forceinline__ void reduce_level(const uint2* src, uint2* dst, int S
 // levels shrink (512, 64, 8, 1 outputs): after the first level only two warps
 // continue (synchronised by a 64-thread named barrier), after the second one.
 // Threads that are no longer needed return, so call this last.
+template <int T = kThreads>
 __device__ __forceinline__ void brick_mips(uint2* s0, uint2* s1, int nlev, uint2* const* gdst,
                                            const cudaSurfaceObject_t* surf, float4* const* pdst, int S0, int bx, int by,
                                            int bz) {
@@ -147,10 +150,10 @@ __device__ __forceinline__ void brick_mips(uint2* s0, uint2* s1, int nlev, uint2
     for (int l = 1; l <= nlev; ++l) {
         const int sub = side / 2;
         const int nout = sub * sub * sub;
-        const int nthr = nout >= kThreads ? kThreads : (nout >= 64 ? 64 : 32);
+        const int nthr = nout >= T ? T : (nout >= 64 ? 64 : 32);
         if ((int)threadIdx.x >= nthr) return;
         reduce_level(a, b, side, gdst[l], surf[l], pdst[l], S0 >> l, bx * sub, by * sub, bz * sub, nthr);
-        if (nthr == kThreads)
+        if (nthr == T)
             __syncthreads();
         else if (nthr == 64)
             asm volatile("bar.sync 1, 64;" ::: "memory");
@@ -183,8 +186,8 @@ __device__ __forceinline__ void brick_mips(uint2* s0, uint2* s1, int nlev, uint2
 // the rasterising voxeliser).  EXACT = true: only the flagged bricks, whose
 // rewritten records hold their sums' float values (bit 31 of the count);
 // a separate instantiation so that the common path keeps its registers.
-template <bool FUSED, bool EXACT, class Scenes>
-__global__ void __launch_bounds__(kThreads, 3) resolve_kernel(const Scenes S) {
+template <bool FUSED, bool EXACT, class Scenes, int T = kThreads>
+__global__ void __launch_bounds__(T, T == kThreads ? 3 : 1) resolve_kernel(const Scenes S) {
     __shared__ uint2 s0[FUSED ? kBrickVox : 1];
     __shared__ uint2 s1[FUSED ? kBrickVox / 8 : 1];
     long long brick;
@@ -197,8 +200,8 @@ __global__ void __launch_bounds__(kThreads, 3) resolve_kernel(const Scenes S) {
     const f3 lvox = FUSED ? light_voxel_index(R.warp, R.light_vox, R.light_tc, R.light_pos, N) : R.light_vox;
     uint32_t uniq = 0, mx = 0, flags = 0;
 #pragma unroll 1
-    for (int it = 0; it < kBrickVox / 4 / kThreads; ++it) {
-        const int q = threadIdx.x + it * kThreads;
+    for (int it = 0; it < kBrickVox / 4 / T; ++it) {
+        const int q = threadIdx.x + it * T;
         const int lx = (q & 3) * 4, ly = (q >> 2) & 15, lz = q >> 6;
         const int x = bx * kBrick + lx, y = by * kBrick + ly, z = bz * kBrick + lz;
         const long long v0 = ((long long)z * N + y) * N + x;
@@ -289,7 +292,7 @@ __global__ void __launch_bounds__(kThreads, 3) resolve_kernel(const Scenes S) {
         // The sampler's copies of level 0 from the brick in shared memory: each
         // half-warp writes one row of 16 texels (256 bytes of the bordered
         // copy, 128 of the texture).
-        for (int t = threadIdx.x; t < kBrickVox; t += kThreads) {
+        for (int t = threadIdx.x; t < kBrickVox; t += T) {
             const int x = bx * kBrick + (t & 15), y = by * kBrick + ((t >> 4) & 15), z = bz * kBrick + (t >> 8);
             const uint2 v = s0[t];
             if (R.pad_levels[0]) R.pad_levels[0][pad_index(x, y, z, N)] = unpack_h4(v);
@@ -298,7 +301,7 @@ __global__ void __launch_bounds__(kThreads, 3) resolve_kernel(const Scenes S) {
     }
     block_stats(P.stats, uniq, mx, flags);
     if (FUSED) {
-        brick_mips(s0, s1, R.mip_levels, R.radiance_levels, R.surf, R.pad_levels, N, bx, by, bz);
+        brick_mips<T>(s0, s1, R.mip_levels, R.radiance_levels, R.surf, R.pad_levels, N, bx, by, bz);
     }
 }
 
@@ -421,14 +424,25 @@ __global__ void __launch_bounds__(kThreads) mip_brick_kernel(const MipLevels M, 
     brick_mips(s0, s1, nlev, M.level + first, M.surf + first, M.pad + first, S, bx, by, bz);
 }
 
-// Small levels (side <= 16): one CTA per scene builds every level after
-// M.first.
+// Small levels (side <= 16): the first CTA of a scene builds every level after
+// M.first.  The others zero the occupancy mask that the resolve before has
+// read, 8192 words each (a memset between the resolve and the trace is 3 us of
+// a frame, mostly waiting).
+constexpr int kTailWords = 8192;
 template <class Scenes>
 __global__ void __launch_bounds__(kThreads) mip_tail_kernel(const Scenes SS) {
     __shared__ uint2 s0[kBrickVox];
     __shared__ uint2 s1[kBrickVox / 8];
-    const MipLevels& M = SS.get(blockIdx.x);
+    const MipLevels& M = SS.get(blockIdx.y);
     const int first = M.first;
+    grid_wait();
+    if (blockIdx.x > 0) {
+        // (at least 128 words, a multiple of four)
+        const int w0 = ((int)blockIdx.x - 1) * kTailWords, w1 = min(w0 + kTailWords, M.occ_words);
+        for (int w = w0 + 4 * (int)threadIdx.x; w < w1; w += 4 * kThreads)
+            *reinterpret_cast<uint4*>(M.occ + w) = make_uint4(0u, 0u, 0u, 0u);
+        return;
+    }
     // Chains of at most five levels are complete after the resolve; the tail
     // (side of level `first` <= 16) only exists for longer ones.
     if (first + 1 >= M.levels) return;
@@ -683,9 +697,15 @@ void launch_inject_mark(const InjectParams& P, cudaStream_t s) {
     note_launches(1);
 }
 
-void launch_resolve(const ResolveParams& R, cudaStream_t s) {
+void launch_resolve(const ResolveParams& R, int num_sms, cudaStream_t s) {
     const int bpa = R.norm.dim / kBrick;
-    resolve_kernel<true, false><<<bpa * bpa * bpa, kThreads, 0, s>>>(OneScene<ResolveParams>{R});
+    // A brick to an SM or less: 512 threads, so that each waits for two rounds of
+    // records instead of four (a 16^3 frame 45.6 -> 43.6 us, a 64^3 one 126 -> 124;
+    // 1024 threads, held to 64 registers, 45.6 and 125.7).
+    if (bpa * bpa * bpa <= num_sms)
+        resolve_kernel<true, false, OneScene<ResolveParams>, 512><<<bpa * bpa * bpa, 512, 0, s>>>(OneScene<ResolveParams>{R});
+    else
+        resolve_kernel<true, false><<<bpa * bpa * bpa, kThreads, 0, s>>>(OneScene<ResolveParams>{R});
     if (R.norm.brick_exact) {
         resolve_kernel<true, true><<<bpa * bpa * bpa, kThreads, 0, s>>>(OneScene<ResolveParams>{R});
         note_launches(1);
@@ -693,26 +713,24 @@ void launch_resolve(const ResolveParams& R, cudaStream_t s) {
     note_launches(1);
 }
 
+static void launch_mip_tail(const MipLevels& M, cudaStream_t s) {
+    const unsigned zeros = (unsigned)((M.occ_words + kTailWords - 1) / kTailWords);
+    launch_overlapped(mip_tail_kernel<OneScene<MipLevels>>, dim3(1u + zeros), kThreads, 0, s, OneScene<MipLevels>{M});
+}
+
 void launch_mips(const MipLevels& M, int first, bool copy, cudaStream_t s) {
     int l = first;
-    while (l + 1 < M.levels) {
-        int S = M.dim >> l;
-        if (S > kBrick) {
-            int nlev = M.levels - 1 - l;
-            if (nlev > 4) nlev = 4;
-            int bpa = S / kBrick;
-            mip_brick_kernel<<<bpa * bpa * bpa, kThreads, 0, s>>>(M, l, nlev, copy && l == first ? 1 : 0);
-            note_launches(1);
-            l += nlev;
-        } else {
-            MipLevels T = M;
-            T.first = l;
-            T.copy_first = copy && l == first ? 1 : 0;
-            mip_tail_kernel<<<1, kThreads, 0, s>>>(OneScene<MipLevels>{T});
-            note_launches(1);
-            break;
-        }
+    while (l + 1 < M.levels && (M.dim >> l) > kBrick) {
+        const int S = M.dim >> l, nlev = std::min(M.levels - 1 - l, 4), bpa = S / kBrick;
+        mip_brick_kernel<<<bpa * bpa * bpa, kThreads, 0, s>>>(M, l, nlev, copy && l == first ? 1 : 0);
+        note_launches(1);
+        l += nlev;
     }
+    if (l + 1 >= M.levels && M.occ_words == 0) return;
+    MipLevels T = M;
+    T.first = l;
+    T.copy_first = copy && l == first ? 1 : 0;
+    launch_mip_tail(T, s);
 }
 
 void launch_inject_mark_batch(const SceneBatch<InjectParams>& B, long long ntexels, cudaStream_t s) {
@@ -731,8 +749,9 @@ void launch_resolve_batch(const SceneBatch<ResolveParams>& B, long long nbricks,
     note_launches(1);
 }
 
-void launch_mip_tail_batch(const SceneBatch<MipLevels>& B, cudaStream_t s) {
-    mip_tail_kernel<<<B.n, kThreads, 0, s>>>(ManyScenes<MipLevels>{B});
+void launch_mip_tail_batch(const SceneBatch<MipLevels>& B, int max_occ_words, cudaStream_t s) {
+    const dim3 grid(1u + (unsigned)((max_occ_words + kTailWords - 1) / kTailWords), (unsigned)B.n);
+    mip_tail_kernel<<<grid, kThreads, 0, s>>>(ManyScenes<MipLevels>{B});
     note_launches(1);
 }
 
