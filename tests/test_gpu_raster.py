@@ -56,6 +56,18 @@ def test_depth_raster_matches_oracle(kind, n):
         assert np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("width", [127, 128, 129, 8192, 16384])
+@pytest.mark.parametrize("kind", ["slivers", "sizes", "far"])
+def test_long_lines_match_oracle(kind, width):
+    """Lines around the length of a piece and beyond 64 of them."""
+    sc = dataclasses.replace(_scene(kind, 67, 16), gbuffer_size=(width, 5), shadow_size=(width, 7))
+    g = GpuScene(sc)
+    sm, gbuf = g.host_inputs()
+    assert np.array_equal(sm, O.render_shadowmap(sc))
+    for got, want in zip(gbuf, O.render_gbuffer(sc)):
+        assert np.array_equal(got, want)
+
+
 @pytest.mark.parametrize("n,dim", [(1, 16), (31, 64), (257, 32), (1500, 128), (300, 256)])
 @pytest.mark.parametrize("kind", ["slivers", "sizes", "far"])
 def test_voxel_raster_matches_oracle(kind, n, dim):

@@ -20,16 +20,21 @@ using namespace lines;
 // One kernel for both passes, over the covered runs of the triangles' lines
 // (lines.cuh).
 //
-// What bounds it is issue (72% of peak; ALU pipe 50%) at some 60 instructions
-// per 32 pixels and 300 per 32 lines.  262,144 triangles into a 2048^2 shadow
-// map (71 M pixels, 3 M lines): 0.35 ms; into a 1920x1080 G-buffer (33 M
-// pixels, 5.5 M lines): 0.27 ms; 1,290 triangles, ten of them walls of a
-// 500^2 / 641x359 image: 0.022 / 0.019 ms.  The form before, a warp per
-// triangle over its whole bounding box with 64-bit divisions and conversions
-// per pixel, took 1.90, 11.1, 0.65 and 1.03 ms: it left one warp with a whole
-// wall, and the columns' slivers with boxes of thousands of pixels around a
-// few hundred.  24 CTAs per SM: with 8, 0.37 and 0.29 ms; grabs of 4 steps 0.40
-// and 0.31, of 16 no faster than of 8.
+// What bounds it is issue (70% of peak, 50% of the ALU pipe) at some 60
+// instructions per 32 pixels and 250 per 32 lines.  262,144 triangles into a
+// 2048^2 shadow map (71 M pixels, 3 M lines): 0.33 ms; into a 1920x1080
+// G-buffer (33 M pixels, 5.5 M lines): 0.24 ms; 1,290 triangles, ten of them
+// walls of a 500^2 / 641x359 image: 0.015 / 0.016 ms.  A warp per triangle over
+// its whole bounding box, with 64-bit divisions and conversions per pixel, took
+// 1.90, 11.1, 0.65 and 1.03 ms: it left one warp with a whole wall, and the
+// columns' slivers with boxes of thousands of pixels around a few hundred.
+// The CTA walk took 0.35, 0.27, 0.022 and 0.020 ms: at 60 instructions a step
+// its warps spend a sixth to a quarter of their time at barriers.  Groups of
+// 96 lines 0.34 and 0.24 ms (four views of 650,000 triangles 0.79 ms; 0.74 with
+// 64, 0.77 with 32), long lines in pieces by the box's width instead of the
+// line's 0.33 and 0.50, one step at a time 0.39 and 0.25, three 0.33 and 0.28.
+// Runs of 8 neighbouring triangles to a CTA 0.34, 0.24, 0.017 and 0.021, of 2
+// 0.33, 0.25, 0.013 and 0.017.
 
 // Keys of two steps at a time: their loads are in flight together.  The keys
 // only fall during the pass, so one that is not below the key it sees needs no
@@ -57,35 +62,36 @@ struct DepthSink {
     }
 };
 
-// `Pass`: setup(t, part, rt, z) sets up part `part` of triangle t (false:
-// nothing to draw), parts(t) counts them (at most kMaxParts), place gives a
-// covered pixel's key and where it goes.
+// `Pass`: setup(t, part, rt, z, more) sets up part `part` of triangle t (false:
+// nothing to draw; more: there is another part, of kMaxParts at most), place
+// gives a covered pixel's key and where it goes.
 template <class Pass>
 __global__ void __launch_bounds__(kLineThreads, 4) depth_raster_kernel(const Pass P, long long ntri) {
-    __shared__ LineShared S;
-    const long long t = my_triangle<8>();
+    __shared__ WarpLines S;
+    const long long t = my_triangle<4>();
+    bool more = t < ntri;
     const DepthSink<Pass> sink = {P};
     for (int part = 0; part < Pass::kMaxParts; ++part) {
-        if (part > 0 && !__syncthreads_or(t < ntri && P.parts(t) > part)) return;
+        if (part > 0 && !__syncthreads_or(more)) return;
         int lines = 0;
         bool big = false;
-        if (t < ntri) {
+        if (more) {
             RasterTri rt;
             float z[3];
-            if (P.setup(t, part, rt, z)) {
-                lines = store_rec(S.recs[threadIdx.x], rt, z, (int)t);
+            if (P.setup(t, part, rt, z, more)) {
+                lines = store_rec<true>(S.recs[threadIdx.x], rt, z, (int)t);
                 big = rt.area >= kBigArea;
             }
         }
-        walk_all<kDepthSteps, 8>(S, lines, big, sink);
+        walk_all<kDepthSteps>(S, lines, big, sink);
     }
 }
 
 struct ShadowPass : ShadowRasterParams {
     using Key = unsigned int;
     static constexpr int kMaxParts = 1;
-    __device__ __forceinline__ int parts(long long) const { return 1; }
-    __device__ __forceinline__ bool setup(long long t, int, RasterTri& rt, float d[3]) const {
+    __device__ __forceinline__ bool setup(long long t, int, RasterTri& rt, float d[3], bool& more) const {
+        more = false;
         const float* Pp = pos + t * 9;
         float wx[3], wy[3];
 #pragma unroll
@@ -119,15 +125,8 @@ struct GbufferPass : GbufferRasterParams {
         for (int k = 0; k < 3; ++k) mat_vec(vp, Pp[3 * k], Pp[3 * k + 1], Pp[3 * k + 2], 1.0f, cv[k]);
     }
     // Two vertices in front of the near plane leave a quadrilateral: two parts.
-    __device__ __forceinline__ int parts(long long t) const {
-        float cv[3][4];
-        clip_space(t, cv);
-        int in = 0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) in += cv[k][2] + cv[k][3] >= 0.0f ? 1 : 0;
-        return in == 2 ? 2 : in == 0 ? 0 : 1;
-    }
-    __device__ __forceinline__ bool setup(long long t, int part, RasterTri& rt, float d[3]) const {
+    __device__ __forceinline__ bool setup(long long t, int part, RasterTri& rt, float d[3], bool& more) const {
+        more = false;
         float cv[3][4];
         clip_space(t, cv);
         bool all_in = true;
@@ -151,6 +150,7 @@ struct GbufferPass : GbufferRasterParams {
                     ++np;
                 }
             }
+            more = np > part + 3;
             if (np < part + 3) return false;
             for (int c = 0; c < 4; ++c) {
                 const float v1 = poly[part + 1][c], v2 = poly[part + 2][c];

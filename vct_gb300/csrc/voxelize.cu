@@ -237,7 +237,7 @@ struct VoxelSink {
 template <class Scenes>
 __global__ void __launch_bounds__(kLineThreads, kRasterBlocksPerSM)
     voxelize_raster_kernel(const Scenes S, long long ntri) {
-    __shared__ LineShared L;
+    __shared__ CtaLines L;
     __shared__ RecordStage stages[kWarps];
     __shared__ unsigned frag_count[kMaxBatchScenes];
     const int nscenes = S.count();
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(kLineThreads, kRasterBlocksPerSM)
         int axis;
         if (project_triangle(S.get(scene), t, rt, z, axis)) {
             TriRec& r = L.recs[threadIdx.x];
-            lines = store_rec(r, rt, z, (int)t);
+            lines = store_rec<false>(r, rt, z, (int)t);
             r.user[0] = (uint32_t)axis;
             r.user[1] = (uint32_t)scene;
             big = rt.area >= kBigArea;
