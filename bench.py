@@ -1072,16 +1072,14 @@ def run_dynamic(args, rank, world):
 # stage, from one ncu capture of the large frame (`bench.py --profile-frames 3`, default
 # launch shapes): accumulate = setup + raster, resolve+mips = resolve + tail; only for the
 # default workload, and only while the frame kernels' sources hash to NCU_CAPTURE_DIGEST.
-NCU_CAPTURE_DIGEST = "438e8eac75de4cad"
+NCU_CAPTURE_DIGEST = "171acd0f9e50d4fb"
 NCU_CAPTURE_SAMPLER = "hybrid"
-NCU_TRAFFIC = {"accumulate": 18.891e6 + 262.704e6 + 161.262e6, "resolve+mips": 258.924e6 + 835.439e6 + 0.047e6,
-               "inject_mark": 18.258e6 + 0.023e6, "trace": 89.188e6 + 12.723e6}
-# Issue-side figures of the cone tracer (hybrid sampler) from its full capture of the same
-# command: it is bound by issue and load latency at its occupancy, not HBM.  (Captured
-# before the accumulator records moved to 2 x 2 slots; the tracer reads no records and its
-# code is unchanged.)
-NCU_TRACE_ISSUE = {"sm_throughput_frac": 0.633, "fma_pipe_frac": 0.437, "l1_hit_rate": 0.971,
-                   "l1_lsu_data_pipe_frac": 0.661, "l1_tex_data_pipe_frac": 0.240}
+NCU_TRAFFIC = {"accumulate": 295.806e6 + 161.277e6, "resolve+mips": 258.935e6 + 839.243e6 + 0.056e6,
+               "inject_mark": 18.255e6 + 0.026e6, "trace": 89.210e6 + 13.008e6}
+# L1- and issue-side figures of the cone tracer (hybrid sampler) from its full capture of the
+# same command: it is bound by the L1 data pipe, not HBM.
+NCU_TRACE_ISSUE = {"sm_throughput_frac": 0.557, "fma_pipe_frac": 0.500, "l1_hit_rate": 0.971,
+                   "l1_lsu_data_pipe_frac": 0.779, "l1_tex_data_pipe_frac": 0.274}
 
 
 def load_peaks() -> dict:

@@ -4,7 +4,6 @@
 // reference, the learned trace with its per-tile or per-pixel fallback).
 #include <cmath>
 #include <cstring>
-#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -19,8 +18,7 @@ struct vct_mlp {
     MlpDev dev = {};
     uint32_t* status = nullptr;  // the word behind the parameters
     int step = 0;
-    std::mutex staging_lock;
-    float* staging = nullptr;  // pinned: the parameters and the status word
+    char* memory = nullptr;  // every device buffer of the network
 };
 
 namespace {
@@ -211,30 +209,38 @@ vct_status vct_mlp_create(int32_t device, uint64_t seed, vct_mlp** out) {
     if (!m) return fail(VCT_ERR_OUT_OF_MEMORY, "host allocation failed");
     m->device = device;
     cudaDeviceGetAttribute(&m->num_sms, cudaDevAttrMultiProcessorCount, device);
+    // one allocation (a dozen small ones take longer than the rest of the call);
+    // all but the parts, which a training pass writes before it reads them, zeroed
     const size_t pf = sizeof(float) * kMlpParams;
     struct {
         void** p;
         size_t bytes;
-    } allocs[] = {{(void**)&m->dev.params, pf + sizeof(uint32_t)}, {(void**)&m->dev.grad, pf},
-                  {(void**)&m->dev.parts, sizeof(float) * kPartStride * (size_t)m->num_sms},
-                  {(void**)&m->dev.m, pf},                {(void**)&m->dev.v, pf},
-                  {(void**)&m->dev.img, (size_t)kImgAll}, {(void**)&m->dev.bias, sizeof(float) * kBiasPad},
-                  {(void**)&m->dev.loss, sizeof(float)}};
-    for (auto& a : allocs) {
-        cudaError_t e = cudaMalloc(a.p, a.bytes);
-        if (e == cudaSuccess) e = cudaMemset(*a.p, 0, a.bytes);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            vct_mlp_destroy(m);
-            return fail(VCT_ERR_OUT_OF_MEMORY, std::string("mlp buffers: ") + cudaGetErrorString(e));
-        }
+    } buffers[] = {{(void**)&m->dev.params, pf + sizeof(uint32_t)},
+                   {(void**)&m->dev.grad, pf},
+                   {(void**)&m->dev.m, pf},
+                   {(void**)&m->dev.v, pf},
+                   {(void**)&m->dev.img, (size_t)kImgAll},
+                   {(void**)&m->dev.bias, sizeof(float) * kBiasPad},
+                   {(void**)&m->dev.loss, sizeof(float)},
+                   {(void**)&m->dev.parts, sizeof(float) * kPartStride * (size_t)m->num_sms}};
+    size_t total = 0, zeroed = 0;
+    for (auto& x : buffers) {
+        zeroed = total;
+        total += (x.bytes + 255) & ~(size_t)255;
     }
-    m->status = reinterpret_cast<uint32_t*>(m->dev.params + kMlpParams);
-    if (cudaMallocHost(reinterpret_cast<void**>(&m->staging), pf + sizeof(uint32_t)) != cudaSuccess) {
+    cudaError_t e = cudaMalloc(&m->memory, total);
+    if (e == cudaSuccess) e = cudaMemset(m->memory, 0, zeroed);
+    if (e != cudaSuccess) {
         cudaGetLastError();
         vct_mlp_destroy(m);
-        return fail(VCT_ERR_OUT_OF_MEMORY, "mlp buffers: pinned host memory");
+        return fail(VCT_ERR_OUT_OF_MEMORY, std::string("mlp buffers: ") + cudaGetErrorString(e));
     }
+    size_t at = 0;
+    for (auto& x : buffers) {
+        *x.p = m->memory + at;
+        at += (x.bytes + 255) & ~(size_t)255;
+    }
+    m->status = reinterpret_cast<uint32_t*>(m->dev.params + kMlpParams);
     std::vector<float> p;
     init_params(seed, p);
     vct_status s = upload_params(m, p.data(), nullptr);
@@ -251,10 +257,7 @@ vct_status vct_mlp_create(int32_t device, uint64_t seed, vct_mlp** out) {
 vct_status vct_mlp_destroy(vct_mlp* m) {
     if (!m) return VCT_OK;
     DeviceScope ds(m->device);
-    void* ptrs[] = {m->dev.params, m->dev.grad, m->dev.parts, m->dev.m, m->dev.v, m->dev.img, m->dev.bias, m->dev.loss};
-    for (void* p : ptrs)
-        if (p) cudaFree(p);
-    if (m->staging) cudaFreeHost(m->staging);
+    if (m->memory) cudaFree(m->memory);
     delete m;
     return VCT_OK;
 }
@@ -279,12 +282,12 @@ vct_status vct_mlp_get_params(vct_mlp* m, float* host, int64_t count, void* stre
     VCT_CUDA(ds.err);
     cudaStream_t st = as_stream(stream);
     // one copy brings the parameters and the status word behind them
-    std::lock_guard<std::mutex> hold(m->staging_lock);
-    VCT_CUDA(cudaMemcpyAsync(m->staging, m->dev.params, sizeof(float) * (kMlpParams + 1), cudaMemcpyDeviceToHost, st));
+    std::vector<float> got(kMlpParams + 1);
+    VCT_CUDA(cudaMemcpyAsync(got.data(), m->dev.params, sizeof(float) * got.size(), cudaMemcpyDeviceToHost, st));
     VCT_CUDA(cudaStreamSynchronize(st));
-    std::memcpy(host, m->staging, sizeof(float) * kMlpParams);
+    std::memcpy(host, got.data(), sizeof(float) * kMlpParams);
     uint32_t h;
-    std::memcpy(&h, m->staging + kMlpParams, sizeof h);
+    std::memcpy(&h, got.data() + kMlpParams, sizeof h);
     return h ? check_status(m, st) : VCT_OK;
 }
 
