@@ -1070,7 +1070,7 @@ def run_dynamic(args, rank, world):
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per launch of each frame
 # stage, from one ncu capture of the large frame (`bench.py --profile-frames 3`, default
-# launch shapes): accumulate = setup + raster, resolve+mips = resolve + tail; only for the
+# launch shapes): accumulate = the raster, resolve+mips = resolve + tail; only for the
 # default workload, and only while the frame kernels' sources hash to NCU_CAPTURE_DIGEST.
 NCU_CAPTURE_DIGEST = "171acd0f9e50d4fb"
 NCU_CAPTURE_SAMPLER = "hybrid"
