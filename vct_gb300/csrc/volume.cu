@@ -112,6 +112,19 @@ __device__ __forceinline__ long long pad_index(int x, int y, int z, int S) {
     return ((long long)(z + 1) * P + (y + 1)) * P + (x + 1);
 }
 
+// Two neighbouring texels of a row, the first at an even x: a whole sector of
+// the bordered copy (a level's interior rows start on sectors) and half of one
+// of the texture's.
+__device__ __forceinline__ void copy2(uint4 v, int x, int y, int z, int S, float4* pad, cudaSurfaceObject_t surf) {
+    if (pad) {
+        const float4 a = unpack_h4(make_uint2(v.x, v.y)), b = unpack_h4(make_uint2(v.z, v.w));
+        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(pad + pad_index(x, y, z, S)), "f"(a.x),
+                     "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                     : "memory");
+    }
+    if (surf) surf3Dwrite(v, surf, x * (int)sizeof(uint2), y, z);
+}
+
 // Reduces a cube of side S (in shared memory, x fastest) into side S/2 with
 // threads [0, nthr), writing the result to shared memory, to the linear level
 // and, when given, to the texture-unit copy (`surf`) and the bordered fp32
@@ -188,7 +201,7 @@ __device__ __forceinline__ void brick_mips(uint2* s0, uint2* s1, int nlev, uint2
 // a separate instantiation so that the common path keeps its registers.
 template <bool FUSED, bool EXACT, class Scenes, int T = kThreads>
 __global__ void __launch_bounds__(T, T == kThreads ? 3 : 1) resolve_kernel(const Scenes S) {
-    __shared__ uint2 s0[FUSED ? kBrickVox : 1];
+    __shared__ __align__(16) uint2 s0[FUSED ? kBrickVox : 2];
     __shared__ uint2 s1[FUSED ? kBrickVox / 8 : 1];
     long long brick;
     const ResolveParams& R = S.get(S.find(blockIdx.x, brick));
@@ -289,15 +302,12 @@ __global__ void __launch_bounds__(T, T == kThreads ? 3 : 1) resolve_kernel(const
     }
     if (FUSED) __syncthreads();
     if (FUSED && (R.pad_levels[0] || R.surf[0])) {
-        // The sampler's copies of level 0 from the brick in shared memory: each
-        // half-warp writes one row of 16 texels (256 bytes of the bordered
+        // The sampler's copies of level 0 from the brick in shared memory: a
+        // quarter-warp writes one row of 16 texels (256 bytes of the bordered
         // copy, 128 of the texture).
-        for (int t = threadIdx.x; t < kBrickVox; t += T) {
-            const int x = bx * kBrick + (t & 15), y = by * kBrick + ((t >> 4) & 15), z = bz * kBrick + (t >> 8);
-            const uint2 v = s0[t];
-            if (R.pad_levels[0]) R.pad_levels[0][pad_index(x, y, z, N)] = unpack_h4(v);
-            if (R.surf[0]) surf3Dwrite(v, R.surf[0], x * (int)sizeof(uint2), y, z);
-        }
+        for (int t = threadIdx.x; t < kBrickVox / 2; t += T)
+            copy2(reinterpret_cast<const uint4*>(s0)[t], bx * kBrick + (t & 7) * 2, by * kBrick + ((t >> 3) & 15),
+                  bz * kBrick + (t >> 7), N, R.pad_levels[0], R.surf[0]);
     }
     block_stats(P.stats, uniq, mx, flags);
     if (FUSED) {
@@ -400,10 +410,12 @@ __global__ void __launch_bounds__(kThreads) inject_mark_kernel(const Scenes S, l
 // written beside them), each half-warp a row.
 //
 // What bounds it: DRAM.  The 256^3 chain with its bordered copy (459 MB, 0.068 ms
-// at the copy rate) takes 0.100 ms; as a pass for the levels and one a level for
-// the copy it took 0.179 (612 MB, ten launches).
+// at the copy rate) takes 0.086 ms; a texel a thread 0.100 with streaming loads
+// (0.095 two texels: they give up the part of the level that is still in the
+// L2); as a pass for the levels and one a level for the copy it took 0.179
+// (612 MB, ten launches).
 __global__ void __launch_bounds__(kThreads) mip_brick_kernel(const MipLevels M, int first, int nlev, int copy) {
-    __shared__ uint2 s0[kBrickVox];
+    __shared__ __align__(16) uint2 s0[kBrickVox];
     __shared__ uint2 s1[kBrickVox / 8];
     const int S = M.dim >> first;
     const int bpa = S / kBrick;
@@ -412,13 +424,12 @@ __global__ void __launch_bounds__(kThreads) mip_brick_kernel(const MipLevels M, 
     float4* pad = copy ? M.pad[first] : nullptr;
     const cudaSurfaceObject_t surf = copy ? M.surf[first] : 0;
 #pragma unroll 4
-    for (int i = 0; i < kBrickVox / kThreads; ++i) {
+    for (int i = 0; i < kBrickVox / 2 / kThreads; ++i) {
         const int t = threadIdx.x + i * kThreads;
-        const int x = bx * kBrick + (t & 15), y = by * kBrick + ((t >> 4) & 15), z = bz * kBrick + (t >> 8);
-        const uint2 v = __ldcs(src + ((long long)z * S + y) * S + x);
-        s0[t] = v;
-        if (pad) pad[pad_index(x, y, z, S)] = unpack_h4(v);
-        if (surf) surf3Dwrite(v, surf, x * (int)sizeof(uint2), y, z);
+        const int x = bx * kBrick + (t & 7) * 2, y = by * kBrick + ((t >> 3) & 15), z = bz * kBrick + (t >> 7);
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(src + ((long long)z * S + y) * S + x));
+        reinterpret_cast<uint4*>(s0)[t] = v;
+        copy2(v, x, y, z, S, pad, surf);
     }
     __syncthreads();
     brick_mips(s0, s1, nlev, M.level + first, M.surf + first, M.pad + first, S, bx, by, bz);
