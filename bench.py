@@ -1072,10 +1072,10 @@ def run_dynamic(args, rank, world):
 # stage, from one ncu capture of the large frame (`bench.py --profile-frames 3`, default
 # launch shapes): accumulate = the raster, resolve+mips = resolve + tail; only for the
 # default workload, and only while the frame kernels' sources hash to NCU_CAPTURE_DIGEST.
-NCU_CAPTURE_DIGEST = "6b55b392b76f616c"
+NCU_CAPTURE_DIGEST = "9fb4aebac12fe4d3"
 NCU_CAPTURE_SAMPLER = "hybrid"
-NCU_TRAFFIC = {"accumulate": 295.682e6 + 161.174e6, "resolve+mips": 258.922e6 + 838.428e6 + 0.057e6,
-               "inject_mark": 18.260e6 + 0.021e6, "trace": 89.218e6 + 12.918e6}
+NCU_TRAFFIC = {"accumulate": 295.790e6 + 161.190e6, "resolve+mips": 258.984e6 + 838.729e6 + 0.057e6,
+               "inject_mark": 18.278e6 + 0.020e6, "trace": 89.177e6 + 12.653e6}
 # L1- and issue-side figures of the cone tracer (hybrid sampler) from its full capture of the
 # same command: it is bound by the L1 data pipe, not HBM.
 NCU_TRACE_ISSUE = {"sm_throughput_frac": 0.557, "fma_pipe_frac": 0.500, "l1_hit_rate": 0.971,

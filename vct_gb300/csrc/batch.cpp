@@ -40,7 +40,7 @@ namespace {
 size_t up256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 struct BatchTotals {
-    long long tris = 0, texels = 0, bricks = 0, tiles = 0;
+    long long tris = 0, marks = 0, bricks = 0, tiles = 0;
     int cones = kConesPlain;  // the kind of the scenes' cone marches
     // The frame's clears, zeroed by one launch before the voxeliser (statistics,
     // lit masks; carry tables and brick flags of the tessellation voxeliser;
@@ -149,11 +149,11 @@ vct_status batch_stage(vct_batch* b, const vct_scene_desc* sc, int n, char* h, B
         std::memcpy(h + b->off_occ + i * sizeof(AccumParams), &O, sizeof O);
         std::memcpy(h + b->off_wmap + i * sizeof(WarpmapArgs), &WM, sizeof WM);
         tri_off[i] = tot.tris;
-        tex_off[i] = tot.texels;
+        tex_off[i] = tot.marks;
         brick_off[i] = tot.bricks;
         tile_off[i] = tot.tiles;
         tot.tris += d.triangles.count;
-        tot.texels += (long long)I.nx * I.ny;
+        tot.marks += (long long)mark_items(I.nx) * I.ny;
         const long long bpa = c->dim / 16;
         tot.bricks += bpa * bpa * bpa;
         tot.tiles += trace_tiles(d.gbuffer.width, d.gbuffer.height, T.tile_w_log2, T.tile_h_log2);
@@ -175,7 +175,7 @@ vct_status batch_stage(vct_batch* b, const vct_scene_desc* sc, int n, char* h, B
         }
     }
     tri_off[n] = tot.tris;
-    tex_off[n] = tot.texels;
+    tex_off[n] = tot.marks;
     brick_off[n] = tot.bricks;
     tile_off[n] = tot.tiles;
     if (tot.tris > 0x7fffffffLL) return fail(VCT_ERR_INVALID_ARGUMENT, "a batch holds at most 2^31-1 triangles");
@@ -248,7 +248,7 @@ vct_status batch_enqueue(vct_batch* b, const char* h, const BatchTotals& tot, cu
     if (timed) VCT_CUDA(cudaEventRecord(b->ev[1], st));
     launch_inject_mark_batch(
         SceneBatch<InjectParams>{reinterpret_cast<const InjectParams*>(b->d_blob + b->off_inject), d_tables + (n + 1), n},
-        tot.texels, st);
+        tot.marks, st);
     VCT_CHECK_LAUNCH("batch: inject mark");
     launch_resolve_batch(SceneBatch<ResolveParams>{reinterpret_cast<const ResolveParams*>(b->d_blob + b->off_resolve),
                                                   d_tables + 2 * (n + 1), n},

@@ -329,6 +329,9 @@ void launch_occupancy(const AccumParams& P, cudaStream_t s);
 void launch_tesselate(const AccumParams& P, cudaStream_t s);
 void launch_normalize(const NormalizeParams& P, cudaStream_t s);
 void launch_inject(const InjectParams& P, cudaStream_t s);
+// Items of inject_mark in a row of the dispatch: a thread takes kMarkTexels texels.
+constexpr int kMarkTexels = 4;
+VCT_HD inline unsigned mark_items(int nx) { return ((unsigned)nx + kMarkTexels - 1) / kMarkTexels; }
 void launch_inject_mark(const InjectParams& P, cudaStream_t s);
 void launch_resolve(const ResolveParams& R, int num_sms, cudaStream_t s);
 // Builds levels [first+1, levels) from level `first`.
@@ -350,7 +353,7 @@ int accumulate_batch_max_scenes();
 void launch_accumulate_batch(const SceneBatch<AccumParams>& B, long long ntri, long long faces, int unit_log2,
                              int num_sms, int blocks_per_sm, cudaStream_t s);
 void launch_tesselate_batch(const SceneBatch<AccumParams>& B, const VoxWork& W, int num_sms, cudaStream_t s);
-void launch_inject_mark_batch(const SceneBatch<InjectParams>& B, long long ntexels, cudaStream_t s);
+void launch_inject_mark_batch(const SceneBatch<InjectParams>& B, long long items, cudaStream_t s);
 void launch_resolve_batch(const SceneBatch<ResolveParams>& B, long long nbricks, bool exact, cudaStream_t s);
 void launch_mip_tail_batch(const SceneBatch<MipLevels>& B, int max_occ_words, cudaStream_t s);
 // A device range of 32-bit words to zero (p 16-byte aligned, as cudaMalloc returns).
