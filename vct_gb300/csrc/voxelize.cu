@@ -175,11 +175,13 @@ __device__ __forceinline__ void shade_fragment(const AccumParams& P, long long t
                 // for a surface turned well away (by more than rounding) the
                 // cosine is: the light then adds +-0, unless its product with
                 // the albedo overflows.  Four point lights of range 0.3-0.8 in a
-                // volume of side 2 leave one in nine fragments inside one.
+                // volume of side 2 leave one in nine fragments inside one.  (A
+                // component each: fmaxf would pass over a NaN, whose product with
+                // 0 is not 0.)
                 const f3 base = mulv(mul(color, L.intensity), L.color);
                 const float d2 = dot(d, d), nd = dot(Nf, d);
                 if ((d2 > L.beyond2 || (nd < 0.0f && nd * nd > 1e-6f * d2 && d2 > 1e-30f && L.beyond2 < 3.0e38f)) &&
-                    fmaxf(fmaxf(fabsf(base.x), fabsf(base.y)), fabsf(base.z)) < 3.0e38f)
+                    fabsf(base.x) < 3.0e38f && fabsf(base.y) < 3.0e38f && fabsf(base.z) < 3.0e38f)
                     continue;
                 float ndl = fmaxf(0.0f, dot(Nf, normalize(d)));
                 lit = mul(base, ndl);
