@@ -4,6 +4,7 @@
 // reference, the learned trace with its per-tile or per-pixel fallback).
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <string>
 #include <vector>
@@ -281,13 +282,17 @@ vct_status vct_mlp_get_params(vct_mlp* m, float* host, int64_t count, void* stre
     DeviceScope ds(m->device);
     VCT_CUDA(ds.err);
     cudaStream_t st = as_stream(stream);
-    // one copy brings the parameters and the status word behind them
-    std::vector<float> got(kMlpParams + 1);
-    VCT_CUDA(cudaMemcpyAsync(got.data(), m->dev.params, sizeof(float) * got.size(), cudaMemcpyDeviceToHost, st));
+    // one copy brings the parameters and the status word behind them; without room for it, two
+    std::unique_ptr<float[]> got(new (std::nothrow) float[kMlpParams + 1]);
+    if (!got) {
+        VCT_CUDA(cudaMemcpyAsync(host, m->dev.params, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost, st));
+        return check_status(m, st);
+    }
+    VCT_CUDA(cudaMemcpyAsync(got.get(), m->dev.params, sizeof(float) * (kMlpParams + 1), cudaMemcpyDeviceToHost, st));
     VCT_CUDA(cudaStreamSynchronize(st));
-    std::memcpy(host, got.data(), sizeof(float) * kMlpParams);
+    std::memcpy(host, got.get(), sizeof(float) * kMlpParams);
     uint32_t h;
-    std::memcpy(&h, got.data() + kMlpParams, sizeof h);
+    std::memcpy(&h, got.get() + kMlpParams, sizeof h);
     return h ? check_status(m, st) : VCT_OK;
 }
 
