@@ -1,15 +1,36 @@
-"""Where the training calls put their results, and without host memory of their own."""
+"""Where the training calls put their results: memory of the host, pinned or
+not, of the network's device, and places that are not a float's."""
 
 from __future__ import annotations
 
+import ctypes as C
 import shutil
 import subprocess
 
 import pytest
 
 from test_c_abi import LIBDIR, ROOT
+from vct_gb300 import _lib as L
+from vct_gb300 import api
 
 pytestmark = pytest.mark.gpu
+
+
+def _get(m, pointer):
+    L.check(L.load().vct_mlp_get_params(m.handle, C.cast(pointer, C.POINTER(C.c_float)), api.Mlp.NPARAMS, 0),
+            "vct_mlp_get_params")
+
+
+def test_parameters_into_any_memory():
+    import torch
+
+    m = api.Mlp(seed=2)
+    want = torch.from_numpy(m.params())
+    assert want.abs().sum() > 0
+    pinned, device = torch.zeros(api.Mlp.NPARAMS).pin_memory(), torch.zeros(api.Mlp.NPARAMS, device="cuda")
+    _get(m, pinned.data_ptr())
+    _get(m, device.data_ptr())
+    assert torch.equal(pinned, want) and torch.equal(device.cpu(), want)
 
 
 _NO_MEMORY = r"""

@@ -282,8 +282,13 @@ vct_status vct_mlp_get_params(vct_mlp* m, float* host, int64_t count, void* stre
     DeviceScope ds(m->device);
     VCT_CUDA(ds.err);
     cudaStream_t st = as_stream(stream);
-    // one copy brings the parameters and the status word behind them; without room for it, two
-    std::unique_ptr<float[]> got(new (std::nothrow) float[kMlpParams + 1]);
+    // One copy brings the parameters and the status word behind them; to memory
+    // that the host does not write (the copy takes any), or without room for it, two.
+    cudaPointerAttributes at;
+    bool hosts = cudaPointerGetAttributes(&at, host) == cudaSuccess;
+    if (!hosts) cudaGetLastError();
+    hosts = hosts && (at.type == cudaMemoryTypeUnregistered || at.type == cudaMemoryTypeHost);
+    std::unique_ptr<float[]> got(hosts ? new (std::nothrow) float[kMlpParams + 1] : nullptr);
     if (!got) {
         VCT_CUDA(cudaMemcpyAsync(host, m->dev.params, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost, st));
         return check_status(m, st);
