@@ -540,7 +540,8 @@ vct_status vct_mlp_gradients(vct_mlp* mlp, const float* rows_dev, const float* t
                              float* grad_dev, float* loss_dev, void* stream);
 /* One Adam step on the n rows index_dev[0..n) of rows_dev / targets_dev
  * (index_dev NULL: rows 0..n); loss_dev (may be NULL) receives the step's
- * loss before the update.  No synchronisation. */
+ * loss before the update: stored by the update kernel in memory of the
+ * network's device, copied to any other.  No synchronisation. */
 vct_status vct_mlp_train_step(vct_mlp* mlp, const float* rows_dev, const float* targets_dev, const int32_t* index_dev,
                               int64_t n, const vct_adam* opt, float* loss_dev, void* stream);
 

@@ -33,6 +33,56 @@ def test_parameters_into_any_memory():
     assert torch.equal(pinned, want) and torch.equal(device.cpu(), want)
 
 
+def test_loss_into_any_memory():
+    """The losses of two steps in memory that the update kernel stores to and
+    in memory that it must not: pinned and pageable host memory, and a place
+    that is not a float's (a copy brings it there, or refuses); then under
+    capture."""
+    import torch
+
+    torch.manual_seed(1)
+    rows, targets = torch.randn(300, 42, device="cuda"), torch.rand(300, 3, device="cuda")
+    opt = L.vct_adam(1e-3, 0.9, 0.999, 1e-8)
+    want = torch.zeros(2, device="cuda")
+    m = api.Mlp(seed=2)
+    for k in range(2):
+        m.train_step(rows, targets, None, 300, 1e-3, want[k:])
+    params = m.params()
+
+    def steps(pointers, stream=0):
+        m = api.Mlp(seed=2)
+        for p in pointers:
+            L.call("vct_mlp_train_step", m.handle, rows.data_ptr(), targets.data_ptr(), 0, 300, C.byref(opt), p, stream)
+        torch.cuda.synchronize()
+        assert (m.params() == params).all()
+
+    pinned = torch.zeros(2).pin_memory()
+    steps([pinned.data_ptr(), pinned.data_ptr() + 4])
+    assert torch.equal(pinned, want.cpu())
+    odd = torch.zeros(9, dtype=torch.uint8, device="cuda")
+    steps([odd.data_ptr() + 1, odd.data_ptr() + 5])
+    assert torch.equal(odd[1:].cpu().view(torch.float32), want.cpu())
+    steps([0, 0])
+    pageable = torch.full((2,), -1.0)
+    m = api.Mlp(seed=2)
+    for k in range(2):
+        try:
+            m.train_step(rows, targets, None, 300, 1e-3, pageable.data_ptr() + 4 * k)
+        except L.VctError as e:
+            assert e.status == L.VCT_ERR_CUDA and pageable[k] == -1.0
+    torch.cuda.synchronize()
+    assert (m.params() == params).all()
+    assert all(p in (-1.0, w) for p, w in zip(pageable.tolist(), want.tolist()))
+
+    m, loss, graph, st = api.Mlp(seed=2), torch.zeros(2, device="cuda"), torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=st):
+        for k in range(2):
+            m.train_step(rows, targets, None, 300, 1e-3, loss[k:])
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(loss, want) and (m.params() == params).all()
+
+
 _NO_MEMORY = r"""
 #include <vct.h>
 #include <cstdio>

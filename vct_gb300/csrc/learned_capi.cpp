@@ -71,6 +71,17 @@ vct_status check_status(vct_mlp* m, cudaStream_t st) {
     return VCT_OK;
 }
 
+// Whether a kernel can store a float at `p`: aligned memory of the network's
+// device.  A copy takes more (another device's memory, the host's, any byte)
+// and turns what is no memory into an error, where a store would fault.
+bool in_float_place(const vct_mlp* m, const float* p) {
+    cudaPointerAttributes at;
+    if (!p || reinterpret_cast<uintptr_t>(p) % sizeof(float)) return false;
+    if (cudaPointerGetAttributes(&at, p) == cudaSuccess) return at.type == cudaMemoryTypeDevice && at.device == m->device;
+    cudaGetLastError();
+    return false;
+}
+
 vct_status validate_rows(const float* rows, int64_t n) {
     if (n < 0 || n > (1LL << 31)) return fail(VCT_ERR_INVALID_ARGUMENT, "row count out of range");
     if (n > 0 && !rows) return fail(VCT_ERR_INVALID_ARGUMENT, "rows is NULL");
@@ -371,12 +382,11 @@ vct_status vct_mlp_train_step(vct_mlp* m, const float* rows, const float* target
     vct_status s = train_launch(m, rows, targets, index, n, st, nparts);
     if (s != VCT_OK) return s;
     ++m->step;
-    // the update stores the loss, unless that is not in a float's place
-    const bool place = reinterpret_cast<uintptr_t>(loss_dev) % sizeof(float) == 0;
+    const bool stores = in_float_place(m, loss_dev);
     launch_mlp_update(m->dev, kUpdateAdam, nparts, m->step, opt->lr, opt->beta1, opt->beta2, opt->eps,
-                      place ? loss_dev : nullptr, st);
+                      stores ? loss_dev : nullptr, st);
     VCT_CHECK_LAUNCH("adam");
-    if (!place) VCT_CUDA(cudaMemcpyAsync(loss_dev, m->dev.loss, sizeof(float), cudaMemcpyDeviceToDevice, st));
+    if (loss_dev && !stores) VCT_CUDA(cudaMemcpyAsync(loss_dev, m->dev.loss, sizeof(float), cudaMemcpyDeviceToDevice, st));
     return VCT_OK;
 }
 
