@@ -873,6 +873,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_kernel(const TrainPar
         }
         first = false;
     }
+    // The update may start; it waits for this kernel's end before it reads anything.
     grid_launch_dependents();
     ok = __syncthreads_and(ok);
     // ---- gradients out: this CTA's part (zeros after a wait that gave up)
@@ -929,15 +930,13 @@ __global__ void __launch_bounds__(kUpdateThreads) mlp_update_kernel(const MlpDev
     const int i = blockIdx.x * kUpdateParams + k;
     float w = 0.0f, m = 0.0f, v = 0.0f;
     const bool mine = slice == 0 && i < kMlpParams;
-    if (mine && what == kUpdateAdam) {
-        // the training kernel, which this one may overlap, started after the
-        // end of everything that writes these
+    grid_wait();
+    grid_launch_dependents();
+    if (mine && what == kUpdateAdam) {  // (in flight with the parts)
         w = M.params[i];
         m = M.m[i];
         v = M.v[i];
     }
-    grid_wait();
-    grid_launch_dependents();
     if (what != kUpdateImages) {
         float g = 0.0f;
         if (i < kMlpParams) {

@@ -306,7 +306,11 @@ struct ManyScenes {
 // grid_launch_dependents (or ended), and waits in grid_wait for that kernel's
 // end before it touches anything that other kernels read or write.  (Read-only
 // loads may be moved before the wait by the compiler: use ordinary ones behind
-// it, or addresses that a barrier behind it makes known.)
+// it, or addresses that a barrier behind it makes known.)  One exception: what
+// was complete when an ordinary launch started, with only kernels that wait
+// between that one and this, may be read before the wait: the triangles of the
+// depth passes (before the fill of their keys) and the G-buffer of a frame's
+// trace (before the resolve).
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
