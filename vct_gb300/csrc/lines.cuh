@@ -469,13 +469,15 @@ __device__ __forceinline__ void walk_all(CtaLines& S, int lines, bool big, Sink&
 }
 
 // Grid of a kernel over `ntri` triangles: as many CTAs to each 256 of them (at
-// most 64) as give `want` in all, but no more than have some `share` pixels
-// each if the triangles cover `pixels`, and at least `least` where there are
-// more sets of 256 than SMs hold CTAs.
-inline dim3 line_grid(long long ntri, long long want, long long pixels, long long share, int num_sms, long long least) {
+// most 64, or what gives `fill` in all) as give `want` in all, but no more than
+// have some `share` pixels each if the triangles cover `pixels`, and at least
+// `least` where there are more sets of 256 than SMs hold CTAs.
+inline dim3 line_grid(long long ntri, long long want, long long pixels, long long share, int num_sms, long long least,
+                      long long fill = 0) {
     const long long ctas = (ntri + kLineThreads - 1) / kLineThreads;
     const long long n = std::min((want + ctas - 1) / ctas, pixels / (ctas * share));
-    return dim3((unsigned)ctas, (unsigned)std::max(ctas > 4LL * num_sms ? least : 1LL, std::min(n, 64LL)));
+    return dim3((unsigned)ctas,
+                (unsigned)std::max(ctas > 4LL * num_sms ? least : 1LL, std::min(n, std::max(64LL, fill / ctas))));
 }
 
 }  // namespace lines

@@ -274,17 +274,28 @@ __global__ void __launch_bounds__(kLineThreads, kRasterBlocksPerSM)
 // By default (units of 512 pixels, 3 CTAs per SM) 9 CTAs per SM, three times
 // as many as are resident; smaller units share the lines out further.  Each
 // CTA that sets the same triangles up again costs some 7 us of latency (loads,
-// projection, scans), each CTA too few leaves SMs idle at the end: with 6, 12
-// and 24 per SM 38,000 triangles in 128^3 take 53, 66 and 96 us, 74,752 in
-// 256^3 0.304, 0.281 and (24 not measured); past 300,000 triangles the least,
-// two to each 256, is best (519,552: 0.497 with one, 0.460 with two).
+// projection, scans), each CTA too few leaves SMs idle at the end: with 3, 6, 9,
+// 12 and 24 per SM 38,040 triangles in 128^3 take 47, 46, 45, 45 and 46 us,
+// 74,752 in 256^3 340, 294, 280, 269 and 275, 262,144 277, 278, 277, 276 and 285;
+// past 300,000 triangles the least, two to each 256, is best (519,552: 0.497 ms
+// with one, 0.460 with two).
+//
+// Where the triangles are few, what they cover is not known before they are set
+// up: they get the CTAs that are resident, or in a large grid, whose walls have
+// that many more pixels, one to 16,384 pixels if they covered its faces 64
+// times.  255 triangles that cover a grid many times over take 0.108 ms in 256^3
+// and 0.331 in 512^3; with no more than 64 CTAs to a set 0.293 and 1.451 (units
+// handed to any CTA by a kernel before it, as once, 0.147 and 0.362), with 9 per
+// SM 0.100 and 0.306; 255 that cover little 0.011 and 0.023, 0.010 and 0.018, 0.024
+// and 0.027.
 template <class Scenes>
 void launch_voxelize(const Scenes& S, long long ntri, long long faces, int unit_log2, int num_sms, int blocks_per_sm,
                      cudaStream_t s) {
     if (ntri <= 0) return;
     const int bps = blocks_per_sm < 1 ? 1 : (blocks_per_sm > kRasterBlocksPerSM ? kRasterBlocksPerSM : blocks_per_sm);
-    const dim3 grid = line_grid(ntri, (((long long)num_sms * bps * 3) << 9) >> unit_log2, 64 * faces, 1LL << (unit_log2 + 1),
-                                num_sms, 2);
+    const long long resident = (long long)num_sms * bps, pixels = 64 * faces;
+    const dim3 grid = line_grid(ntri, (3 * resident << 9) >> unit_log2, pixels, 2LL << unit_log2, num_sms, 2,
+                                std::max(resident, pixels >> 14));
     voxelize_raster_kernel<Scenes><<<grid, kLineThreads, 0, s>>>(S, ntri);
     note_launches(1);
 }
