@@ -235,8 +235,7 @@ vct_status batch_enqueue(vct_batch* b, const char* h, const BatchTotals& tot, cu
             AccumParams W;
             W.ntri = tot.tris;
             tess_bind_scratch(W, b->work);
-            launch_tesselate_batch(SB, VoxWork{W.tri_rec, W.tri_units, W.tri_scan, W.block_off, tot.tris, tess_run_log2(tot.tris)},
-                                   b->num_sms, st);
+            launch_tesselate_batch(SB, VoxWork{W.tri_rec, W.tri_units, W.tri_scan, W.block_off, tot.tris}, b->num_sms, st);
         } else {
             long long faces = 0;
             for (const vct_ctx* c : b->ctx) faces += (long long)c->dim * c->dim;

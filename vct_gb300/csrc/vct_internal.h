@@ -101,9 +101,9 @@ struct AccumParams {
     float max_tess_level;   // GL_MAX_TESS_GEN_LEVEL
     // Work distribution scratch of the tessellation voxeliser (sized for ntri).
     uint4* tri_rec;          // uint4 per triangle
-    uint32_t* tri_units;     // work units per triangle
+    uint32_t* tri_units;     // work units per triangle, of items << 16 | of points
     uint32_t* tri_scan;      // block-local exclusive scan of tri_units
-    uint32_t* block_off;     // exclusive scan of per-block unit totals (+ total at [nblocks])
+    uint4* block_off;        // exclusive scan of per-block unit totals (+ totals at [nblocks])
 };
 
 // Several independent scenes processed by one launch per stage: `off` is the
@@ -124,21 +124,19 @@ struct VoxWork {
     uint4* tri_rec;
     uint32_t* tri_units;
     uint32_t* tri_scan;
-    uint32_t* block_off;
+    uint4* block_off;
     long long ntri;
-    int run_log2;  // log2 of the most points of an edge that one item holds
 };
-int tess_run_log2(long long ntri);
 
 constexpr int kSetupThreads = 256;  // triangles per setup block
 constexpr long long align256(long long b) { return (b + 255) & ~255LL; }
 // Scratch bytes the tessellation voxeliser needs for `ntri` triangles: a
-// 16-byte set-up record, a unit count and a scan entry per triangle, one
-// offset per block (+ the total), an 8-byte work counter.  The rasterising
+// 16-byte set-up record, a word of unit counts and one of scans per triangle,
+// 16 bytes of offsets per block (+ the totals), an 8-byte work counter.  The rasterising
 // voxeliser needs none.
 constexpr long long tess_scratch_bytes(long long ntri) {
     return align256(ntri * 16) + align256(ntri * 4) * 2 +
-           align256(((ntri + kSetupThreads - 1) / kSetupThreads + 2) * 4 + 8);
+           align256(((ntri + kSetupThreads - 1) / kSetupThreads + 1) * 16 + 8);
 }
 // Carves the scratch buffer into the AccumParams work arrays.
 void tess_bind_scratch(AccumParams& P, void* scratch);

@@ -430,26 +430,38 @@ __global__ void __launch_bounds__(kOccThreads) occupancy_kernel(const Scenes S, 
 }
 
 // ====================================================== tessellation voxeliser
-// testTesselation.tesc/.tese (Application.cpp:585-662) in three launches:
-// per-triangle tessellation levels and edge counts (tess_setup_kernel), the
-// scan of the block totals, and a persistent kernel (tess_points_kernel).
+// testTesselation.tesc/.tese (Application.cpp:585-662) in four launches:
+// per-triangle tessellation levels and unit counts (tess_setup_kernel), the
+// scan of the block totals, and two persistent kernels of which one ends at
+// once (tess_walks): single points, or the walk.
 //
-// The points of a patch fall into few voxels (on the 262,144-triangle scene, 14
-// points to each voxel that a triangle reaches), but not in the order of its
-// rings.  A lane therefore walks a sequence of points that is likely to stay in
-// one voxel (TessItem) and sums it in registers while it does; a finished run
-// goes to a queue in shared memory, and 32 queued runs are added to the records
-// together.  Integer sums: any grouping gives the same record.
+// Single points (tess_points_kernel): one to a lane, neighbours of a ring edge
+// that fall into one voxel added together.  For triangles of ordinary shape,
+// whose points are about a voxel apart in every direction: 24,576 box triangles
+// (14.7 M points) in 256^3 take 0.37 ms, bound by the reductions.
 //
-// What bounds it is issue (82% of peak), some 300 instructions per 32 points:
-// half of them the exact position, a tenth each the normal, the runs' queue and
-// their additions, the rest each item's set-up.  53,248 column slivers and
-// 24,576 box triangles (181 M points, 38 M runs) in 256^3: 1.89 ms.  The form
-// before, one point per lane with neighbouring pairs merged, spent 4.85 ms on 28
-// times as many reductions; lanes that walk whole ring edges, which finish a
-// run every 1.6 points, 2.65 ms.  Triangles of ordinary shape, whose points are
-// about a voxel apart in every direction, have nothing to gain: 3,568 of them
-// take 0.095 against 0.076 ms.
+// The walk (tess_walk_kernel).  The points of slivers fall into few voxels (on
+// the 262,144-triangle scene, 14 points to each voxel that a triangle reaches),
+// but not in the order of a patch's rings.  A lane therefore walks a sequence of
+// points that is likely to stay in one voxel (TessItem) and sums it in registers
+// while it does; a finished run goes to a queue in shared memory, and 32 queued
+// runs are added to the records together.  Integer sums: any grouping gives the
+// same record.  What bounds it is issue (82% of peak), some 300 instructions per
+// 32 points: half of them the exact position, a tenth each the normal, the runs'
+// queue and their additions, the rest each item's set-up.  53,248 column
+// slivers and 24,576 box triangles (180 M points, 38 M runs) in 256^3: 1.85 ms,
+// 4.46 as single points; lanes that walk whole ring edges, which finish a run
+// every 1.6 points, 2.65.
+//
+// The walk's constants, by three scenes of column slivers and boxes (22,000 in
+// 64^3, 30,000 in 128^3, 78,000 in 256^3; us): units taken at a time 2, 4, 8, 16, 32: 857, 788, 760,
+// 764, 782; 934, 860, 832, 815, 870; 2,225, 2,006, 1,893, 1,852, 1,867 (16
+// cost 16,000 slivers up to a tenth more).  Points of an edge to an item 4, 8, 16:
+// 815, 760, 789; 888, 832, 858; 2,052, 1,893, 1,962.  Places in turn 1, 512, 2,048,
+// 8,192, 32,768: 760, 763, 767, 760, 762; 828, 853, 852, 832, 828; 1,869, 1,950,
+// 1,935, 1,893, 1,875, and 78,000 triangles in 16^3, whose units all add to
+// the same few records, 311, 295, 289, 285, 286.  The inner level from which a sliver is
+// walked across, 4 to 16: no difference.
 //
 // Tessellation levels after GL's equal_spacing rounding, packed 7 bits each:
 // inner n | outer[0] << 7 | outer[1] << 14 | outer[2] << 21 (1..64 each) |
@@ -457,14 +469,23 @@ __global__ void __launch_bounds__(kOccThreads) occupancy_kernel(const Scenes S, 
 constexpr int kTessUnit = 32;  // items per work unit
 constexpr int kTessBlocksPerSM = 3;
 constexpr int kTessSliver = 8; // inner level from which slivers are walked across
+constexpr float kTessThin = 12.0f;  // inner level, in lengths of the shortest edge, of the slivers that decide for the walk
+constexpr int kTessRunLog2 = 3;     // log2 of the most points of an edge that one item holds
 constexpr int kTessGrab = 8;  // units a warp takes at a time, when there are that many
 constexpr int kTessSpread = 8192;  // places in the unit order that are worked on at a time
 constexpr int kMaxTess = VCT_MAX_TESS_LEVEL;
 
+// Work units, 32 items or 32 points of one triangle each.  A triangle's counts
+// are in one word: its items' in the high half, its points' in the low one (at
+// most 100, of 256 triangles 25,600).
+__device__ __forceinline__ uint32_t item_units(uint32_t x) { return x >> 16; }
+__device__ __forceinline__ uint32_t point_units(uint32_t x) { return x & 0xffffu; }
+
 // Block-local exclusive scan of the per-triangle unit counts of one setup
-// block into tri_scan, and the block's total into block_off[blockIdx.x].
-__device__ __forceinline__ void block_scan_units(const VoxWork& W, long long g, uint32_t units) {
-    __shared__ uint32_t warp_tot[kSetupThreads / 32];
+// block into tri_scan, and the block's totals {items, points, points of
+// slivers} into block_off[blockIdx.x].
+__device__ __forceinline__ void block_scan_units(const VoxWork& W, long long g, uint32_t units, bool sliver) {
+    __shared__ uint32_t warp_tot[kSetupThreads / 32], warp_slivers[kSetupThreads / 32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     uint32_t incl = units;
 #pragma unroll
@@ -472,52 +493,104 @@ __device__ __forceinline__ void block_scan_units(const VoxWork& W, long long g, 
         uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += v;
     }
-    if (lane == 31) warp_tot[wid] = incl;
+    const uint32_t slivers = __reduce_add_sync(0xffffffffu, sliver ? point_units(units) : 0u);
+    if (lane == 31) {
+        warp_tot[wid] = incl;
+        warp_slivers[wid] = slivers;
+    }
     __syncthreads();
-    uint32_t before = 0, total = 0;
+    uint32_t before = 0, total = 0, total_slivers = 0;
 #pragma unroll
     for (int w = 0; w < kSetupThreads / 32; ++w) {
         before += (w < wid) ? warp_tot[w] : 0u;
         total += warp_tot[w];
+        total_slivers += warp_slivers[w];
     }
     if (g < W.ntri) W.tri_scan[g] = before + incl - units;
-    if (threadIdx.x == 0) W.block_off[blockIdx.x] = total;
+    if (threadIdx.x == 0) W.block_off[blockIdx.x] = make_uint4(item_units(total), point_units(total), total_slivers, 0u);
 }
 
-__global__ void __launch_bounds__(1024) voxelize_scan_kernel(uint32_t* block_off, int nblocks) {
-    __shared__ uint32_t warp_tot[32];
-    __shared__ uint32_t carry;
-    if (threadIdx.x == 0) carry = 0;
+__global__ void __launch_bounds__(1024) voxelize_scan_kernel(uint4* block_off, int nblocks) {
+    __shared__ uint4 warp_tot[32];
+    __shared__ uint4 carry;
+    auto add = [](uint4 a, uint4 b) { return make_uint4(a.x + b.x, a.y + b.y, a.z + b.z, 0u); };
+    const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+    if (threadIdx.x == 0) carry = none;
     __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     for (int base = 0; base < nblocks; base += 1024) {
         const int i = base + threadIdx.x;
-        const uint32_t v = i < nblocks ? block_off[i] : 0u;
-        uint32_t incl = v;
+        const uint4 v = i < nblocks ? block_off[i] : none;
+        uint4 incl = v;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            uint32_t s = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += s;
+            const uint4 u = make_uint4(__shfl_up_sync(0xffffffffu, incl.x, o), __shfl_up_sync(0xffffffffu, incl.y, o),
+                                       __shfl_up_sync(0xffffffffu, incl.z, o), 0u);
+            if (lane >= o) incl = add(incl, u);
         }
         if (lane == 31) warp_tot[wid] = incl;
         __syncthreads();
-        uint32_t before = carry, total = 0;
+        uint4 before = carry, total = none;
         for (int w = 0; w < 32; ++w) {
-            before += (w < wid) ? warp_tot[w] : 0u;
-            total += warp_tot[w];
+            if (w < wid) before = add(before, warp_tot[w]);
+            total = add(total, warp_tot[w]);
         }
-        if (i < nblocks) block_off[i] = before + incl - v;
+        if (i < nblocks)
+            block_off[i] = make_uint4(before.x + incl.x - v.x, before.y + incl.y - v.y, before.z + incl.z - v.z, 0u);
         __syncthreads();
-        if (threadIdx.x == 0) carry += total;
+        if (threadIdx.x == 0) carry = add(carry, total);
         __syncthreads();
     }
     if (threadIdx.x == 0) block_off[nblocks] = carry;
 }
 
-template <class Scenes>
-__device__ __forceinline__ long long unit_start(const VoxWork& W, long long g) {
-    return (long long)W.block_off[g / kSetupThreads] + W.tri_scan[g];
-}
+// The triangle that a unit belongs to: its number, its first unit and how many
+// it has, of the units of items or of points.
+template <bool ITEMS>
+struct UnitOwner {
+    long long g;
+    uint32_t start, units;
+    static __device__ __forceinline__ uint32_t part(uint32_t x) { return ITEMS ? item_units(x) : point_units(x); }
+    static __device__ __forceinline__ uint32_t block(const VoxWork& W, long long b) {
+        return reinterpret_cast<const uint32_t*>(W.block_off + b)[ITEMS ? 0 : 1];
+    }
+    __device__ __forceinline__ void at(const VoxWork& W, long long t) {
+        g = t;
+        start = block(W, g / kSetupThreads) + part(W.tri_scan[g]);
+        units = part(W.tri_units[g]);
+    }
+    __device__ __forceinline__ bool holds(uint32_t u) const { return u - start < units; }
+    // By a search over the block offsets, then the block-local scan, 8 entries
+    // per lane: the number of entries <= u is one past the last triangle starting
+    // at or before u.
+    __device__ __forceinline__ void find(const VoxWork& W, int nblocks, uint32_t u, int lane) {
+        int lo = 0, hi = nblocks - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (block(W, mid) <= u)
+                lo = mid;
+            else
+                hi = mid - 1;
+        }
+        const long long gbase = (long long)lo * kSetupThreads;
+        const int in_block = (int)min((long long)kSetupThreads, W.ntri - gbase);
+        const uint32_t rel = u - block(W, lo);
+        int below = 0;
+#pragma unroll
+        for (int j = 0; j < kSetupThreads / 32; ++j) {
+            const int k = lane * (kSetupThreads / 32) + j;
+            below += (k < in_block && part(__ldg(W.tri_scan + gbase + k)) <= rel) ? 1 : 0;
+        }
+        below = __reduce_add_sync(0xffffffffu, below);
+        at(W, gbase + max(below - 1, 0));
+    }
+    // The owner of the unit after one of this triangle's: often this one or the next.
+    __device__ __forceinline__ void follow(const VoxWork& W, int nblocks, uint32_t u, int lane) {
+        if (holds(u)) return;
+        at(W, min(g + 1, W.ntri - 1));
+        if (!holds(u)) find(W, nblocks, u, lane);
+    }
+};
 
 // Float-to-int truncation of ivec3(): NaN -> 0, saturating (cvt.rzi.s32.f32).
 __device__ __forceinline__ int trunc_sat(float x) { return __float2int_rz(x); }
@@ -542,7 +615,8 @@ __device__ __forceinline__ uint32_t tess_point_count(int n, int m0, int m1, int 
 
 // testTesselation.tesc:33-78: levels of one triangle; false if discarded
 // (all three vertices truncate to one voxel: levels 0).
-__device__ __forceinline__ bool tess_levels(const AccumParams& P, const float* Pp, uint32_t& packed, uint32_t& npts) {
+__device__ __forceinline__ bool tess_levels(const AccumParams& P, const float* Pp, uint32_t& packed, uint32_t& npts,
+                                            bool& sliver) {
     const f3 a = ld3(Pp), b = ld3(Pp + 3), c = ld3(Pp + 6);
     const float fN = (float)P.dim;
     const f3 vtx[3] = {a, b, c};
@@ -583,6 +657,7 @@ __device__ __forceinline__ bool tess_levels(const AccumParams& P, const float* P
         if (4.0f * ly < fminf(lx, lz)) across = 3;
     }
     packed = (uint32_t)n | ((uint32_t)m0 << 7) | ((uint32_t)m1 << 14) | ((uint32_t)m2 << 21) | (across << 28);
+    sliver = (float)n >= kTessThin * fminf(ox, fminf(oy, oz));  // (lengths in voxels, 1 at least)
     npts = tess_point_count(n, m0, m1, m2);
     return true;
 }
@@ -681,37 +756,127 @@ __device__ __forceinline__ TessItem tess_item(uint32_t packed, int i, int rl) {
     return t;
 }
 
-// The points warps' shared work counter: 8 bytes after block_off[nblocks].
-__device__ __forceinline__ unsigned long long* grab_counter(const VoxWork& W, int nblocks) {
-    return reinterpret_cast<unsigned long long*>(W.block_off + (((long long)nblocks + 2) & ~1LL));
+// Point `i` of a patch in the order of tess_point_count: the corners, the
+// outer edges' inner points, then ring by ring.
+__device__ __forceinline__ f3 tess_coord(uint32_t packed, int i) {
+    const int n = (int)(packed & 127u), m0 = (int)((packed >> 7) & 127u), m1 = (int)((packed >> 14) & 127u),
+              m2 = (int)((packed >> 21) & 127u);
+    if (i < 3) return i == 0 ? mk(1.0f, 0.0f, 0.0f) : i == 1 ? mk(0.0f, 1.0f, 0.0f) : mk(0.0f, 0.0f, 1.0f);
+    i -= 3;
+    if (i < m0 - 1) {
+        const float s = __fdiv_rn((float)(i + 1), (float)m0);
+        return mk(0.0f, 1.0f - s, s);
+    }
+    i -= m0 - 1;
+    if (i < m1 - 1) {
+        const float s = __fdiv_rn((float)(i + 1), (float)m1);
+        return mk(s, 0.0f, 1.0f - s);
+    }
+    i -= m1 - 1;
+    if (i < m2 - 1) {
+        const float s = __fdiv_rn((float)(i + 1), (float)m2);
+        return mk(1.0f - s, s, 0.0f);
+    }
+    i -= m2 - 1;
+    int k = 1, q = n - 2;
+    while (q > 0 && i >= 3 * q) {
+        i -= 3 * q;
+        ++k;
+        q -= 2;
+    }
+    if (q <= 0) {  // the centre of an even inner level
+        const float third = __fdiv_rn(1.0f, 3.0f);
+        return mk(third, third, third);
+    }
+    const float t = __fdiv_rn((float)(2 * k), (float)(3 * n));
+    const float h = 1.0f - 2.0f * t;
+    const int e = i / q, j = i - e * q;
+    const float s = __fdiv_rn((float)j, (float)q);
+    // corners c_e and c_{e+1} of the ring: c0 = (h,t,t), c1 = (t,h,t), c2 = (t,t,h)
+    const int e1 = e == 2 ? 0 : e + 1;
+    const float a0 = e == 0 ? h : t, a1 = e == 1 ? h : t, a2 = e == 2 ? h : t;
+    const float b0 = e1 == 0 ? h : t, b1 = e1 == 1 ? h : t, b2 = e1 == 2 ? h : t;
+    return mk(a0 + s * (b0 - a0), a1 + s * (b1 - a1), a2 + s * (b2 - a2));
 }
 
-// Record of a triangle: {packed levels, items, scene, index within its scene}.
+// Whether the items are walked: where thin slivers have most of the points, and
+// at least some 1.3 M of them (totals: {items, points, points of slivers}, in
+// units of 32).  Otherwise every point is taken singly.  A walk costs some 13 us
+// before it gains, and on ordinary triangles it always loses.  Points against
+// walk, with set-up and scan (us; slivers' points of all): columns of slivers and
+// a few boxes in 16^3 (1.3 M of 1.3 M) 191 and 65, in 64^3 (1.4 of 1.6) 100 and
+// 60, in 256^3 (1.7 of 3.6) 124 and 132; columns between 24,576 box
+// triangles in 256^3 (26 of 40) 976 and 585; the boxes alone in 64^3 (0.1 of
+// 1.2) 53 and 131, in 256^3 (1 of 15) 374 and 398; scattered slivers, which
+// share no voxels, in 128^3 (1.2 of 1.2) 41 and 57, (12 of 12) 248 and 194, and
+// where the rule loses, in 64^3 (3 of 3) 80 and 114.
+__device__ __forceinline__ bool tess_walks(const uint4 total) {
+    return total.z >= 40000u && (float)total.z >= 0.6f * (float)total.y;
+}
+
+// The walking warps' shared work counter: the 8 bytes after block_off[nblocks].
+__device__ __forceinline__ unsigned long long* grab_counter(const VoxWork& W, int nblocks) {
+    return reinterpret_cast<unsigned long long*>(W.block_off + nblocks + 1);
+}
+
+// Record of a triangle: {packed levels, items << 16 | points, scene, index within its scene}.
 template <class Scenes>
 __global__ void __launch_bounds__(kSetupThreads) tess_setup_kernel(const Scenes S, const VoxWork W) {
     const long long g = (long long)blockIdx.x * kSetupThreads + threadIdx.x;
     uint32_t units = 0;
+    bool sliver = false;
     if (g < W.ntri) {
         long long t;
         const int scene = S.find(g, t);
         const AccumParams& P = S.get(scene);
         uint32_t packed = 0, npts = 0;
-        if (!tess_levels(P, P.pos + t * 9, packed, npts)) npts = 0;
-        const uint32_t items = npts ? tess_item_count(packed, W.run_log2) : 0u;
-        W.tri_rec[g] = make_uint4(packed, items, (uint32_t)scene, (uint32_t)t);
-        units = (items + kTessUnit - 1) / kTessUnit;
+        if (!tess_levels(P, P.pos + t * 9, packed, npts, sliver)) npts = 0;
+        const uint32_t items = npts ? tess_item_count(packed, kTessRunLog2) : 0u;
+        W.tri_rec[g] = make_uint4(packed, items << 16 | npts, (uint32_t)scene, (uint32_t)t);
+        units = ((items + kTessUnit - 1) / kTessUnit) << 16 | ((npts + kTessUnit - 1) / kTessUnit);
         W.tri_units[g] = units;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) *grab_counter(W, gridDim.x) = 0ull;
-    block_scan_units(W, g, units);
+    block_scan_units(W, g, units, sliver);
 }
 
-// A warp's queued items, and its finished runs of points on their way to the
+// A warp's queued items or points.
+struct TessQueue {
+    int tri[2 * kTessUnit];        // triangle index within its scene
+    uint32_t item[2 * kTessUnit];  // item or point of the triangle | scene << 16
+    uint32_t lev[2 * kTessUnit];   // packed levels
+};
+// Queues unit `unit` of a triangle's `n` items or points; `full` works on 32
+// of them.  qn: the number queued (warp-uniform).
+template <class F>
+__device__ __forceinline__ void queue_unit(TessQueue& q, int& qn, const uint4 rec, uint32_t n, uint32_t unit, int lane,
+                                           F full) {
+    const int base = (int)unit * kTessUnit;
+    const int cnt = min(kTessUnit, (int)n - base);
+    if (lane < cnt) {
+        q.tri[qn + lane] = (int)rec.w;
+        q.item[qn + lane] = (uint32_t)(base + lane) | (rec.z << 16);
+        q.lev[qn + lane] = rec.x;
+    }
+    __syncwarp();
+    qn += cnt;
+    if (qn >= kTessUnit) {
+        full(kTessUnit);
+        __syncwarp();
+        if (lane < qn - kTessUnit) {
+            q.tri[lane] = q.tri[kTessUnit + lane];
+            q.item[lane] = q.item[kTessUnit + lane];
+            q.lev[lane] = q.lev[kTessUnit + lane];
+        }
+        __syncwarp();
+        qn -= kTessUnit;
+    }
+}
+
+// A walking warp's queue, and its finished runs of points on their way to the
 // records (a ring): the four 64-bit words of each, its voxel and scene.
 struct TessStage {
-    int tri[2 * kTessUnit];        // triangle index within its scene
-    uint32_t item[2 * kTessUnit];  // item of the triangle | scene << 16
-    uint32_t lev[2 * kTessUnit];   // packed levels
+    TessQueue q;
     ulonglong2 words[64][2];
     uint32_t vox[64], scene[64];
 };
@@ -776,11 +941,100 @@ __device__ __forceinline__ void fill_tables(TessTables& T) {
     }
 }
 
-// testTesselation.tese:101-133 for the queued items, one per lane (lanes >=
-// nact idle).
+// testTesselation.tese:101-133: the voxel of a point at `pos`; false outside.
+__device__ __forceinline__ bool tess_voxel(const AccumParams& P, f3 pos, uint32_t& v) {
+    const int N = P.dim;
+    const float fN = (float)N;
+    f3 tc;  // times N
+    if (P.warp.mode == VCT_WARP_PERSPECTIVE) {  // voxelTesselationWarpedPosition
+        tc = mul(perspective_tc(P.warp, pos), fN);
+    } else {  // voxelLinearPosition (the evaluation shader passes warpVoxels = false)
+        tc = sub(sub(pos, P.vcenter), P.vmin);
+        if (P.ext_rcp != 0.0f)  // the extents are a power of two, as N is: the product is the quotient's
+            tc = mul(tc, P.ext_rcp * fN);
+        else
+            tc = mul(mk(__fdiv_rn(tc.x, P.ext.x), __fdiv_rn(tc.y, P.ext.y), __fdiv_rn(tc.z, P.ext.z)), fN);
+    }
+    const int vx = trunc_sat(tc.x), vy = trunc_sat(tc.y), vz = trunc_sat(tc.z);
+    if ((uint32_t)(vx | vy | vz) >= (uint32_t)N) return false;  // not all in [0, N): N is a power of two
+    v = (uint32_t)((vz * N + vy) * N + vx);
+    return true;
+}
+// voxelStore: normalize(normal) * 0.5 + 0.5.
+__device__ __forceinline__ void tess_normal(f3 nrm, uint32_t& qx, uint32_t& qy, uint32_t& qz) {
+    const f3 Nf = normalize(nrm);
+    qx = quant16(Nf.x * 0.5f + 0.5f);
+    qy = quant16(Nf.y * 0.5f + 0.5f);
+    qz = quant16(Nf.z * 0.5f + 0.5f);
+}
+
+// The queued points, one per lane (lanes >= nact idle), stored with 64-bit
+// reductions.  Neighbouring points of a ring edge often share a voxel: an even
+// lane takes its odd neighbour's sums when both hit the same voxel (one shuffle
+// per word), so the pair costs one set of reductions.  Exact as tess_flush is.
+template <class Scenes>
+__device__ __forceinline__ void tess_store32(const Scenes& S, const TessQueue& q, int nact, int lane) {
+    const unsigned FULL = 0xffffffffu;
+    bool valid = false;
+    uint32_t v = 0, qr = 0, qg = 0, qb = 0, qx = 0, qy = 0, qz = 0;
+    const AccumParams& P = S.get(lane < nact ? (int)(q.item[lane] >> 16) : 0);
+    if (lane < nact) {
+        const long long t = q.tri[lane];
+        const f3 bc = tess_coord(q.lev[lane], (int)(q.item[lane] & 0xffffu));
+        const float* Pp = P.pos + t * 9;
+        const float* Pn = P.nrm + t * 9;
+        const f3 p0 = ld3(Pp), p1 = ld3(Pp + 3), p2 = ld3(Pp + 6);
+        const f3 n0 = ld3(Pn), n1 = ld3(Pn + 3), n2 = ld3(Pn + 6);
+        valid = tess_voxel(P, add(add(mul(p0, bc.x), mul(p1, bc.y)), mul(p2, bc.z)), v);
+        if (valid) {
+            const f3 col = ld3(P.albedo + t * 3);
+            qr = quant16(col.x);
+            qg = quant16(col.y);
+            qb = quant16(col.z);
+            tess_normal(add(add(mul(n0, bc.x), mul(n1, bc.y)), mul(n2, bc.z)), qx, qy, qz);
+        }
+    }
+    const unsigned key = valid ? v : 0xffffffffu;
+    const unsigned partner = __shfl_xor_sync(FULL, key, 1);  // every lane takes part
+    const bool pair = valid && partner == key;
+    const uint32_t pr = __shfl_xor_sync(FULL, qr, 1), pg = __shfl_xor_sync(FULL, qg, 1), pb = __shfl_xor_sync(FULL, qb, 1),
+                   px = __shfl_xor_sync(FULL, qx, 1), py = __shfl_xor_sync(FULL, qy, 1), pz = __shfl_xor_sync(FULL, qz, 1);
+    if (!valid || (pair && (lane & 1))) return;
+    unsigned long long cnt = 1;
+    if (pair) {
+        cnt = 2;
+        qr += pr;
+        qg += pg;
+        qb += pb;
+        qx += px;
+        qy += py;
+        qz += pz;
+    }
+    unsigned long long* rec = reinterpret_cast<unsigned long long*>(P.acc + kAccWords * record_slot(v, P.dim));
+    const unsigned long long a0 = cnt | ((unsigned long long)qr << 32);
+    const unsigned long long a1 = (unsigned long long)qg | ((unsigned long long)qb << 32);
+    const unsigned long long a2 = (unsigned long long)qx | ((unsigned long long)qy << 32);
+    const unsigned long long was = atomicAdd(rec + 0, a0);
+    const uint32_t c0 = (uint32_t)was;
+    if (P.carry) {
+        const unsigned long long w1 = atomicAdd(rec + 1, a1), w2 = atomicAdd(rec + 2, a2);
+        atomicAdd(rec + 3, (unsigned long long)qz);
+        const uint32_t ev[kCarryEvents] = {wrap_hi(was, a0), carry_lo(w1, a1), wrap_hi(w1, a1), carry_lo(w2, a2),
+                                           wrap_hi(w2, a2)};
+        if ((ev[0] | ev[1] | ev[2] | ev[3] | ev[4]) || (c0 <= 65536u && c0 + (uint32_t)cnt > 65536u))
+            carry_add(P.carry, v, ev, P.stats);
+    } else {
+        atomicAdd(rec + 1, a1);
+        atomicAdd(rec + 2, a2);
+        atomicAdd(rec + 3, (unsigned long long)qz);
+    }
+    if (c0 == 0u) atomicOr(P.occ + (v >> 5), 1u << (v & 31));
+}
+
+// The queued items, one per lane (lanes >= nact idle).
 template <class Scenes>
 __device__ __forceinline__ uint32_t tess_walk32(const Scenes& S, TessStage& st, const TessTables& T, int nact, int lane,
-                                                int rl, int& head, int& count) {
+                                                int& head, int& count) {
     const unsigned FULL = 0xffffffffu;
     constexpr uint32_t kNone = 0xffffffffu;
     f3 p0 = mk(0.f, 0.f, 0.f), p1 = p0, p2 = p0, n0 = p0, n1 = p0, n2 = p0;
@@ -790,11 +1044,11 @@ __device__ __forceinline__ uint32_t tess_walk32(const Scenes& S, TessStage& st, 
     const float* ring = T.ring[1];
     float third = 0.0f;  // the centre's coordinates
     if (lane < nact) {
-        scene = (int)(st.item[lane] >> 16);
+        scene = (int)(st.q.item[lane] >> 16);
         const AccumParams& P = S.get(scene);
-        const long long t = st.tri[lane];
-        const uint32_t packed = st.lev[lane];
-        it = tess_item(packed, (int)(st.item[lane] & 0xffffu), rl);
+        const long long t = st.q.tri[lane];
+        const uint32_t packed = st.q.lev[lane];
+        it = tess_item(packed, (int)(st.q.item[lane] & 0xffffu), kTessRunLog2);
         const int n = (int)(packed & 127u);
         ring = T.ring[n] + it.k;
         // (an outer edge's segments: outer[0] from corner 1, outer[1] from 2, outer[2] from 0)
@@ -816,8 +1070,6 @@ __device__ __forceinline__ uint32_t tess_walk32(const Scenes& S, TessStage& st, 
     }
     const int cnt = it.cnt;
     const AccumParams& P = S.get(scene);
-    const int N = P.dim;
-    const float fN = (float)N;
     uint32_t cur = kNone, run = 0, sx = 0, sy = 0, sz = 0;
     // Queues the finished runs of the lanes with `push`; 32 queued ones go out.
     auto finish = [&](bool push) {
@@ -854,25 +1106,10 @@ __device__ __forceinline__ uint32_t tess_walk32(const Scenes& S, TessStage& st, 
             at += step;
             if (it.dk) step += 36;
             ring += it.dk;
-            const f3 pos = add(add(mul(p0, bc.x), mul(p1, bc.y)), mul(p2, bc.z));
-            f3 tc;  // times N
-            if (P.warp.mode == VCT_WARP_PERSPECTIVE) {  // voxelTesselationWarpedPosition
-                tc = mul(perspective_tc(P.warp, pos), fN);
-            } else {  // voxelLinearPosition (the evaluation shader passes warpVoxels = false)
-                tc = sub(sub(pos, P.vcenter), P.vmin);
-                if (P.ext_rcp != 0.0f)  // the extents are a power of two, as N is: the product is the quotient's
-                    tc = mul(tc, P.ext_rcp * fN);
-                else
-                    tc = mul(mk(__fdiv_rn(tc.x, P.ext.x), __fdiv_rn(tc.y, P.ext.y), __fdiv_rn(tc.z, P.ext.z)), fN);
-            }
-            const int vx = trunc_sat(tc.x), vy = trunc_sat(tc.y), vz = trunc_sat(tc.z);
-            if ((uint32_t)(vx | vy | vz) < (uint32_t)N) {  // all in [0, N): N is a power of two
-                v = (uint32_t)((vz * N + vy) * N + vx);
-                const f3 nrm = add(add(mul(n0, bc.x), mul(n1, bc.y)), mul(n2, bc.z));
-                const f3 Nf = normalize(nrm);  // voxelStore: normalize(normal) * 0.5 + 0.5
-                qx = quant16(Nf.x * 0.5f + 0.5f);
-                qy = quant16(Nf.y * 0.5f + 0.5f);
-                qz = quant16(Nf.z * 0.5f + 0.5f);
+            uint32_t at_voxel;
+            if (tess_voxel(P, add(add(mul(p0, bc.x), mul(p1, bc.y)), mul(p2, bc.z)), at_voxel)) {
+                v = at_voxel;
+                tess_normal(add(add(mul(n0, bc.x), mul(n1, bc.y)), mul(n2, bc.z)), qx, qy, qz);
             }
         }
         const bool change = i < cnt && v != cur;
@@ -921,109 +1158,115 @@ __global__ void __launch_bounds__(256) carry_fixup_kernel(const Scenes S) {
     P.brick_exact[((z / 16) * bpa + y / 16) * bpa + x / 16] = 1u;
 }
 
-// Warps take units from a shared counter, whose values are
-// spread over the unit order (kTessSpread places in turn): neighbouring units,
-// which belong to neighbouring triangles and add to the same records, are then
-// not worked on at the same time.
+// Adds a warp's counts of generated points (this lane's `points` of a single
+// scene; or a scene's by point_count) to the scenes' statistics.
 template <class Scenes>
-__global__ void __launch_bounds__(kWarps * 32, kTessBlocksPerSM) tess_points_kernel(const Scenes S, const VoxWork W, int nblocks) {
+__device__ __forceinline__ void add_points(const Scenes& S, unsigned* point_count, uint32_t points) {
+    if (points) atomicAdd(&point_count[0], points);
+    __syncthreads();
+    for (int i = threadIdx.x; i < S.count(); i += blockDim.x)
+        if (point_count[i] && S.get(i).stats) atomicAdd(&S.get(i).stats->total_voxel_fragments, point_count[i]);
+}
+
+// The walk.  Warps take units from a shared counter (their first by their own
+// number), whose values are spread over the unit order (kTessSpread places in
+// turn): neighbouring units, which belong to neighbouring triangles and add to
+// the same records, are then not worked on at the same time.
+template <class Scenes>
+__global__ void __launch_bounds__(kWarps * 32, kTessBlocksPerSM) tess_walk_kernel(const Scenes S, const VoxWork W, int nblocks) {
     __shared__ TessStage stages[kWarps];
     __shared__ TessTables tables;
-    __shared__ unsigned point_count[kMaxBatchScenes];      // generated points per scene
+    __shared__ unsigned point_count[kMaxBatchScenes];  // generated points per scene
+    grid_launch_dependents();  // the other kernel, of which one ends at once, reads nothing of this one
+    const uint4 total = W.block_off[nblocks];
+    if (!tess_walks(total)) return;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    TessStage& q = stages[threadIdx.x >> 5];
+    TessStage& st = stages[threadIdx.x >> 5];
     const int nscenes = S.count();
     for (int i = threadIdx.x; i < nscenes; i += blockDim.x) point_count[i] = 0;
     fill_tables(tables);
     __syncthreads();
-    const long long total = W.block_off[nblocks];
-    const int grab = (int)max(1LL, min((long long)kTessGrab, total / ((long long)gridDim.x * kWarps)));
-    const long long grabs = (total + grab - 1) / grab, stretch = (grabs + kTessSpread - 1) / kTessSpread;
+    const long long nw = (long long)gridDim.x * kWarps, warp = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5);
+    const int grab = (int)max(1LL, min((long long)kTessGrab, total.x / nw));
+    const long long grabs = ((long long)total.x + grab - 1) / grab, spread = min((long long)kTessSpread, grabs),
+                    stretch = (grabs + spread - 1) / spread;
     unsigned long long* counter = grab_counter(W, nblocks);
     int qn = 0;               // queued items (warp-uniform)
     int head = 0, count = 0;  // the ring of finished runs (warp-uniform)
     uint32_t points = 0;      // this lane's, of a single scene
     auto walk = [&](int nact) {
-        const int scene = lane < nact ? (int)(q.item[lane] >> 16) : 0;
-        const uint32_t pts = tess_walk32(S, q, tables, nact, lane, W.run_log2, head, count);
+        const int scene = lane < nact ? (int)(st.q.item[lane] >> 16) : 0;
+        const uint32_t pts = tess_walk32(S, st, tables, nact, lane, head, count);
         if (nscenes > 1) {
             if (pts) atomicAdd(&point_count[scene], pts);
         } else {
             points += pts;
         }
     };
-    for (;;) {
-        unsigned long long gu = 0;
-        if (lane == 0) gu = atomicAdd(counter, 1ull);
-        const long long c = (long long)__shfl_sync(FULL, gu, 0);
-        if (c >= stretch * kTessSpread) break;
-        const long long u0 = ((c % kTessSpread) * stretch + c / kTessSpread) * grab, u1 = min(u0 + grab, total);
-        if (u0 >= total) continue;
-        long long g = 0, start = 0;
-        uint32_t nunits = 0;
-        for (long long u = u0; u < u1; ++u) {
-            if (u != u0 && u >= start + nunits) {  // often the next triangle's
-                g = min(g + 1, W.ntri - 1);
-                start = unit_start<Scenes>(W, g);
-                nunits = W.tri_units[g];
-            }
-            if (u == u0 || u >= start + nunits) {
-                // Triangle owning unit u: binary search over the block offsets,
-                // then the block-local scan, 8 entries per lane: the number of
-                // entries <= u is one past the last triangle starting at or
-                // before u.
-                int lo = 0, hi = nblocks - 1;
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if ((long long)W.block_off[mid] <= u)
-                        lo = mid;
-                    else
-                        hi = mid - 1;
-                }
-                const long long gbase = (long long)lo * kSetupThreads;
-                const int in_block = (int)min((long long)kSetupThreads, W.ntri - gbase);
-                const uint32_t rel = (uint32_t)(u - W.block_off[lo]);
-                int below = 0;
-#pragma unroll
-                for (int j = 0; j < kSetupThreads / 32; ++j) {
-                    const int k = lane * (kSetupThreads / 32) + j;
-                    below += (k < in_block && __ldg(W.tri_scan + gbase + k) <= rel) ? 1 : 0;
-                }
-                below = __reduce_add_sync(FULL, below);
-                g = gbase + max(below - 1, 0);
-                start = unit_start<Scenes>(W, g);
-                nunits = W.tri_units[g];
-            }
-            const uint4 r = __ldg(W.tri_rec + g);
-            const int base = (int)(u - start) * kTessUnit;
-            const int cnt = min(kTessUnit, (int)r.y - base);
-            if (lane < cnt) {
-                q.tri[qn + lane] = (int)r.w;
-                q.item[qn + lane] = (uint32_t)(base + lane) | (r.z << 16);
-                q.lev[qn + lane] = r.x;
-            }
-            __syncwarp();
-            qn += cnt;
-            if (qn >= kTessUnit) {
-                walk(kTessUnit);
-                __syncwarp();
-                if (lane < qn - kTessUnit) {
-                    q.tri[lane] = q.tri[kTessUnit + lane];
-                    q.item[lane] = q.item[kTessUnit + lane];
-                    q.lev[lane] = q.lev[kTessUnit + lane];
-                }
-                __syncwarp();
-                qn -= kTessUnit;
+    UnitOwner<true> o = {0, 0u, 0u};
+    for (long long c = warp; c < stretch * spread;) {
+        const long long u0 = ((c % spread) * stretch + c / spread) * grab;
+        if (u0 < total.x) {
+            const uint32_t u1 = (uint32_t)min(u0 + grab, (long long)total.x);
+            o.find(W, nblocks, (uint32_t)u0, lane);
+            for (uint32_t u = (uint32_t)u0; u < u1; ++u) {
+                o.follow(W, nblocks, u, lane);
+                const uint4 r = __ldg(W.tri_rec + o.g);
+                queue_unit(st.q, qn, r, r.y >> 16, u - o.start, lane, walk);
             }
         }
+        if (nw >= stretch * spread) break;
+        unsigned long long next = 0;
+        if (lane == 0) next = atomicAdd(counter, 1ull);
+        c = nw + (long long)__shfl_sync(FULL, next, 0);
     }
     walk(qn);
-    tess_flush(S, q, head, count, lane);
-    if (points) atomicAdd(&point_count[0], points);
+    tess_flush(S, st, head, count, lane);
+    add_points(S, point_count, points);
+}
+
+// The points, where nothing is walked: an equal range of units to each warp.
+template <class Scenes>
+__global__ void __launch_bounds__(kWarps * 32, 4) tess_points_kernel(const Scenes S, const VoxWork W, int nblocks) {
+    __shared__ TessQueue queues[kWarps];
+    __shared__ unsigned point_count[kMaxBatchScenes];
+    const uint4 total = W.block_off[nblocks];
+    if (tess_walks(total)) {
+        grid_wait();  // (this kernel's end is the walk's for the ones behind it)
+        return;
+    }
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    TessQueue& q = queues[threadIdx.x >> 5];
+    const int nscenes = S.count();
+    for (int i = threadIdx.x; i < nscenes; i += blockDim.x) point_count[i] = 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < nscenes; i += blockDim.x)
-        if (point_count[i] && S.get(i).stats) atomicAdd(&S.get(i).stats->total_voxel_fragments, point_count[i]);
+    const long long nw = (long long)gridDim.x * kWarps, warp = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5);
+    const uint32_t u0 = (uint32_t)((unsigned long long)total.y * warp / nw),
+                   u1 = (uint32_t)((unsigned long long)total.y * (warp + 1) / nw);
+    int qn = 0;
+    uint32_t points = 0;
+    auto store = [&](int nact) {
+        tess_store32(S, q, nact, lane);
+        if (nscenes > 1) {
+            const int scene = lane < nact ? (int)(q.item[lane] >> 16) : -1;
+            const unsigned same = __match_any_sync(FULL, scene);
+            if (scene >= 0 && lane == __ffs(same) - 1) atomicAdd(&point_count[scene], (unsigned)__popc(same));
+        } else {
+            points += lane < nact ? 1u : 0u;
+        }
+    };
+    UnitOwner<false> o = {0, 0u, 0u};
+    if (u0 < u1) o.find(W, nblocks, u0, lane);
+    for (uint32_t u = u0; u < u1; ++u) {
+        o.follow(W, nblocks, u, lane);
+        const uint4 r = __ldg(W.tri_rec + o.g);
+        queue_unit(q, qn, r, r.y & 0xffffu, u - o.start, lane, store);
+    }
+    store(qn);
+    add_points(S, point_count, points);
+    grid_wait();
 }
 
 template <class Scenes>
@@ -1032,19 +1275,16 @@ void launch_tess(const Scenes& S, const VoxWork& W, int num_sms, cudaStream_t s)
     const int nblocks = (int)((W.ntri + kSetupThreads - 1) / kSetupThreads);
     tess_setup_kernel<Scenes><<<nblocks, kSetupThreads, 0, s>>>(S, W);
     voxelize_scan_kernel<<<1, 1024, 0, s>>>(W.block_off, nblocks);
-    tess_points_kernel<Scenes><<<num_sms * kTessBlocksPerSM, kWarps * 32, 0, s>>>(S, W, nblocks);
+    tess_walk_kernel<Scenes><<<num_sms * kTessBlocksPerSM, kWarps * 32, 0, s>>>(S, W, nblocks);
+    launch_overlapped(tess_points_kernel<Scenes>, dim3((unsigned)(num_sms * 4)), kWarps * 32, 0, s, S, W, nblocks);
     note_launches(3);
 }
 
 }  // namespace
 
-// Points of an edge item: with few triangles, the fewer the more warps have any.
-int tess_run_log2(long long ntri) { return ntri < 16384 ? 2 : 3; }
-
-// The tessellation voxeliser: setup, scan, points (the same scratch as the
-// rasteriser's).
+// The tessellation voxeliser: setup, scan, the walk and the points.
 void launch_tesselate(const AccumParams& P, cudaStream_t s) {
-    const VoxWork W = {P.tri_rec, P.tri_units, P.tri_scan, P.block_off, P.ntri, tess_run_log2(P.ntri)};
+    const VoxWork W = {P.tri_rec, P.tri_units, P.tri_scan, P.block_off, P.ntri};
     launch_tess(OneScene<AccumParams>{P}, W, P.num_sms, s);
     if (P.carry) {
         carry_fixup_kernel<<<dim3(kCarrySlots / 256, 1), 256, 0, s>>>(OneScene<AccumParams>{P});
@@ -1067,7 +1307,7 @@ void tess_bind_scratch(AccumParams& P, void* scratch) {
     p += align256(ntri * 4);
     P.tri_scan = reinterpret_cast<uint32_t*>(p);
     p += align256(ntri * 4);
-    P.block_off = reinterpret_cast<uint32_t*>(p);
+    P.block_off = reinterpret_cast<uint4*>(p);
 }
 
 void launch_occupancy(const AccumParams& P, cudaStream_t s) {
