@@ -357,9 +357,8 @@ vct_status build_warpmap(vct_ctx* ctx, const AccumParams& A, cudaStream_t st) {
 // tessellating (testTesselation.tesc/.tese).
 void launch_voxelizer(const vct_ctx* ctx, const AccumParams& P, cudaStream_t st) {
     if (ctx->params.voxelize_tesselation) {
-        // (errors of these clears surface at the launch check)
-        cudaMemsetAsync(P.carry, 0, (size_t)kCarryBytes, st);
-        cudaMemsetAsync(P.brick_exact, 0, (size_t)(ctx->nv / 4096 + 1) * 4, st);
+        // (an error of this clear surfaces at the launch check)
+        cudaMemsetAsync(P.carry, 0, (size_t)kCarryBytes + (size_t)(ctx->nv / 4096 + 1) * 4, st);
         launch_tesselate(P, st);
     } else {
         launch_accumulate(P, st);
@@ -751,8 +750,7 @@ vct_status vct_create(const vct_config* cfg, vct_ctx** out) {
         {(void**)&c->occ32, (size_t)(VCT_WARP_DIM * VCT_WARP_DIM * VCT_WARP_DIM / 32) * 4},
         {(void**)&c->warpmap, (size_t)VCT_WARP_DIM * VCT_WARP_DIM * VCT_WARP_DIM * 8},
         {(void**)&c->warpmap_f, (size_t)(VCT_WARP_DIM + 2) * (VCT_WARP_DIM + 2) * (VCT_WARP_DIM + 2) * 16},
-        {(void**)&c->carry, (size_t)kCarryBytes},
-        {(void**)&c->brick_exact, (size_t)(c->nv / 4096 + 1) * 4},
+        {(void**)&c->carry, (size_t)kCarryBytes + (size_t)(c->nv / 4096 + 1) * 4},
     };
     for (auto& a : allocs) {
         cudaError_t e = cudaMalloc(a.p, a.bytes);
@@ -764,6 +762,7 @@ vct_status vct_create(const vct_config* cfg, vct_ctx** out) {
             return fail(e == cudaErrorMemoryAllocation ? VCT_ERR_OUT_OF_MEMORY : VCT_ERR_CUDA, msg);
         }
     }
+    c->brick_exact = c->carry + kCarryBytes / 4;  // behind the table: one clear of both
     cudaError_t e = cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming);
@@ -790,8 +789,7 @@ vct_status vct_destroy(vct_ctx* c) {
     for (auto sf : c->surf)
         if (sf) cudaDestroySurfaceObject(sf);
     void* ptrs[] = {c->acc,    c->occ,   c->lit,         c->color,  c->normal,  c->radiance, c->stats,
-                    c->vox_scratch, c->pchain, c->learned, c->occ32, c->warpmap, c->warpmap_f, c->carry,
-                    c->brick_exact};
+                    c->vox_scratch, c->pchain, c->learned, c->occ32, c->warpmap, c->warpmap_f, c->carry};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     delete c;
