@@ -60,3 +60,35 @@ def test_captured_depth_passes(size):
         graph.replay()
         torch.cuda.synchronize()
         assert all(torch.equal(a, b) for a, b in zip(planes, want))
+
+
+@pytest.mark.parametrize("columns", [1, 4], ids=["points", "walk"])
+def test_captured_tessellation(columns):
+    """Both kernels of the tessellation voxeliser, which start before the kernel
+    in front of them has ended, in frames under capture: one of columns of
+    slivers, one of boxes, in turn."""
+    import torch
+
+    sc = scenes.large_family(3, dim=64, shadow=64, gbuffer=(64, 48), n_boxes=200, n_cyl=columns, cyl_segments=columns * 75)
+    g = GpuScene(sc)
+    with api.Context(api.config_for(sc)) as ctx:
+        ctx.set_params(api.scene_params(sc, voxelize_tesselation=1))
+        out = g.new_outputs()
+
+        def frame():
+            ctx.frame(g.tris, g.lights, g.shadow, sc.eye, g.gb, api.trace_out(*out))
+
+        frame()
+        torch.cuda.synchronize()
+        want, stats = [t.clone() for t in out[:3]], ctx.stats()
+        graph, st = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        with torch.cuda.graph(graph, stream=st):
+            frame()
+        for _ in range(4):
+            for t in out:
+                t.zero_()
+            graph.replay()
+        torch.cuda.synchronize()
+        assert float(want[0].abs().sum()) > 0
+        assert all(torch.equal(a, b) for a, b in zip(out, want))
+        assert ctx.stats() == stats
