@@ -52,13 +52,16 @@ __device__ __forceinline__ f3 mul(f3 a, float s) { return {a.x * s, a.y * s, a.z
 __device__ __forceinline__ f3 mulv(f3 a, f3 b) { return {a.x * b.x, a.y * b.y, a.z * b.z}; }
 __device__ __forceinline__ float dot(f3 a, f3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 __device__ __forceinline__ f3 ld3(const float* p) { return {p[0], p[1], p[2]}; }
-// a / b rounded to nearest, given y = RN(1 / b): the quotient a y is within a
-// unit in the last place, its remainder is exact in one fused multiply-add, and
-// the corrected quotient is the rounded one (P. Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev.
-// 34, 1990), as long as nothing on the way overflows or underflows; a = 0 gives
-// 0.  Cheaper than the division where y is at hand or shared, and above all for
-// a = 0, which takes the division's slow path.
+// a / b rounded to nearest, given y = RN(1 / b): the quotient a y is within 1.5
+// units in the last place, its remainder is exact or off by one part in 2^24 in
+// one fused multiply-add, and the corrected quotient is the rounded one (after
+// P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34, 1990, which supposes a first quotient within
+// one unit; the operands whose quotient lies near enough to a rounding boundary
+// to matter are enumerated in tests/test_quotient.py), as long as nothing on
+// the way overflows or underflows; a = 0 gives 0.  Cheaper than the division
+// where y is at hand or shared, and above all for a = 0, which takes the
+// division's slow path.
 __device__ __forceinline__ float quotient(float a, float b, float y) {
     const float q = a * y;
     return fmaf(fmaf(-q, b, a), y, q);
