@@ -101,11 +101,16 @@ __device__ __forceinline__ int store_rec(TriRec& r, const RasterTri& t, const fl
 // The covered pixels of piece `k` of a triangle's lines, which are contiguous:
 // the line, how many, the first one, and the edge functions there in the caller's vertex
 // order (modulo 2^32 unless BIG).  The triangle's crossings of the line are
-// computed in fp32, within 2^-21 of the coordinates' magnitude (the
-// differences' conversion, the division, the product and the sum each round
-// at 2^-24 or 2^-22).  Pixel centres further than 2^-20 of it and half a
-// sub-pixel unit from a crossing are decided by it; the few nearer ones by the
-// exact edge functions.
+// computed in fp32; pixel centres further than eps from one are decided by it,
+// the few nearer ones by the exact edge functions.
+//
+// With M the largest coordinate along the line, at most 2^28 sub-pixel units: an edge's extent (up to 2M), its extent
+// across and the line's distance convert within 2^-24 each and the quotient is
+// within 2^-22 (two units in the last place), so their product is within 14 x
+// 2^-24 M, and with the first end's conversion within 15 x 2^-24 M.  Where a crossing
+// matters, within the image's 2^23 units, it, its sum with eps and that with half
+// a pixel round within 1/4 each.  eps = 16 x 2^-24 M + 1/2 covers that from M = 2^23
+// on; below, all but the quotient and the roundings (which shrink with M) is exact.
 template <bool BIG>
 __device__ __forceinline__ int line_pixels(const TriRec& r, int k, int& line, int& first, long long base[3]) {
     const uint4 v0 = r.v0, v1 = r.v1;
