@@ -124,17 +124,30 @@ void launch_sampler_rate(const TraceParams& P, int filter, int blocks, int iters
 
 namespace {
 
-// Up to this many tiles per SM (two rounds of the CTAs that it holds) a launch
-// takes the split kernel.  1,200 tiles (640 x 480): 139 us against 173 with the
-// software sampler over 64^3, 130 against 138 with the hybrid one over 256^3;
-// 1,450 tiles 127 against 166 and 121 against 110, 2,040 tiles 174 against 174 and
-// 160 against 153.
-constexpr long long kSplitTilesPerSM = 8;
+// Tiles per SM up to which a launch takes the split kernel: two rounds of the
+// CTAs that an SM holds, fewer where a sample takes less time, so that the shorter
+// chain gains less, and where the march checks every footprint.  The plain texture
+// sampler's unsplit kernel holds five CTAs to an SM, which ends badly on few
+// rounds: it splits up to 16.  Unsplit and split (us):
+//   software, 64^3: 1,200 tiles 173 and 139, 1,450 166 and 127, 2,040 174 and 174;
+//   hybrid, 256^3: 1,200 tiles 138 and 130, 1,450 110 and 121, 2,040 153 and 160;
+//     any warp, 32^3: 1,040 tiles 73 and 70, 1,200 76 and 83;
+//   texture by level, 32^3: 920 tiles 36 and 37, 1,200 43 and 52, 128^3 74 and 76;
+//     any warp: 756 tiles 41 and 40, 128^3 56 and 51, 1,040 45 and 52, 60 and 68;
+//   texture, 128^3: 1,250 tiles 69 and 50, 2,432 102 and 92, 3,600 124 and 134;
+//     warp map, 32^3: 1,040 tiles 67 and 63, 1,200 68 and 76;
+//     any warp, 32^3: 756 tiles 37 and 39, 128^3 51 and 49, 1,200 48 and 60, 73 and 80.
+int split_tiles_per_sm(int filter, int kind) {
+    if (filter == VCT_FILTER_SOFTWARE) return 8;
+    if (filter == VCT_FILTER_HYBRID) return kind == kConesAny ? 7 : 8;
+    if (filter == VCT_FILTER_HARDWARE && kind == kConesPlain) return 16;
+    return kind == kConesAny ? 6 : 7;
+}
 
 template <class Scenes>
 void launch_trace_set(const Scenes& S, int filter, int kind, long long tiles, int num_sms, bool overlap, cudaStream_t s) {
     if (tiles <= 0) return;
-    if (tiles <= kSplitTilesPerSM * num_sms) {
+    if (tiles <= (long long)split_tiles_per_sm(filter, kind) * num_sms) {
         launch_trace_split(S, filter, kind, tiles, num_sms, overlap, s);
         return;
     }
