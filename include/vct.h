@@ -420,7 +420,7 @@ uint64_t vct_launch_count(void);
 /* No counterpart in the reference (it renders one scene per frame).  A batch
  * owns one context per scene (grids may differ, each <= 256^3, all on one
  * device) and runs vct_frame for every scene with one launch per stage:
- * the voxeliser's work units, the shadow texels, the resolve bricks and the
+ * the triangles, the shadow texels, the resolve bricks and the
  * pixel tiles of all scenes are concatenated and each launch maps a global
  * work index back to its scene.  Results equal vct_frame per scene. */
 typedef struct vct_batch vct_batch;

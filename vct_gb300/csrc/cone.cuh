@@ -5,7 +5,9 @@
 //
 // Every fused multiply-add is written out (fmaf, __ffma2_rn); the including
 // translation units are compiled without FMA contraction, so every
-// instantiation rounds the same way.
+// instantiation rounds the same way.  The one exception is the warp map's lookup
+// (warp.cuh), whose packed products and sums the compiler fuses all the same, in
+// every instantiation: the tests compare them bit for bit.
 #pragma once
 
 #include "vct_device.cuh"

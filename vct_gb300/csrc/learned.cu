@@ -1075,7 +1075,8 @@ void launch_learned_probe(const LearnedParams& P, cudaStream_t s) {
 void launch_trace16(const LearnedParams& P, bool listed, int num_sms, cudaStream_t s) {
     const long long tiles = (long long)((P.T.width + kLearnTile - 1) / kLearnTile) *
                             ((P.T.height + kLearnTile - 1) / kLearnTile);
-    // Persistent over the listed tiles: as many CTAs as fit (8 per SM).
+    // Over the listed tiles a grid of twice the CTAs that fit (four per SM), whose
+    // CTAs take tiles in turn; over all tiles a CTA to each.
     const long long cap = (long long)num_sms * 8;
     const long long grid = listed ? cap : tiles;
     with_kind(P, [&](auto kind) {

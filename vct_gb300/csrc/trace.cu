@@ -15,8 +15,9 @@
 // filter weights).
 //
 // The file is compiled without FMA contraction: every fused multiply-add is
-// written out (fmaf, __ffma2_rn), so the single-scene and the batched
-// instantiations of the kernel give bit-identical results.
+// written out (fmaf, __ffma2_rn; but for the warp map's lookup, see cone.cuh), so
+// the single-scene and the batched instantiations of the kernel give bit-identical
+// results.
 #include <algorithm>
 
 #include "trace.cuh"

@@ -389,8 +389,8 @@ constexpr int kOffW1 = 0, kOffB1 = 2688, kOffW2 = 2752, kOffB2 = 6848, kOffW3 = 
 // mean squared error of the irradiance).
 constexpr float kMlpConfidenceWeight = 0.5f;
 // BF16 operand images in the tensor core's shared-memory tile layout: W1
-// (64 x 48), W2, W3 (64 x 64), W4 (16 x 64); the forward passes' B operands,
-// and the backward pass's transposed ones.
+// (64 x 48), W2, W3 (64 x 64), W4 (16 x 64): the forward passes' B operands,
+// which the backward pass reads transposed.
 constexpr int kImgW1 = 0, kImgW2 = 6144, kImgW3 = 14336, kImgW4 = 22528, kImgAll = 24576;
 // Bias vector padded for the kernels: b1 | b2 | b3 | b4 (16).
 constexpr int kBiasPad = 208;
