@@ -19,7 +19,8 @@ namespace {
 // 1920 x 1080 over 256^3 675 (560).
 //
 // PAIRS: the marches take two steps at a time.  For launches of a CTA to an SM
-// at most, which have the registers: the 47 x 31 pixels' frame 37 us (43).
+// at most, which have the registers: the 47 x 31 pixels' frame 37 us (43).  The
+// software sampler without a warp only; the others have not been tried.
 constexpr int kSplit = 4;
 template <int MODE, int KIND, bool PAIRS, class Scenes>
 __global__ void __launch_bounds__(256, PAIRS ? 1 : 4) trace_split_kernel(const Scenes S) {
