@@ -8,6 +8,7 @@
 // multiply-adds out.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <type_traits>
 
@@ -281,25 +282,32 @@ __device__ __forceinline__ void load_dirs(const LearnedParams& P, float (*s_dirs
     if (threadIdx.x < 64) s_dirs[threadIdx.x >> 2][threadIdx.x & 3] = P.dirs16[threadIdx.x >> 2][threadIdx.x & 3];
 }
 
-// 16-cone irradiance of whole 16x16 tiles (every tile, or the listed ones).
-template <int KIND>
-__global__ void __launch_bounds__(256, 4) trace16_kernel(const LearnedParams P, int listed) {
+// 16-cone irradiance of whole 16x16 tiles (every tile, or the listed ones), half
+// a tile to a CTA and six of them to an SM, eight of the listed ones': an image of
+// a few tiles to an SM otherwise ends with some SMs a heavy tile behind the others.
+// 128^3 at 320x180, 640x360, 800x450 and 1920x1080: 142, 232, 379 and 1,673 us;
+// whole tiles, four to an SM, 167, 294, 470 and 1,677, and before the cones' step
+// tables, three to an SM, 185, 266, 401 and 1,754.
+constexpr int kTile16Threads = 128;  // (the cones' table takes that many)
+template <int KIND, bool LISTED>
+__global__ void __launch_bounds__(kTile16Threads, LISTED ? 8 : 6) trace16_kernel(const LearnedParams P) {
     __shared__ cone::Level s_lv[VCT_MAX_LEVELS];
     __shared__ cone::ConeTable s_cone;
     __shared__ float s_dirs[16][4];
+    const TraceParams& T = P.T;
+    const int tiles_x = (T.width + kLearnTile - 1) / kLearnTile;
+    const long long total = LISTED ? (long long)*P.count : (long long)tiles_x * ((T.height + kLearnTile - 1) / kLearnTile);
+    if (blockIdx.x >= 2 * total) return;  // past the list
     cone::fill_levels(P.T, s_lv);
     cone::fill_cone(P.T, P.ref_cone, P.T.max_distance, s_cone, 64);
     load_dirs(P, s_dirs);
     __syncthreads();
-    const TraceParams& T = P.T;
-    const int tiles_x = (T.width + kLearnTile - 1) / kLearnTile;
-    const long long total = listed ? (long long)*P.count : (long long)tiles_x * ((T.height + kLearnTile - 1) / kLearnTile);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     unsigned ns = 0;
-    for (long long t = blockIdx.x; t < total; t += gridDim.x) {
-        const long long tile = listed ? (long long)P.list[t] : t;
+    for (long long t = blockIdx.x; t < 2 * total; t += gridDim.x) {
+        const long long tile = LISTED ? (long long)P.list[t >> 1] : t >> 1;
         const int x = (int)(tile % tiles_x) * kLearnTile + (wid & 1) * 8 + cone::lane_x(lane, 3);
-        const int y = (int)(tile / tiles_x) * kLearnTile + (wid >> 1) * 4 + cone::lane_y(lane, 3);
+        const int y = (int)(tile / tiles_x) * kLearnTile + (int)(t & 1) * 8 + (wid >> 1) * 4 + cone::lane_y(lane, 3);
         if (x >= T.width || y >= T.height) continue;
         const long long pix = (long long)y * T.width + x;
         const float4 gp = __ldg(T.gpos + pix);
@@ -1078,12 +1086,14 @@ void launch_learned_probe(const LearnedParams& P, cudaStream_t s) {
 void launch_trace16(const LearnedParams& P, bool listed, int num_sms, cudaStream_t s) {
     const long long tiles = (long long)((P.T.width + kLearnTile - 1) / kLearnTile) *
                             ((P.T.height + kLearnTile - 1) / kLearnTile);
-    // Over the listed tiles a grid of twice the CTAs that fit (four per SM), whose
-    // CTAs take tiles in turn; over all tiles a CTA to each.
-    const long long cap = (long long)num_sms * 8;
-    const long long grid = listed ? cap : tiles;
+    // Over all tiles a CTA to each half; over the listed ones, whose number is known
+    // on the device, as many, or six times the CTAs that fit, which take halves in turn
+    // (twice: 128^3, 1080p 1.76 ms, 1.74; a 256^3 scene of many small tiles 1.27, 1.17).
     with_kind(P, [&](auto kind) {
-        trace16_kernel<kind.value><<<(unsigned)(grid > 0 ? grid : 1), 256, 0, s>>>(P, listed ? 1 : 0);
+        if (listed)
+            trace16_kernel<kind.value, true><<<(unsigned)std::min(num_sms * 48LL, 2 * tiles), kTile16Threads, 0, s>>>(P);
+        else
+            trace16_kernel<kind.value, false><<<(unsigned)(2 * tiles), kTile16Threads, 0, s>>>(P);
     });
     note_launches(1);
 }
@@ -1092,7 +1102,9 @@ void launch_trace16_pixels(const LearnedParams& P, cudaStream_t s) {
     const long long n = (long long)P.T.width * P.T.height;
     const long long tiles = (long long)((P.T.width + 15) / 16) * ((P.T.height + 15) / 16);  // one CTA each
     learned_flag_kernel<<<(unsigned)tiles, 256, 0, s>>>(P);
-    with_kind(P, [&](auto kind) { trace16_pixels_kernel<kind.value><<<(unsigned)((n + kListThreads - 1) / kListThreads), kListThreads, 0, s>>>(P); });
+    with_kind(P, [&](auto kind) {
+        trace16_pixels_kernel<kind.value><<<(unsigned)((n + kListThreads - 1) / kListThreads), kListThreads, 0, s>>>(P);
+    });
     note_launches(2);
 }
 
