@@ -147,6 +147,14 @@ __device__ __forceinline__ void flush_stage(const RecordStage& st, int lane) {
     }
 }
 
+// The largest magnitude of three; NaN if one is, which fmaxf passes over and
+// whose product with 0 is not 0.
+__device__ __forceinline__ float largest(f3 v) {
+    float m;
+    asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(v.x), "f"(v.y), "f"(v.z));
+    return m;
+}
+
 // voxelize.frag:186-280 for one fragment: triangle t of the scene, pixel
 // (px, py) of its dominant axis' view, weights l and depth z.
 __device__ __forceinline__ void shade_fragment(const AccumParams& P, long long t, int axis, int px, int py,
@@ -175,13 +183,11 @@ __device__ __forceinline__ void shade_fragment(const AccumParams& P, long long t
                 // for a surface turned well away (by more than rounding) the
                 // cosine is: the light then adds +-0, unless its product with
                 // the albedo overflows.  Four point lights of range 0.3-0.8 in a
-                // volume of side 2 leave one in nine fragments inside one.  (A
-                // component each: fmaxf would pass over a NaN, whose product with
-                // 0 is not 0.)
+                // volume of side 2 leave one in nine fragments inside one.
                 const f3 base = mulv(mul(color, L.intensity), L.color);
                 const float d2 = dot(d, d), nd = dot(Nf, d);
                 if ((d2 > L.beyond2 || (nd < 0.0f && nd * nd > 1e-6f * d2 && d2 > 1e-30f && L.beyond2 < 3.0e38f)) &&
-                    fabsf(base.x) < 3.0e38f && fabsf(base.y) < 3.0e38f && fabsf(base.z) < 3.0e38f)
+                    largest(base) < 3.0e38f)
                     continue;
                 float ndl = fmaxf(0.0f, dot(Nf, normalize(d)));
                 lit = mul(base, ndl);
